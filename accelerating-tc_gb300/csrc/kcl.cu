@@ -3,24 +3,34 @@
 // The reference (k-clique/kcl.cu:147-215, Pangolin) materialises every level of the
 // embedding list in HBM: per level it counts extensions (extend_alloc, :16-50), scans
 // them (thrust::exclusive_scan, :197) and writes the next level (extend_insert,
-// :115-145), counting instead of writing at level k-2.  Here each warp walks the
-// search tree of one oriented edge (u, v) depth first, so nothing but a small stack of
-// candidate sets is ever stored:
+// :115-145), counting instead of writing at level k-2.  Here a warp or a CTA takes one
+// source u and builds, once for all its edges, the graph that the CSR induces on N+(u) as
+// bitmap rows in shared memory: row i = the members of N+(u) that are in N+(S[i]), S = N+(u).
+// Row i is then C0 = N+(u) ∩ N+(S[i]) of the edge u -> S[i], and every deeper level of the
+// search is an AND / popc of rows:
 //
-//   C0 = N+(u) ∩ N+(v);  C(l+1) = C(l) ∩ N+(w) for the w chosen from C(l);
-//   with k-1 vertices chosen, every element of the current candidate set completes a
-//   k-clique, so the last level is counted, never stored.
-// When |C0| <= 64 (every RGG edge, most R-MAT edges) the warp instead builds the 64-bit
-// successor masks of the DAG induced on C0 with one ballot per member, and each lane
-// counts the remaining (k-2)-cliques of its first member with AND / popc on registers.
-// From k = 5 on, edges with 64 < |C0| <= 1024 go to a second kernel, a CTA per edge, that
-// counts the (k-2)-cliques of C0 from bitmap rows in shared memory (kcl_dense_kernel).
+//   cliq(1, M) = |M|,  cliq(t, M) = sum_{j in M} cliq(t - 1, M & row[j]),
+//   k-cliques whose first edge is u -> S[i]: cliq(k - 2, row[i]).
+//
+//   rows of 2..32 and (up to k = 5) 33..64 members (kcl_rows_warp_kernel): a warp per u, 32-
+//     and 64-bit rows; the induced edges are listed in shared memory as they are found and dealt over
+//     the lanes, each lane counting the (k-3)-cliques of its edge's common row;
+//   longer rows up to kRowMax members (kcl_rows_block_kernel): a CTA per u, rows of 64-bit
+//     words; at k = 4 each induced edge is one AND / popc over the words, from k = 5 on a row's
+//     C0 is renumbered into shorter rows of its own by a warp (up to kRowWarp members) or, at
+//     k = 5, by the CTA; what is left goes to kcl_dense_kernel, a CTA per edge;
+//   longer rows still: a warp walks the search tree of one oriented edge depth first with
+//     binary searches in global memory (kcl_kernel), its C0 of 65..1024 members counted by
+//     kcl_dense_kernel from k = 5 on.  atc_tuning.kcl_dense = -1 puts every edge on that warp
+//     search, without the dense kernel.
 //
 // Orientation is acyclic, so every k-clique is found once, from its first two vertices
-// in orientation order — the same count kcl_gpu_solver accumulates.  Intersections:
-// lanes take the elements of the candidate set (a subset of N+(u)), binary-search each
-// in N+(w), and ballot/popc compact the hits in order into the next level, which lives
-// in the warp's slice of a scratch buffer ((k-2) x max out-degree ints per warp).
+// in orientation order — the same count kcl_gpu_solver accumulates.
+//
+// Measured (ms, one call; the per-edge walk with its dense kernel -> rows): RGG 2^20 of mean
+// degree 32, k = 4 / 5 / 6 / 7: 22.0 / 25.2 / 39.7 / 72.8 -> 0.87 / 1.25 / 4.3 / 16.4; R-MAT
+// scale 18, k = 4 / 5 / 6: 53.7 / 69.4 / 360 -> 3.8 / 17.8 / 174; scale 20, k = 4 / 5 / 6: 424 /
+// 547 / 3697 -> 25.2 / 215 / 2339; scale 14, k = 6 / 7: 3.8 / 37.5 -> 2.4 / 28.9.
 #include <algorithm>
 
 #include "internal.cuh"
@@ -58,17 +68,23 @@ constexpr int kMaxK = 16;
 constexpr int kMaskMax = 64;     // candidate sets up to this size use the warp's bitmask path
 constexpr int kDenseMax = 1024;  // larger ones up to this size: a CTA per edge, bitmaps in shared memory
 constexpr int kDenseWords = kDenseMax / 64;
+constexpr int kDensePad = 4;
 constexpr int kDenseThreads = 1024;  // 256: R-MAT s20 k = 6 4.84 s; 512: 3.81 s; 1024: 3.70 s
 
 // d-cliques inside `mask` of the DAG whose successor sets (within C0) are adj[]:
 // cliq(1, M) = |M|, cliq(d, M) = sum_{i in M} cliq(d-1, M & adj[i]).  Iterative, one
 // lane, an explicit stack of (remaining mask, candidate mask) per depth.
-__device__ __forceinline__ unsigned long long mask_cliques(const unsigned long long* adj, unsigned long long mask,
-                                                           int d) {
+__device__ __forceinline__ int first_bit(uint32_t x) { return __ffs((int)x) - 1; }
+__device__ __forceinline__ int first_bit(unsigned long long x) { return __ffsll((long long)x) - 1; }
+__device__ __forceinline__ int popc_of(uint32_t x) { return __popc(x); }
+__device__ __forceinline__ int popc_of(unsigned long long x) { return __popcll(x); }
+
+template <class M>
+__device__ __forceinline__ unsigned long long mask_cliques(const M* adj, M mask, int d) {
   if (d <= 0) return 1ull;
-  if (d == 1) return (unsigned long long)__popcll(mask);
+  if (d == 1) return (unsigned long long)popc_of(mask);
   unsigned long long total = 0;
-  unsigned long long rem[kMaxK], cand[kMaxK];
+  M rem[kMaxK], cand[kMaxK];
   int top = 0;
   rem[0] = mask;
   cand[0] = mask;
@@ -77,13 +93,13 @@ __device__ __forceinline__ unsigned long long mask_cliques(const unsigned long l
       --top;
       continue;
     }
-    int i = __ffsll(rem[top]) - 1;
+    int i = first_bit(rem[top]);
     rem[top] &= rem[top] - 1;
-    unsigned long long nm = cand[top] & adj[i];
+    M nm = cand[top] & adj[i];
     int left = d - 1 - top;  // vertices still to choose after i
     if (left == 1) {
-      total += (unsigned long long)__popcll(nm);
-    } else if (__popcll(nm) >= left) {
+      total += (unsigned long long)popc_of(nm);
+    } else if (popc_of(nm) >= left) {
       ++top;
       rem[top] = nm;
       cand[top] = nm;
@@ -92,11 +108,18 @@ __device__ __forceinline__ unsigned long long mask_cliques(const unsigned long l
   return total;
 }
 
+// Edges of sources with more than min_ud members (the shorter ones go by rows, below).
+// Intersections: lanes take the elements of the candidate set (a subset of N+(u)),
+// binary-search each in N+(w), and ballot/popc compact the hits in order into the next level,
+// which lives in the warp's slice of a scratch buffer ((k-2) x max out-degree ints per warp).
+// C0 of at most 64 members: the warp builds the 64-bit successor masks of the DAG induced on
+// it with one ballot per member, and each lane counts the (k-2)-cliques of its first member.
 // dense (nullable): edges whose C0 has kMaskMax < |C0| <= kDenseMax are appended to
 // dense[1 + ...] (count in dense[0]) for kcl_dense_kernel instead of being walked here.
 __global__ void __launch_bounds__(kKcWarps * 32) kcl_kernel(const int64_t* off, const int32_t* cols, const int32_t* esrc,
-                                                          int64_t e0, int64_t e1, int k, int cap, int32_t* scratch,
-                                                          unsigned long long* dense, unsigned long long* out) {
+                                                          int64_t e0, int64_t e1, int k, int cap, int min_ud,
+                                                          int32_t* scratch, unsigned long long* dense,
+                                                          unsigned long long* out) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t gw = (int64_t)blockIdx.x * kKcWarps + w;
   const int64_t warps = (int64_t)gridDim.x * kKcWarps;
@@ -109,6 +132,7 @@ __global__ void __launch_bounds__(kKcWarps * 32) kcl_kernel(const int64_t* off, 
   for (int64_t e = e0 + gw; e < e1; e += warps) {
     int32_t u = esrc[e], v = cols[e];
     int64_t ub = off[u], ud = off[u + 1] - ub;
+    if (ud <= min_ud) continue;
     int64_t vb = off[v], vd = off[v + 1] - vb;
     bytes += 4ull * (unsigned long long)vd;
     // C0 = N+(u) ∩ N+(v), in the order of N+(u)
@@ -261,6 +285,46 @@ __device__ unsigned long long pair_cliques(const unsigned long long* U, int word
   return total;
 }
 
+// The same count with the candidate sets in registers: rows of at most W words, D members to
+// choose from M.  Rows hold higher members only, so every set below is above the last one chosen.
+// Words past a row's end are read (the rows are padded) and masked off by M's zero words.
+template <int W, int D>
+__device__ __forceinline__ unsigned long long word_cliques(const unsigned long long* U, int stride,
+                                                           const unsigned long long (&M)[W]) {
+  unsigned c = 0;
+  if constexpr (D == 1) {
+#pragma unroll
+    for (int w = 0; w < W; ++w) c += __popcll(M[w]);
+    return c;
+  } else {
+    unsigned long long total = 0;
+#pragma unroll
+    for (int w = 0; w < W; ++w)
+      for (unsigned long long r = M[w]; r; r &= r - 1) {
+        const unsigned long long* Rx = U + (size_t)(w * 64 + first_bit(r)) * stride;
+        unsigned long long N[W];
+#pragma unroll
+        for (int v = 0; v < W; ++v) N[v] = v < w ? 0ull : M[v] & Rx[v];
+        total += word_cliques<W, D - 1>(U, stride, N);
+      }
+    return total;
+  }
+}
+template <int W>
+__device__ __forceinline__ unsigned long long pair_word_cliques(const unsigned long long* U, int stride, int i, int j,
+                                                                int d) {
+  unsigned long long M[W];
+#pragma unroll
+  for (int w = 0; w < W; ++w) M[w] = U[(size_t)i * stride + w] & U[(size_t)j * stride + w];
+  if (stride < W)
+#pragma unroll
+    for (int w = 0; w < W; ++w)
+      if (w >= stride) M[w] = 0ull;
+  if (d == 1) return word_cliques<W, 1>(U, stride, M);
+  if (d == 2) return word_cliques<W, 2>(U, stride, M);
+  return word_cliques<W, 3>(U, stride, M);
+}
+
 // Edges whose C0 = N+(u) ∩ N+(v) holds kMaskMax < |C0| <= kDenseMax members, a CTA per
 // edge.  C0 goes to shared memory (sorted by id, as N+(u) is) and the graph induced on it
 // to bitmap rows: row i = the members above i adjacent to C0[i] (each oriented edge
@@ -276,7 +340,7 @@ __global__ void __launch_bounds__(kDenseThreads) kcl_dense_kernel(const int64_t*
                                                                   const int32_t* esrc, const unsigned long long* dense,
                                                                   int k, int cmax, unsigned long long* next,
                                                                   unsigned long long* out) {
-  extern __shared__ unsigned long long dsm[];  // rows: cmax * words
+  extern __shared__ unsigned long long dsm[];  // rows: cmax * words, and kDensePad words read past them
   __shared__ int32_t C[kDenseMax];
   __shared__ int pre[kDenseMax + 1];
   __shared__ int wcount[kDenseThreads / 32];
@@ -385,7 +449,480 @@ __global__ void __launch_bounds__(kDenseThreads) kcl_dense_kernel(const int64_t*
         r -= pc;
       }
       const int j = x * 64 + select_bit(Ri[x], r);
-      cnt += pair_cliques(dsm, words, i, j, k - 4);
+      if (words <= 2 && k <= 7) cnt += pair_word_cliques<2>(dsm, words, i, j, k - 4);
+      else if (words <= 4 && k <= 7) cnt += pair_word_cliques<4>(dsm, words, i, j, k - 4);
+      else cnt += pair_cliques(dsm, words, i, j, k - 4);
+    }
+    __syncthreads();
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+    bytes += __shfl_xor_sync(0xffffffffu, bytes, o);
+  }
+  if (lane == 0) {
+    if (cnt) atomicAdd(out, cnt);
+    if (bytes) atomicAdd(out + 1, bytes);
+  }
+}
+
+// ============================== rows of one source ===================================
+// What bounds these kernels: building the rows streams N+(x) for every member x of N+(u) (W
+// elements over the graph, mostly L2 hits) with one search in shared memory each, and is issue
+// bound; the counting after it is AND / popc on shared memory.  Every search per edge that
+// the walk above makes in global memory (dependent loads) is gone.
+constexpr int kRowMax = 960;       // rows of 960 x 15 words (115 KB) and everything below fit
+constexpr int kRowWarp = 128;      // C0 up to this size is renumbered and counted by one warp
+constexpr int kRowBlock = 512;     // k = 5: C0 up to this size by the CTA that holds its rows
+constexpr int kRowThreads = 512;
+constexpr int kRowBuckets = 4;     // lists by length, longest first (row_bucket)
+constexpr int kRowSearch = 128;    // lists longer than this are searched for the members of
+                                   // N+(u), not streamed, where N+(u) fits one warp's masks
+
+// D-cliques inside m of the DAG with successor rows `rows` (D levels unrolled into nested
+// loops, nothing on a stack); D > kRowUnroll: `d` levels by mask_cliques' explicit stack.
+constexpr int kRowUnroll = 5;
+template <int D, class M>
+__device__ __forceinline__ unsigned long long row_cliques(const M* rows, M m, int d) {
+  if constexpr (D == 0) {
+    return 1ull;
+  } else if constexpr (D == 1) {
+    return (unsigned long long)popc_of(m);
+  } else if constexpr (D == 2) {
+    unsigned c = 0;
+    for (M r = m; r; r &= r - 1) c += popc_of((M)(m & rows[first_bit(r)]));
+    return c;
+  } else if constexpr (D <= kRowUnroll) {
+    unsigned long long c = 0;
+    for (M r = m; r; r &= r - 1) {
+      const M nm = m & rows[first_bit(r)];
+      if (popc_of(nm) >= D - 1) c += row_cliques<D - 1, M>(rows, nm, d);
+    }
+    return c;
+  } else {
+    return mask_cliques(rows, m, d);
+  }
+}
+
+// Position of y in the sorted S[0, d), padded to R = 2^j entries with INT_MAX; -1 if absent.
+template <int R>
+__device__ __forceinline__ int member_of(const int32_t* S, int d, int32_t y) {
+  int p = 0;
+#pragma unroll
+  for (int step = R / 2; step > 0; step >>= 1)
+    if (S[p + step - 1] < y) p += step;
+  return p < d && S[p] == y ? p : -1;
+}
+
+// Calls f(y, k, valid) on all 32 lanes for every element y of the lists [xb, xb + xd) held by
+// the lanes (k = the lane holding y's list): lists of 32 or more elements are walked by the
+// whole warp, shorter ones laid end to end and dealt 32 elements a round.
+template <class F>
+__device__ __forceinline__ void for_members(const int32_t* cols, int64_t xb, int xd, int lane, F f) {
+  unsigned longm = __ballot_sync(0xffffffffu, xd >= 32);
+  while (longm) {
+    const int k = __ffs(longm) - 1;
+    longm &= longm - 1;
+    const int32_t* P = cols + __shfl_sync(0xffffffffu, xb, k);
+    const int ln = __shfl_sync(0xffffffffu, xd, k);
+    int j0 = 0;
+    for (; j0 + 64 <= ln; j0 += 64) {
+      const int32_t y0 = __ldg(P + j0 + lane), y1 = __ldg(P + j0 + 32 + lane);
+      f(y0, k, true);
+      f(y1, k, true);
+    }
+    for (; j0 < ln; j0 += 32) {
+      const bool v = j0 + lane < ln;
+      f(v ? __ldg(P + j0 + lane) : 0, k, v);
+    }
+  }
+  const int slen = xd < 32 ? xd : 0;
+  int incl = slen;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  const int total = __shfl_sync(0xffffffffu, incl, 31);
+  const int start = incl - slen;
+  for (int t0 = 0; t0 < total; t0 += 32) {
+    const int t = t0 + lane;
+    int k = 0;  // the last lane whose list starts at or before t
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1)
+      if (__shfl_sync(0xffffffffu, start, k + step) <= t) k += step;
+    const int64_t kb = __shfl_sync(0xffffffffu, xb, k);
+    const int ks = __shfl_sync(0xffffffffu, start, k);
+    const bool v = t < total;
+    f(v ? __ldg(cols + kb + (t - ks)) : 0, k, v);
+  }
+}
+
+// A warp per source u with lo < |N+(u)| <= R (R = bits of M), k - 1 <= |N+(u)|, over the edges
+// of [e0, e1).  KD = k - 3: the members to choose below an induced edge (0: k = 3; above
+// kRowUnroll: any k).  Sources are taken `grab` (<= 32) at a time from `queue`.
+template <class M, int KD>
+__global__ void __launch_bounds__(kKcWarps * 32) kcl_rows_warp_kernel(const int64_t* off, const int32_t* cols, int64_t n,
+                                                                    int64_t e0, int64_t e1, int k, int lo, int grab,
+                                                                    int* queue, unsigned long long* out) {
+  constexpr int R = 8 * (int)sizeof(M);
+  constexpr int kPairs = R * (R - 1) / 2;  // induced edges of a DAG; other digraphs may hold more
+  __shared__ int32_t Ssm[kKcWarps][R];
+  __shared__ M rsm[kKcWarps][R];
+  __shared__ uint16_t psm[kKcWarps][KD ? kPairs : 1];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int32_t* S = Ssm[w];
+  M* rows = rsm[w];
+  uint32_t* row32 = reinterpret_cast<uint32_t*>(rows);
+  uint16_t* pairs = psm[w];
+  const unsigned below = (1u << lane) - 1;
+  unsigned long long cnt = 0, bytes = 0;
+  for (;;) {
+    int chunk = 0;
+    if (lane == 0) chunk = atomicAdd(queue, 1);
+    chunk = __shfl_sync(0xffffffffu, chunk, 0);
+    if ((int64_t)chunk * grab >= n) break;
+    const int64_t row = min((int64_t)chunk * grab + lane, n);
+    const int64_t rb = __ldg(off + row), re = __ldg(off + min(row + 1, n));
+    unsigned todo = __ballot_sync(0xffffffffu, lane < grab && re - rb > lo && re - rb <= R && re - rb >= k - 1 &&
+                                                   min(re, e1) > max(rb, e0));
+    while (todo) {
+      const int q = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const int64_t ub = __shfl_sync(0xffffffffu, rb, q);
+      const int d = (int)(__shfl_sync(0xffffffffu, re, q) - ub);
+      const int ia = (int)max(e0 - ub, (int64_t)0), ib = (int)min(e1 - ub, (int64_t)d);  // edges counted
+      for (int j = lane; j < R; j += 32) {
+        S[j] = j < d ? __ldg(cols + ub + j) : INT32_MAX;
+        rows[j] = 0;
+      }
+      __syncwarp();
+      int np = 0;
+      // an induced edge S[i] -> S[j] on the lanes with `hit` (all 32 lanes call)
+      auto found = [&](bool hit, int i, int j) {
+        if constexpr (KD == 0) {
+          cnt += hit && i >= ia && i < ib;
+        } else {
+          if (hit) atomicOr(&row32[R == 32 ? i : 2 * i + (j >> 5)], 1u << (j & 31));
+          hit = hit && i >= ia && i < ib;
+          const unsigned b = __ballot_sync(0xffffffffu, hit);
+          const int at = np + __popc(b & below);
+          if (hit && at < kPairs) pairs[at] = (uint16_t)(i << 8 | j);
+          np += __popc(b);
+        }
+      };
+      for (int base = 0; base < d; base += 32) {
+        int64_t xb = 0;
+        int xd = 0;
+        if (base + lane < d) {
+          const int32_t x = S[base + lane];
+          xb = __ldg(off + x);
+          xd = (int)(__ldg(off + x + 1) - xb);
+        }
+        bytes += 4ull * (unsigned long long)xd;
+        unsigned far = __ballot_sync(0xffffffffu, xd > kRowSearch);
+        while (far) {  // long lists: the members of N+(u) are searched in them
+          const int kk = __ffs(far) - 1;
+          far &= far - 1;
+          const int64_t kb = __shfl_sync(0xffffffffu, xb, kk);
+          const int kd = __shfl_sync(0xffffffffu, xd, kk);
+          for (int j = lane; j < R; j += 32)
+            found(j < d && kc_has(cols + kb, kd, S[j]), base + kk, j);
+        }
+        for_members(cols, xb, xd > kRowSearch ? 0 : xd, lane, [&](int32_t y, int kk, bool v) {
+          const int j = member_of<R>(S, d, y);
+          found(v && j >= 0, base + kk, j & (R - 1));
+        });
+      }
+      __syncwarp();
+      if constexpr (KD > 0) {
+        if (np <= kPairs) {
+          for (int p = lane; p < np; p += 32) {
+            const int ij = pairs[p];
+            cnt += row_cliques<KD, M>(rows, rows[ij >> 8] & rows[ij & 255], k - 3);
+          }
+        } else {  // not a DAG: every bit of every row
+          for (int i = ia; i < ib; ++i)
+            for (int j = lane; j < R; j += 32)
+              if ((rows[i] >> j) & 1) cnt += row_cliques<KD, M>(rows, rows[i] & rows[j], k - 3);
+        }
+        __syncwarp();
+      }
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+    bytes += __shfl_xor_sync(0xffffffffu, bytes, o);
+  }
+  if (lane == 0) {
+    if (cnt) atomicAdd(out, cnt);
+    if (bytes) atomicAdd(out + 1, bytes);
+  }
+}
+
+// Sources with lo < |N+(u)| <= hi and an edge in [e0, e1), longest bucket first:
+// lists[b * cap ...], counts[b].
+__device__ __forceinline__ int row_bucket(int64_t d) { return d > 384 ? 0 : d > 192 ? 1 : d > 96 ? 2 : 3; }
+__global__ void kcl_rows_list_kernel(const int64_t* off, int64_t n, int64_t e0, int64_t e1, int lo, int hi, int64_t cap,
+                                     int32_t* lists, int* counts) {
+  const int lane = threadIdx.x & 31;
+  const int64_t n_pad = (n + 31) & ~31ll;
+  for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < n_pad; u += (int64_t)gridDim.x * blockDim.x) {
+    int mine = -1;
+    if (u < n) {
+      const int64_t b = off[u], e = off[u + 1];
+      if (e - b > lo && e - b <= hi && min(e, e1) > max(b, e0)) mine = row_bucket(e - b);
+    }
+    for (int q = 0; q < kRowBuckets; ++q) {  // one atomic per warp and bucket
+      const unsigned m = __ballot_sync(0xffffffffu, mine == q);
+      int at = 0;
+      if (m && lane == 0) at = atomicAdd(&counts[q], __popc(m));
+      at = __shfl_sync(0xffffffffu, at, 0);
+      if (mine == q) lists[q * cap + at + __popc(m & ((1u << lane) - 1))] = (int32_t)u;
+    }
+  }
+}
+
+// Shared memory of kcl_rows_block_kernel for sources of up to dmax members.  MODE as there.
+__host__ __device__ inline int row_stride(int d) { return ((d + 63) >> 6) | 1; }  // odd: rows of random j spread over the banks
+constexpr int kRowWarpWords = kRowWarp * 3;  // rows of two words, three apart
+struct RowsSmem {
+  size_t rows, rows2, wrows, s, wmem, mem, rcnt, bytes;  // byte offsets of the parts, and their end
+  __host__ __device__ RowsSmem(int dmax, int mode) {
+    const int d2 = dmax < kRowBlock ? dmax : kRowBlock;
+    const size_t list = (size_t)((dmax + 8) & ~7);
+    rows = 0;
+    rows2 = rows + sizeof(unsigned long long) * (size_t)dmax * row_stride(dmax);
+    wrows = rows2 + (mode == 2 ? sizeof(unsigned long long) * (size_t)d2 * row_stride(d2) : 0);
+    s = wrows + (mode >= 2 ? sizeof(unsigned long long) * kRowWarpWords * (kRowThreads / 32) : 0);
+    wmem = s + sizeof(int32_t) * list;
+    mem = wmem + (mode >= 2 ? sizeof(uint16_t) * kRowWarp * (kRowThreads / 32) : 0);
+    rcnt = mem + (mode == 2 ? sizeof(uint16_t) * kRowBlock : 0);
+    bytes = rcnt + (mode == 2 ? sizeof(uint16_t) * list : 0);
+  }
+};
+
+// The members of row `Ri` (32-bit halves r32, `halves` of them) in order, by one warp.
+__device__ __forceinline__ void row_members(const uint32_t* r32, int halves, uint16_t* M, int lane) {
+  for (int h = 0, at = 0; h < halves; ++h) {
+    const uint32_t bits = r32[h];
+    if ((bits >> lane) & 1) M[at + __popc(bits & ((1u << lane) - 1))] = (uint16_t)(h * 32 + lane);
+    at += __popc(bits);
+  }
+  __syncwarp();
+}
+
+// A CTA per source u too long for a warp.  MODE 0: k = 3 (the hits are the count), 1:
+// k = 4, 2: k = 5, 3: k >= 6.  Rows are built from the lists of the members, a batch of 32
+// members a warp.  From k = 5 on, with few sources, each is split over several CTAs (every
+// nsplit-th of its edges): the rows are cheap to build again next to the search below them, and
+// a dense core's few sources would otherwise leave most CTAs idle.  Edges whose row is too long
+// for the warps (and at k = 5 for the CTA) go on the dense list.
+template <int MODE>
+__global__ void __launch_bounds__(kRowThreads) kcl_rows_block_kernel(const int64_t* off, const int32_t* cols, int64_t e0,
+                                                                    int64_t e1, int k, const int32_t* lists, int64_t cap,
+                                                                    const int* counts, int dmax, int* queue,
+                                                                    unsigned long long* dense,
+                                                                    unsigned long long* out) {
+  extern __shared__ __align__(16) unsigned char rsm[];
+  const RowsSmem at(dmax, MODE);
+  unsigned long long* rows = reinterpret_cast<unsigned long long*>(rsm + at.rows);
+  int32_t* S = reinterpret_cast<int32_t*>(rsm + at.s);
+  __shared__ int item, next_batch, next_row;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = kRowThreads / 32;
+  int first[kRowBuckets + 1];
+  first[0] = 0;
+#pragma unroll
+  for (int b = 0; b < kRowBuckets; ++b) first[b + 1] = first[b] + counts[b];
+  const int sources = first[kRowBuckets];
+  const int nsplit = MODE < 2 ? 1 : min(max(8 * (int)gridDim.x / max(sources, 1), 1), 32);
+  unsigned long long cnt = 0, bytes = 0;
+  for (;;) {
+    if (threadIdx.x == 0) {
+      item = atomicAdd(queue, 1);
+      next_batch = 0;
+      next_row = 0;
+    }
+    __syncthreads();
+    const int it = item / nsplit, part = item - it * nsplit;
+    if (it >= sources) break;
+    int b = 0, fb = 0;
+#pragma unroll
+    for (int q = 1; q < kRowBuckets; ++q)
+      if (it >= first[q]) {
+        b = q;
+        fb = first[q];
+      }
+    const int64_t u = lists[b * cap + (it - fb)];
+    const int64_t ub = off[u];
+    const int d = (int)(off[u + 1] - ub);
+    const int ia = (int)max(e0 - ub, (int64_t)0), ib = (int)min(e1 - ub, (int64_t)d);
+    const int words = (d + 63) >> 6, st = row_stride(d);
+    for (int j = threadIdx.x; j < d; j += kRowThreads) S[j] = __ldg(cols + ub + j);
+    if (MODE > 0)
+      for (int t = threadIdx.x; t < d * st; t += kRowThreads) rows[t] = 0ull;
+    __syncthreads();
+    const int32_t s_lo = S[0], s_hi = S[d - 1];
+    uint32_t* r32 = reinterpret_cast<uint32_t*>(rows);
+    for (;;) {
+      int base = 0;
+      if (lane == 0) base = atomicAdd(&next_batch, 32);
+      base = __shfl_sync(0xffffffffu, base, 0);
+      if (base >= d) break;
+      int64_t xb = 0;
+      int xd = 0;
+      if (base + lane < d) {
+        const int32_t x = S[base + lane];
+        xb = __ldg(off + x);
+        xd = (int)(__ldg(off + x + 1) - xb);
+      }
+      bytes += 4ull * (unsigned long long)xd;
+      for_members(cols, xb, xd, lane, [&](int32_t y, int kk, bool v) {
+        if (!v || y < s_lo || y > s_hi) return;
+        int lo = 0, len = d;  // branch-free lower bound
+        while (len > 1) {
+          const int half = len >> 1;
+          lo = S[lo + half - 1] < y ? lo + half : lo;
+          len -= half;
+        }
+        if (S[lo] != y) return;
+        const int i = base + kk;
+        if constexpr (MODE == 0) cnt += i >= ia && i < ib;
+        else atomicOr(&r32[2 * ((size_t)i * st + (lo >> 6)) + ((lo >> 5) & 1)], 1u << (lo & 31));
+      });
+    }
+    __syncthreads();
+    if constexpr (MODE == 1) {
+      // a warp per row: the lanes holding a successor j take |row i AND row j|
+      for (int i = ia + w; i < ib; i += nw) {
+        const unsigned long long* Ri = rows + (size_t)i * st;
+        for (int h = 0; h < 2 * words; ++h) {
+          const uint32_t bits = r32[2 * (size_t)i * st + h];
+          if ((bits >> lane) & 1) {
+            const unsigned long long* Rj = rows + (size_t)(h * 32 + lane) * st;
+            unsigned c = 0;
+            for (int x = 0; x < words; ++x) c += __popcll(Ri[x] & Rj[x]);
+            cnt += c;
+          }
+        }
+      }
+    }
+    if constexpr (MODE >= 2) {
+      auto has = [&](int i, int j) { return (r32[2 * ((size_t)i * st) + (j >> 5)] >> (j & 31)) & 1u; };
+      uint16_t* rcnt = reinterpret_cast<uint16_t*>(rsm + at.rcnt);
+      // a warp per row: its members renumbered into rows A of one or two words, then the
+      // (k-2)-cliques of the induced graph: an edge a -> c a lane, with the (k-4)-cliques of
+      // the two rows' common members
+      unsigned long long* A = reinterpret_cast<unsigned long long*>(rsm + at.wrows) + w * kRowWarpWords;
+      uint16_t* Mw = reinterpret_cast<uint16_t*>(rsm + at.wmem) + w * kRowWarp;
+      for (;;) {
+        int t = 0;
+        if (lane == 0) t = atomicAdd(&next_row, 1);
+        t = __shfl_sync(0xffffffffu, t, 0);
+        const int i = ia + part + t * nsplit;
+        if (i >= ib) break;
+        const int r = __reduce_add_sync(0xffffffffu, lane < words ? __popcll(rows[(size_t)i * st + lane]) : 0);
+        if (MODE == 2 && lane == 0) rcnt[i] = (uint16_t)r;
+        const bool two = r > kMaskMax && r <= kRowWarp && k <= 7;
+        if (r > kMaskMax && !two && (MODE == 3 || r > kRowBlock) && lane == 0)
+          dense[1 + atomicAdd(dense, 1ull)] = (unsigned long long)(ub + i);
+        if (r < k - 2 || (r > kMaskMax && !two)) continue;
+        row_members(r32 + 2 * (size_t)i * st, 2 * words, Mw, lane);
+        if (!two) {
+          const int m0 = lane < r ? Mw[lane] : -1, m1 = lane + 32 < r ? Mw[lane + 32] : -1;
+          for (int a = 0; a < r; ++a) {
+            const int ma = Mw[a];
+            const unsigned lo = __ballot_sync(0xffffffffu, m0 >= 0 && has(ma, m0));
+            const unsigned hi = __ballot_sync(0xffffffffu, m1 >= 0 && has(ma, m1));
+            if (lane == 0) A[a] = ((unsigned long long)hi << 32) | lo;
+          }
+          __syncwarp();
+          for (int a = 0; a < r; ++a) {
+            const unsigned long long Ra = A[a];
+            if (__popcll(Ra) < k - 3) continue;
+            for (int c = lane; c < r; c += 32)
+              if ((Ra >> c) & 1) {
+                const unsigned long long m = Ra & A[c];
+                if (MODE == 2) cnt += __popcll(m);
+                else if (k == 6) cnt += row_cliques<2, unsigned long long>(A, m, 0);
+                else if (k == 7) cnt += row_cliques<3, unsigned long long>(A, m, 0);
+                else cnt += mask_cliques(A, m, k - 4);
+              }
+          }
+        } else {  // an induced edge is kept at the lower position of the two, as kcl_dense_kernel does
+          uint32_t* A32 = reinterpret_cast<uint32_t*>(A);
+          for (int a = 0; a < r; ++a) {
+            const int ma = Mw[a];
+            for (int h = 0; h < 4; ++h) {
+              const int c = h * 32 + lane;
+              bool in = false;
+              if (c >= a && c < r) {
+                const int mc = Mw[c];
+                in = has(ma, mc) || has(mc, ma);
+              }
+              const unsigned bits = __ballot_sync(0xffffffffu, in);
+              if (lane == 0) A32[6 * a + h] = bits;
+            }
+          }
+          __syncwarp();
+          for (int a = 0; a < r; ++a)
+            for (int c = (a & ~31) + lane; c < r; c += 32)
+              if ((A32[6 * a + (c >> 5)] >> (c & 31)) & 1) {
+                if (MODE == 2) {
+                  cnt += (unsigned)(__popcll(A[3 * a] & A[3 * c]) + __popcll(A[3 * a + 1] & A[3 * c + 1]));
+                } else {
+                  cnt += pair_word_cliques<2>(A, 3, a, c, k - 4);
+                }
+              }
+        }
+        __syncwarp();
+      }
+    }
+    if constexpr (MODE == 2) {
+      // longer rows by the whole CTA, renumbered the same way; an induced edge is one AND / popc
+      auto has = [&](int i, int j) { return (r32[2 * ((size_t)i * st) + (j >> 5)] >> (j & 31)) & 1u; };
+      const uint16_t* rcnt = reinterpret_cast<const uint16_t*>(rsm + at.rcnt);
+      uint16_t* mem = reinterpret_cast<uint16_t*>(rsm + at.mem);
+      unsigned long long* rows2 = reinterpret_cast<unsigned long long*>(rsm + at.rows2);
+      uint32_t* q32 = reinterpret_cast<uint32_t*>(rows2);
+      __syncthreads();
+      for (int i = ia + part; i < ib; i += nsplit) {
+        const int r = rcnt[i];
+        if (r <= kRowWarp || r > kRowBlock) continue;
+        const unsigned long long* Ri = rows + (size_t)i * st;
+        for (int j = threadIdx.x; j < d; j += kRowThreads)
+          if (has(i, j)) {
+            int pos = __popcll(Ri[j >> 6] & ((1ull << (j & 63)) - 1));
+            for (int x = 0; x < (j >> 6); ++x) pos += __popcll(Ri[x]);
+            mem[pos] = (uint16_t)j;
+          }
+        __syncthreads();
+        const int w2 = (r + 63) >> 6, st2 = row_stride(r);
+        for (int a = w; a < r; a += nw) {
+          const int ma = mem[a];
+          for (int h = 0; h < 2 * w2; ++h) {
+            const int c = h * 32 + lane;
+            bool in = false;
+            if (c >= a && c < r) {
+              const int mc = mem[c];
+              in = has(ma, mc) || has(mc, ma);
+            }
+            const unsigned bits = __ballot_sync(0xffffffffu, in);
+            if (lane == 0) q32[2 * (size_t)a * st2 + h] = bits;
+          }
+        }
+        __syncthreads();
+        for (int a = w; a < r; a += nw) {
+          const unsigned long long* Ra = rows2 + (size_t)a * st2;
+          for (int c = (a & ~31) + lane; c < r; c += 32)
+            if ((q32[2 * (size_t)a * st2 + (c >> 5)] >> (c & 31)) & 1) {
+              const unsigned long long* Rc = rows2 + (size_t)c * st2;
+              unsigned n = 0;
+              for (int x = c >> 6; x < w2; ++x) n += __popcll(Ra[x] & Rc[x]);
+              cnt += n;
+            }
+        }
+        __syncthreads();
+      }
     }
     __syncthreads();
   }
@@ -405,43 +942,109 @@ __global__ void __launch_bounds__(kDenseThreads) kcl_dense_kernel(const int64_t*
 
 using namespace atc;
 
-// k-cliques whose first two vertices (in orientation order) form an edge of [e0, e1).
+// Rows of up to R = 32 or 64 members (M's bits): one warp launch for the given k.
+template <class M>
+static atc_status launch_rows_warp(const atc_csr* csr, int64_t e0, int64_t e1, int k, int lo, int* queue,
+                                   unsigned long long* out, cudaStream_t s) {
+  using Kernel = void (*)(const int64_t*, const int32_t*, int64_t, int64_t, int64_t, int, int, int, int*,
+                          unsigned long long*);
+  static const Kernel kernels[kRowUnroll + 2] = {
+      kcl_rows_warp_kernel<M, 0>, kcl_rows_warp_kernel<M, 1>, kcl_rows_warp_kernel<M, 2>, kcl_rows_warp_kernel<M, 3>,
+      kcl_rows_warp_kernel<M, 4>, kcl_rows_warp_kernel<M, 5>, kcl_rows_warp_kernel<M, kRowUnroll + 1>};
+  const Kernel kern = kernels[std::min(k - 3, kRowUnroll + 1)];
+  int bps = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, kKcWarps * 32, 0);
+  // a grab of 32 sources (one coalesced read of their offsets) unless that would leave warps
+  // without work
+  const int64_t warps = (int64_t)sm_count() * std::max(bps, 1) * kKcWarps;
+  const int grab = (int)std::min<int64_t>(std::max<int64_t>(csr->n / (4 * warps), 1), 32);
+  const int64_t grid = std::min<int64_t>(warps, (csr->n + grab - 1) / grab) / kKcWarps + 1;
+  kern<<<(unsigned)grid, kKcWarps * 32, 0, s>>>(csr->offsets, csr->cols, csr->n, e0, e1, k, lo, grab, queue, out);
+  ATC_CK(cudaGetLastError());
+  return ATC_OK;
+}
+
+template <int MODE>
+static atc_status launch_rows_block(const atc_csr* csr, int64_t e0, int64_t e1, int k, int dmax, const int32_t* lists,
+                                    int64_t cap, int* counts, int* queue, unsigned long long* dense,
+                                    unsigned long long* out, cudaStream_t s) {
+  const size_t smem = RowsSmem(dmax, MODE).bytes;
+  ATC_CK(cudaFuncSetAttribute((const void*)kcl_rows_block_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)smem));
+  int bps = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kcl_rows_block_kernel<MODE>, kRowThreads, smem);
+  kcl_rows_block_kernel<MODE><<<(unsigned)(sm_count() * std::max(bps, 1)), kRowThreads, smem, s>>>(
+      csr->offsets, csr->cols, e0, e1, k, lists, cap, counts, dmax, queue, dense, out);
+  ATC_CK(cudaGetLastError());
+  return ATC_OK;
+}
+
+// k-cliques whose first two vertices (in orientation order) form an edge of [e0, e1).  by_rows:
+// sources of up to kRowMax members by rows, longer ones by the walk;
+// otherwise every edge by the walk alone.
 static atc_status kcl_window(const atc_csr* csr, uint32_t k, int64_t e0, int64_t e1, uint64_t* count, atc_stats* stats,
-                             cudaStream_t s, bool allow_dense = true) {
+                             cudaStream_t s, bool by_rows = true) {
   *count = 0;
   unsigned long long h[2] = {0, 0};
   EventTimer tm;
   int launches = 0;
   if (e1 > e0) {
     CsrPriv* pv = static_cast<CsrPriv*>(csr->priv);
-    int cap = std::max(csr->max_outdeg, 1);
-    int levels = (int)k - 2;
-    int bps = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kcl_kernel, kKcWarps * 32, 0);
-    if (bps < 1) bps = 1;
-    int64_t grid = (int64_t)sm_count() * bps;
-    // keep the scratch within 4 GiB
-    int64_t per_warp = (int64_t)levels * cap * 4;
-    while (grid > sm_count() && grid * kKcWarps * per_warp > (4ll << 30)) grid /= 2;
-    DevBuf<int32_t> scratch;
-    ATC_TRY(scratch.alloc((size_t)grid * kKcWarps * levels * cap, s));
-    // edges with mid-sized C0 go to the dense kernel from k = 5 on (at k = 4 the count is
-    // one intersection per member of C0, which the warp path does as fast: R-MAT scale 20
-    // took 562 ms dense, 422 ms without)
-    const bool use_dense = allow_dense && k >= 5 && cap > kMaskMax;
+    const int cap = std::max(csr->max_outdeg, 1);
+    const int levels = (int)k - 2;
+    const int row_max = by_rows ? kRowMax : 0;
+    const bool walk = cap > row_max;  // some source is too long for rows
+    int64_t grid = 0;
+    DevBuf<int32_t> scratch, lists;
     DevBuf<unsigned long long> dense;
+    DevBuf<int> q;  // queues: 32-bit rows, 64-bit rows, block rows; [4..7] the block lists' counts
+    if (walk) {
+      int bps = 0;
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kcl_kernel, kKcWarps * 32, 0);
+      if (bps < 1) bps = 1;
+      grid = (int64_t)sm_count() * bps;
+      // keep the scratch within 4 GiB
+      int64_t per_warp = (int64_t)levels * cap * 4;
+      while (grid > sm_count() && grid * kKcWarps * per_warp > (4ll << 30)) grid /= 2;
+      ATC_TRY(scratch.alloc((size_t)grid * kKcWarps * levels * cap, s));
+    }
+    // edges with 65..1024 members in C0 go to the dense kernel from k = 5 on (at k = 4 the walk
+    // does one intersection per member of C0 as fast)
+    const bool use_dense = by_rows && k >= 5 && cap > kMaskMax;
     if (use_dense) ATC_TRY(dense.alloc((size_t)csr->m + 2, s));
+    // k >= 6: the search below one source of 33..64 members is long enough for a CTA (one warp
+    // of it held R-MAT scale 14's k = 6 count at 12.8 ms, 3.8 by the walk)
+    const int warp_max = k >= 6 ? 32 : kMaskMax;  // longest rows a warp takes
+    const int64_t lcap = csr->m / (warp_max + 1) + 1;
+    const bool blocks = by_rows && cap > warp_max;
+    ATC_TRY(q.alloc(8, s));
+    if (blocks) ATC_TRY(lists.alloc((size_t)lcap * kRowBuckets, s));
     tm.start(s);
     ATC_CK(cudaMemsetAsync(pv->counter, 0, 2 * sizeof(unsigned long long), s));
+    ATC_CK(cudaMemsetAsync(q.p, 0, 8 * sizeof(int), s));
     if (use_dense) ATC_CK(cudaMemsetAsync(dense.p, 0, 2 * sizeof(unsigned long long), s));
-    kcl_kernel<<<(unsigned)grid, kKcWarps * 32, 0, s>>>(csr->offsets, csr->cols, pv->esrc, e0, e1, (int)k, cap,
-                                                         scratch.p, use_dense ? dense.p + 1 : nullptr, pv->counter);
-    ATC_CK(cudaGetLastError());
-    launches = 1;
+    if (walk) {
+      kcl_kernel<<<(unsigned)grid, kKcWarps * 32, 0, s>>>(csr->offsets, csr->cols, pv->esrc, e0, e1, (int)k, cap,
+                                                           row_max, scratch.p, use_dense ? dense.p + 1 : nullptr,
+                                                           pv->counter);
+      ATC_CK(cudaGetLastError());
+      ++launches;
+    }
+    if (blocks) {
+      const int dmax = std::min(cap, row_max);
+      kcl_rows_list_kernel<<<grid_for(csr->n, 256), 256, 0, s>>>(csr->offsets, csr->n, e0, e1, warp_max, row_max, lcap,
+                                                                lists.p, q.p + 4);
+      ATC_CK(cudaGetLastError());
+      const auto launch = k == 3 ? launch_rows_block<0> : k == 4 ? launch_rows_block<1>
+                          : k == 5 ? launch_rows_block<2> : launch_rows_block<3>;
+      ATC_TRY(launch(csr, e0, e1, (int)k, dmax, lists.p, lcap, q.p + 4, q.p + 2, use_dense ? dense.p + 1 : nullptr,
+                     pv->counter, s));
+      launches += 2;
+    }
     if (use_dense) {
       // rows for the largest C0 this graph can have
       const int cmax = std::min(cap, kDenseMax);
-      const size_t smem = sizeof(unsigned long long) * (size_t)cmax * ((cmax + 63) / 64);
+      const size_t smem = sizeof(unsigned long long) * ((size_t)cmax * ((cmax + 63) / 64) + kDensePad);
       ATC_CK(cudaFuncSetAttribute((const void*)kcl_dense_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)smem));
       int dbps = 0;
@@ -450,7 +1053,15 @@ static atc_status kcl_window(const atc_csr* csr, uint32_t k, int64_t e0, int64_t
       kcl_dense_kernel<<<(unsigned)(sm_count() * dbps), kDenseThreads, smem, s>>>(
           csr->offsets, csr->cols, pv->esrc, dense.p + 1, (int)k, cmax, dense.p, pv->counter);
       ATC_CK(cudaGetLastError());
-      launches = 2;
+      ++launches;
+    }
+    if (by_rows && cap > 32 && warp_max > 32) {
+      ATC_TRY(launch_rows_warp<unsigned long long>(csr, e0, e1, (int)k, 32, q.p + 1, pv->counter, s));
+      ++launches;
+    }
+    if (by_rows) {
+      ATC_TRY(launch_rows_warp<uint32_t>(csr, e0, e1, (int)k, 0, q.p, pv->counter, s));
+      ++launches;
     }
     tm.stop(s);
     ATC_CK(cudaMemcpyAsync(h, pv->counter, sizeof(h), cudaMemcpyDeviceToHost, s));
