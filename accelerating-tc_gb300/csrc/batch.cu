@@ -351,16 +351,16 @@ atc_status build_pipeline(atc_batch* b, const ItemShape& sh, cudaStream_t s) {
                                                               skip, 0);
   kernels += 3;  // items, block, warp
   stage("batch.items");
-  bisson_block_kernel<CompactItems, kDefaultSlots><<<grid_block, kBgWarps * 32, smem, c>>>(g, plist, bitems, 0, b->counters + 1,
+  bisson_block_kernel<CompactItems, kDefaultSlots><<<grid_block, kBgWarps * 32, smem, c>>>(g, ListPartners{plist}, bitems, 0, b->counters + 1,
                                                                             b->counters + 5, words, tags, b->gcounts);
   stage("batch.block");
   if (any_big) {
     bisson_block_kernel<CompactItems, kDefaultSlots><<<grid_big, kBgWarps * 32, smem_big, c>>>(
-        g, plist, litems, 0, b->counters + 2, b->counters + 6, words_big, tags, b->gcounts);
+        g, ListPartners{plist}, litems, 0, b->counters + 2, b->counters + 6, words_big, tags, b->gcounts);
     kernels += 1;
     stage("batch.block.long");
   }
-  bisson_warp_kernel<CompactItems, kDefaultSlots><<<grid_warp, kBgWarps * 32, 0, c>>>(g, plist, witems, 0, b->counters,
+  bisson_warp_kernel<CompactItems, kDefaultSlots><<<grid_warp, kBgWarps * 32, 0, c>>>(g, ListPartners{plist}, witems, 0, b->counters,
                                                                        b->counters + 4, tags, b->gcounts);
   stage("batch.warp");
   if (mixed && nrows > 0) {
@@ -370,16 +370,16 @@ atc_status build_pipeline(atc_batch* b, const ItemShape& sh, cudaStream_t s) {
     kernels += 3;
     stage("batch.rows.items");
     bisson_block_kernel<CompactItems, kDefaultSlots><<<grid_block, kBgWarps * 32, smem, c>>>(
-        g, b->cols, bitems_r, 0, b->counters_r + 1, b->counters_r + 5, words, tags, b->gcounts);
+        g, ListPartners{b->cols}, bitems_r, 0, b->counters_r + 1, b->counters_r + 5, words, tags, b->gcounts);
     stage("batch.rows.block");
     if (any_big) {
       bisson_block_kernel<CompactItems, kDefaultSlots><<<grid_big, kBgWarps * 32, smem_big, c>>>(
-          g, b->cols, litems_r, 0, b->counters_r + 2, b->counters_r + 6, words_big, tags, b->gcounts);
+          g, ListPartners{b->cols}, litems_r, 0, b->counters_r + 2, b->counters_r + 6, words_big, tags, b->gcounts);
       kernels += 1;
       stage("batch.rows.block.long");
     }
     bisson_warp_kernel<CompactItems, kDefaultSlots><<<grid_warp, kBgWarps * 32, 0, c>>>(
-        g, b->cols, witems_r, 0, b->counters_r, b->counters_r + 4, tags, b->gcounts);
+        g, ListPartners{b->cols}, witems_r, 0, b->counters_r, b->counters_r + 4, tags, b->gcounts);
     stage("batch.rows.warp");
   }
   cudaError_t launch_err = cudaGetLastError();

@@ -559,7 +559,26 @@ struct HashQueueProber {
   }
 };
 
-// Streams the lists of the partners plist[base, base+32) for every batch start `base`
+// Where a work item's partners come from.  ListPartners: a partner's whole list.
+// PrefixPartners: (first element, length) of the part of a list to stream (csrc/ranked.cu).
+struct ListPartners {
+  const int32_t* __restrict__ p;
+  __device__ __forceinline__ void get(const CsrView& g, int64_t i, int64_t* pb, int* len) const {
+    const int32_t v = __ldg(p + i);
+    *pb = __ldg(g.off + v);
+    *len = (int)(__ldg(g.off + v + 1) - *pb);
+  }
+};
+struct PrefixPartners {
+  const uint2* __restrict__ p;
+  __device__ __forceinline__ void get(const CsrView&, int64_t i, int64_t* pb, int* len) const {
+    const uint2 q = __ldg(p + i);
+    *pb = q.x;
+    *len = (int)q.y;
+  }
+};
+
+// Streams the lists of the partners [base, base+32) for every batch start `base`
 // that `next_batch()` hands out (until it reaches i1) through the prober, and returns
 // the hits.  Lists of 32 or more elements are walked by the whole warp, one list at a
 // time, four coalesced loads in flight per lane.  Shorter lists are laid end to end by
@@ -567,19 +586,15 @@ struct HashQueueProber {
 // the list holding its element by a 5-step binary search over the lanes' start offsets,
 // done with shuffles so that every lane runs the same steps.  Every probe call is made
 // by all 32 lanes together.
-template <class NextBatch, class Prober>
-__device__ __forceinline__ unsigned stream_partners(const CsrView& g, const int32_t* __restrict__ plist, int64_t i1,
-                                                    int lane, NextBatch next_batch, Prober& pr) {
+template <class Partners, class NextBatch, class Prober>
+__device__ __forceinline__ unsigned stream_partners(const CsrView& g, const Partners& partners, int64_t i1, int lane,
+                                                    NextBatch next_batch, Prober& pr) {
   unsigned cnt = 0;
   for (int64_t base = next_batch(); base < i1; base = next_batch()) {
     int64_t i = base + lane;
     int len = 0;
     int64_t pb = 0;
-    if (i < i1) {
-      int32_t p = __ldg(plist + i);
-      pb = __ldg(g.off + p);
-      len = (int)(__ldg(g.off + p + 1) - pb);
-    }
+    if (i < i1) partners.get(g, i, &pb, &len);
     unsigned longm = __ballot_sync(0xffffffffu, len >= 32);
     while (longm) {
       const int k = __ffs(longm) - 1;
@@ -629,8 +644,8 @@ __device__ __forceinline__ unsigned stream_partners(const CsrView& g, const int3
 }
 
 // nitems_dev (nullable): the item count read from device memory instead of `nitems`.
-template <class Items, int S = 1>
-__global__ void __launch_bounds__(kBgWarps * 32, Items::kMinBlocks) bisson_warp_kernel(CsrView g, const int32_t* __restrict__ plist,
+template <class Items, int S = 1, class Partners = ListPartners>
+__global__ void __launch_bounds__(kBgWarps * 32, Items::kMinBlocks) bisson_warp_kernel(CsrView g, Partners partners,
                                                                   Items items, int nitems,
                                                                   const int* nitems_dev, int* next, GraphTags tags,
                                                                   unsigned long long* out) {
@@ -674,7 +689,7 @@ __global__ void __launch_bounds__(kBgWarps * 32, Items::kMinBlocks) bisson_warp_
         }
         return T[lo] == x;
       });
-      cnt = stream_partners(g, plist, gi.e, lane, nb, pr);
+      cnt = stream_partners(g, partners, gi.e, lane, nb, pr);
       __syncwarp();
       for (int j = lane; j < dh; j += 32) T[j] = -1;
     } else {
@@ -684,7 +699,7 @@ __global__ void __launch_bounds__(kBgWarps * 32, Items::kMinBlocks) bisson_warp_
       for (int j = lane; j < dh; j += 32) hash_insert<S>(T, mask, __ldg(g.cols + hb + j));
       __syncwarp();
       HashQueueProber<S> pr{T, mask, qx[w], qs[w], 0, lane};
-      cnt = stream_partners(g, plist, gi.e, lane, nb, pr);
+      cnt = stream_partners(g, partners, gi.e, lane, nb, pr);
       __syncwarp();
       for (int j = lane; j < dh; j += 32) hash_erase<S>(T, mask, __ldg(g.cols + hb + j));
     }
@@ -696,8 +711,8 @@ __global__ void __launch_bounds__(kBgWarps * 32, Items::kMinBlocks) bisson_warp_
   warp_add_count(total, out);
 }
 
-template <class Items, int S = 1>
-__global__ void __launch_bounds__(kBgWarps * 32, Items::kMinBlocks) bisson_block_kernel(CsrView g, const int32_t* __restrict__ plist,
+template <class Items, int S = 1, class Partners = ListPartners>
+__global__ void __launch_bounds__(kBgWarps * 32, Items::kMinBlocks) bisson_block_kernel(CsrView g, Partners partners,
                                                                    Items items, int nitems,
                                                                    const int* nitems_dev, int* next, uint32_t tab_words,
                                                                    GraphTags tags, unsigned long long* out) {
@@ -738,7 +753,7 @@ __global__ void __launch_bounds__(kBgWarps * 32, Items::kMinBlocks) bisson_block
       for (int64_t j = threadIdx.x; j < dh; j += blockDim.x) hash_insert<S>(tab, mask, Nh[j]);
       __syncthreads();
       HashQueueProber<S> pr{tab, mask, qx[w], qs[w], 0, lane};
-      cnt = stream_partners(g, plist, gi.e, lane, nb, pr);
+      cnt = stream_partners(g, partners, gi.e, lane, nb, pr);
       __syncthreads();
       for (int64_t j = threadIdx.x; j < dh; j += blockDim.x) hash_erase<S>(tab, mask, Nh[j]);
     } else if (gi.mode == 1) {
@@ -757,7 +772,7 @@ __global__ void __launch_bounds__(kBgWarps * 32, Items::kMinBlocks) bisson_block
         x -= lo;
         return (bits[x >> 5] >> (x & 31)) & 1u;
       });
-      cnt = stream_partners(g, plist, gi.e, lane, nb, pr);
+      cnt = stream_partners(g, partners, gi.e, lane, nb, pr);
       __syncthreads();
       for (int j = threadIdx.x; j < words; j += blockDim.x) bits[j] = 0xffffffffu;  // back to empty slots (-1)
     } else {
@@ -769,7 +784,7 @@ __global__ void __launch_bounds__(kBgWarps * 32, Items::kMinBlocks) bisson_block
         }
         return lo < dh && Nh[lo] == x;
       });
-      cnt = stream_partners(g, plist, gi.e, lane, nb, pr);
+      cnt = stream_partners(g, partners, gi.e, lane, nb, pr);
     }
     __syncthreads();
     if constexpr (Items::kBatch) graph_acc_add(tags, &acc[w], gi.h, cnt);

@@ -12,6 +12,8 @@ namespace atc {
 // Sorts n keys on bits [begin_bit, end_bit).  `keys` and `alt` are two buffers of n
 // elements; on return `keys` points at the sorted data (the two may be swapped).
 atc_status sort_keys_u64(uint64_t*& keys, uint64_t*& alt, size_t n, int begin_bit, int end_bit, cudaStream_t s);
+atc_status sort_keys_u64_tmp(void* tmp, size_t* bytes, uint64_t* keys, uint64_t* alt, size_t n, int begin_bit,
+                             int end_bit, uint64_t** sorted, cudaStream_t s);
 // Stable sort of n (key, value) pairs on key bits [begin_bit, end_bit); on return `keys` /
 // `vals` point at the sorted data (each may be swapped with its alternate buffer).
 atc_status sort_pairs_u64_i32(uint64_t*& keys, uint64_t*& kalt, int32_t*& vals, int32_t*& valt, size_t n, int begin_bit,
@@ -100,11 +102,19 @@ atc_status part_edge_range(const atc_csr* csr, uint32_t part, uint32_t nparts, i
 // lookup (n_v ints, device) = new id of every id in [0, n_v).
 atc_status gro_lookup(const int2* pairs, uint64_t ne, int64_t n_v, int32_t* lookup, cudaStream_t s);
 
+// Counts the triangles of a CSR with in-degrees (CsrPriv::indeg) on a degree-ranked copy of its
+// edges (csrc/ranked.cu), added to *out (device).  *done = false: no room for the copy, or a row
+// too long for it, and *out is not to be used.
+atc_status count_ranked(const atc_csr* csr, unsigned long long* out, bool* done, cudaStream_t s, int* launches);
+
 // Private part of an atc_csr.
 struct CsrPriv {
   int32_t* esrc = nullptr;       // m: source vertex of every edge, in edge order
   unsigned long long* counter = nullptr;  // 2 x u64 scratch for counting kernels
   int bits = 1;
+  // n: in-degrees of a CSR built by preTC, which orients every edge of a simple graph once;
+  // null for a CSR loaded from a file, whose rows may be any sorted lists
+  int32_t* indeg = nullptr;
   // cols and esrc live in pinned host memory mapped into the device's address space
   // (atc_csr_host_resident / atc_csr_load_host); these are the host allocations
   int32_t* host_cols = nullptr;

@@ -495,6 +495,7 @@ static atc_status pretc_impl(const int2* pairs, uint64_t np, atc_dir dir, atc_or
   pv->esrc = esrc.detach();
   pv->counter = counter.detach();
   pv->bits = bout;
+  pv->indeg = indeg.detach();
   out->n = n;
   out->m = m;
   out->offsets = off.detach();
@@ -575,6 +576,7 @@ extern "C" atc_status atc_csr_free(atc_csr* csr) try {
   }
   if (pv) {
     if (pv->counter) cudaFree(pv->counter);
+    if (pv->indeg) cudaFree(pv->indeg);
     delete pv;
   }
   *csr = atc_csr{};

@@ -26,6 +26,16 @@ atc_status sort_keys_u64(uint64_t*& keys, uint64_t*& alt, size_t n, int begin_bi
   return ATC_OK;
 }
 
+// The same with caller-provided temporary storage; *sorted = the buffer that holds the result.
+// tmp == nullptr: *bytes receives the size needed.
+atc_status sort_keys_u64_tmp(void* tmp, size_t* bytes, uint64_t* keys, uint64_t* alt, size_t n, int begin_bit,
+                             int end_bit, uint64_t** sorted, cudaStream_t s) {
+  cub::DoubleBuffer<uint64_t> db(keys, alt);
+  ATC_CK(cub::DeviceRadixSort::SortKeys(tmp, *bytes, db, (int64_t)n, begin_bit, end_bit, s));
+  if (sorted) *sorted = db.Current();
+  return ATC_OK;
+}
+
 atc_status sort_pairs_u64_i32(uint64_t*& keys, uint64_t*& kalt, int32_t*& vals, int32_t*& valt, size_t n, int begin_bit,
                              int end_bit, cudaStream_t s) {
   if (n <= 1) return ATC_OK;

@@ -1,0 +1,756 @@
+// Triangle counting on a degree-ranked copy of the edges: the Bisson-style count of a whole
+// CSR built by preTC (Bisson/tc.cu:18-104: a bitmap of N+(u), other lists streamed through it).
+//
+// The count does not depend on the orientation, so this path picks its own.  Vertices are
+// numbered by descending degree (rank 0 = the largest) and every edge points from its endpoint
+// of higher rank to the one of lower rank; rows are sorted.  For an edge u -> v the common
+// successors w all have rank(w) < rank(v), so they lie in the part of row u before v: only that
+// prefix is tested against N+(v).  Over all edges these are sum_u C(d+(u), 2) tests, 0.6 of the
+// sum of min(d+u, d+v) that the grouping of whole lists streams (R-MAT scales 16..20), and
+// rows are short, so a row's later reads hit in L2.  And N+(v) lies in [0, rank(v)): the targets
+// that take nearly all tests have small ranks, and their N+(v) is a bitmap in shared memory
+// addressed by the id itself: one 4-byte shared load and a shift per test, against a hash, a
+// 16-byte bucket, four compares and a queue (about 8 instructions per 32 tests against 31).
+//
+//   passes: degrees -> rank (radix sort on the degree bits) -> out-degrees and group sizes ->
+//   scans -> rows (scatter, then sorted in registers) -> entries (row start, prefix length)
+//   grouped by target -> work items -> count.  Nothing waits on the host before the count.
+//   targets of rank below 2^16: a warp per chunk of entries, its own bitmap of 4 or 8 KB, rows
+//   read as 16-bit ids; below 2^17 with enough entries: a CTA of four warps per chunk, a bitmap
+//   of 16 KB; the rest (a tenth of the tests at R-MAT scale 24): the hash kernels of bisson.cuh
+//   over the same entries, or a CTA's 64 KB bitmap for rows too long for a warp's table.
+//
+// Measured (R-MAT scale 24, A-direction + A-order; whole lists grouped at the longer endpoint ->
+// this path): 117.5 -> 47.4 ms, of which the passes take 13.7 ms (entries 5.8, group sizes 2.5,
+// row sorts 3.2, rows 1.4) and the count 33.5: ranks below 2^15 15.6, 2^16 5.5, 2^17 3.2, hash 9.2.
+// DRAM 14 %, L1 77 %, issue 63 % of peak in the 2^15 kernel at scale 22: bound by the shared
+// and L1 pipe (two wavefronts per 32 tests, one of them bank conflicts) and by issue (10 warp
+// instructions per 32 tests).  Scale 20: 4.45 -> 1.82 ms; Chung-Lu n = 700 001: 1.95 -> 1.18.
+// Tried: 32-bit rows and one entry a warp at a time 68 ms; 32-lane scans of short prefixes
+// instead of lane groups 88 ms; rows on 128-byte lines 1-4 % for twice the copy; 2 or 4 lanes a
+// prefix 73 / 57 ms.
+#include <algorithm>
+
+#include "bisson.cuh"
+
+namespace atc {
+
+namespace {
+
+constexpr int kHub = 8192;              // group sizes of the lowest ranks are counted in shared memory
+constexpr int kHubEntry = 1024;         // ranks whose group cursors are reserved once per tile
+constexpr int kTile = 4096;             // edges per tile of the entry pass
+constexpr int kRank15 = (1 << 15) - 1;  // targets below: a warp's bitmap of 4 KB
+constexpr int kRank16 = (1 << 16) - 1;  // below: a warp's bitmap of 8 KB; ids in 16 bits
+constexpr int kRank17 = 1 << 17;        // below, with entries: a small CTA's bitmap of 16 KB
+constexpr int kRank19 = kTabWords * 32; // below, with a row too long for a warp's hash table: 64 KB
+constexpr int kRankBlockChunk = 1024;   // entries per CTA item
+constexpr int kRankMidMin = 24;         // fewer entries than these do not pay for a CTA's bitmap
+constexpr int kRankBlockMin = 48;
+constexpr int64_t kWideMean = 224;      // mean of min(d+u, d+v) from which 16 lanes read a prefix, below it
+                                        // eight: R-MAT scale 20 (mean 132) 1.88 ms with 8, 2.09 with 16;
+                                        // scale 22 (187) 8.6 and 9.1; scale 24 (270) 50.6 and 47.7
+constexpr int kRankRowMax = kTabWords;  // longest row the CTA sort holds (64 KB)
+constexpr int kRankWarpRow = 1024;      // longest row a warp sorts in registers
+
+// counters of one count
+enum { kc15, kc16, kc17, kc19, kcHashWarp, kcHashBlock, kcNext15, kcNext16, kcNext17, kcNext19, kcNextHashWarp,
+       kcNextHashBlock, kcMid, kcBig, kcNextMid, kcNextBig, kcTooLong, kcCount };
+
+__global__ void rank_keys_kernel(const int64_t* off, const int32_t* indeg, int64_t n, int B, int db, uint64_t* keys) {
+  const uint64_t top = (1ull << db) - 1;
+  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
+    const uint64_t d = (uint64_t)(off[v + 1] - off[v]) + (uint64_t)indeg[v];
+    keys[v] = (top - d) << B | (uint64_t)v;
+  }
+}
+
+__global__ void rank_scatter_kernel(const uint64_t* sorted, int64_t n, int B, int32_t* rank) {
+  const uint64_t mask = (1ull << B) - 1;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    rank[sorted[i] & mask] = (int32_t)i;
+}
+
+// Out-degrees by rank, every edge's slot in its row, and the edges per target.  Edges of one
+// source are contiguous, so a warp takes each run of one row with one atomic; the targets are
+// hubs, whose counters would serialise: the lowest ranks are counted per CTA.
+__global__ void __launch_bounds__(512) rank_count_kernel(const int32_t* esrc, const int32_t* cols, int64_t m,
+                                                         const int32_t* rank, int32_t* deg, int32_t* cnt, uint32_t* slot) {
+  __shared__ int hub[kHub];
+  for (int j = threadIdx.x; j < kHub; j += blockDim.x) hub[j] = 0;
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const int64_t m_pad = (m + 31) & ~31ll;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m_pad; i += (int64_t)gridDim.x * blockDim.x) {
+    int32_t hi = -1, lo = 0;
+    if (i < m) {
+      const int32_t a = __ldg(rank + esrc[i]), b = __ldg(rank + cols[i]);
+      hi = max(a, b);
+      lo = min(a, b);
+      if (lo < kHub) atomicAdd(&hub[lo], 1);
+      else atomicAdd(&cnt[lo], 1);
+    }
+    const unsigned same = __match_any_sync(0xffffffffu, hi);
+    const int lead = __ffs(same) - 1;
+    int base = 0;
+    if (hi >= 0 && lane == lead) base = atomicAdd(&deg[hi], __popc(same));
+    base = __shfl_sync(0xffffffffu, base, lead);
+    if (hi >= 0) slot[i] = (uint32_t)(base + __popc(same & ((1u << lane) - 1)));
+  }
+  __syncthreads();
+  for (int j = threadIdx.x; j < kHub; j += blockDim.x)
+    if (hub[j]) atomicAdd(&cnt[j], hub[j]);
+}
+
+// Rows of the 16-bit copy start at multiples of eight ids: their lengths in such pieces.
+__global__ void rank_pieces_kernel(const int32_t* deg, int64_t n, int32_t* pieces) {
+  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v <= n; v += (int64_t)gridDim.x * blockDim.x)
+    pieces[v] = v < n ? (deg[v] + 7) >> 3 : 0;
+}
+
+__global__ void rank_rows_kernel(const int32_t* esrc, const int32_t* cols, int64_t m, const int32_t* rank,
+                                 const uint32_t* slot, const int64_t* roff, int32_t* rcols) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t a = __ldg(rank + esrc[i]), b = __ldg(rank + cols[i]);
+    rcols[__ldg(roff + max(a, b)) + slot[i]] = min(a, b);
+  }
+}
+
+// Rows of up to 32 elements: a warp takes 32 consecutive rows, cuts them into windows of whole
+// rows of at most 32 elements together and sorts each window by (row, id) across its lanes.
+// Longer rows go on a list each for the warp and the CTA sort.
+__global__ void rank_sort_small_kernel(const int64_t* roff, int64_t n, int32_t* rcols, int32_t* mid, int32_t* big,
+                                       int* ctr) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t rb = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; rb * 32 < n; rb += warps) {
+    const int64_t row = min(rb * 32 + lane, n);
+    const int64_t start = __ldg(roff + row), end = __ldg(roff + min(row + 1, n));
+    const int len = (int)(end - start);
+    const unsigned mm = __ballot_sync(0xffffffffu, len > 32 && len <= kRankWarpRow);
+    const unsigned mb = __ballot_sync(0xffffffffu, len > kRankWarpRow);
+    if (mm) {
+      int at = 0;
+      if (lane == 0) at = atomicAdd(&ctr[kcMid], __popc(mm));
+      at = __shfl_sync(0xffffffffu, at, 0);
+      if (len > 32 && len <= kRankWarpRow) mid[at + __popc(mm & ((1u << lane) - 1))] = (int32_t)row;
+    }
+    if (mb) {
+      int at = 0;
+      if (lane == 0) at = atomicAdd(&ctr[kcBig], __popc(mb));
+      at = __shfl_sync(0xffffffffu, at, 0);
+      if (len > kRankWarpRow) big[at + __popc(mb & ((1u << lane) - 1))] = (int32_t)row;
+    }
+    const unsigned multi = __ballot_sync(0xffffffffu, len >= 2 && len <= 32);
+    int c = 0;  // first row of the window
+    while (c < 32 && (multi >> c)) {
+      c += __ffs(multi >> c) - 1;  // rows of fewer than two elements need no sort
+      const int64_t s0 = __shfl_sync(0xffffffffu, start, c);
+      const unsigned fit = __ballot_sync(0xffffffffu, lane >= c && end - s0 <= 32);
+      const int last = 31 - __clz(fit);  // rows c..last; row c fits
+      const int64_t e0 = __shfl_sync(0xffffffffu, end, last);
+      const bool valid = s0 + lane < e0;
+      int k = 0;  // the last row that starts at or before this element
+      const int rel = (int)(start - s0);  // negative for rows before the window
+#pragma unroll
+      for (int step = 16; step > 0; step >>= 1)
+        if (__shfl_sync(0xffffffffu, rel, k + step) <= lane) k += step;
+      uint64_t key = valid ? (uint64_t)k << 32 | (uint32_t)rcols[s0 + lane] : ~0ull;
+#pragma unroll
+      for (int kk = 2; kk <= 32; kk <<= 1)
+#pragma unroll
+        for (int j = kk >> 1; j > 0; j >>= 1) {
+          const uint64_t y = __shfl_xor_sync(0xffffffffu, key, j);
+          const bool keep_min = ((lane & j) == 0) == ((lane & kk) == 0);
+          key = keep_min == (key < y) ? key : y;
+        }
+      if (valid) rcols[s0 + lane] = (int32_t)(uint32_t)key;
+      c = last + 1;
+    }
+  }
+}
+
+// Ascending bitonic sort of R * 32 values held R a lane (element i = register i / 32, lane
+// i % 32).
+template <int R>
+__device__ __forceinline__ void warp_sort(int32_t (&x)[R], int lane) {
+#pragma unroll
+  for (int k = 2; k <= 32 * R; k <<= 1)
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      if (j >= 32) {
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+          if (!(r & (j / 32))) {
+            const int q = r | (j / 32);
+            const bool up = !(r & (k / 32));
+            const int32_t lo = min(x[r], x[q]), hi = max(x[r], x[q]);
+            x[r] = up ? lo : hi;
+            x[q] = up ? hi : lo;
+          }
+      } else {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const int32_t y = __shfl_xor_sync(0xffffffffu, x[r], j);
+          const bool up = k >= 32 ? !(r & (k / 32)) : !(lane & k);
+          x[r] = up == ((lane & j) == 0) ? min(x[r], y) : max(x[r], y);
+        }
+      }
+    }
+}
+
+template <int R>
+__device__ __forceinline__ void warp_sort_row(int32_t* p, int len, int lane) {
+  int32_t x[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) x[r] = r * 32 + lane < len ? p[r * 32 + lane] : INT32_MAX;
+  warp_sort<R>(x, lane);
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (r * 32 + lane < len) p[r * 32 + lane] = x[r];
+}
+
+__global__ void __launch_bounds__(256) rank_sort_mid_kernel(const int64_t* roff, const int32_t* mid, int32_t* rcols,
+                                                            int* ctr) {
+  const int lane = threadIdx.x & 31;
+  const int total = ctr[kcMid];
+  for (;;) {
+    int it = 0;
+    if (lane == 0) it = atomicAdd(&ctr[kcNextMid], 1);
+    it = __shfl_sync(0xffffffffu, it, 0);
+    if (it >= total) break;
+    const int32_t u = mid[it];
+    const int64_t b = __ldg(roff + u);
+    const int len = (int)(__ldg(roff + u + 1) - b);
+    int32_t* p = rcols + b;
+    if (len <= 64) warp_sort_row<2>(p, len, lane);
+    else if (len <= 128) warp_sort_row<4>(p, len, lane);
+    else if (len <= 256) warp_sort_row<8>(p, len, lane);
+    else if (len <= 512) warp_sort_row<16>(p, len, lane);
+    else warp_sort_row<32>(p, len, lane);
+  }
+}
+
+// Rows beyond kRankWarpRow, in shared memory; one beyond kRankRowMax gives the count up
+// (ctr[kcTooLong]: the caller counts by whole lists instead).
+__global__ void __launch_bounds__(1024) rank_sort_big_kernel(const int64_t* roff, const int32_t* big, int32_t* rcols,
+                                                             int* ctr) {
+  extern __shared__ __align__(16) int32_t sm[];  // kRankRowMax
+  __shared__ int item;
+  const int total = ctr[kcBig];
+  for (;;) {
+    if (threadIdx.x == 0) item = atomicAdd(&ctr[kcNextBig], 1);
+    __syncthreads();
+    const int it = item;
+    if (it >= total) break;
+    const int32_t u = big[it];
+    const int64_t b = roff[u], len = roff[u + 1] - b;
+    if (len > kRankRowMax) {
+      if (threadIdx.x == 0) ctr[kcTooLong] = 1;
+      __syncthreads();
+      continue;
+    }
+    int pow2 = 2 * kRankWarpRow;
+    while (pow2 < (int)len) pow2 <<= 1;
+    for (int j = threadIdx.x; j < pow2; j += blockDim.x) sm[j] = j < len ? rcols[b + j] : INT32_MAX;
+    __syncthreads();
+    for (int k = 2; k <= pow2; k <<= 1)
+      for (int j = k >> 1; j > 0; j >>= 1) {
+        for (int t = threadIdx.x; t < pow2 / 2; t += blockDim.x) {
+          const int i = (t / j) * 2 * j + (t & (j - 1)), q = i + j;
+          const bool up = (i & k) == 0;
+          const int32_t x = sm[i], y = sm[q];
+          if ((x > y) == up) {
+            sm[i] = y;
+            sm[q] = x;
+          }
+        }
+        __syncthreads();
+      }
+    for (int j = threadIdx.x; j < len; j += blockDim.x) rcols[b + j] = sm[j];
+    __syncthreads();
+  }
+}
+
+// tile_row[t] = the row that holds element t * kTile.
+__global__ void rank_tile_rows_kernel(const int64_t* roff, int64_t n, int32_t* tile_row) {
+  for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t b = roff[u], e = roff[u + 1];
+    for (int64_t t = (b + kTile - 1) / kTile; t * kTile < e; ++t) tile_row[t] = (int32_t)u;
+  }
+}
+
+// Entry of every edge in its target's group: where the source's row starts and how much of it
+// lies before the target.  Targets below kRank16 read the 16-bit copy of the rows (r16, starts in
+// pieces of eight ids), written here; the others the rows themselves.  A tile's entries of the
+// most contended targets take their places with one atomic per tile and target.
+constexpr int kEntryThreads = 1024;
+constexpr int kEntryEach = kTile / kEntryThreads;
+__global__ void __launch_bounds__(kEntryThreads, 2) rank_entries_kernel(const int64_t* roff, int64_t n, int64_t m,
+                                                                     const int32_t* rcols, const int32_t* tile_row,
+                                                                     const int64_t* gstart, const int64_t* roff8,
+                                                                     int32_t* gcur, uint16_t* r16, uint2* ent) {
+  __shared__ int hub[kHubEntry];
+  const int64_t tiles = (m + kTile - 1) / kTile;
+  for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+    for (int j = threadIdx.x; j < kHubEntry; j += kEntryThreads) hub[j] = 0;
+    __syncthreads();
+    const int32_t r0 = tile_row[t];
+    const int32_t r1 = t + 1 < tiles ? tile_row[t + 1] : (int32_t)(n - 1);
+    int32_t lo[kEntryEach];
+    uint32_t st[kEntryEach], len[kEntryEach];
+    int pos[kEntryEach];
+#pragma unroll
+    for (int q = 0; q < kEntryEach; ++q) {
+      const int64_t p = t * kTile + q * kEntryThreads + threadIdx.x;
+      lo[q] = -1;
+      if (p < m) {
+        int32_t a = r0, b = r1;  // the last row that starts at or before p
+        while (a < b) {
+          const int32_t mid = a + ((b - a + 1) >> 1);
+          if (__ldg(roff + mid) <= p) a = mid; else b = mid - 1;
+        }
+        lo[q] = rcols[p];
+        st[q] = (uint32_t)__ldg(roff + a);
+        len[q] = (uint32_t)p - st[q];
+        if (lo[q] < kRank16) {
+          const int64_t r8 = __ldg(roff8 + a);
+          st[q] = (uint32_t)r8;
+          r16[8 * r8 + len[q]] = (uint16_t)lo[q];
+        }
+        pos[q] = lo[q] < kHubEntry ? atomicAdd(&hub[lo[q]], 1) : atomicAdd(&gcur[lo[q]], 1);
+      }
+    }
+    __syncthreads();
+    for (int j = threadIdx.x; j < kHubEntry; j += kEntryThreads)
+      if (hub[j]) hub[j] = atomicAdd(&gcur[j], hub[j]);
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kEntryEach; ++q)
+      if (lo[q] >= 0) {
+        const int at = pos[q] + (lo[q] < kHubEntry ? hub[lo[q]] : 0);
+        ent[__ldg(gstart + lo[q]) + at] = make_uint2(st[q], len[q]);
+      }
+    __syncthreads();
+  }
+}
+
+// Work items (target, chunk) of the five kinds of targets; hash: the targets no bitmap takes
+// (warp items from the front, block items from the back).
+struct RankItemLists {
+  int2 *t15, *t16, *t17, *t19, *hash;
+  int64_t hcap;
+  int chunk;  // entries per warp item
+};
+__global__ void rank_items_kernel(const int64_t* roff, const int64_t* gstart, int64_t n, RankItemLists li, int* ctr) {
+  const int64_t n_pad = (n + 31) & ~31ll;
+  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n_pad; v += (int64_t)gridDim.x * blockDim.x) {
+    int64_t ne = 0, dv = 0;
+    if (v < n) {
+      ne = gstart[v + 1] - gstart[v];
+      dv = roff[v + 1] - roff[v];
+    }
+    const bool any = ne > 0 && dv > 0;
+    const int kind = !any ? -1
+                     : v < kRank15 ? kc15
+                     : v < kRank16 ? kc16
+                     : v < kRank17 && ne >= kRankMidMin ? kc17
+                     : dv <= kWarpHashMax ? kcHashWarp  // R-MAT scale 24, ranks 2^17..2^19: 9.2 ms by hash
+                                                        // tables, 21 ms by 64 KB bitmaps a CTA
+                     : v < kRank19 && ne >= kRankBlockMin ? kc19 : kcHashBlock;
+    const int64_t chunk = kind <= kc16 ? li.chunk : kind <= kc19 ? kRankBlockChunk
+                          : kind == kcHashWarp ? kWarpChunk : kBlockChunk;
+    const int k = any ? (int)((ne + chunk - 1) / chunk) : 0;
+#pragma unroll
+    for (int q = kc15; q <= kcHashBlock; ++q) {
+      if (!__any_sync(0xffffffffu, kind == q)) continue;
+      const int at = warp_reserve(&ctr[q], kind == q ? k : 0);
+      if (kind != q) continue;
+      int2* to = q == kc15 ? li.t15 : q == kc16 ? li.t16 : q == kc17 ? li.t17 : q == kc19 ? li.t19 : li.hash;
+      for (int c = 0; c < k; ++c)
+        to[q == kcHashBlock ? li.hcap - 1 - (at + c) : (int64_t)(at + c)] = make_int2((int32_t)v, c);
+    }
+  }
+}
+
+// Items of the hash kernels.
+struct RankedItems {
+  static constexpr bool kBatch = false;
+  static constexpr int kMinBlocks = 0;
+  const int2* p;
+  const int64_t* gstart;
+  int64_t cap;
+  bool block;
+  __device__ __forceinline__ GroupItem get(const CsrView& g, int i) const {
+    const int2 c = block ? p[cap - 1 - i] : p[i];
+    const int64_t chunk = block ? kBlockChunk : kWarpChunk;
+    const int64_t b = gstart[c.x] + c.y * chunk, e = min(gstart[c.x + 1], b + chunk);
+    const int64_t hb = g.off[c.x], dh = g.off[c.x + 1] - hb;
+    int32_t mode;
+    if (!block) mode = dh <= 8 ? 0 : 1;
+    else mode = dh <= kHashMax ? 0 : (g.cols[hb + dh - 1] - g.cols[hb] < kTabWords * 32 ? 1 : 2);
+    return GroupItem{c.x, mode, b, e};
+  }
+};
+
+// Streams the prefixes of entries [base, base + 32) for every batch that next() hands out through
+// the bitmap T of N+(v): a bit is 0 for a member, 1 otherwise (the empty table is all ones, and
+// members are put back by storing whole words).  Prefixes of 32 or more are walked by the whole
+// warp, up to four loads in flight per lane; lanes past the end test v itself, which is
+// never a member, so no load or test is predicated.
+template <class Next>
+__device__ __forceinline__ unsigned stream_bitmap(const int32_t* __restrict__ cols, const uint2* __restrict__ ent,
+                                                  int64_t e1, int lane, const uint32_t* T, int32_t v, Next next) {
+  unsigned cnt = 0;
+  auto test = [&](int32_t x) { cnt += ~(T[(uint32_t)x >> 5] >> (x & 31)) & 1u; };
+  for (int64_t base = next(); base < e1; base = next()) {
+    uint2 q = make_uint2(0u, 0u);
+    if (base + lane < e1) q = __ldg(ent + base + lane);
+    unsigned longm = __ballot_sync(0xffffffffu, q.y >= 32);
+    while (longm) {
+      const int k = __ffs(longm) - 1;
+      longm &= longm - 1;
+      const int32_t* P = cols + __shfl_sync(0xffffffffu, q.x, k) + lane;
+      int left = (int)__shfl_sync(0xffffffffu, q.y, k) - lane;  // elements from this lane's first on
+      const int ln = left + lane;
+      for (int j0 = 0; j0 < ln; j0 += 128, P += 128, left -= 128) {
+        const int32_t x0 = left > 0 ? __ldg(P) : v;
+        if (j0 + 64 < ln) {
+          const int32_t x1 = __ldg(P + 32);
+          const int32_t x2 = left > 64 ? __ldg(P + 64) : v;
+          const int32_t x3 = left > 96 ? __ldg(P + 96) : v;
+          test(x0);
+          test(x1);
+          test(x2);
+          test(x3);
+        } else {
+          const int32_t x1 = left > 32 ? __ldg(P + 32) : v;
+          test(x0);
+          test(x1);
+        }
+      }
+    }
+    const int slen = q.y < 32 ? (int)q.y : 0;
+    int incl = slen;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    const int start = incl - slen;
+    const uint32_t at = q.x - (uint32_t)start;
+    for (int t0 = 0; t0 < total; t0 += 32) {
+      const int t = t0 + lane;
+      int k = 0;  // the last lane whose prefix starts at or before t
+#pragma unroll
+      for (int step = 16; step > 0; step >>= 1)
+        if (__shfl_sync(0xffffffffu, start, k + step) <= t) k += step;
+      const uint32_t kp = __shfl_sync(0xffffffffu, at, k);
+      test(t < total ? __ldg(cols + (kp + (uint32_t)t)) : v);
+    }
+  }
+  return cnt;
+}
+
+// Targets below kRank15 (BITS = 2^15) or kRank16 (2^16): a warp per chunk of entries, N+(v) as
+// the warp's own bitmap.  Prefixes are read from the 16-bit rows by groups of kLanes lanes, 16
+// bytes (eight ids) a lane: 32 / kLanes entries are under way at once, so that short prefixes fill
+// the warp without a search for the owner of each element, and each group has the next piece
+// loading while it tests the last.  Ids past a prefix's end are masked off by position.
+template <int BITS, int WARPS, int kLanes>
+__global__ void __launch_bounds__(WARPS * 32) rank_warp_kernel(const int64_t* __restrict__ roff,
+                                                               const int32_t* __restrict__ rcols,
+                                                               const uint4* __restrict__ r16,
+                                                               const uint2* __restrict__ ent,
+                                                               const int2* __restrict__ items,
+                                                               const int64_t* __restrict__ gstart, int chunk,
+                                                               const int* nitems_dev, int* next, const int* too_long,
+                                                               unsigned long long* out) {
+  constexpr uint32_t kBytes = BITS / 8;
+  __shared__ __align__(16) unsigned char smem[WARPS * kBytes];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const uint32_t base = w * kBytes;
+  uint32_t* T = reinterpret_cast<uint32_t*>(smem + base);
+  for (int j = lane; j < (int)(kBytes / 4); j += 32) T[j] = 0u;
+  __syncwarp();
+  const int nitems = *too_long ? 0 : *nitems_dev;  // an unsorted row's prefix is no prefix
+  const int sub = lane % kLanes;
+  // the bit of id x is bit 31 - x % 32 of word x / 32: shifting the word left by x brings it to the
+  // top, and a funnel shift moves it into acc, two instructions after the load
+  auto word = [&](uint32_t r) {  // r: the id in its low 16 bits
+    return *reinterpret_cast<const uint32_t*>(smem + (((r >> 3) & (kBytes - 4)) | base));
+  };
+  auto tests = [&](const uint4& d, int valid) -> unsigned {  // members among the first `valid` ids
+    const uint32_t x1 = d.x >> 16, y1 = d.y >> 16, z1 = d.z >> 16, w1 = d.w >> 16;
+    const uint32_t b0 = word(d.x), b1 = word(x1), b2 = word(d.y), b3 = word(y1), b4 = word(d.z), b5 = word(z1),
+                   b6 = word(d.w), b7 = word(w1);
+    auto fold = [](uint32_t acc, uint32_t b, uint32_t r) {
+      return __funnelshift_l(__funnelshift_l(b, b, r), acc, 1);
+    };
+    uint32_t acc = fold(0u, b0, d.x), acc2 = fold(0u, b4, d.z);
+    acc = fold(acc, b1, x1);
+    acc2 = fold(acc2, b5, z1);
+    acc = fold(acc, b2, d.y);
+    acc2 = fold(acc2, b6, d.w);
+    acc = fold(acc, b3, y1);
+    acc2 = fold(acc2, b7, w1);
+    return __popc((acc << 4 | acc2) & (0xff00u >> min(max(valid, 0), 8)) & 0xffu);
+  };
+  unsigned long long total = 0;
+  for (;;) {
+    int it = 0;
+    if (lane == 0) it = atomicAdd(next, 1);
+    it = __shfl_sync(0xffffffffu, it, 0);
+    if (it >= nitems) break;
+    const int2 c = __ldg(items + it);
+    const int32_t v = c.x;
+    const int64_t g0 = __ldg(gstart + v) + (int64_t)c.y * chunk;
+    const int ne = (int)min(__ldg(gstart + v + 1) - g0, (int64_t)chunk);
+    const uint2* en = ent + g0;
+    const int64_t hb = __ldg(roff + v);
+    const int dh = (int)(__ldg(roff + v + 1) - hb);
+    int i = lane / kLanes;
+    uint2 nq = i < ne ? __ldg(en + i) : make_uint2(0u, 0u);
+    for (int j = lane; j < dh; j += 32) {
+      const int32_t x = __ldg(rcols + hb + j);
+      atomicOr(&T[x >> 5], 0x80000000u >> (x & 31));
+    }
+    __syncwarp();
+    uint32_t at = 0;  // the lane's next piece
+    int left = 0;     // ids from the lane's next piece to the end of the group's prefix
+    unsigned cnt = 0;
+    // loads the lane's next piece; returns its valid ids (<= 0: none)
+    auto fetch = [&](uint4& d) -> int {
+      if (left + 8 * sub <= 0 && i < ne) {  // the group's prefix is done
+        at = nq.x + sub;
+        left = (int)nq.y - 8 * sub;
+        i += 32 / kLanes;
+        if (i < ne) nq = __ldg(en + i);
+      }
+      const int valid = left;
+      d = make_uint4(0u, 0u, 0u, 0u);
+      if (valid > 0) d = __ldg(r16 + at);
+      at += kLanes;
+      left -= 8 * kLanes;
+      return valid;
+    };
+    uint4 d0, d1;
+    int v0 = fetch(d0), v1;
+    do {
+      v1 = fetch(d1);
+      cnt += tests(d0, v0);
+      v0 = fetch(d0);
+      cnt += tests(d1, v1);
+    } while (__any_sync(0xffffffffu, v0 > 0 || left > 0 || i < ne));
+    total += cnt;
+    __syncwarp();
+    for (int j = lane; j < dh; j += 32) T[__ldg(rcols + hb + j) >> 5] = 0u;
+    __syncwarp();
+  }
+  warp_add_count(total, out);
+}
+
+// Targets of larger rank: a CTA per chunk of entries, ids in 32 bits.
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) rank_block_kernel(CsrView g, const uint2* __restrict__ ent,
+                                                             const int2* __restrict__ items,
+                                                             const int64_t* __restrict__ gstart, uint32_t words,
+                                                             const int* nitems_dev, int* next, const int* too_long,
+                                                             unsigned long long* out) {
+  extern __shared__ __align__(16) uint32_t T[];  // words
+  __shared__ int item;
+  __shared__ unsigned long long bnext;
+  const int lane = threadIdx.x & 31;
+  for (uint32_t j = threadIdx.x; j < words; j += blockDim.x) T[j] = ~0u;
+  const int nitems = *too_long ? 0 : *nitems_dev;  // an unsorted row holds ids beyond the bitmap
+  unsigned long long total = 0;
+  for (;;) {
+    if (threadIdx.x == 0) {
+      item = atomicAdd(next, 1);
+      bnext = 0;
+    }
+    __syncthreads();
+    const int it = item;
+    if (it >= nitems) break;
+    const int2 c = __ldg(items + it);
+    const int32_t v = c.x;
+    const int64_t b = __ldg(gstart + v) + (int64_t)c.y * kRankBlockChunk;
+    const int64_t e = min(__ldg(gstart + v + 1), b + kRankBlockChunk);
+    const int64_t hb = __ldg(g.off + v);
+    const int dh = (int)(__ldg(g.off + v + 1) - hb);
+    for (int j = threadIdx.x; j < dh; j += blockDim.x) {
+      const int32_t x = __ldg(g.cols + hb + j);
+      atomicAnd(&T[x >> 5], ~(1u << (x & 31)));
+    }
+    __syncthreads();
+    total += stream_bitmap(g.cols, ent, e, lane, T, v, [&]() {
+      unsigned long long r = 0;
+      if (lane == 0) r = atomicAdd(&bnext, 32ull);
+      return b + (int64_t)__shfl_sync(0xffffffffu, r, 0);
+    });
+    __syncthreads();
+    for (int j = threadIdx.x; j < dh; j += blockDim.x) T[__ldg(g.cols + hb + j) >> 5] = ~0u;
+    __syncthreads();
+  }
+  warp_add_count(total, out);
+}
+
+// Byte offsets of the buffers of one count in a single allocation.
+struct Arena {
+  size_t bytes = 0;
+  template <class T>
+  size_t add(size_t count) {
+    const size_t at = bytes;
+    bytes += (sizeof(T) * (count ? count : 1) + 255) & ~size_t(255);
+    return at;
+  }
+};
+
+}  // namespace
+
+atc_status count_ranked(const atc_csr* csr, unsigned long long* out, bool* done, cudaStream_t s, int* launches) {
+  *done = false;
+  const CsrPriv* pv = static_cast<const CsrPriv*>(csr->priv);
+  const int64_t n = csr->n, m = csr->m;
+  std::optional<Phase> ph;
+  ph.emplace("tc.group", s);
+  const int B = id_bits(n), db = id_bits(n);  // degrees are below n
+  size_t sort_tmp = 0, scan_tmp = 0;
+  ATC_TRY(sort_keys_u64_tmp(nullptr, &sort_tmp, nullptr, nullptr, (size_t)n, B, B + db, nullptr, s));
+  ATC_TRY(exclusive_scan_i32_to_i64_tmp(nullptr, &scan_tmp, nullptr, nullptr, (size_t)n + 1, s));
+  const int64_t tiles = (m + kTile - 1) / kTile;
+  // a warp item holds at most 512 entries (the bitmap costs d+(v) of them to set up), fewer where
+  // that would leave warps without work
+  const int64_t warps = (int64_t)sm_count() * 48;
+  const int chunk = (int)std::min<int64_t>(std::max<int64_t>((m / (8 * warps)) & ~31ll, 64), 512);
+  auto item_cap = [&](int64_t below, int64_t per) { return std::min<int64_t>(n, below) + m / per + 1; };
+  const int64_t cap15 = item_cap(kRank15, chunk), cap16 = n > kRank15 ? item_cap(kRank16, chunk) : 0;
+  const int64_t cap17 = n > kRank16 ? item_cap(kRank17, kRankBlockChunk) : 0;
+  const int64_t cap19 = n > kRank17 ? item_cap(kRank19, kRankBlockChunk) : 0;
+  const int64_t hcap = n > kRank16 ? max_items(n, m, std::min(kWarpChunk, kBlockChunk)) : 0;
+  Arena ar;
+  const size_t a_ka = ar.add<uint64_t>(n), a_kb = ar.add<uint64_t>(n);
+  const size_t a_tmp = ar.add<char>(std::max(sort_tmp, scan_tmp));
+  const size_t a_rank = ar.add<int32_t>(n);
+  const size_t a_zero = ar.bytes;  // from here on zeroed
+  const size_t a_ctr = ar.add<int>(kcCount), a_deg = ar.add<int32_t>(n + 1), a_cnt = ar.add<int32_t>(n + 1),
+               a_gcur = ar.add<int32_t>(n);
+  const size_t zero_end = ar.bytes;
+  const size_t a_roff = ar.add<int64_t>(n + 1), a_gstart = ar.add<int64_t>(n + 1);
+  const size_t a_rcols = ar.add<int32_t>(m + 16), a_ent = ar.add<uint2>(m), a_tile = ar.add<int32_t>(tiles + 1);
+  const size_t a_mid = ar.add<int32_t>(m / 33 + 1), a_big = ar.add<int32_t>(m / (kRankWarpRow + 1) + 1);
+  const size_t a_15 = ar.add<int2>(cap15), a_16 = ar.add<int2>(cap16), a_17 = ar.add<int2>(cap17),
+               a_19 = ar.add<int2>(cap19), a_hash = ar.add<int2>(hcap);
+  const size_t a_pieces = ar.add<int32_t>(n + 1), a_roff8 = ar.add<int64_t>(n + 1);
+  const size_t a_r16 = ar.add<uint16_t>(m + 8 * std::min(n, m));
+  DevBuf<char> mem;
+  if (mem.alloc(ar.bytes, s) != ATC_OK) {  // no room for the copy: the caller counts in place
+    cudaGetLastError();
+    return ATC_OK;
+  }
+  char* p = mem.p;
+  uint64_t* ka = reinterpret_cast<uint64_t*>(p + a_ka);
+  uint64_t* kb = reinterpret_cast<uint64_t*>(p + a_kb);
+  int32_t* rank = reinterpret_cast<int32_t*>(p + a_rank);
+  int* ctr = reinterpret_cast<int*>(p + a_ctr);
+  int32_t* deg = reinterpret_cast<int32_t*>(p + a_deg);
+  int32_t* cnt = reinterpret_cast<int32_t*>(p + a_cnt);
+  int32_t* gcur = reinterpret_cast<int32_t*>(p + a_gcur);
+  int64_t* roff = reinterpret_cast<int64_t*>(p + a_roff);
+  int64_t* gstart = reinterpret_cast<int64_t*>(p + a_gstart);
+  int32_t* rcols = reinterpret_cast<int32_t*>(p + a_rcols);
+  uint2* ent = reinterpret_cast<uint2*>(p + a_ent);
+  uint32_t* slot = reinterpret_cast<uint32_t*>(ent);  // until the entries are written
+  int32_t* tile_row = reinterpret_cast<int32_t*>(p + a_tile);
+  int32_t* mid = reinterpret_cast<int32_t*>(p + a_mid);
+  int32_t* big = reinterpret_cast<int32_t*>(p + a_big);
+  int32_t* pieces = reinterpret_cast<int32_t*>(p + a_pieces);
+  int64_t* roff8 = reinterpret_cast<int64_t*>(p + a_roff8);
+  uint16_t* r16 = reinterpret_cast<uint16_t*>(p + a_r16);
+  const RankItemLists li{reinterpret_cast<int2*>(p + a_15), reinterpret_cast<int2*>(p + a_16),
+                         reinterpret_cast<int2*>(p + a_17), reinterpret_cast<int2*>(p + a_19),
+                         reinterpret_cast<int2*>(p + a_hash), hcap, chunk};
+  ATC_CK(cudaMemsetAsync(p + a_zero, 0, zero_end - a_zero, s));
+  rank_keys_kernel<<<grid_for(n, 256), 256, 0, s>>>(csr->offsets, pv->indeg, n, B, db, ka);
+  ATC_CK(cudaGetLastError());
+  uint64_t* sorted = nullptr;
+  ATC_TRY(sort_keys_u64_tmp(p + a_tmp, &sort_tmp, ka, kb, (size_t)n, B, B + db, &sorted, s));
+  rank_scatter_kernel<<<grid_for(n, 256), 256, 0, s>>>(sorted, n, B, rank);
+  rank_count_kernel<<<grid_for(m, 512, 4), 512, 0, s>>>(pv->esrc, csr->cols, m, rank, deg, cnt, slot);
+  ATC_CK(cudaGetLastError());
+  ATC_TRY(exclusive_scan_i32_to_i64_tmp(p + a_tmp, &scan_tmp, deg, roff, (size_t)n + 1, s));
+  ATC_TRY(exclusive_scan_i32_to_i64_tmp(p + a_tmp, &scan_tmp, cnt, gstart, (size_t)n + 1, s));
+  rank_pieces_kernel<<<grid_for(n + 1, 256), 256, 0, s>>>(deg, n, pieces);
+  ATC_TRY(exclusive_scan_i32_to_i64_tmp(p + a_tmp, &scan_tmp, pieces, roff8, (size_t)n + 1, s));
+  rank_rows_kernel<<<grid_for(m, 256), 256, 0, s>>>(pv->esrc, csr->cols, m, rank, slot, roff, rcols);
+  rank_sort_small_kernel<<<grid_for(n, 256), 256, 0, s>>>(roff, n, rcols, mid, big, ctr);
+  rank_sort_mid_kernel<<<sm_count() * blocks_per_sm((const void*)rank_sort_mid_kernel, 256, 0), 256, 0, s>>>(
+      roff, mid, rcols, ctr);
+  const size_t big_smem = sizeof(int32_t) * kRankRowMax;
+  ATC_CK(cudaFuncSetAttribute((const void*)rank_sort_big_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)big_smem));
+  const int64_t long_rows = m / (kRankWarpRow + 1);
+  if (long_rows) {
+    rank_sort_big_kernel<<<(unsigned)std::min<int64_t>(long_rows, sm_count() * 2), 1024, big_smem, s>>>(roff, big, rcols,
+                                                                                                      ctr);
+    *launches += 1;
+  }
+  rank_tile_rows_kernel<<<grid_for(n, 256), 256, 0, s>>>(roff, n, tile_row);
+  rank_entries_kernel<<<grid_for(m, kTile, 2), kEntryThreads, 0, s>>>(roff, n, m, rcols, tile_row, gstart, roff8,
+                                                                        gcur, r16, ent);
+  rank_items_kernel<<<grid_for(n, 256), 256, 0, s>>>(roff, gstart, n, li, ctr);
+  ATC_CK(cudaGetLastError());
+  *launches += 14;
+  ph.reset();
+  ph.emplace("tc.count", s);
+  const CsrView g = csr_view(roff, rcols, nullptr, n, m);
+  const int* too = ctr + kcTooLong;
+  auto block_launch = [&](auto kern, int threads, int64_t bits, const int2* items, int kind, int nxt) -> atc_status {
+    const size_t smem = (size_t)bits / 8;
+    ATC_CK(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<sm_count() * blocks_per_sm((const void*)kern, threads, smem), threads, smem, s>>>(
+        g, ent, items, gstart, (uint32_t)(bits / 32), ctr + kind, ctr + nxt, too, out);
+    ATC_CK(cudaGetLastError());
+    *launches += 1;
+    return ATC_OK;
+  };
+  if (n > kRank17) ATC_TRY(block_launch(rank_block_kernel<256>, 256, kRank19, li.t19, kc19, kcNext19));
+  if (n > kRank16) {
+    ATC_TRY(block_launch(rank_block_kernel<128>, 128, kRank17, li.t17, kc17, kcNext17));
+    const auto hw = bisson_warp_kernel<RankedItems, kDefaultSlots, PrefixPartners>;
+    const auto hb = bisson_block_kernel<RankedItems, kDefaultSlots, PrefixPartners>;
+    const size_t hsmem = sizeof(int32_t) * kTabWords;
+    ATC_CK(cudaFuncSetAttribute((const void*)hb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsmem));
+    hb<<<sm_count() * blocks_per_sm((const void*)hb, kBgWarps * 32, hsmem), kBgWarps * 32, hsmem, s>>>(
+        g, PrefixPartners{ent}, RankedItems{li.hash, gstart, hcap, true}, 0, ctr + kcHashBlock, ctr + kcNextHashBlock,
+        (uint32_t)kTabWords, GraphTags{nullptr, 0, nullptr}, out);
+    hw<<<sm_count() * blocks_per_sm((const void*)hw, kBgWarps * 32, 0), kBgWarps * 32, 0, s>>>(
+        g, PrefixPartners{ent}, RankedItems{li.hash, gstart, hcap, false}, 0, ctr + kcHashWarp, ctr + kcNextHashWarp,
+        GraphTags{nullptr, 0, nullptr}, out);
+    ATC_CK(cudaGetLastError());
+    *launches += 2;
+  }
+  const uint4* q16 = reinterpret_cast<const uint4*>(r16);
+  const bool wide = csr->wedges_min >= kWideMean * m;
+  if (n > kRank15) {
+    const auto kern = wide ? rank_warp_kernel<1 << 16, 4, 16> : rank_warp_kernel<1 << 16, 4, 8>;
+    kern<<<sm_count() * blocks_per_sm((const void*)kern, 128, 0), 128, 0, s>>>(
+        roff, rcols, q16, ent, li.t16, gstart, chunk, ctr + kc16, ctr + kcNext16, too, out);
+    *launches += 1;
+  }
+  const auto kern = wide ? rank_warp_kernel<1 << 15, 8, 16> : rank_warp_kernel<1 << 15, 8, 8>;
+  kern<<<sm_count() * blocks_per_sm((const void*)kern, 256, 0), 256, 0, s>>>(
+      roff, rcols, q16, ent, li.t15, gstart, chunk, ctr + kc15, ctr + kcNext15, too, out);
+  ATC_CK(cudaGetLastError());
+  *launches += 1;
+  int too_long = 0;
+  if (long_rows) {
+    ATC_CK(cudaMemcpyAsync(&too_long, ctr + kcTooLong, sizeof(int), cudaMemcpyDeviceToHost, s));
+    ATC_CK(cudaStreamSynchronize(s));
+  }
+  *done = too_long == 0;
+  return ATC_OK;
+}
+
+}  // namespace atc

@@ -479,7 +479,7 @@ __global__ void __launch_bounds__(kBgWarps * 32) sorted_warp_kernel(CsrView g, c
     int64_t cur = gi.b;
     auto nb = [&]() { int64_t r = cur; cur += 32; return r; };
     SortedProber<KIND> pr{L, piv[w], dh, L[dh - 1], 0, INT32_MIN, 16, 31 - __clz((dh + 31) >> 5)};
-    total += stream_partners(g, plist, gi.e, lane, nb, pr);
+    total += stream_partners(g, ListPartners{plist}, gi.e, lane, nb, pr);
     __syncwarp();  // the next item overwrites the copy
   }
   warp_add_count(total, out);
@@ -539,7 +539,7 @@ __global__ void __launch_bounds__(kBgWarps * 32) sorted_block_kernel(CsrView g, 
     };
     SortedProber<KIND> pr{L, piv, (int)dh, __ldg(g.cols + hb + dh - 1), 0, INT32_MIN, 16,
                           31 - __clz((int)((dh + 31) >> 5))};
-    total += stream_partners(g, plist, gi.e, lane, nb, pr);
+    total += stream_partners(g, ListPartners{plist}, gi.e, lane, nb, pr);
     __syncthreads();  // the next item overwrites the copy
   }
   warp_add_count(total, out);
@@ -666,14 +666,14 @@ static atc_status launch_bisson(const CsrView& g, const int32_t* plist, const Gr
     int bps = blocks_per_sm((const void*)bisson_block_kernel<FullItems, S>, kBgWarps * 32, smem);
     int grid = std::min(hc[1], sm_count() * bps);
     bisson_block_kernel<FullItems, S><<<grid, kBgWarps * 32, smem, s>>>(
-        g, plist, FullItems{bitems}, hc[1], nullptr, counters + 5, words, GraphTags{nullptr, 0, nullptr}, ctr);
+        g, ListPartners{plist}, FullItems{bitems}, hc[1], nullptr, counters + 5, words, GraphTags{nullptr, 0, nullptr}, ctr);
     ATC_CK(cudaGetLastError());
     *launches += 1;
   }
   if (hc[0]) {
     int bps = blocks_per_sm((const void*)bisson_warp_kernel<FullItems, S>, kBgWarps * 32, 0);
     int grid = (int)std::min<int64_t>((hc[0] + kBgWarps - 1) / kBgWarps, (int64_t)sm_count() * bps);
-    bisson_warp_kernel<FullItems, S><<<grid, kBgWarps * 32, 0, s>>>(g, plist, FullItems{witems}, hc[0], nullptr,
+    bisson_warp_kernel<FullItems, S><<<grid, kBgWarps * 32, 0, s>>>(g, ListPartners{plist}, FullItems{witems}, hc[0], nullptr,
                                                                    counters + 4, GraphTags{nullptr, 0, nullptr}, ctr);
     ATC_CK(cudaGetLastError());
     *launches += 1;
@@ -783,6 +783,18 @@ static atc_status group_edges(const CsrView& g, const ItemShape& sh, Grouping* g
   ATC_CK(cudaStreamSynchronize(s));
   *launches += 5;
   return ATC_OK;
+}
+
+// The ranked count (csrc/ranked.cu) takes whole counts of CSRs that preTC built and that live on
+// the device.  Parts keep the CSR's own orientation (their counts are defined by it), as do CSRs
+// read from files (any sorted rows are accepted there); CSRs in host memory count in bounded
+// scratch; an item shape asked for by tuning is one of the grouped lists.  Entries hold 32-bit
+// positions.
+static bool ranked_applies(const atc_csr* csr, int64_t e0, int64_t e1, const atc_tuning* t) {
+  const CsrPriv* pv = static_cast<const CsrPriv*>(csr->priv);
+  if (!pv->indeg || pv->host_cols || e0 != 0 || e1 != csr->m || csr->m > (int64_t)INT32_MAX) return false;
+  return !t || (t->bisson_cutover <= 0 && t->bisson_warp_max <= 0 && t->bisson_warp_chunk <= 0 &&
+                t->bisson_block_chunk <= 0 && t->bisson_slots == 0);
 }
 
 static atc_status run_bisson(const CsrView& g, const atc_tuning* t, unsigned long long* ctr, cudaStream_t s,
@@ -1028,23 +1040,26 @@ atc_status atc::part_edge_range(const atc_csr* csr, uint32_t part, uint32_t npar
 }
 
 // Counts the edges [e0, e1) of the CSR (every edge for the whole count).
-// ATC_KERNEL_AUTO: the Bisson-style or the Hu-style count, whichever this cost model of
-// their GB300 times predicts is faster for the CSR.  Bisson-style: 1.232 ps per probe of the
-// shorter lists (W_min) + 117.5 ps per edge (grouping, items) + 0.3 ms per call (two more
-// passes and one more host synchronisation); Hu-style: 1.097 ps per wedge (W) + 103.5 ps per
-// edge.  Fitted to R-MAT scale 24 (117 / 231 ms) and Chung-Lu graphs of 4M-46M edges; the
-// learned selector (atc_select) chooses among all kernels and pipelines instead.
-static atc_kernel auto_kernel(const atc_csr* csr) {
+// ATC_KERNEL_AUTO: the Bisson-style or the Hu-style count, whichever this cost model of their
+// GB300 times predicts is faster.  Hu-style: 1.2 ps per wedge (W) + 45 ps per edge + 0.06 ms.
+// Bisson-style, ranked: 0.37 ps per element of the shorter lists (W_min) + 85 ps per edge (the
+// ranked copy) + 0.17 ms of launches.  By whole lists (parts, loaded CSRs): 1.232 ps per
+// element of W_min + 117.5 ps per edge + 0.3 ms, against Hu's 1.097 ps and 103.5 ps, the fit of
+// the two that it was made with.  Measured Hu / ranked in ms: R-MAT scale 14 0.15 / 0.21, 16 0.37 /
+// 0.26, 18 1.30 / 0.55, 20 6.2 / 1.8, 24 231 / 47; Chung-Lu 1.3M edges 0.21 / 0.33, 9.6M 1.39 /
+// 1.18; RGG 1.6M 0.14 / 0.36, 16M 0.93 / 1.9.
+static atc_kernel auto_kernel(const atc_csr* csr, bool ranked) {
   const double m = (double)csr->m, w = (double)csr->wedges, wmin = (double)csr->wedges_min;
-  const double bisson_ps = 1.232 * wmin + 117.5 * m + 3.0e8;
-  const double hu_ps = 1.097 * w + 103.5 * m;
+  const double bisson_ps = ranked ? 0.37 * wmin + 85.0 * m + 1.7e8 : 1.232 * wmin + 117.5 * m + 3.0e8;
+  const double hu_ps = ranked ? 1.2 * w + 45.0 * m + 6.0e7 : 1.097 * w + 103.5 * m;
   return hu_ps < bisson_ps ? ATC_KERNEL_HU : ATC_KERNEL_BISSON;
 }
 
 static atc_status tc_window(const atc_csr* csr, atc_kernel kernel, const atc_tuning* tuning, int64_t e0, int64_t e1,
                             uint64_t* count, atc_stats* stats, cudaStream_t s) {
-  if (kernel == ATC_KERNEL_AUTO) kernel = auto_kernel(csr);
   CsrPriv* pv = static_cast<CsrPriv*>(csr->priv);
+  const bool ranked = pv && ranked_applies(csr, e0, e1, tuning);
+  if (kernel == ATC_KERNEL_AUTO) kernel = auto_kernel(csr, ranked);
   int launches = 0;
   EventTimer tm;
   if (e1 > e0) {
@@ -1057,7 +1072,15 @@ static atc_status tc_window(const atc_csr* csr, atc_kernel kernel, const atc_tun
     ATC_CK(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), s));
     switch (kernel) {
       case ATC_KERNEL_HU: ATC_TRY(run_hu(g, tuning, ctr, s, &launches)); break;
-      case ATC_KERNEL_BISSON: ATC_TRY(run_bisson(g, tuning, ctr, s, &launches)); break;
+      case ATC_KERNEL_BISSON: {
+        bool done = false;
+        if (ranked) ATC_TRY(count_ranked(csr, ctr, &done, s, &launches));
+        if (!done) {
+          ATC_CK(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), s));
+          ATC_TRY(run_bisson(g, tuning, ctr, s, &launches));
+        }
+        break;
+      }
       case ATC_KERNEL_FOX:
         if (tuning && tuning->edge_kernels) ATC_TRY(run_fox(g, tuning, ctr, s, &launches));
         else ATC_TRY(run_sorted<1>(g, csr->max_outdeg, pv->host_cols == nullptr, ctr, s, &launches));
