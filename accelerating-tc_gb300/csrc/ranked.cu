@@ -31,7 +31,7 @@
 // prefix 73 / 57 ms.
 #include <algorithm>
 
-#include "bisson.cuh"
+#include "ranked.cuh"
 
 namespace atc {
 
@@ -52,10 +52,6 @@ constexpr int64_t kWideMean = 224;      // mean of min(d+u, d+v) from which 16 l
                                         // scale 22 (187) 8.6 and 9.1; scale 24 (270) 50.6 and 47.7
 constexpr int kRankRowMax = kTabWords;  // longest row the CTA sort holds (64 KB)
 constexpr int kRankWarpRow = 1024;      // longest row a warp sorts in registers
-
-// counters of one count
-enum { kc15, kc16, kc17, kc19, kcHashWarp, kcHashBlock, kcNext15, kcNext16, kcNext17, kcNext19, kcNextHashWarp,
-       kcNextHashBlock, kcMid, kcBig, kcNextMid, kcNextBig, kcTooLong, kcCount };
 
 __global__ void rank_keys_kernel(const int64_t* off, const int32_t* indeg, int64_t n, int B, int db, uint64_t* keys) {
   const uint64_t top = (1ull << db) - 1;
@@ -281,7 +277,7 @@ __global__ void rank_tile_rows_kernel(const int64_t* roff, int64_t n, int32_t* t
 }
 
 // Entry of every edge in its target's group: where the source's row starts and how much of it
-// lies before the target.  Targets below kRank16 read the 16-bit copy of the rows (r16, starts in
+// lies before the target.  Targets below below16 read the 16-bit copy of the rows (r16, starts in
 // pieces of eight ids), written here; the others the rows themselves.  A tile's entries of the
 // most contended targets take their places with one atomic per tile and target.
 constexpr int kEntryThreads = 1024;
@@ -289,7 +285,8 @@ constexpr int kEntryEach = kTile / kEntryThreads;
 __global__ void __launch_bounds__(kEntryThreads, 2) rank_entries_kernel(const int64_t* roff, int64_t n, int64_t m,
                                                                      const int32_t* rcols, const int32_t* tile_row,
                                                                      const int64_t* gstart, const int64_t* roff8,
-                                                                     int32_t* gcur, uint16_t* r16, uint2* ent) {
+                                                                     int32_t below16, int32_t* gcur, uint16_t* r16,
+                                                                     uint2* ent) {
   __shared__ int hub[kHubEntry];
   const int64_t tiles = (m + kTile - 1) / kTile;
   for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
@@ -313,7 +310,7 @@ __global__ void __launch_bounds__(kEntryThreads, 2) rank_entries_kernel(const in
         lo[q] = rcols[p];
         st[q] = (uint32_t)__ldg(roff + a);
         len[q] = (uint32_t)p - st[q];
-        if (lo[q] < kRank16) {
+        if (lo[q] < below16) {
           const int64_t r8 = __ldg(roff8 + a);
           st[q] = (uint32_t)r8;
           r16[8 * r8 + len[q]] = (uint16_t)lo[q];
@@ -335,14 +332,9 @@ __global__ void __launch_bounds__(kEntryThreads, 2) rank_entries_kernel(const in
   }
 }
 
-// Work items (target, chunk) of the five kinds of targets; hash: the targets no bitmap takes
-// (warp items from the front, block items from the back).
-struct RankItemLists {
-  int2 *t15, *t16, *t17, *t19, *hash;
-  int64_t hcap;
-  int chunk;  // entries per warp item
-};
-__global__ void rank_items_kernel(const int64_t* roff, const int64_t* gstart, int64_t n, RankItemLists li, int* ctr) {
+// bitmaps: targets by kind; otherwise every target as a list.  ctr[kcMaxRow] = the longest N+(v).
+__global__ void rank_items_kernel(const int64_t* roff, const int64_t* gstart, int64_t n, RankItemLists li, bool bitmaps,
+                                  int* ctr) {
   const int64_t n_pad = (n + 31) & ~31ll;
   for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n_pad; v += (int64_t)gridDim.x * blockDim.x) {
     int64_t ne = 0, dv = 0;
@@ -352,46 +344,29 @@ __global__ void rank_items_kernel(const int64_t* roff, const int64_t* gstart, in
     }
     const bool any = ne > 0 && dv > 0;
     const int kind = !any ? -1
+                     : !bitmaps ? (dv <= li.warp_max ? kcWarp : kcBlock)
                      : v < kRank15 ? kc15
                      : v < kRank16 ? kc16
                      : v < kRank17 && ne >= kRankMidMin ? kc17
-                     : dv <= kWarpHashMax ? kcHashWarp  // R-MAT scale 24, ranks 2^17..2^19: 9.2 ms by hash
-                                                        // tables, 21 ms by 64 KB bitmaps a CTA
-                     : v < kRank19 && ne >= kRankBlockMin ? kc19 : kcHashBlock;
+                     : dv <= li.warp_max ? kcWarp  // R-MAT scale 24, ranks 2^17..2^19: 9.2 ms by hash
+                                                   // tables, 21 ms by 64 KB bitmaps a CTA
+                     : v < kRank19 && ne >= kRankBlockMin ? kc19 : kcBlock;
     const int64_t chunk = kind <= kc16 ? li.chunk : kind <= kc19 ? kRankBlockChunk
-                          : kind == kcHashWarp ? kWarpChunk : kBlockChunk;
+                          : kind == kcWarp ? li.warp_chunk : li.block_chunk;
     const int k = any ? (int)((ne + chunk - 1) / chunk) : 0;
+    const int longest = __reduce_max_sync(0xffffffffu, any ? (int)dv : 0);
+    if ((threadIdx.x & 31) == 0 && longest) atomicMax(&ctr[kcMaxRow], longest);
 #pragma unroll
-    for (int q = kc15; q <= kcHashBlock; ++q) {
+    for (int q = kc15; q <= kcBlock; ++q) {
       if (!__any_sync(0xffffffffu, kind == q)) continue;
       const int at = warp_reserve(&ctr[q], kind == q ? k : 0);
       if (kind != q) continue;
-      int2* to = q == kc15 ? li.t15 : q == kc16 ? li.t16 : q == kc17 ? li.t17 : q == kc19 ? li.t19 : li.hash;
+      int2* to = q == kc15 ? li.t15 : q == kc16 ? li.t16 : q == kc17 ? li.t17 : q == kc19 ? li.t19 : li.list;
       for (int c = 0; c < k; ++c)
-        to[q == kcHashBlock ? li.hcap - 1 - (at + c) : (int64_t)(at + c)] = make_int2((int32_t)v, c);
+        to[q == kcBlock ? li.lcap - 1 - (at + c) : (int64_t)(at + c)] = make_int2((int32_t)v, c);
     }
   }
 }
-
-// Items of the hash kernels.
-struct RankedItems {
-  static constexpr bool kBatch = false;
-  static constexpr int kMinBlocks = 0;
-  const int2* p;
-  const int64_t* gstart;
-  int64_t cap;
-  bool block;
-  __device__ __forceinline__ GroupItem get(const CsrView& g, int i) const {
-    const int2 c = block ? p[cap - 1 - i] : p[i];
-    const int64_t chunk = block ? kBlockChunk : kWarpChunk;
-    const int64_t b = gstart[c.x] + c.y * chunk, e = min(gstart[c.x + 1], b + chunk);
-    const int64_t hb = g.off[c.x], dh = g.off[c.x + 1] - hb;
-    int32_t mode;
-    if (!block) mode = dh <= 8 ? 0 : 1;
-    else mode = dh <= kHashMax ? 0 : (g.cols[hb + dh - 1] - g.cols[hb] < kTabWords * 32 ? 1 : 2);
-    return GroupItem{c.x, mode, b, e};
-  }
-};
 
 // Streams the prefixes of entries [base, base + 32) for every batch that next() hands out through
 // the bitmap T of N+(v): a bit is 0 for a member, 1 otherwise (the empty table is all ones, and
@@ -609,12 +584,9 @@ struct Arena {
 
 }  // namespace
 
-atc_status count_ranked(const atc_csr* csr, unsigned long long* out, bool* done, cudaStream_t s, int* launches) {
-  *done = false;
+atc_status build_ranked(const atc_csr* csr, bool bitmaps, RankedCopy* rc, cudaStream_t s, int* launches) {
   const CsrPriv* pv = static_cast<const CsrPriv*>(csr->priv);
   const int64_t n = csr->n, m = csr->m;
-  std::optional<Phase> ph;
-  ph.emplace("tc.group", s);
   const int B = id_bits(n), db = id_bits(n);  // degrees are below n
   size_t sort_tmp = 0, scan_tmp = 0;
   ATC_TRY(sort_keys_u64_tmp(nullptr, &sort_tmp, nullptr, nullptr, (size_t)n, B, B + db, nullptr, s));
@@ -625,10 +597,13 @@ atc_status count_ranked(const atc_csr* csr, unsigned long long* out, bool* done,
   const int64_t warps = (int64_t)sm_count() * 48;
   const int chunk = (int)std::min<int64_t>(std::max<int64_t>((m / (8 * warps)) & ~31ll, 64), 512);
   auto item_cap = [&](int64_t below, int64_t per) { return std::min<int64_t>(n, below) + m / per + 1; };
-  const int64_t cap15 = item_cap(kRank15, chunk), cap16 = n > kRank15 ? item_cap(kRank16, chunk) : 0;
-  const int64_t cap17 = n > kRank16 ? item_cap(kRank17, kRankBlockChunk) : 0;
-  const int64_t cap19 = n > kRank17 ? item_cap(kRank19, kRankBlockChunk) : 0;
-  const int64_t hcap = n > kRank16 ? max_items(n, m, std::min(kWarpChunk, kBlockChunk)) : 0;
+  const int64_t cap15 = bitmaps ? item_cap(kRank15, chunk) : 0;
+  const int64_t cap16 = bitmaps && n > kRank15 ? item_cap(kRank16, chunk) : 0;
+  const int64_t cap17 = bitmaps && n > kRank16 ? item_cap(kRank17, kRankBlockChunk) : 0;
+  const int64_t cap19 = bitmaps && n > kRank17 ? item_cap(kRank19, kRankBlockChunk) : 0;
+  // with bitmaps few targets are left for lists, and they have few entries
+  const int warp_chunk = bitmaps ? kWarpChunk : chunk, block_chunk = bitmaps ? kBlockChunk : 4 * chunk;
+  const int64_t lcap = !bitmaps || n > kRank16 ? max_items(n, m, std::min(warp_chunk, block_chunk)) : 0;
   Arena ar;
   const size_t a_ka = ar.add<uint64_t>(n), a_kb = ar.add<uint64_t>(n);
   const size_t a_tmp = ar.add<char>(std::max(sort_tmp, scan_tmp));
@@ -641,15 +616,14 @@ atc_status count_ranked(const atc_csr* csr, unsigned long long* out, bool* done,
   const size_t a_rcols = ar.add<int32_t>(m + 16), a_ent = ar.add<uint2>(m), a_tile = ar.add<int32_t>(tiles + 1);
   const size_t a_mid = ar.add<int32_t>(m / 33 + 1), a_big = ar.add<int32_t>(m / (kRankWarpRow + 1) + 1);
   const size_t a_15 = ar.add<int2>(cap15), a_16 = ar.add<int2>(cap16), a_17 = ar.add<int2>(cap17),
-               a_19 = ar.add<int2>(cap19), a_hash = ar.add<int2>(hcap);
-  const size_t a_pieces = ar.add<int32_t>(n + 1), a_roff8 = ar.add<int64_t>(n + 1);
-  const size_t a_r16 = ar.add<uint16_t>(m + 8 * std::min(n, m));
-  DevBuf<char> mem;
-  if (mem.alloc(ar.bytes, s) != ATC_OK) {  // no room for the copy: the caller counts in place
+               a_19 = ar.add<int2>(cap19), a_list = ar.add<int2>(lcap);
+  const size_t a_pieces = ar.add<int32_t>(bitmaps ? n + 1 : 0), a_roff8 = ar.add<int64_t>(bitmaps ? n + 1 : 0);
+  const size_t a_r16 = ar.add<uint16_t>(bitmaps ? m + 8 * std::min(n, m) : 0);
+  if (rc->mem.alloc(ar.bytes, s) != ATC_OK) {  // no room for the copy: the caller counts in place
     cudaGetLastError();
     return ATC_OK;
   }
-  char* p = mem.p;
+  char* p = rc->mem.p;
   uint64_t* ka = reinterpret_cast<uint64_t*>(p + a_ka);
   uint64_t* kb = reinterpret_cast<uint64_t*>(p + a_kb);
   int32_t* rank = reinterpret_cast<int32_t*>(p + a_rank);
@@ -670,7 +644,8 @@ atc_status count_ranked(const atc_csr* csr, unsigned long long* out, bool* done,
   uint16_t* r16 = reinterpret_cast<uint16_t*>(p + a_r16);
   const RankItemLists li{reinterpret_cast<int2*>(p + a_15), reinterpret_cast<int2*>(p + a_16),
                          reinterpret_cast<int2*>(p + a_17), reinterpret_cast<int2*>(p + a_19),
-                         reinterpret_cast<int2*>(p + a_hash), hcap, chunk};
+                         reinterpret_cast<int2*>(p + a_list), lcap, chunk, warp_chunk, block_chunk,
+                         bitmaps ? kWarpHashMax : kWarpMax};
   ATC_CK(cudaMemsetAsync(p + a_zero, 0, zero_end - a_zero, s));
   rank_keys_kernel<<<grid_for(n, 256), 256, 0, s>>>(csr->offsets, pv->indeg, n, B, db, ka);
   ATC_CK(cudaGetLastError());
@@ -681,30 +656,58 @@ atc_status count_ranked(const atc_csr* csr, unsigned long long* out, bool* done,
   ATC_CK(cudaGetLastError());
   ATC_TRY(exclusive_scan_i32_to_i64_tmp(p + a_tmp, &scan_tmp, deg, roff, (size_t)n + 1, s));
   ATC_TRY(exclusive_scan_i32_to_i64_tmp(p + a_tmp, &scan_tmp, cnt, gstart, (size_t)n + 1, s));
-  rank_pieces_kernel<<<grid_for(n + 1, 256), 256, 0, s>>>(deg, n, pieces);
-  ATC_TRY(exclusive_scan_i32_to_i64_tmp(p + a_tmp, &scan_tmp, pieces, roff8, (size_t)n + 1, s));
+  if (bitmaps) {
+    rank_pieces_kernel<<<grid_for(n + 1, 256), 256, 0, s>>>(deg, n, pieces);
+    ATC_TRY(exclusive_scan_i32_to_i64_tmp(p + a_tmp, &scan_tmp, pieces, roff8, (size_t)n + 1, s));
+    *launches += 3;
+  }
   rank_rows_kernel<<<grid_for(m, 256), 256, 0, s>>>(pv->esrc, csr->cols, m, rank, slot, roff, rcols);
   rank_sort_small_kernel<<<grid_for(n, 256), 256, 0, s>>>(roff, n, rcols, mid, big, ctr);
   rank_sort_mid_kernel<<<sm_count() * blocks_per_sm((const void*)rank_sort_mid_kernel, 256, 0), 256, 0, s>>>(
       roff, mid, rcols, ctr);
-  const size_t big_smem = sizeof(int32_t) * kRankRowMax;
-  ATC_CK(cudaFuncSetAttribute((const void*)rank_sort_big_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)big_smem));
   const int64_t long_rows = m / (kRankWarpRow + 1);
   if (long_rows) {
+    const size_t big_smem = sizeof(int32_t) * kRankRowMax;
+    ATC_CK(cudaFuncSetAttribute((const void*)rank_sort_big_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)big_smem));
     rank_sort_big_kernel<<<(unsigned)std::min<int64_t>(long_rows, sm_count() * 2), 1024, big_smem, s>>>(roff, big, rcols,
                                                                                                       ctr);
     *launches += 1;
   }
   rank_tile_rows_kernel<<<grid_for(n, 256), 256, 0, s>>>(roff, n, tile_row);
   rank_entries_kernel<<<grid_for(m, kTile, 2), kEntryThreads, 0, s>>>(roff, n, m, rcols, tile_row, gstart, roff8,
-                                                                        gcur, r16, ent);
-  rank_items_kernel<<<grid_for(n, 256), 256, 0, s>>>(roff, gstart, n, li, ctr);
+                                                                        bitmaps ? kRank16 : 0, gcur, r16, ent);
+  rank_items_kernel<<<grid_for(n, 256), 256, 0, s>>>(roff, gstart, n, li, bitmaps, ctr);
   ATC_CK(cudaGetLastError());
-  *launches += 14;
+  *launches += 17;
+  rc->n = n;
+  rc->m = m;
+  rc->roff = roff;
+  rc->rcols = rcols;
+  rc->r16 = reinterpret_cast<const uint4*>(r16);
+  rc->gstart = gstart;
+  rc->ent = ent;
+  rc->ctr = ctr;
+  rc->li = li;
+  rc->long_rows = long_rows != 0;
+  return ATC_OK;
+}
+
+atc_status count_ranked(const atc_csr* csr, unsigned long long* out, bool* done, cudaStream_t s, int* launches) {
+  *done = false;
+  RankedCopy rc;
+  std::optional<Phase> ph;
+  ph.emplace("tc.group", s);
+  ATC_TRY(build_ranked(csr, true, &rc, s, launches));
+  if (!rc.mem.p) return ATC_OK;
   ph.reset();
   ph.emplace("tc.count", s);
-  const CsrView g = csr_view(roff, rcols, nullptr, n, m);
+  const int64_t n = rc.n, m = rc.m;
+  const CsrView g = csr_view(rc.roff, rc.rcols, nullptr, n, m);
+  const RankItemLists& li = rc.li;
+  const int64_t* gstart = rc.gstart;
+  const uint2* ent = rc.ent;
+  int* ctr = rc.ctr;
   const int* too = ctr + kcTooLong;
   auto block_launch = [&](auto kern, int threads, int64_t bits, const int2* items, int kind, int nxt) -> atc_status {
     const size_t smem = (size_t)bits / 8;
@@ -723,29 +726,30 @@ atc_status count_ranked(const atc_csr* csr, unsigned long long* out, bool* done,
     const size_t hsmem = sizeof(int32_t) * kTabWords;
     ATC_CK(cudaFuncSetAttribute((const void*)hb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsmem));
     hb<<<sm_count() * blocks_per_sm((const void*)hb, kBgWarps * 32, hsmem), kBgWarps * 32, hsmem, s>>>(
-        g, PrefixPartners{ent}, RankedItems{li.hash, gstart, hcap, true}, 0, ctr + kcHashBlock, ctr + kcNextHashBlock,
+        g, PrefixPartners{ent}, RankedItems{li.list, gstart, li.lcap, li.block_chunk, true}, 0, ctr + kcBlock,
+        ctr + kcNextBlock,
         (uint32_t)kTabWords, GraphTags{nullptr, 0, nullptr}, out);
     hw<<<sm_count() * blocks_per_sm((const void*)hw, kBgWarps * 32, 0), kBgWarps * 32, 0, s>>>(
-        g, PrefixPartners{ent}, RankedItems{li.hash, gstart, hcap, false}, 0, ctr + kcHashWarp, ctr + kcNextHashWarp,
+        g, PrefixPartners{ent}, RankedItems{li.list, gstart, li.lcap, li.warp_chunk, false}, 0, ctr + kcWarp,
+        ctr + kcNextWarp,
         GraphTags{nullptr, 0, nullptr}, out);
     ATC_CK(cudaGetLastError());
     *launches += 2;
   }
-  const uint4* q16 = reinterpret_cast<const uint4*>(r16);
   const bool wide = csr->wedges_min >= kWideMean * m;
   if (n > kRank15) {
     const auto kern = wide ? rank_warp_kernel<1 << 16, 4, 16> : rank_warp_kernel<1 << 16, 4, 8>;
     kern<<<sm_count() * blocks_per_sm((const void*)kern, 128, 0), 128, 0, s>>>(
-        roff, rcols, q16, ent, li.t16, gstart, chunk, ctr + kc16, ctr + kcNext16, too, out);
+        rc.roff, rc.rcols, rc.r16, ent, li.t16, gstart, li.chunk, ctr + kc16, ctr + kcNext16, too, out);
     *launches += 1;
   }
   const auto kern = wide ? rank_warp_kernel<1 << 15, 8, 16> : rank_warp_kernel<1 << 15, 8, 8>;
   kern<<<sm_count() * blocks_per_sm((const void*)kern, 256, 0), 256, 0, s>>>(
-      roff, rcols, q16, ent, li.t15, gstart, chunk, ctr + kc15, ctr + kcNext15, too, out);
+      rc.roff, rc.rcols, rc.r16, ent, li.t15, gstart, li.chunk, ctr + kc15, ctr + kcNext15, too, out);
   ATC_CK(cudaGetLastError());
   *launches += 1;
   int too_long = 0;
-  if (long_rows) {
+  if (rc.long_rows) {
     ATC_CK(cudaMemcpyAsync(&too_long, ctr + kcTooLong, sizeof(int), cudaMemcpyDeviceToHost, s));
     ATC_CK(cudaStreamSynchronize(s));
   }

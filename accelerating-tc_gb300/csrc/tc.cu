@@ -25,7 +25,7 @@
 #include <mutex>
 #include <vector>
 
-#include "bisson.cuh"
+#include "ranked.cuh"
 
 namespace atc {
 
@@ -259,75 +259,50 @@ __global__ void fox_deal_kernel(const uint64_t* keys, const int64_t* list, int64
 // per item as a sorted copy in shared memory, and every streamed element is searched in
 // it.  The reference kernels search the longer list in global memory, one dependent load
 // per step, per edge; here only lists too long for shared memory are searched there.
-//   KIND 0, TriCore-style (tricount_gpu.cu:215-290): 32 samples of the longer list (the
-//     reference's per-warp pivot cache) sit contiguous in shared memory, so the first five
-//     levels of every search touch 32 distinct banks; the sample bracket holding the
-//     element is then binary-searched.  Every bracket of a list holds at most ceil(d/32)
-//     elements, so the bracket search is a fixed run of halving steps, the same number on
-//     every lane, without a loop test or a bound test per step (a read past the list is
-//     clamped to its last element, which is not below the element searched).
+//   KIND 0, TriCore-style (tricount_gpu.cu:215-290): the reference's pivot cache (32 samples of
+//     the longer list per warp) becomes a table over the list's id range: the range is cut into
+//     up to kPivots equal parts, twice as many as the list has elements, and the table gives the
+//     elements of each part.  One read brackets an element to a part, whose few elements are
+//     then binary-searched.  (Samples at equal positions took five steps to find the bracket
+//     and log2(d/32) + 1 more inside it, each a shared load with bank conflicts.)
 //   KIND 1, Fox-style (Fox/tc.cu:64-125): a lane's successive elements of a list ascend, so
 //     each search gallops forward from where the lane's previous one ended (restarting
 //     when the element is smaller than the previous one), then binary-searches the last
 //     step.
-constexpr int kLiftMax = 11;  // the unrolled bracket search covers brackets of up to 4095
+constexpr int kWarpPivots = 256;    // parts of a warp item's table (lists of up to kWarpMax)
+constexpr int kBlockPivots = 2048;  // and of a block item's
 
 template <int KIND>
 struct SortedProber {
-  const int32_t* T;    // sorted N+(h) (shared memory, or global for lists beyond it)
-  const int32_t* piv;  // 32 samples piv[i] = T[i * d / 32] (shared memory)
+  const int32_t* T;     // sorted N+(h) (shared memory, or global for lists beyond it)
+  const uint32_t* part; // TriCore: first element | end << 16 of every part (null: the whole list)
   int d;
   int32_t hi;    // T[d - 1]
+  int32_t base;  // TriCore: T[0]
+  uint32_t range;  // TriCore: T[d - 1] - T[0]
+  int shift;     // TriCore: log2 of a part's ids
   int prev;      // Fox: lower bound of the lane's previous element
   int32_t last;  // Fox: the lane's previous element
   int gap;       // Fox: how far the lane's previous forward search moved
-  int lg = -1;   // TriCore: floor(log2(ceil(d/32))), the first halving step of the bracket search
-                 // (the same for the whole list); -1: the bracket is searched by a loop
   __device__ __forceinline__ unsigned probe(int32_t x, bool valid) {
     if (!valid) return 0u;
-    if (x > hi) return 0u;  // above the longer list: no search
     if constexpr (KIND == 0) {
-      int k = 0;  // number of samples <= x: five fixed steps, then the last sample
-#pragma unroll
-      for (int step = 16; step > 0; step >>= 1)
-        if (piv[k + step - 1] <= x) k += step;
-      if (piv[k] <= x) ++k;
-      if (k == 0) return 0u;  // x < T[0]
-      if (piv[k - 1] == x) return 1u;
-      int b = (int)(((int64_t)(k - 1) * d) >> 5) + 1;  // strictly inside the bracket
-      int e = k == 32 ? d : (int)(((int64_t)k * d) >> 5);
-      if (lg >= 0 && lg <= kLiftMax) {
-        // the last index below x: T[b-1] (the sample) is below x, and 2^(lg+1) - 1 steps cover
-        // the bracket; T[e] (the next sample, or past the list) is not below x
-        int lo = b - 1;
-#define ATC_LIFT(t) \
-  case t: {        \
-    const int c = lo + (1 << t); \
-    if (T[min(c, d - 1)] < x) lo = c; \
-  }
-        switch (lg) {  // enters at the first step and falls through the rest
-          ATC_LIFT(11) [[fallthrough]];
-          ATC_LIFT(10) [[fallthrough]];
-          ATC_LIFT(9) [[fallthrough]];
-          ATC_LIFT(8) [[fallthrough]];
-          ATC_LIFT(7) [[fallthrough]];
-          ATC_LIFT(6) [[fallthrough]];
-          ATC_LIFT(5) [[fallthrough]];
-          ATC_LIFT(4) [[fallthrough]];
-          ATC_LIFT(3) [[fallthrough]];
-          ATC_LIFT(2) [[fallthrough]];
-          ATC_LIFT(1) [[fallthrough]];
-          ATC_LIFT(0)
-        }
-#undef ATC_LIFT
-        return lo + 1 < d && T[lo + 1] == x;
+      const uint32_t r = (uint32_t)(x - base);
+      if (r > range) return 0u;  // outside the longer list: no search
+      int lo = 0, n = d;
+      if (part) {
+        const uint32_t pe = part[r >> shift];
+        lo = (int)(pe & 0xffffu);
+        n = (int)(pe >> 16) - lo;
       }
-      while (b < e) {
-        const int mid = (b + e) >> 1;
-        if (T[mid] < x) b = mid + 1; else e = mid;
+      while (n > 1) {  // branch-free lower bound inside the part
+        const int half = n >> 1;
+        lo = T[lo + half - 1] < x ? lo + half : lo;
+        n -= half;
       }
-      return b < d && T[b] == x;
+      return n == 1 && T[lo] == x;
     } else {
+      if (x > hi) return 0u;  // above the longer list: no search
       if (x < last) {
         // a new list (or an earlier element): its lower bound lies in [0, prev]
         int a = 0, b = prev;
@@ -361,6 +336,31 @@ struct SortedProber {
   }
   __device__ __forceinline__ unsigned finish() { return 0u; }
 };
+
+// The part table of the sorted list T[0, d), d <= 65535, built by `threads` threads (this one `t`)
+// with sync() between the steps: start[b] = the first element of part b or above, then part[].
+// Returns the shift.
+template <class Sync>
+__device__ __forceinline__ int build_parts(const int32_t* T, int d, int max_parts, uint16_t* start, uint32_t* part, int t,
+                                           int threads, Sync sync) {
+  const int32_t base = T[0];
+  const uint32_t range = (uint32_t)(T[d - 1] - base);
+  int parts = 32;
+  while (parts < 2 * d && parts < max_parts) parts <<= 1;
+  int shift = 0;
+  while ((range >> shift) >= (uint32_t)parts) ++shift;
+  for (int j = t; j < d; j += threads) {
+    const int c = (int)((uint32_t)(T[j] - base) >> shift);
+    const int p = j ? (int)((uint32_t)(T[j - 1] - base) >> shift) : -1;
+    for (int b = p + 1; b <= c; ++b) start[b] = (uint16_t)j;
+    if (j == d - 1) start[c + 1] = (uint16_t)d;
+  }
+  sync();
+  const int used = (int)(range >> shift) + 1;
+  for (int b = t; b < used; b += threads) part[b] = (uint32_t)start[b] | (uint32_t)start[b + 1] << 16;
+  sync();
+  return shift;
+}
 
 // ---- 1-D bulk copies into shared memory (the TMA unit's untiled mode) -------------
 // One thread issues cp.async.bulk of a whole list; its completion is counted in bytes on an
@@ -435,13 +435,13 @@ __device__ __forceinline__ void bulk_window(int64_t hb, int64_t dh, int64_t* a0,
 
 // bulk: stage N+(h) with bulk copies (device-resident cols); otherwise with loads (cols in
 // mapped host memory).  err: set to 1 when a bulk wait runs out.
-template <int KIND>
-__global__ void __launch_bounds__(kBgWarps * 32) sorted_warp_kernel(CsrView g, const int32_t* __restrict__ plist,
-                                                                    const GroupItem* __restrict__ items, int nitems,
-                                                                    int* next, bool bulk, int* err,
+template <int KIND, class Items, class Partners>
+__global__ void __launch_bounds__(kBgWarps * 32) sorted_warp_kernel(CsrView g, Partners partners, Items items,
+                                                                    int nitems, int* next, bool bulk, int* err,
                                                                     unsigned long long* out) {
   __shared__ __align__(16) int32_t T[kBgWarps][kWarpMax + 8];
-  __shared__ int32_t piv[kBgWarps][32];
+  __shared__ uint32_t part[kBgWarps][KIND == 0 ? kWarpPivots : 1];
+  __shared__ uint16_t start[kBgWarps][KIND == 0 ? kWarpPivots + 1 : 1];
   __shared__ __align__(8) uint64_t bar[kBgWarps];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (lane == 0) mbar_init(&bar[w]);
@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(kBgWarps * 32) sorted_warp_kernel(CsrView g, c
     if (lane == 0) it = atomicAdd(next, 1);
     it = __shfl_sync(0xffffffffu, it, 0);
     if (it >= nitems) break;
-    const GroupItem gi = items[it];
+    const GroupItem gi = items.get(g, it);
     const int64_t hb = g.off[gi.h];
     const int dh = (int)(g.off[gi.h + 1] - hb);  // 1 .. kWarpMax
     const int32_t* L = T[w];
@@ -474,24 +474,24 @@ __global__ void __launch_bounds__(kBgWarps * 32) sorted_warp_kernel(CsrView g, c
       for (int j = lane; j < dh; j += 32) T[w][j] = __ldg(g.cols + hb + j);
       __syncwarp();
     }
-    piv[w][lane] = L[(lane * dh) >> 5];
-    __syncwarp();
+    int shift = 0;
+    if (KIND == 0) shift = build_parts(L, dh, kWarpPivots, start[w], part[w], lane, 32, [] { __syncwarp(); });
     int64_t cur = gi.b;
     auto nb = [&]() { int64_t r = cur; cur += 32; return r; };
-    SortedProber<KIND> pr{L, piv[w], dh, L[dh - 1], 0, INT32_MIN, 16, 31 - __clz((dh + 31) >> 5)};
-    total += stream_partners(g, ListPartners{plist}, gi.e, lane, nb, pr);
+    SortedProber<KIND> pr{L, part[w], dh, L[dh - 1], L[0], (uint32_t)(L[dh - 1] - L[0]), shift, 0, INT32_MIN, 16};
+    total += stream_partners(g, partners, gi.e, lane, nb, pr);
     __syncwarp();  // the next item overwrites the copy
   }
   warp_add_count(total, out);
 }
 
-template <int KIND>
-__global__ void __launch_bounds__(kBgWarps * 32) sorted_block_kernel(CsrView g, const int32_t* __restrict__ plist,
-                                                                     const GroupItem* __restrict__ items, int nitems,
-                                                                     int* next, uint32_t tab_words, bool bulk,
-                                                                     int* err, unsigned long long* out) {
+template <int KIND, class Items, class Partners>
+__global__ void __launch_bounds__(kBgWarps * 32) sorted_block_kernel(CsrView g, Partners partners, Items items,
+                                                                     int nitems, int* next, uint32_t tab_words,
+                                                                     bool bulk, int* err, unsigned long long* out) {
   extern __shared__ __align__(16) int32_t T[];  // tab_words + 8
-  __shared__ int32_t piv[32];
+  __shared__ uint32_t part[KIND == 0 ? kBlockPivots : 1];
+  __shared__ uint16_t start[KIND == 0 ? kBlockPivots + 1 : 1];
   __shared__ int cur_item;
   __shared__ unsigned long long bnext;
   __shared__ __align__(8) uint64_t bar;
@@ -508,7 +508,7 @@ __global__ void __launch_bounds__(kBgWarps * 32) sorted_block_kernel(CsrView g, 
     __syncthreads();
     const int it = cur_item;
     if (it >= nitems) break;
-    const GroupItem gi = items[it];
+    const GroupItem gi = items.get(g, it);
     const int64_t hb = g.off[gi.h];
     const int64_t dh = g.off[gi.h + 1] - hb;
     const bool staged = dh <= (int64_t)tab_words;
@@ -530,16 +530,19 @@ __global__ void __launch_bounds__(kBgWarps * 32) sorted_block_kernel(CsrView g, 
       for (int64_t j = threadIdx.x; j < dh; j += blockDim.x) T[j] = __ldg(g.cols + hb + j);
       L = T;
     }
-    if (threadIdx.x < 32) piv[threadIdx.x] = __ldg(g.cols + hb + (((int64_t)threadIdx.x * dh) >> 5));
-    __syncthreads();
+    if (staged && !bulk) __syncthreads();
+    int shift = 0;
+    if (KIND == 0 && staged)
+      shift = build_parts(L, (int)dh, kBlockPivots, start, part, threadIdx.x, kBgWarps * 32, [] { __syncthreads(); });
     auto nb = [&]() {
       unsigned long long r = 0;
       if (lane == 0) r = atomicAdd(&bnext, 32ull);
       return gi.b + (int64_t)__shfl_sync(0xffffffffu, r, 0);
     };
-    SortedProber<KIND> pr{L, piv, (int)dh, __ldg(g.cols + hb + dh - 1), 0, INT32_MIN, 16,
-                          31 - __clz((int)((dh + 31) >> 5))};
-    total += stream_partners(g, ListPartners{plist}, gi.e, lane, nb, pr);
+    const int32_t t0 = __ldg(g.cols + hb), t1 = __ldg(g.cols + hb + dh - 1);
+    SortedProber<KIND> pr{L, KIND == 0 && staged ? part : nullptr, (int)dh, t1, t0, (uint32_t)(t1 - t0), shift, 0,
+                          INT32_MIN, 16};
+    total += stream_partners(g, partners, gi.e, lane, nb, pr);
     __syncthreads();  // the next item overwrites the copy
   }
   warp_add_count(total, out);
@@ -785,6 +788,16 @@ static atc_status group_edges(const CsrView& g, const ItemShape& sh, Grouping* g
   return ATC_OK;
 }
 
+// Whether the ranked copy pays for its passes: the passes cost about 60 ps an edge and 0.1 ms more
+// than grouping whole lists, which in turn is slow where hubs are (contended group cursors, long
+// lists).  Measured whole lists / ranked in ms: Bisson on R-MAT of 5K, 23K, 910K, 16M edges 0.12 /
+// 0.16, 0.19 / 0.16, 0.64 / 0.28, 4.8 / 1.9, Chung-Lu of 35K, 1.3M, 14M 0.21 / 0.18, 0.73 / 0.34,
+// 2.25 / 1.66, RGG (mean degree 32, W = 1.04 W_min) of 45K, 1.6M, 16M 0.11 / 0.18, 0.21 / 0.39,
+// 1.19 / 1.96.  Even degrees with long lists pay too: a test costs a third.
+static bool ranked_pays(const atc_csr* csr) {
+  return csr->m >= 16384 && (csr->wedges >= csr->wedges_min + csr->wedges_min / 2 || csr->wedges_min >= 48 * csr->m);
+}
+
 // The ranked count (csrc/ranked.cu) takes whole counts of CSRs that preTC built and that live on
 // the device.  Parts keep the CSR's own orientation (their counts are defined by it), as do CSRs
 // read from files (any sorted rows are accepted there); CSRs in host memory count in bounded
@@ -811,7 +824,44 @@ static atc_status run_bisson(const CsrView& g, const atc_tuning* t, unsigned lon
   return launch_slots(slots, g, gr.plist.p, gr.witems.p, gr.bitems.p, gr.hc, gr.counters.p, ctr, s, launches);
 }
 
-// TriCore-style (KIND 0) and Fox-style (KIND 1) searches of the staged longer lists.
+// Launches the searched kernels of one family over warp items [0, hc0) and block items
+// [0, hc1), and checks their bulk waits.  next: the items' cursors (warp, block); err: zeroed.
+template <int KIND, class Items, class Partners>
+static atc_status launch_sorted(const CsrView& g, const Partners& partners, const Items& witems, const Items& bitems,
+                                int hc0, int hc1, int max_row, bool bulk, int* next_w, int* next_b, int* err_d,
+                                unsigned long long* ctr, cudaStream_t s, int* launches) {
+  if (hc1) {
+    const auto kern = sorted_block_kernel<KIND, Items, Partners>;
+    uint32_t words = (uint32_t)std::min(std::max(max_row, kWarpMax + 1), kTabWords);
+    words = (words + 31) & ~31u;
+    const size_t smem = sizeof(int32_t) * (words + 8);  // + the bulk window's rounding
+    ATC_CK(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int bps = blocks_per_sm((const void*)kern, kBgWarps * 32, smem);
+    const int grid = std::min(hc1, sm_count() * bps);
+    kern<<<grid, kBgWarps * 32, smem, s>>>(g, partners, bitems, hc1, next_b, words, bulk, err_d, ctr);
+    ATC_CK(cudaGetLastError());
+    *launches += 1;
+  }
+  if (hc0) {
+    const auto kern = sorted_warp_kernel<KIND, Items, Partners>;
+    const int bps = blocks_per_sm((const void*)kern, kBgWarps * 32, 0);
+    const int grid = (int)std::min<int64_t>((hc0 + kBgWarps - 1) / kBgWarps, (int64_t)sm_count() * bps);
+    kern<<<grid, kBgWarps * 32, 0, s>>>(g, partners, witems, hc0, next_w, bulk, err_d, ctr);
+    ATC_CK(cudaGetLastError());
+    *launches += 1;
+  }
+  int err = 0;
+  ATC_CK(cudaMemcpyAsync(&err, err_d, sizeof(int), cudaMemcpyDeviceToHost, s));
+  ATC_CK(cudaStreamSynchronize(s));
+  if (err) {
+    set_error("a bulk copy into shared memory did not complete within its wait limit");
+    return ATC_ERR_TIMEOUT;
+  }
+  return ATC_OK;
+}
+
+// TriCore-style (KIND 0) and Fox-style (KIND 1) searches of the staged longer lists, on the
+// Bisson-style grouping of whole lists.
 // max_outdeg sizes the block kernels' shared copy (lists above kTabWords stay in global).
 // bulk: the lists are staged by TMA bulk copies (cols in device memory); with cols in mapped
 // host memory they are staged with loads.
@@ -825,35 +875,40 @@ static atc_status run_sorted(const CsrView& g, int max_outdeg, bool bulk, unsign
   ATC_TRY(group_edges(g, sh, &gr, s, launches));
   ph.reset();
   ph.emplace("tc.count", s);
-  if (gr.hc[1]) {
-    uint32_t words = (uint32_t)std::min(std::max(max_outdeg, kWarpMax + 1), kTabWords);
-    words = (words + 31) & ~31u;
-    const size_t smem = sizeof(int32_t) * (words + 8);  // + the bulk window's rounding
-    ATC_CK(cudaFuncSetAttribute((const void*)sorted_block_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem));
-    const int bps = blocks_per_sm((const void*)sorted_block_kernel<KIND>, kBgWarps * 32, smem);
-    const int grid = std::min(gr.hc[1], sm_count() * bps);
-    sorted_block_kernel<KIND><<<grid, kBgWarps * 32, smem, s>>>(g, gr.plist.p, gr.bitems.p, gr.hc[1],
-                                                                 gr.counters.p + 5, words, bulk, gr.counters.p + 7,
-                                                                 ctr);
-    ATC_CK(cudaGetLastError());
-    *launches += 1;
-  }
-  if (gr.hc[0]) {
-    const int bps = blocks_per_sm((const void*)sorted_warp_kernel<KIND>, kBgWarps * 32, 0);
-    const int grid = (int)std::min<int64_t>((gr.hc[0] + kBgWarps - 1) / kBgWarps, (int64_t)sm_count() * bps);
-    sorted_warp_kernel<KIND><<<grid, kBgWarps * 32, 0, s>>>(g, gr.plist.p, gr.witems.p, gr.hc[0],
-                                                            gr.counters.p + 4, bulk, gr.counters.p + 7, ctr);
-    ATC_CK(cudaGetLastError());
-    *launches += 1;
-  }
-  int err = 0;
-  ATC_CK(cudaMemcpyAsync(&err, gr.counters.p + 7, sizeof(int), cudaMemcpyDeviceToHost, s));
+  return launch_sorted<KIND>(g, ListPartners{gr.plist.p}, FullItems{gr.witems.p}, FullItems{gr.bitems.p}, gr.hc[0],
+                             gr.hc[1], max_outdeg, bulk, gr.counters.p + 4, gr.counters.p + 5, gr.counters.p + 7, ctr,
+                             s, launches);
+}
+
+// The same searches on the degree-ranked copy: for every edge u -> v the part of row u before v is
+// searched in N+(v) (sum of C(d+(u), 2) searches instead of the sum of min(d+u, d+v), in lists
+// that are shorter too).  TriCore-style with the part tables, R-MAT scale 20: 10.4 ms by whole lists
+// and 32 samples, 8.7 with the tables, 6.9 on the ranked copy with samples, 3.6 with both; scale 24:
+// 290 -> 97 ms.  Fox-style: 11.8 -> 7.6 and 304 -> 200 ms.  Both are bound by the shared-memory
+// reads of the searches (three to four a test, with conflicts).
+// *done = false: no room for the copy, or a row too long for it.
+template <int KIND>
+static atc_status run_sorted_ranked(const atc_csr* csr, unsigned long long* ctr, bool* done, cudaStream_t s,
+                                    int* launches) {
+  *done = false;
+  std::optional<Phase> ph;
+  ph.emplace("tc.group", s);
+  RankedCopy rc;
+  ATC_TRY(build_ranked(csr, false, &rc, s, launches));
+  if (!rc.mem.p) return ATC_OK;
+  int h[kcCount];
+  ATC_CK(cudaMemcpyAsync(h, rc.ctr, sizeof(h), cudaMemcpyDeviceToHost, s));
   ATC_CK(cudaStreamSynchronize(s));
-  if (err) {
-    set_error("a bulk copy into shared memory did not complete within its wait limit");
-    return ATC_ERR_TIMEOUT;
-  }
+  if (h[kcTooLong]) return ATC_OK;
+  ph.reset();
+  ph.emplace("tc.count", s);
+  const CsrView g = csr_view(rc.roff, rc.rcols, nullptr, rc.n, rc.m);
+  const RankItemLists& li = rc.li;
+  ATC_TRY(launch_sorted<KIND>(g, PrefixPartners{rc.ent}, RankedItems{li.list, rc.gstart, li.lcap, li.warp_chunk, false},
+                              RankedItems{li.list, rc.gstart, li.lcap, li.block_chunk, true}, h[kcWarp], h[kcBlock],
+                              h[kcMaxRow], true, rc.ctr + kcNextWarp, rc.ctr + kcNextBlock, rc.ctr + kcError, ctr, s,
+                              launches));
+  *done = true;
   return ATC_OK;
 }
 
@@ -1041,7 +1096,8 @@ atc_status atc::part_edge_range(const atc_csr* csr, uint32_t part, uint32_t npar
 
 // Counts the edges [e0, e1) of the CSR (every edge for the whole count).
 // ATC_KERNEL_AUTO: the Bisson-style or the Hu-style count, whichever this cost model of their
-// GB300 times predicts is faster.  Hu-style: 1.2 ps per wedge (W) + 45 ps per edge + 0.06 ms.
+// GB300 times predicts is faster.  Hu-style: 2 ps per wedge (W; 1.2 at scale 20 and above, where
+// it loses anyway) + 45 ps per edge + 0.06 ms.
 // Bisson-style, ranked: 0.37 ps per element of the shorter lists (W_min) + 85 ps per edge (the
 // ranked copy) + 0.17 ms of launches.  By whole lists (parts, loaded CSRs): 1.232 ps per
 // element of W_min + 117.5 ps per edge + 0.3 ms, against Hu's 1.097 ps and 103.5 ps, the fit of
@@ -1051,14 +1107,14 @@ atc_status atc::part_edge_range(const atc_csr* csr, uint32_t part, uint32_t npar
 static atc_kernel auto_kernel(const atc_csr* csr, bool ranked) {
   const double m = (double)csr->m, w = (double)csr->wedges, wmin = (double)csr->wedges_min;
   const double bisson_ps = ranked ? 0.37 * wmin + 85.0 * m + 1.7e8 : 1.232 * wmin + 117.5 * m + 3.0e8;
-  const double hu_ps = ranked ? 1.2 * w + 45.0 * m + 6.0e7 : 1.097 * w + 103.5 * m;
+  const double hu_ps = ranked ? 2.0 * w + 45.0 * m + 6.0e7 : 1.097 * w + 103.5 * m;
   return hu_ps < bisson_ps ? ATC_KERNEL_HU : ATC_KERNEL_BISSON;
 }
 
 static atc_status tc_window(const atc_csr* csr, atc_kernel kernel, const atc_tuning* tuning, int64_t e0, int64_t e1,
                             uint64_t* count, atc_stats* stats, cudaStream_t s) {
   CsrPriv* pv = static_cast<CsrPriv*>(csr->priv);
-  const bool ranked = pv && ranked_applies(csr, e0, e1, tuning);
+  const bool ranked = pv && ranked_applies(csr, e0, e1, tuning) && ranked_pays(csr);
   if (kernel == ATC_KERNEL_AUTO) kernel = auto_kernel(csr, ranked);
   int launches = 0;
   EventTimer tm;
@@ -1081,14 +1137,23 @@ static atc_status tc_window(const atc_csr* csr, atc_kernel kernel, const atc_tun
         }
         break;
       }
-      case ATC_KERNEL_FOX:
-        if (tuning && tuning->edge_kernels) ATC_TRY(run_fox(g, tuning, ctr, s, &launches));
-        else ATC_TRY(run_sorted<1>(g, csr->max_outdeg, pv->host_cols == nullptr, ctr, s, &launches));
+      default: {
+        const bool fox = kernel == ATC_KERNEL_FOX;
+        if (tuning && tuning->edge_kernels) {
+          ATC_TRY(fox ? run_fox(g, tuning, ctr, s, &launches) : run_tricore(g, tuning, ctr, s, &launches));
+          break;
+        }
+        bool done = false;
+        if (ranked)
+          ATC_TRY(fox ? run_sorted_ranked<1>(csr, ctr, &done, s, &launches)
+                      : run_sorted_ranked<0>(csr, ctr, &done, s, &launches));
+        if (!done) {
+          const bool bulk = pv->host_cols == nullptr;
+          ATC_TRY(fox ? run_sorted<1>(g, csr->max_outdeg, bulk, ctr, s, &launches)
+                      : run_sorted<0>(g, csr->max_outdeg, bulk, ctr, s, &launches));
+        }
         break;
-      default:
-        if (tuning && tuning->edge_kernels) ATC_TRY(run_tricore(g, tuning, ctr, s, &launches));
-        else ATC_TRY(run_sorted<0>(g, csr->max_outdeg, pv->host_cols == nullptr, ctr, s, &launches));
-        break;
+      }
     }
     tm.stop(s);
     unsigned long long h = 0;

@@ -60,6 +60,18 @@ def test_equals_the_grouped_lists(dir, tuning):
     csr.free()
 
 
+@pytest.mark.parametrize("n", [3, 17, 33, 34, 65, 129, 181, 183, 257, 258, 600, 1100, 2100])
+@pytest.mark.parametrize("kernel", [K.TRICORE, K.FOX])
+def test_searched_families(n, kernel):
+    """Complete graphs (lists of every length up to n - 1) with their ids scattered over 2^20, so
+    that the part tables are sparse; from 16384 edges on the ranked copy, otherwise whole lists."""
+    ids = np.random.default_rng(n).choice(1 << 20, n, replace=False).astype(np.int32)
+    csr = atc.pretc(ids[_complete(n)], atc.Dir.DEGREE)
+    assert atc.tc(csr, kernel)[0] == comb(n, 3)
+    assert atc.tc(csr, kernel, tuning={"bisson_slots": 4})[0] == comb(n, 3)
+    csr.free()
+
+
 def test_loaded_rows_that_are_no_orientation(tmp_path):
     """A cache file may hold any sorted rows: its count stays the sum over its rows' edges."""
     n = 50
