@@ -465,7 +465,7 @@ static atc_status pretc_impl(const int2* pairs, uint64_t np, atc_dir dir, atc_or
   ATC_TRY(off.alloc(n + 1, s));
   ATC_TRY(cols.alloc(m + 16, s));
   ATC_TRY(esrc.alloc(m + 16, s));
-  ATC_TRY(counter.alloc(4, s));
+  ATC_TRY(counter.alloc(kCsrCounters, s));
   ATC_CK(cudaMemsetAsync(cols.p + m, 0, sizeof(int32_t) * 16, s));
   offsets_kernel<<<grid_for(n + 1, 256), 256, 0, s>>>(ka, m, bout, n, off.p);
   ATC_CK(cudaGetLastError());
@@ -474,7 +474,7 @@ static atc_status pretc_impl(const int2* pairs, uint64_t np, atc_dir dir, atc_or
   // W = sum_v indeg(v) * outdeg(v) and the largest out-degree
   ATC_TRY(indeg.alloc(n + 1, s));
   ATC_CK(cudaMemsetAsync(indeg.p, 0, sizeof(int32_t) * (n + 1), s));
-  ATC_CK(cudaMemsetAsync(counter.p, 0, sizeof(unsigned long long) * 4, s));
+  ATC_CK(cudaMemsetAsync(counter.p, 0, sizeof(unsigned long long) * kCsrCounters, s));
   if (m) indeg_kernel<<<grid_for(m, 256), 256, 0, s>>>(cols.p, m, indeg.p);
   if (n) wedge_kernel<<<grid_for(n, 256), 256, 0, s>>>(off.p, indeg.p, n, counter.p, (int*)(counter.p + 1));
   if (m) wedge_min_kernel<<<grid_for(m, 256), 256, 0, s>>>(off.p, cols.p, esrc.p, m, counter.p + 2);
@@ -859,7 +859,8 @@ static atc_status csr_load_impl(const char* path, bool host_resident, atc_csr* o
   DevBuf<unsigned long long> counter;
   HostMapped hcols, hesrc;
   ATC_TRY(doff.alloc(n + 1, s));
-  ATC_TRY(counter.alloc(4, s));
+  ATC_TRY(counter.alloc(kCsrCounters, s));
+  ATC_CK(cudaMemsetAsync(counter.p, 0, sizeof(unsigned long long) * kCsrCounters, s));
   ATC_CK(cudaMemcpyAsync(doff.p, off.data(), sizeof(int64_t) * (n + 1), cudaMemcpyHostToDevice, s));
   int32_t* cols_dev;
   int32_t* esrc_dev;

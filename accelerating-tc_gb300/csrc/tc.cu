@@ -252,6 +252,57 @@ __global__ void fox_deal_kernel(const uint64_t* keys, const int64_t* list, int64
   }
 }
 
+// ============================== small counts =======================================
+// Graphs of a few thousand edges are counted before a launch's items could be made: G lanes take
+// an edge, each every G-th element of the shorter list, and binary-search it in the longer
+// one, where both lists sit in L1 or L2 (Hu/tc.cu:69-201 searches a staged run the same way).  One
+// launch, no scratch, no item lists, no wait before the result, and no memset: the last block
+// to end stores the total and leaves the accumulator and the ticket at zero.
+// Measured, the whole call, items -> this kernel (us): R-MAT of 4.9K, 23K, 102K, 441K edges 55 -> 30,
+// 78 -> 31, 118 -> 50, 232 -> 175; Chung-Lu of 35K, 380K 93 -> 31, 115 -> 69; RGG of 45K, 473K
+// 80 -> 30, 106 -> 70, 1.6M 160 -> 180.  Bound by launches below 50K edges, then by the searches'
+// dependent loads.
+constexpr int64_t kSmallEdges = 1 << 19;
+template <int G>
+__global__ void __launch_bounds__(256) small_edges_kernel(CsrView g, unsigned long long* out, unsigned long long* acc) {
+  const int sub = threadIdx.x % G;
+  const int64_t groups = (int64_t)gridDim.x * 256 / G;
+  unsigned cnt = 0;
+  for (int64_t e = g.e0 + (blockIdx.x * 256ll + threadIdx.x) / G; e < g.e1; e += groups) {
+    const int32_t u = __ldg(g.esrc + e), v = __ldg(g.cols + e);
+    const int64_t au = __ldg(g.off + u), av = __ldg(g.off + v);
+    const int du = (int)(__ldg(g.off + u + 1) - au), dv = (int)(__ldg(g.off + v + 1) - av);
+    const int32_t* L = g.cols + (du >= dv ? au : av);
+    const int32_t* S = g.cols + (du >= dv ? av : au);
+    const int dl = max(du, dv), ds = min(du, dv);
+    for (int j = sub; j < ds; j += G) {
+      const int32_t x = __ldg(S + j);
+      int lo = 0, n = dl;
+      while (n > 1) {  // branch-free lower bound
+        const int half = n >> 1;
+        lo = __ldg(L + lo + half - 1) < x ? lo + half : lo;
+        n -= half;
+      }
+      cnt += __ldg(L + lo) == x;
+    }
+  }
+  __shared__ unsigned long long part[8];
+  const unsigned w = __reduce_add_sync(0xffffffffu, cnt);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = w;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned long long t = 0;
+    for (int i = 0; i < 8; ++i) t += part[i];
+    if (t) atomicAdd(&acc[0], t);
+    __threadfence();
+    if (atomicAdd(&acc[1], 1ull) == gridDim.x - 1) {  // the last block
+      __threadfence();
+      *out = atomicExch(&acc[0], 0ull);
+      acc[1] = 0ull;
+    }
+  }
+}
+
 // ============================== sorted-copy searches ===============================
 // TriCore-style and Fox-style counts on the Bisson-style grouping: every edge goes to its
 // endpoint h with the longer list and the partner's shorter list is streamed (sum of
@@ -743,6 +794,31 @@ static atc_status run_hu(const CsrView& g, const atc_tuning* t, unsigned long lo
   return launch_slots(slots, g, g.cols, witems.p, bitems.p, hc, counters.p, ctr, s, launches);
 }
 
+// Whether the window's Hu-style count goes to the small kernel: 5.5 ps per element of W_min and 60
+// ps per edge (dependent loads) against 2 ps per wedge, 45 ps per edge and 47 us more of launches
+// and waits.  Dense graphs of few edges (K_1000: 0.9 ms here, 0.4 by items) are not small.
+static bool small_pays(const atc_csr* csr, int64_t edges) {
+  if (edges > kSmallEdges) return false;
+  const double part = (double)edges / (double)csr->m;
+  return part * (5.5 * (double)csr->wedges_min + 15.0 * (double)csr->m) < part * 2.0 * (double)csr->wedges + 4.7e7;
+}
+
+static atc_status run_small(const CsrView& g, int64_t mean_min, unsigned long long* ctr, unsigned long long* acc,
+                            cudaStream_t s, int* launches) {
+  Phase ph("tc.count", s);
+  const int64_t edges = g.e1 - g.e0;
+  auto launch = [&](auto kern, int lanes) {
+    const int64_t want = (edges * lanes + 255) / 256;
+    kern<<<(unsigned)std::min<int64_t>(want, (int64_t)sm_count() * 8), 256, 0, s>>>(g, ctr, acc);
+  };
+  if (mean_min <= 8) launch(small_edges_kernel<8>, 8);
+  else if (mean_min <= 32) launch(small_edges_kernel<16>, 16);
+  else launch(small_edges_kernel<32>, 32);
+  ATC_CK(cudaGetLastError());
+  *launches += 1;
+  return ATC_OK;
+}
+
 // The Bisson-style grouping of the edges of [e0, e1): every edge {u, v} at its endpoint h
 // with the longer list, the partners of each h contiguous in plist, cut into warp and block
 // items.  hc = {warp items, block items, -, longest hashed block list}.
@@ -803,11 +879,14 @@ static bool ranked_pays(const atc_csr* csr) {
 // read from files (any sorted rows are accepted there); CSRs in host memory count in bounded
 // scratch; an item shape asked for by tuning is one of the grouped lists.  Entries hold 32-bit
 // positions.
+static bool shaped(const atc_tuning* t) {  // an item shape is asked for
+  return t && (t->bisson_cutover > 0 || t->bisson_warp_max > 0 || t->bisson_warp_chunk > 0 ||
+               t->bisson_block_chunk > 0 || t->bisson_slots != 0);
+}
 static bool ranked_applies(const atc_csr* csr, int64_t e0, int64_t e1, const atc_tuning* t) {
   const CsrPriv* pv = static_cast<const CsrPriv*>(csr->priv);
   if (!pv->indeg || pv->host_cols || e0 != 0 || e1 != csr->m || csr->m > (int64_t)INT32_MAX) return false;
-  return !t || (t->bisson_cutover <= 0 && t->bisson_warp_max <= 0 && t->bisson_warp_chunk <= 0 &&
-                t->bisson_block_chunk <= 0 && t->bisson_slots == 0);
+  return !shaped(t);
 }
 
 static atc_status run_bisson(const CsrView& g, const atc_tuning* t, unsigned long long* ctr, cudaStream_t s,
@@ -1107,7 +1186,8 @@ atc_status atc::part_edge_range(const atc_csr* csr, uint32_t part, uint32_t npar
 static atc_kernel auto_kernel(const atc_csr* csr, bool ranked) {
   const double m = (double)csr->m, w = (double)csr->wedges, wmin = (double)csr->wedges_min;
   const double bisson_ps = ranked ? 0.37 * wmin + 85.0 * m + 1.7e8 : 1.232 * wmin + 117.5 * m + 3.0e8;
-  const double hu_ps = ranked ? 2.0 * w + 45.0 * m + 6.0e7 : 1.097 * w + 103.5 * m;
+  double hu_ps = ranked ? 2.0 * w + 45.0 * m + 6.0e7 : 1.097 * w + 103.5 * m;
+  if (small_pays(csr, csr->m)) hu_ps = std::min(hu_ps, 5.5 * wmin + 60.0 * m + 1.3e7);
   return hu_ps < bisson_ps ? ATC_KERNEL_HU : ATC_KERNEL_BISSON;
 }
 
@@ -1125,9 +1205,13 @@ static atc_status tc_window(const atc_csr* csr, atc_kernel kernel, const atc_tun
     unsigned long long* ctr = pv->counter;
     Phase ph("tc", s);
     tm.start(s);
-    ATC_CK(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), s));
+    const bool small = kernel == ATC_KERNEL_HU && !shaped(tuning) && small_pays(csr, e1 - e0);
+    if (!small) ATC_CK(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), s));
     switch (kernel) {
-      case ATC_KERNEL_HU: ATC_TRY(run_hu(g, tuning, ctr, s, &launches)); break;
+      case ATC_KERNEL_HU:
+        if (small) ATC_TRY(run_small(g, csr->wedges_min / csr->m, ctr, pv->counter + 4, s, &launches));
+        else ATC_TRY(run_hu(g, tuning, ctr, s, &launches));
+        break;
       case ATC_KERNEL_BISSON: {
         bool done = false;
         if (ranked) ATC_TRY(count_ranked(csr, ctr, &done, s, &launches));

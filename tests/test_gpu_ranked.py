@@ -126,3 +126,23 @@ def test_long_rows_beyond_the_bitmaps():
     assert csr.max_outdeg > 512
     assert atc.tc(csr, K.BISSON)[0] == atc.tc(csr, K.HU)[0]
     csr.free()
+
+
+@pytest.mark.parametrize("n", [3, 9, 20, 33, 70, 200, 300])
+def test_small_counts(n):
+    """The small Hu-style kernel (8, 16 and 32 lanes an edge by the mean list), on one CSR several
+    times over (its accumulator is left at zero), whole and in parts, beside the item kernels."""
+    rng = np.random.default_rng(n)
+    e = rng.integers(0, 4 * n, (6 * n, 2))
+    hub = np.stack([np.zeros(3 * n, np.int64), np.arange(1, 3 * n + 1)], 1)
+    g = np.concatenate([_complete(n), e, hub]).astype(np.int32)
+    want = oracle.tc_count(g)
+    for d in (atc.Dir.ID, atc.Dir.DEGREE):
+        csr = atc.pretc(g, d)
+        for _ in range(3):
+            assert atc.tc(csr, K.HU)[0] == want
+        assert sum(atc.tc_part(csr, p, 5, K.HU)[0] for p in range(5)) == want
+        assert atc.tc(csr, K.BISSON)[0] == want
+        assert atc.tc(csr, K.HU, tuning={"bisson_slots": 2})[0] == want
+        assert atc.tc(csr, K.AUTO)[0] == want
+        csr.free()
