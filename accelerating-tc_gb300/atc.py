@@ -561,7 +561,9 @@ class MLP:
         x = np.ascontiguousarray(x, dtype=np.float32).reshape(-1, self.n_in)
         t = np.ascontiguousarray(t, dtype=np.float32).reshape(-1, self.n_out)
         mask = None if mask is None else np.ascontiguousarray(mask, dtype=np.float32)
-        g = np.empty(self.params().size, dtype=np.float32)
+        cnt = C.c_int64(0)
+        _check(lib().atc_mlp_params(self._h, None, None, C.byref(cnt)))
+        g = np.empty(cnt.value, dtype=np.float32)
         loss = np.zeros(1, dtype=np.float32)
         _check(lib().atc_mlp_gradients(self._h, _ptr(x), _ptr(t), _ptr(mask), x.shape[0], _ptr(g), _ptr(loss), None))
         return float(loss[0]), g

@@ -102,3 +102,25 @@ def test_selector_gains_over_cost_function():
     pol = res["policies"]
     assert pol["learned"]["ms"] < pol["cost_function"]["ms"], pol
     assert pol["learned"]["ms"] <= pol["fixed_default"]["ms"], pol
+
+
+@pytest.mark.parametrize("B", [1, 7, 8, 9, 480, 1217, 1300])
+@pytest.mark.parametrize("I,H,O", [(6, 64, 24), (6, 64, 60), (3, 33, 7), (6, 100, 60), (1, 1, 1), (6, 160, 24)])
+def test_fused_gradients_match_oracle(B, I, H, O):
+    """Rows at the edges of the tiles and of a CTA's share of them, odd and even layers, and a
+    network beyond shared memory (layer kernels).  Tolerance: sums of up to 1300 rows and 160
+    units in FP32, about 1e-7 each, relative to the largest gradient."""
+    rng = np.random.default_rng(B * 1000 + H)
+    net = atc.MLP(I, H, O, seed=B)
+    mean = rng.normal(size=I).astype(np.float32)
+    std = (rng.random(I) + 0.5).astype(np.float32)
+    net.scaling(mean, std)
+    x, t, mask = _problem(rng, B, I, O)
+    for mk in (mask, None):
+        loss, g = net.gradients(x, t, mk)
+        rloss, rg = oracle.mlp_grad(net.params(), I, H, O, mean, std, x, t, mk)
+        assert abs(loss - rloss) <= 1e-4 * max(1.0, abs(rloss))
+        assert np.abs(g - rg).max() <= 2e-4 * max(np.abs(rg).max(), 1e-3)
+        loss2, g2 = net.gradients(x, t, mk)
+        assert loss2 == loss and np.array_equal(g, g2)  # fixed order of every sum
+    assert net.forward(x).shape == (B, O)
