@@ -18,8 +18,8 @@ atc_status sort_keys_u64_tmp(void* tmp, size_t* bytes, uint64_t* keys, uint64_t*
 // `vals` point at the sorted data (each may be swapped with its alternate buffer).
 atc_status sort_pairs_u64_i32(uint64_t*& keys, uint64_t*& kalt, int32_t*& vals, int32_t*& valt, size_t n, int begin_bit,
                              int end_bit, cudaStream_t s);
-// Unique over sorted keys; *n_out (host) receives the count.
-atc_status unique_u64(const uint64_t* in, uint64_t* out, size_t n, size_t* n_out, cudaStream_t s);
+// Unique over n sorted keys; *count (device) receives their number.
+atc_status unique_u64_async(const uint64_t* in, uint64_t* out, size_t n, int64_t* count, cudaStream_t s);
 // out[i] = sum_{j<i} in[j], for n elements.
 atc_status exclusive_scan_i64(const int64_t* in, int64_t* out, size_t n, cudaStream_t s);
 atc_status exclusive_scan_i32_to_i64(const int32_t* in, int64_t* out, size_t n, cudaStream_t s);

@@ -57,19 +57,12 @@ atc_status sort_pairs_u64_i32(uint64_t*& keys, uint64_t*& kalt, int32_t*& vals, 
   return ATC_OK;
 }
 
-atc_status unique_u64(const uint64_t* in, uint64_t* out, size_t n, size_t* n_out, cudaStream_t s) {
-  if (n == 0) { *n_out = 0; return ATC_OK; }
-  DevBuf<int64_t> cnt;
-  ATC_TRY(cnt.alloc(1, s));
+atc_status unique_u64_async(const uint64_t* in, uint64_t* out, size_t n, int64_t* count, cudaStream_t s) {
   size_t tmp = 0;
-  ATC_CK(cub::DeviceSelect::Unique(nullptr, tmp, in, out, cnt.p, (int64_t)n, s));
+  ATC_CK(cub::DeviceSelect::Unique(nullptr, tmp, in, out, count, (int64_t)n, s));
   DevBuf<char> t;
   ATC_TRY(t.alloc(tmp, s));
-  ATC_CK(cub::DeviceSelect::Unique(t.p, tmp, in, out, cnt.p, (int64_t)n, s));
-  int64_t h = 0;
-  ATC_CK(cudaMemcpyAsync(&h, cnt.p, sizeof(h), cudaMemcpyDeviceToHost, s));
-  ATC_CK(cudaStreamSynchronize(s));
-  *n_out = (size_t)h;
+  ATC_CK(cub::DeviceSelect::Unique(t.p, tmp, in, out, count, (int64_t)n, s));
   return ATC_OK;
 }
 
