@@ -28,12 +28,15 @@
 // in orientation order — the same count kcl_gpu_solver accumulates.
 //
 // Measured (ms, one call; the per-edge walk with its dense kernel -> rows): RGG 2^20 of mean
-// degree 32, k = 4 / 5 / 6 / 7: 22.0 / 25.2 / 39.7 / 72.8 -> 0.87 / 1.25 / 4.3 / 16.4; R-MAT
-// scale 18, k = 4 / 5 / 6: 53.7 / 69.4 / 360 -> 3.8 / 17.8 / 174; scale 20, k = 4 / 5 / 6: 424 /
-// 547 / 3697 -> 25.2 / 215 / 2339; scale 14, k = 6 / 7: 3.8 / 37.5 -> 2.4 / 28.9.
+// degree 32, k = 4 / 5 / 6 / 7: 22.0 / 25.2 / 39.7 / 72.8 -> 0.87 / 1.25 / 4.3 / 16.8; R-MAT
+// scale 18, k = 4 / 5 / 6: 53.7 / 69.4 / 360 -> 2.7 / 15.0 / 171; scale 20, k = 4 / 5 / 6: 424 /
+// 547 / 3697 -> 16.2 / 169 / 2464; scale 14, k = 6 / 7: 3.8 / 37.5 -> 2.3 / 30.5.  Of that, the CTA
+// kernel's binary searches in all of N+(u) and its grabs of 32 lists (few of its warps had any)
+// took scale 18, k = 4 from 3.8 to 2.7 when a part table and smaller grabs replaced them.
 #include <algorithm>
 
 #include "internal.cuh"
+#include "parts.cuh"
 
 namespace atc {
 
@@ -474,6 +477,7 @@ constexpr int kRowMax = 960;       // rows of 960 x 15 words (115 KB) and everyt
 constexpr int kRowWarp = 128;      // C0 up to this size is renumbered and counted by one warp
 constexpr int kRowBlock = 512;     // k = 5: C0 up to this size by the CTA that holds its rows
 constexpr int kRowThreads = 512;
+constexpr int kRowParts = 2048;    // part table of N+(u): two parts a member
 constexpr int kRowBuckets = 4;     // lists by length, longest first (row_bucket)
 constexpr int kRowSearch = 128;    // lists longer than this are searched for the members of
                                    // N+(u), not streamed, where N+(u) fits one warp's masks
@@ -728,6 +732,8 @@ __global__ void __launch_bounds__(kRowThreads) kcl_rows_block_kernel(const int64
   unsigned long long* rows = reinterpret_cast<unsigned long long*>(rsm + at.rows);
   int32_t* S = reinterpret_cast<int32_t*>(rsm + at.s);
   __shared__ int item, next_batch, next_row;
+  __shared__ uint32_t ptab[kRowParts];
+  __shared__ uint16_t part_start[kRowParts + 1];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = kRowThreads / 32;
   int first[kRowBuckets + 1];
   first[0] = 0;
@@ -761,25 +767,32 @@ __global__ void __launch_bounds__(kRowThreads) kcl_rows_block_kernel(const int64
     if (MODE > 0)
       for (int t = threadIdx.x; t < d * st; t += kRowThreads) rows[t] = 0ull;
     __syncthreads();
-    const int32_t s_lo = S[0], s_hi = S[d - 1];
+    const int shift = build_parts(S, d, kRowParts, part_start, ptab, threadIdx.x, kRowThreads, [] { __syncthreads(); });
+    const int32_t s_lo = S[0];
+    const uint32_t s_range = (uint32_t)(S[d - 1] - s_lo);
+    // lists a warp takes at a time: at least two rounds for every warp, where there are that many
+    const int grab = min(max(d / (2 * nw), 1), 32);
     uint32_t* r32 = reinterpret_cast<uint32_t*>(rows);
     for (;;) {
       int base = 0;
-      if (lane == 0) base = atomicAdd(&next_batch, 32);
+      if (lane == 0) base = atomicAdd(&next_batch, grab);
       base = __shfl_sync(0xffffffffu, base, 0);
       if (base >= d) break;
       int64_t xb = 0;
       int xd = 0;
-      if (base + lane < d) {
+      if (lane < grab && base + lane < d) {
         const int32_t x = S[base + lane];
         xb = __ldg(off + x);
         xd = (int)(__ldg(off + x + 1) - xb);
       }
       bytes += 4ull * (unsigned long long)xd;
       for_members(cols, xb, xd, lane, [&](int32_t y, int kk, bool v) {
-        if (!v || y < s_lo || y > s_hi) return;
-        int lo = 0, len = d;  // branch-free lower bound
-        while (len > 1) {
+        const uint32_t r = (uint32_t)(y - s_lo);
+        if (!v || r > s_range) return;
+        const uint32_t pe = ptab[r >> shift];
+        int lo = (int)(pe & 0xffffu), len = (int)(pe >> 16) - lo;
+        if (len == 0) return;
+        while (len > 1) {  // branch-free lower bound inside the part
           const int half = len >> 1;
           lo = S[lo + half - 1] < y ? lo + half : lo;
           len -= half;

@@ -29,7 +29,7 @@ def test_row_lengths(d):
     csr.free()
 
 
-@pytest.mark.parametrize("d,k", [(832, 5), (833, 5), (1280, 4), (1281, 4), (1279, 3), (1281, 3), (900, 6)])
+@pytest.mark.parametrize("d,k", [(832, 5), (833, 5), (960, 5), (961, 5), (960, 6), (960, 4), (1280, 4), (1281, 4), (1279, 3), (1281, 3), (900, 6)])
 def test_longest_rows(d, k):
     g = _hub(d, d, 0.03)
     csr = atc.pretc(g, atc.Dir.ID)
