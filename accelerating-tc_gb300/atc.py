@@ -621,7 +621,7 @@ def adirection(pairs, want_prio=False, stream=None):
     if want_prio:
         prio = np.empty(int(p.max()) + 1 if p.size else 1, dtype=np.int32)
     _check(lib().atc_adirection(_ptr(p), p.shape[0], _ptr(out), C.byref(n), _ptr(prio), stream))
-    res = out[: n.value].copy()
+    res = out[: n.value]
     return (res, prio) if want_prio else res
 
 
