@@ -45,7 +45,7 @@ struct atc_batch {
   int64_t* vbase_d = nullptr;
   unsigned long long* gcounts = nullptr;
   void* scan_tmp = nullptr;
-  int64_t built_n = -1, built_m = -1, items_cap = 0;
+  int64_t built_n = -1, built_m = -1, items_cap = 0, rows_cap = 0;
   int built_graphs = -1;
   atc::ItemShape built_shape{};
   cudaStream_t cap_stream = nullptr;
@@ -215,6 +215,9 @@ ItemShape shape_from(const atc_tuning* t, const ItemShape& base) {
   if (t->bisson_warp_chunk > 0) sh.warp_chunk = t->bisson_warp_chunk;
   if (t->bisson_block_chunk > 0) sh.block_chunk = t->bisson_block_chunk;
   if (t->group_by_source > 0) sh.by_source = t->group_by_source >= 2 ? 2 : 1;
+  // every partner list is streamed through a row's set: the sorted copy only for the shortest rows,
+  // as in the single-graph Hu count, unless the tuning says otherwise
+  if (sh.by_source == 1 && t->bisson_cutover <= 0) sh.cutover = std::min(sh.cutover, 8);
   if (sh.cutover > sh.warp_max) sh.cutover = sh.warp_max;
   return sh;
 }
@@ -228,8 +231,16 @@ atc_status build_pipeline(atc_batch* b, const ItemShape& sh, cudaStream_t s) {
   // block items of lists longer than kBlockSmallList: one per such list (at most
   // m / (kBlockSmallList + 1) of them) plus one per chunk boundary
   const int64_t big_cap = m / (kBlockSmallList + 1) + m / sh.block_chunk + 1;
+  // rows items of mode 2: a row's partners are its own members, so a chunk is a share of one row
+  // and the longest rows set the tail; 64 partners an item (Chung-Lu batch of 26M edges: rows items
+  // of 512 4.36 ms, of 64 4.22)
+  ItemShape shr = sh;
+  shr.by_source = 1;
+  shr.cutover = std::min(sh.cutover, 8);  // the rows items' sorted copy, as the single-graph Hu count
+  shr.warp_chunk = std::min(sh.warp_chunk, 64);
+  const int64_t cap_rows = max_items(n, m, std::min(shr.warp_chunk, shr.block_chunk));
   if (b->built_n != n || b->built_m != m || b->built_graphs != ng || b->items_cap < cap_items ||
-      b->big_cap < big_cap) {
+      b->rows_cap < cap_rows || b->big_cap < big_cap) {
     free_pipeline(b);
     ATC_TRY(dev_alloc(&b->cnt, (size_t)n + 1));
     ATC_TRY(dev_alloc(&b->cur, (size_t)n + 1));
@@ -237,7 +248,7 @@ atc_status build_pipeline(atc_batch* b, const ItemShape& sh, cudaStream_t s) {
     ATC_TRY(dev_alloc(&b->plist, (size_t)m + 32));
     ATC_TRY(dev_alloc(&b->items, (size_t)cap_items));
     ATC_TRY(dev_alloc(&b->counters, kBatchCounters));
-    ATC_TRY(dev_alloc(&b->items_r, (size_t)cap_items));
+    ATC_TRY(dev_alloc(&b->items_r, (size_t)cap_rows));
     ATC_TRY(dev_alloc(&b->counters_r, 8));
     ATC_TRY(dev_alloc(&b->vrows, (size_t)n + 1));
     ATC_TRY(dev_alloc(&b->big, (size_t)big_cap));
@@ -252,6 +263,7 @@ atc_status build_pipeline(atc_batch* b, const ItemShape& sh, cudaStream_t s) {
     b->built_m = m;
     b->built_graphs = ng;
     b->items_cap = cap_items;
+    b->rows_cap = cap_rows;
     b->big_cap = big_cap;
   } else if (b->exec) {
     cudaGraphExecDestroy(b->exec);
@@ -293,18 +305,19 @@ atc_status build_pipeline(atc_batch* b, const ItemShape& sh, cudaStream_t s) {
   // whichever the per-graph cost model of the two kernels predicts faster (the per-call terms
   // of the single-graph model do not apply inside one replay)
   const bool mixed = sh.by_source == 2;
-  ItemShape shr = sh;
-  shr.by_source = 1;
-  shr.cutover = std::min(sh.cutover, 8);  // the rows items' sorted copy, as the single-graph Hu count
-  CompactItems witems_r{b->items_r, b->off, cap_items, false, false, shr};
-  CompactItems bitems_r{b->items_r, b->off, cap_items, true, true, shr};
+  CompactItems witems_r{b->items_r, b->off, cap_rows, false, false, shr};
+  CompactItems bitems_r{b->items_r, b->off, cap_rows, true, true, shr};
   CompactItems litems_r{b->big_r, b->off, big_cap, false, true, shr};
   int nrows = 0;
   if (mixed) {
     ATC_CK(cudaMemsetAsync(b->vrows, 0, (size_t)n + 1, s));
     for (int q = 0; q < ng; ++q) {
       const double m_q = (double)b->gm[q];
-      const bool rows = 1.097 * (double)b->gw[q] + 103.5 * m_q < 1.232 * (double)b->gwmin[q] + 117.5 * m_q;
+      // ps, fitted to R-MAT and Chung-Lu graphs alone and in batches.  Grouping's 250 ps an edge
+      // holds the contended cursors of the hubs: measured by rows / grouped, R-MAT scale 18 342 / 330 ps
+      // an edge in all, scale 20 395 / 305, scale 24 890 / 450, Chung-Lu 1M vertices 151 / 163, batches
+      // of 48 Chung-Lu graphs 120-130 / 165-196
+      const bool rows = 1.25 * (double)b->gw[q] + 60.0 * m_q < 1.2 * (double)b->gwmin[q] + 250.0 * m_q;
       if (rows && b->vbase[q + 1] > b->vbase[q]) {
         ATC_CK(cudaMemsetAsync(b->vrows + b->vbase[q], 1, (size_t)(b->vbase[q + 1] - b->vbase[q]), s));
         ++nrows;
@@ -365,7 +378,7 @@ atc_status build_pipeline(atc_batch* b, const ItemShape& sh, cudaStream_t s) {
   stage("batch.warp");
   if (mixed && nrows > 0) {
     cudaMemsetAsync(b->counters_r, 0, sizeof(int) * 8, c);
-    group_items_compact_kernel<<<grid_for(n, 256), 256, 0, c>>>(g, b->off, b->items_r, cap_items, b->big_r,
+    group_items_compact_kernel<<<grid_for(n, 256), 256, 0, c>>>(g, b->off, b->items_r, cap_rows, b->big_r,
                                                                 b->counters_r, shr, b->vrows, 1);
     kernels += 3;
     stage("batch.rows.items");
