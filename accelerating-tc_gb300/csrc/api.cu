@@ -34,6 +34,21 @@ int sm_count() {
   return cached_sms;
 }
 
+bool host_stores() {
+  static thread_local int cached_dev = -1;
+  static thread_local bool cached = false;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  if (dev != cached_dev) {
+    int access = 0, tables = 0;
+    cudaDeviceGetAttribute(&access, cudaDevAttrPageableMemoryAccess, dev);
+    cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev);
+    cached_dev = dev;
+    cached = access && tables;
+  }
+  return cached;
+}
+
 // ---- device allocation budget ----------------------------------------------------
 static std::atomic<int64_t> g_budget{-1};  // bytes left; -1 = unlimited
 

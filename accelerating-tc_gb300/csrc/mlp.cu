@@ -321,6 +321,13 @@ atc_status fused_gradients(const atc_mlp* net, const FusedArgs& a, float* grads,
   return ATC_OK;
 }
 
+// Whether the tile kernels read their rows from host memory in place and the results are stored
+// there: one pass over the CPU-GPU link inside the kernel instead of a copy before and after it.
+// For calls of up to a megabyte; larger ones keep the copies.
+bool direct_io(int rows, const atc_mlp* net) {
+  return host_stores() && (size_t)rows * (net->I + 2 * net->O) <= (1u << 18);
+}
+
 // One host array of the call's inputs, so that they take one copy: mean, 1 / std, x, t, mask.
 std::vector<float> pack_inputs(const atc_mlp* net, const float* x, const float* t, const float* mask, int B) {
   const size_t I = net->I, O = net->O, nx = (size_t)B * I, nt = t ? (size_t)B * O : 0;
@@ -581,18 +588,25 @@ extern "C" atc_status atc_mlp_forward(atc_mlp* net, const float* x, int32_t rows
   cudaStream_t s = as_stream(st);
   if (fused_fits(net, false)) {
     const std::vector<float> in = pack_inputs(net, x, nullptr, nullptr, rows);
+    const size_t ny = (size_t)rows * net->O;
+    const bool direct = direct_io(rows, net);
+    std::vector<float> out(direct ? ny : 0);  // touched pages: y may be fresh memory
     DevBuf<float> mem;
-    ATC_TRY(mem.alloc(in.size() + (size_t)rows * net->O, s));
-    ATC_CK(cudaMemcpyAsync(mem.p, in.data(), sizeof(float) * in.size(), cudaMemcpyHostToDevice, s));
+    if (!direct) {
+      ATC_TRY(mem.alloc(in.size() + ny, s));
+      ATC_CK(cudaMemcpyAsync(mem.p, in.data(), sizeof(float) * in.size(), cudaMemcpyHostToDevice, s));
+    }
+    const float* src = direct ? in.data() : mem.p;
     FusedArgs a{};
-    a.mean = mem.p;
-    a.inv = mem.p + net->I;
-    a.x = mem.p + 2 * net->I;
+    a.mean = src;
+    a.inv = src + net->I;
+    a.x = src + 2 * net->I;
     a.B = rows;
-    a.y = mem.p + in.size();
-    ATC_TRY(launch_tiles<false>(net, a, s));
-    ATC_CK(cudaMemcpyAsync(y, a.y, sizeof(float) * rows * net->O, cudaMemcpyDeviceToHost, s));
-    ATC_CK(cudaStreamSynchronize(s));
+    a.y = direct ? out.data() : mem.p + in.size();
+    const atc_status st2 = launch_tiles<false>(net, a, s);
+    ATC_TRY(read_bytes(y, a.y, sizeof(float) * ny, direct, s));
+    ATC_TRY(st2);
+    if (direct) memcpy(y, out.data(), sizeof(float) * ny);
     return ATC_OK;
   }
   Scratch sc;
@@ -611,22 +625,24 @@ extern "C" atc_status atc_mlp_gradients(atc_mlp* net, const float* x, const floa
   if (fused_fits(net, true)) {
     const std::vector<float> in = pack_inputs(net, x, t, mask, rows);
     const size_t np = (size_t)net->nparams, nx = (size_t)rows * net->I, nt = (size_t)rows * net->O;
+    const bool direct = direct_io(rows, net);
+    std::vector<float> out(np + 1);
     DevBuf<float> mem;
-    ATC_TRY(mem.alloc(in.size() + np + 1 + (size_t)fused_ctas(rows) * (np + 2), s));
-    ATC_CK(cudaMemcpyAsync(mem.p, in.data(), sizeof(float) * in.size(), cudaMemcpyHostToDevice, s));
+    ATC_TRY(mem.alloc((direct ? 0 : in.size() + np + 1) + (size_t)fused_ctas(rows) * (np + 2), s));
+    float* g = direct ? out.data() : mem.p + in.size();
+    if (!direct) ATC_CK(cudaMemcpyAsync(mem.p, in.data(), sizeof(float) * in.size(), cudaMemcpyHostToDevice, s));
+    const float* src = direct ? in.data() : mem.p;
     FusedArgs a{};
-    a.mean = mem.p;
-    a.inv = mem.p + net->I;
-    a.x = mem.p + 2 * net->I;
+    a.mean = src;
+    a.inv = src + net->I;
+    a.x = src + 2 * net->I;
     a.t = a.x + nx;
     a.mask = mask ? a.t + nt : nullptr;
     a.B = rows;
-    float* g = mem.p + in.size();
-    a.partial = g + np + 1;
-    ATC_TRY(fused_gradients(net, a, g, s));
-    std::vector<float> out(np + 1);
-    ATC_CK(cudaMemcpyAsync(out.data(), g, sizeof(float) * (np + 1), cudaMemcpyDeviceToHost, s));
-    ATC_CK(cudaStreamSynchronize(s));
+    a.partial = direct ? mem.p : g + np + 1;
+    const atc_status st2 = fused_gradients(net, a, g, s);
+    ATC_TRY(read_bytes(out.data(), g, sizeof(float) * (np + 1), direct, s));
+    ATC_TRY(st2);
     if (grads) memcpy(grads, out.data(), sizeof(float) * np);
     if (loss) *loss = out[np];
     return ATC_OK;

@@ -21,8 +21,10 @@ namespace {
 
 constexpr uint64_t kSentinel = ~0ull;
 
-// mx = the largest id as unsigned (a negative id is above INT_MAX), *mn = the smallest where asked.
-__global__ void max_id_kernel(const int2* p, uint64_t np, unsigned* mx, int* mn) {
+// mx[0] = the largest id as unsigned (a negative id is above INT_MAX), *mn = the smallest where
+// asked.  mx[1]: blocks that have ended, zeroed with mx[0]; the last one stores the result to
+// host (nullable: the caller's variable, host_stores()).
+__global__ void max_id_kernel(const int2* p, uint64_t np, unsigned* mx, int* mn, volatile unsigned* host) {
   unsigned hi = 0;
   int lo = INT_MAX;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -36,6 +38,14 @@ __global__ void max_id_kernel(const int2* p, uint64_t np, unsigned* mx, int* mn)
   if (mn) {
     lo = __reduce_min_sync(0xffffffffu, lo);
     if ((threadIdx.x & 31) == 0) atomicMin(mn, lo);
+  }
+  if (host) {
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(mx + 1, 1u) == gridDim.x - 1) {
+      __threadfence();
+      *host = *(volatile unsigned*)mx;
+    }
   }
 }
 
@@ -52,8 +62,12 @@ __global__ void canon_kernel(const int2* p, uint64_t np, int B, uint64_t* keys) 
   }
 }
 
-__global__ void drop_sentinel_kernel(const uint64_t* keys, int64_t* count) {
-  if (*count > 0 && keys[*count - 1] == kSentinel) *count -= 1;
+// host (nullable): the caller's variable, stored too (host_stores()).
+__global__ void drop_sentinel_kernel(const uint64_t* keys, int64_t* count, volatile int64_t* host) {
+  int64_t n = *count;
+  if (n > 0 && keys[n - 1] == kSentinel) --n;
+  *count = n;
+  if (host) *host = n;
 }
 
 // Degrees of the simple graph from its sorted keys.  Keys of one smaller endpoint are
@@ -202,8 +216,10 @@ __global__ void indeg_kernel(const int32_t* cols, int64_t m, int32_t* indeg) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += stride) atomicAdd(&indeg[cols[i]], 1);
 }
 
+// w: [0] = W, [1] = the largest out-degree (int), [2] = split_kernel's sum, [3] = blocks that have
+// ended (all zeroed, [3] again at the end).  The last block stores [0..2] to host (nullable).
 __global__ void wedge_kernel(const int64_t* off, const int32_t* indeg, int64_t n, unsigned long long* w,
-                             int* maxout) {
+                             volatile unsigned long long* host) {
   unsigned long long s = 0;
   int mo = 0;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -218,7 +234,16 @@ __global__ void wedge_kernel(const int64_t* off, const int32_t* indeg, int64_t n
   }
   if ((threadIdx.x & 31) == 0) {
     atomicAdd(w, s);
-    atomicMax(maxout, mo);
+    atomicMax(reinterpret_cast<int*>(w + 1), mo);
+  }
+  if (host) {
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(w + 3, 1ull) == gridDim.x - 1) {
+      __threadfence();
+      for (int i = 0; i < 3; ++i) host[i] = *(volatile unsigned long long*)(w + i);
+      w[3] = 0ull;
+    }
   }
 }
 
@@ -297,18 +322,18 @@ atc_status build_simple_edges(const int2* pairs, uint64_t np, SimpleEdges* out, 
   out->bits = 1;
   if (np == 0) return ATC_OK;
   DevBuf<unsigned> mx;
-  ATC_TRY(mx.alloc(2, s));
-  ATC_CK(cudaMemsetAsync(mx.p, 0, sizeof(unsigned), s));
-  max_id_kernel<<<grid_for(np, 256), 256, 0, s>>>(pairs, np, mx.p, nullptr);
-  ATC_CK(cudaGetLastError());
-  unsigned top = 0;
-  ATC_CK(cudaMemcpyAsync(&top, mx.p, sizeof(top), cudaMemcpyDeviceToHost, s));
-  ATC_CK(cudaStreamSynchronize(s));
+  ATC_TRY(mx.alloc(3, s));
+  ATC_CK(cudaMemsetAsync(mx.p, 0, 2 * sizeof(unsigned), s));
+  unsigned top_here = 0;
+  const bool stored = host_stores();
+  max_id_kernel<<<grid_for(np, 256), 256, 0, s>>>(pairs, np, mx.p, nullptr, stored ? &top_here : nullptr);
+  ATC_TRY(read_bytes(&top_here, mx.p, sizeof(top_here), stored, s));
+  const unsigned top = *static_cast<volatile unsigned*>(&top_here);
   if (top > (unsigned)INT_MAX) {
     int least = INT_MAX;
-    int* mn = reinterpret_cast<int*>(mx.p + 1);
+    int* mn = reinterpret_cast<int*>(mx.p + 2);
     ATC_CK(cudaMemcpyAsync(mn, &least, sizeof(least), cudaMemcpyHostToDevice, s));
-    max_id_kernel<<<grid_for(np, 256), 256, 0, s>>>(pairs, np, mx.p, mn);
+    max_id_kernel<<<grid_for(np, 256), 256, 0, s>>>(pairs, np, mx.p, mn, nullptr);
     ATC_CK(cudaGetLastError());
     ATC_CK(cudaMemcpyAsync(&least, mn, sizeof(least), cudaMemcpyDeviceToHost, s));
     ATC_CK(cudaStreamSynchronize(s));
@@ -329,10 +354,10 @@ atc_status build_simple_edges(const int2* pairs, uint64_t np, SimpleEdges* out, 
   DevBuf<int64_t> nu;
   ATC_TRY(nu.alloc(1, s));
   ATC_TRY(unique_u64_async(ka, kb, np, nu.p, s));
-  drop_sentinel_kernel<<<1, 1, 0, s>>>(kb, nu.p);
-  ATC_CK(cudaGetLastError());
-  ATC_CK(cudaMemcpyAsync(&out->m, nu.p, sizeof(out->m), cudaMemcpyDeviceToHost, s));
-  ATC_CK(cudaStreamSynchronize(s));
+  int64_t unique = 0;
+  drop_sentinel_kernel<<<1, 1, 0, s>>>(kb, nu.p, stored ? &unique : nullptr);
+  ATC_TRY(read_bytes(&unique, nu.p, sizeof(unique), stored, s));
+  out->m = *static_cast<volatile int64_t*>(&unique);
   // keep whichever buffer holds the unique keys
   if (kb == b.p) { out->keys = std::move(b); } else { out->keys = std::move(a); }
   return ATC_OK;
@@ -503,10 +528,10 @@ static atc_status pretc_impl(const int2* pairs, uint64_t np, atc_dir dir, atc_or
   } else if (n) {
     indeg_from_degrees_kernel<<<grid_for(n, 256), 256, 0, s>>>(off.p, deg.p, perm.p, n, indeg.p);
   }
-  if (n) wedge_kernel<<<grid_for(n, 256), 256, 0, s>>>(off.p, indeg.p, n, counter.p, (int*)(counter.p + 1));
-  ATC_CK(cudaGetLastError());
   unsigned long long hw[3] = {0, 0, 0};
-  ATC_CK(cudaMemcpyAsync(hw, counter.p, sizeof(hw), cudaMemcpyDeviceToHost, s));
+  const bool stored = n > 0 && host_stores();
+  if (n) wedge_kernel<<<grid_for(n, 256), 256, 0, s>>>(off.p, indeg.p, n, counter.p, stored ? hw : nullptr);
+  ATC_TRY(read_bytes(hw, counter.p, sizeof(hw), stored, s));
   if (perm_out && order != ATC_ORDER_NONE && n_in)
     ATC_CK(cudaMemcpyAsync(perm_out, perm.p, sizeof(int32_t) * n_in, cudaMemcpyDeviceToHost, s));
   else if (perm_out && n_in) {
@@ -527,12 +552,13 @@ static atc_status pretc_impl(const int2* pairs, uint64_t np, atc_dir dir, atc_or
   out->offsets = off.detach();
   out->cols = cols.detach();
   out->n_input = n_in;
-  out->wedges = (int64_t)hw[0];
+  const volatile unsigned long long* stats = hw;
+  out->wedges = (int64_t)stats[0];
   out->dir = (int32_t)dir;
   out->order = (int32_t)order;
   out->pruned = prune ? 1 : 0;
-  out->max_outdeg = (int32_t)(hw[1] & 0xffffffffu);
-  out->wedges_min = (int64_t)hw[2];
+  out->max_outdeg = (int32_t)(stats[1] & 0xffffffffu);
+  out->wedges_min = (int64_t)stats[2];
   out->priv = pv;
   return ATC_OK;
 }

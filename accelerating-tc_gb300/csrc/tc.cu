@@ -265,7 +265,8 @@ __global__ void fox_deal_kernel(const uint64_t* keys, const int64_t* list, int64
 // dependent loads.
 constexpr int64_t kSmallEdges = 1 << 19;
 template <int G>
-__global__ void __launch_bounds__(256) small_edges_kernel(CsrView g, unsigned long long* out, unsigned long long* acc) {
+__global__ void __launch_bounds__(256) small_edges_kernel(CsrView g, unsigned long long* out, unsigned long long* acc,
+                                                         volatile unsigned long long* host) {
   const int sub = threadIdx.x % G;
   const int64_t groups = (int64_t)gridDim.x * 256 / G;
   unsigned cnt = 0;
@@ -298,7 +299,9 @@ __global__ void __launch_bounds__(256) small_edges_kernel(CsrView g, unsigned lo
     __threadfence();
     if (atomicAdd(&acc[1], 1ull) == gridDim.x - 1) {  // the last block
       __threadfence();
-      *out = atomicExch(&acc[0], 0ull);
+      const unsigned long long total = atomicExch(&acc[0], 0ull);
+      *out = total;
+      if (host) *host = total;
       acc[1] = 0ull;
     }
   }
@@ -779,20 +782,20 @@ static bool small_pays(const atc_csr* csr, int64_t edges) {
   return part * (5.5 * (double)csr->wedges_min + 15.0 * (double)csr->m) < part * 2.0 * (double)csr->wedges + 4.7e7;
 }
 
+// host (nullable): the caller's variable, stored by the kernel (host_stores()).
 static atc_status run_small(const CsrView& g, int64_t mean_min, unsigned long long* ctr, unsigned long long* acc,
-                            cudaStream_t s, int* launches) {
+                            unsigned long long* host, cudaStream_t s, int* launches) {
   Phase ph("tc.count", s);
   const int64_t edges = g.e1 - g.e0;
   auto launch = [&](auto kern, int lanes) {
     const int64_t want = (edges * lanes + 255) / 256;
-    kern<<<(unsigned)std::min<int64_t>(want, (int64_t)sm_count() * 8), 256, 0, s>>>(g, ctr, acc);
+    kern<<<(unsigned)std::min<int64_t>(want, (int64_t)sm_count() * 8), 256, 0, s>>>(g, ctr, acc, host);
   };
   if (mean_min <= 8) launch(small_edges_kernel<8>, 8);
   else if (mean_min <= 32) launch(small_edges_kernel<16>, 16);
   else launch(small_edges_kernel<32>, 32);
-  ATC_CK(cudaGetLastError());
   *launches += 1;
-  return ATC_OK;
+  return ATC_OK;  // the caller's read_bytes checks the launch
 }
 
 // The Bisson-style grouping of the edges of [e0, e1): every edge {u, v} at its endpoint h
@@ -1182,10 +1185,12 @@ static atc_status tc_window(const atc_csr* csr, atc_kernel kernel, const atc_tun
     Phase ph("tc", s);
     tm.start(s);
     const bool small = kernel == ATC_KERNEL_HU && !shaped(tuning) && small_pays(csr, e1 - e0);
+    const bool stored = small && host_stores();  // the kernel itself stores the count to h
+    unsigned long long h = 0;
     if (!small) ATC_CK(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), s));
     switch (kernel) {
       case ATC_KERNEL_HU:
-        if (small) ATC_TRY(run_small(g, csr->wedges_min / csr->m, ctr, pv->counter + 4, s, &launches));
+        if (small) ATC_TRY(run_small(g, csr->wedges_min / csr->m, ctr, pv->counter + 4, stored ? &h : nullptr, s, &launches));
         else ATC_TRY(run_hu(g, tuning, ctr, s, &launches));
         break;
       case ATC_KERNEL_BISSON: {
@@ -1216,13 +1221,11 @@ static atc_status tc_window(const atc_csr* csr, atc_kernel kernel, const atc_tun
       }
     }
     tm.stop(s);
-    unsigned long long h = 0;
     {
       Phase ph_rb("tc.readback", s);
-      ATC_CK(cudaMemcpyAsync(&h, ctr, sizeof(h), cudaMemcpyDeviceToHost, s));
+      ATC_TRY(read_bytes(&h, ctr, sizeof(h), stored, s));
     }
-    ATC_CK(cudaStreamSynchronize(s));
-    *count = h;
+    *count = *static_cast<volatile unsigned long long*>(&h);
   }
   if (stats) {
     stats->kernel_ms = e1 > e0 ? tm.ms() : 0.0f;
