@@ -8,7 +8,7 @@
 
 namespace atc {
 
-// ---- device primitives (prims.cu; CUB radix sort / scan / select) ----------------
+// ---- device primitives (prims.cu; radix.cuh's sort, CUB scan / select) ----------------
 // Sorts n keys on bits [begin_bit, end_bit).  `keys` and `alt` are two buffers of n
 // elements; on return `keys` points at the sorted data (the two may be swapped).
 atc_status sort_keys_u64(uint64_t*& keys, uint64_t*& alt, size_t n, int begin_bit, int end_bit, cudaStream_t s);

@@ -1,5 +1,5 @@
-// Device-wide sort / unique / scan used by preTC.  These are plain library
-// primitives (CUB, shipped with the CUDA toolkit), in the role thrust::sort /
+// Device-wide sort / unique / scan used by preTC.  The key sort is radix.cuh's; the rest are plain
+// library primitives (CUB, shipped with the CUDA toolkit), in the role thrust::sort /
 // thrust::unique / thrust::exclusive_scan play in the reference preprocessing
 // (Hu/preTC.cu:208-212, tricount_gpu.cu:172-174, kcl.cu:197).
 #include <cub/device/device_radix_sort.cuh>
@@ -8,31 +8,41 @@
 #include <thrust/iterator/transform_iterator.h>
 
 #include "internal.cuh"
+#include "radix.cuh"
 
 namespace atc {
 
-atc_status sort_keys_u64(uint64_t*& keys, uint64_t*& alt, size_t n, int begin_bit, int end_bit, cudaStream_t s) {
-  if (n <= 1) return ATC_OK;
-  cub::DoubleBuffer<uint64_t> db(keys, alt);
-  size_t tmp = 0;
-  ATC_CK(cub::DeviceRadixSort::SortKeys(nullptr, tmp, db, (int64_t)n, begin_bit, end_bit, s));
-  DevBuf<char> t;
-  ATC_TRY(t.alloc(tmp, s));
-  ATC_CK(cub::DeviceRadixSort::SortKeys(t.p, tmp, db, (int64_t)n, begin_bit, end_bit, s));
-  if (db.Current() != keys) {
-    alt = keys;
-    keys = db.Current();
-  }
-  return ATC_OK;
-}
+// The framework's own sort (radix.cuh) from here on: it needs a histogram, an offsets and a clearing
+// launch besides its passes, so below this CUB's single-tile or smaller-tile kernels are as fast or
+// faster (figures in radix.cuh; the two cross between 16000 and 32000 keys).
+constexpr size_t kOwnSort = 1 << 15;
 
-// The same with caller-provided temporary storage; *sorted = the buffer that holds the result.
+// Sorts with caller-provided temporary storage; *sorted = the buffer that holds the result.
 // tmp == nullptr: *bytes receives the size needed.
 atc_status sort_keys_u64_tmp(void* tmp, size_t* bytes, uint64_t* keys, uint64_t* alt, size_t n, int begin_bit,
                              int end_bit, uint64_t** sorted, cudaStream_t s) {
+  if (n >= kOwnSort && end_bit > begin_bit) {
+    ATC_CK(radix_sort_keys(tmp, bytes, keys, alt, n, begin_bit, end_bit, sorted, s));
+    return ATC_OK;
+  }
   cub::DoubleBuffer<uint64_t> db(keys, alt);
   ATC_CK(cub::DeviceRadixSort::SortKeys(tmp, *bytes, db, (int64_t)n, begin_bit, end_bit, s));
   if (sorted) *sorted = db.Current();
+  return ATC_OK;
+}
+
+atc_status sort_keys_u64(uint64_t*& keys, uint64_t*& alt, size_t n, int begin_bit, int end_bit, cudaStream_t s) {
+  if (n <= 1) return ATC_OK;
+  size_t tmp = 0;
+  ATC_TRY(sort_keys_u64_tmp(nullptr, &tmp, keys, alt, n, begin_bit, end_bit, nullptr, s));
+  DevBuf<char> t;
+  ATC_TRY(t.alloc(tmp, s));
+  uint64_t* sorted = nullptr;
+  ATC_TRY(sort_keys_u64_tmp(t.p, &tmp, keys, alt, n, begin_bit, end_bit, &sorted, s));
+  if (sorted != keys) {
+    alt = keys;
+    keys = sorted;
+  }
   return ATC_OK;
 }
 
