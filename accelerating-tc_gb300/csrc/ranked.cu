@@ -13,23 +13,27 @@
 // 16-byte bucket, four compares and a queue (about 8 instructions per 32 tests against 31).
 //
 //   passes: degrees -> rank (radix sort on the degree bits) -> out-degrees and group sizes ->
-//   scans -> rows (scatter, then sorted in registers) -> entries (row start, prefix length)
-//   grouped by target -> work items -> count.  Nothing waits on the host before the count.
+//   scans -> rows (scatter, then sorted in registers) -> rows of the lowest ranks as bitmaps ->
+//   entries (row start, prefix length) grouped by target -> work items -> count.  Nothing waits on
+//   the host before the count.
+//   a long prefix before a target of low rank: the source's and the target's rows as bitmaps, ANDed
+//   word by word, 128 candidates per 16 bytes against eight ids; such edges need no entry.  Other
 //   targets of rank below 2^16: a warp per chunk of entries, its own bitmap of 4 or 8 KB, rows
 //   read as 16-bit ids; below 2^17 with enough entries: a CTA of four warps per chunk, a bitmap
 //   of 16 KB; the rest (a tenth of the tests at R-MAT scale 24): the hash kernels of bisson.cuh
 //   over the same entries, or a CTA's 64 KB bitmap for rows too long for a warp's table.
 //
 // Measured (R-MAT scale 24, A-direction + A-order; whole lists grouped at the longer endpoint ->
-// this path): 117.5 -> 47.4 ms, of which the passes take 13.7 ms (entries 5.8, group sizes 2.5,
-// row sorts 3.2, rows 1.4) and the count 33.5: ranks below 2^15 15.6, 2^16 5.5, 2^17 3.2, hash 9.2.
-// DRAM 14 %, L1 77 %, issue 63 % of peak in the 2^15 kernel at scale 22: bound by the shared
-// and L1 pipe (two wavefronts per 32 tests, one of them bank conflicts) and by issue (10 warp
-// instructions per 32 tests).  Scale 20: 4.45 -> 1.82 ms; Chung-Lu n = 700 001: 1.95 -> 1.18.
+// this path): 117.5 -> 40.0 ms, of which the passes take 12.8 ms (entries 4.9, group sizes 2.3,
+// row sorts 3.1, rows 1.4) and the count 27.1: words 4, other ranks below 2^15 6, 2^16 5.5, 2^17 3.2,
+// hash 9.2.  Without the words the ranks below 2^15 took 15.7 and the entries 5.7 (47.1 in all):
+// bound by the shared and L1 pipe (two wavefronts per 32 tests, one of them bank conflicts) and by
+// issue (10 warp instructions per 32 tests).  Scale 22: 8.6 -> 7.0 ms by the words, scale 20: 1.86 ->
+// 1.47 (4.45 by whole lists); Chung-Lu n = 700 001, which has few dense rows: 1.30 -> 1.26.
 // Tried: 32-bit rows and one entry a warp at a time 68 ms; 32-lane scans of short prefixes
-// instead of lane groups 88 ms; rows on 128-byte lines 1-4 % for twice the copy; 2 or 4 lanes a
-// prefix 73 / 57 ms.
+// instead of lane groups 88 ms; rows on 128-byte lines 1-4 % for twice the copy.
 #include <algorithm>
+#include <cmath>
 
 #include "ranked.cuh"
 
@@ -47,9 +51,12 @@ constexpr int kRank19 = kTabWords * 32; // below, with a row too long for a warp
 constexpr int kRankBlockChunk = 1024;   // entries per CTA item
 constexpr int kRankMidMin = 24;         // fewer entries than these do not pay for a CTA's bitmap
 constexpr int kRankBlockMin = 48;
-constexpr int64_t kWideMean = 224;      // mean of min(d+u, d+v) from which 16 lanes read a prefix, below it
-                                        // eight: R-MAT scale 20 (mean 132) 1.88 ms with 8, 2.09 with 16;
-                                        // scale 22 (187) 8.6 and 9.1; scale 24 (270) 50.6 and 47.7
+// Lanes that read a prefix, by the mean of min(d+u, d+v).  Targets below 2^15, whose long prefixes are
+// words: four, from kWideMean15 eight (R-MAT scale 20, mean 132: 1.47 and 1.51 ms; scale 22, 187: 7.1 and
+// 7.0; scale 24, 270: 41.0 and 40.2; Chung-Lu 1.26 and 1.31).  Below 2^16: eight, from kWideMean 16.
+constexpr int64_t kWideMean15 = 160, kWideMean = 224;
+constexpr int kDenseRows = 1 << 15;     // rows that may be kept as bitmaps
+constexpr int kDenseSources = 4;        // times as many rows are looked at for targets among them
 constexpr int kRankRowMax = kTabWords;  // longest row the CTA sort holds (64 KB)
 constexpr int kRankWarpRow = 1024;      // longest row a warp sorts in registers
 
@@ -276,17 +283,59 @@ __global__ void rank_piece_rows_kernel(const int64_t* roff, int64_t n, int32_t* 
   }
 }
 
+// Rows of the ranks below `rows` (at most 2^15) once more as bitmaps, in pieces of 128 bits: row v
+// has v / 128 + 1 of them, from dense_start(v) on.
+__host__ __device__ __forceinline__ uint32_t dense_start(uint32_t v) {
+  const uint32_t a = v >> 7, b = v & 127;
+  return (a + 1) * (64 * a + b);
+}
+
+// Whether the prefix of len ids before target v is better tested as words, by ANDing the rows of
+// the source and of v: a piece of 128 bits against kWordGain times a piece of eight ids, which costs
+// a look at every id and the edge's entry.  Gains of 2, 3, 4, 6, 8, 12 and 24: 41.8, 40.2, 39.9, 39.9, 40.2,
+// 40.2 and 40.3 ms at R-MAT scale 24; 3, 6, 12 and 24 at scale 20: 1.55, 1.47, 1.52 and 1.61.
+constexpr int kWordGain = 6;
+__device__ __forceinline__ bool words_pay(uint32_t len, uint32_t v) {
+  return kWordGain * ((len + 7) >> 3) > (v >> 7) + 1;
+}
+
+constexpr int kDenseWarps = 8;
+__global__ void __launch_bounds__(kDenseWarps * 32) rank_dense_kernel(const int64_t* roff, const int32_t* rcols, int rows,
+                                                                      uint4* dense) {
+  __shared__ __align__(16) uint32_t smem[kDenseWarps][1 << 10];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  uint32_t* T = smem[w];
+  uint4* T4 = reinterpret_cast<uint4*>(T);
+  const int warps = gridDim.x * kDenseWarps;
+  for (int u = blockIdx.x * kDenseWarps + w; u < rows; u += warps) {
+    const int pieces = (u >> 7) + 1;
+    for (int j = lane; j < pieces; j += 32) T4[j] = make_uint4(0u, 0u, 0u, 0u);
+    __syncwarp();
+    const int64_t e = __ldg(roff + u + 1);
+    for (int64_t j = __ldg(roff + u) + lane; j < e; j += 32) {
+      const int32_t x = __ldg(rcols + j);
+      atomicOr(&T[x >> 5], 1u << (x & 31));
+    }
+    __syncwarp();
+    uint4* to = dense + dense_start(u);
+    for (int j = lane; j < pieces; j += 32) to[j] = T4[j];
+    __syncwarp();
+  }
+}
+
 // Entry of every edge in its target's group: where the source's row starts and how much of it
 // lies before the target.  Targets below below16 read the 16-bit copy of the rows (r16, starts in
 // pieces of eight ids), written here; the others the rows themselves.  A tile's entries of the
-// most contended targets take their places with one atomic per tile and target.
+// most contended targets take their places with one atomic per tile and target.  Edges that
+// are tested as words have none: those of the first `sources` rows to targets below `rows` for
+// which that pays.
 constexpr int kEntryThreads = 1024;
 constexpr int kEntryEach = kTile / kEntryThreads;
 __global__ void __launch_bounds__(kEntryThreads, 2) rank_entries_kernel(const int64_t* roff, int64_t n, int64_t m,
                                                                      const int32_t* rcols, const int32_t* piece_row,
                                                                      const int64_t* gstart, const int64_t* roff8,
-                                                                     int32_t below16, int32_t* gcur, uint16_t* r16,
-                                                                     uint2* ent) {
+                                                                     int32_t below16, int32_t rows, int32_t sources,
+                                                                     int32_t* gcur, uint16_t* r16, uint2* ent) {
   __shared__ int hub[kHubEntry];
   const int64_t tiles = (m + kTile - 1) / kTile;
   for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
@@ -316,7 +365,8 @@ __global__ void __launch_bounds__(kEntryThreads, 2) rank_entries_kernel(const in
           st[q] = (uint32_t)r8;
           r16[8 * r8 + len[q]] = (uint16_t)lo[q];
         }
-        pos[q] = lo[q] < kHubEntry ? atomicAdd(&hub[lo[q]], 1) : atomicAdd(&gcur[lo[q]], 1);
+        if (a < sources && lo[q] < rows && words_pay(len[q], (uint32_t)lo[q])) lo[q] = -1;
+        else pos[q] = lo[q] < kHubEntry ? atomicAdd(&hub[lo[q]], 1) : atomicAdd(&gcur[lo[q]], 1);
       }
     }
     __syncthreads();
@@ -334,14 +384,14 @@ __global__ void __launch_bounds__(kEntryThreads, 2) rank_entries_kernel(const in
 }
 
 // bitmaps: targets by kind; otherwise every target as a list.  ctr[kcMaxRow] = the longest N+(v).
-__global__ void rank_items_kernel(const int64_t* roff, const int64_t* gstart, int64_t n, RankItemLists li, bool bitmaps,
-                                  int* ctr) {
+__global__ void rank_items_kernel(const int64_t* roff, const int64_t* gstart, const int32_t* gcur, int64_t n,
+                                  RankItemLists li, bool bitmaps, int* ctr) {
   const int64_t n_pad = (n + 31) & ~31ll;
   int longest = 0;
   for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n_pad; v += (int64_t)gridDim.x * blockDim.x) {
     int64_t ne = 0, dv = 0;
     if (v < n) {
-      ne = gstart[v + 1] - gstart[v];
+      ne = gcur[v];
       dv = roff[v + 1] - roff[v];
     }
     const bool any = ne > 0 && dv > 0;
@@ -442,7 +492,8 @@ __global__ void __launch_bounds__(WARPS * 32) rank_warp_kernel(const int64_t* __
                                                                const uint4* __restrict__ r16,
                                                                const uint2* __restrict__ ent,
                                                                const int2* __restrict__ items,
-                                                               const int64_t* __restrict__ gstart, int chunk,
+                                                               const int64_t* __restrict__ gstart,
+                                                               const int32_t* __restrict__ nids, int chunk,
                                                                const int* nitems_dev, int* next, const int* too_long,
                                                                unsigned long long* out) {
   constexpr uint32_t kBytes = BITS / 8;
@@ -484,7 +535,7 @@ __global__ void __launch_bounds__(WARPS * 32) rank_warp_kernel(const int64_t* __
     const int2 c = __ldg(items + it);
     const int32_t v = c.x;
     const int64_t g0 = __ldg(gstart + v) + (int64_t)c.y * chunk;
-    const int ne = (int)min(__ldg(gstart + v + 1) - g0, (int64_t)chunk);
+    const int ne = min(__ldg(nids + v) - c.y * chunk, chunk);
     const uint2* en = ent + g0;
     const int64_t hb = __ldg(roff + v);
     const int dh = (int)(__ldg(roff + v + 1) - hb);
@@ -525,6 +576,84 @@ __global__ void __launch_bounds__(WARPS * 32) rank_warp_kernel(const int64_t* __
     __syncwarp();
     for (int j = lane; j < dh; j += 32) T[__ldg(rcols + hb + j) >> 5] = 0u;
     __syncwarp();
+  }
+  warp_add_count(total, out);
+}
+
+// The edges tested as words: a warp per row u, its ids below 2^15 as a bitmap in shared memory,
+// ANDed with the bitmap rows of its targets.  Eight lanes take a target, 16 bytes a lane and four
+// loads in flight; the row ascends, so the four targets under way have about as many pieces.  Bits of u
+// from v on meet no bit of N+(v).  The bitmap rows take 64 MB at most and stay in L2: bound by issue
+// (72 % of peak at scale 20, L1 66 %, DRAM 2 %).  A target's bitmap against the sources' rows instead
+// had 192 MB of them to read, at 8 TB/s, and needed entries: 42.9 ms at R-MAT scale 24 to 40.0.
+__global__ void __launch_bounds__(256) rank_words_kernel(const int64_t* __restrict__ roff,
+                                                         const int32_t* __restrict__ rcols,
+                                                         const uint4* __restrict__ dense, int rows, int sources, int* next,
+                                                         const int* too_long, unsigned long long* out) {
+  __shared__ __align__(16) uint32_t smem[8][1 << 10];
+  __shared__ int32_t lists[8][32];
+  const int lane = threadIdx.x & 31, sub = lane & 7, grp = lane >> 3;
+  int32_t* list = lists[threadIdx.x >> 5];
+  uint32_t* T = smem[threadIdx.x >> 5];
+  const uint4* T4 = reinterpret_cast<const uint4*>(T);
+  for (int j = lane; j < (1 << 10); j += 32) T[j] = 0u;
+  __syncwarp();
+  if (*too_long) return;  // an unsorted row's prefix is no prefix
+  unsigned long long total = 0;
+  for (;;) {
+    int u = 0;
+    if (lane == 0) u = atomicAdd(next, 1);
+    u = __shfl_sync(0xffffffffu, u, 0);
+    if (u >= sources) break;
+    const int64_t b = __ldg(roff + u);
+    const int du = (int)(__ldg(roff + u + 1) - b);
+    bool filled = false;
+    unsigned cnt = 0;
+    for (int j0 = 0; j0 < du; j0 += 32) {
+      const int32_t v = j0 + lane < du ? __ldg(rcols + b + j0 + lane) : rows;
+      unsigned left = __ballot_sync(0xffffffffu, v < rows && words_pay((uint32_t)(j0 + lane), (uint32_t)v));
+      if (left && !filled) {
+        for (int j = lane; j < du; j += 32) {
+          const int32_t x = __ldg(rcols + b + j);
+          if (x < (1 << 15)) atomicOr(&T[x >> 5], 1u << (x & 31));
+        }
+        __syncwarp();
+        filled = true;
+      }
+      const int nt = __popc(left);
+      if ((left >> lane) & 1u) list[__popc(left & ((1u << lane) - 1))] = v;
+      __syncwarp();
+      for (int k = 0; k < nt; k += 4) {
+        const uint32_t x = (uint32_t)list[min(k + grp, nt - 1)];
+        const int most = (list[min(k + 3, nt - 1)] >> 7) + 1;  // of the four, which ascend
+        const int pieces = k + grp < nt ? (int)(x >> 7) + 1 : 0;
+        const uint4* row = dense + dense_start(x) + sub;
+        for (int p = 0; p < most; p += 32) {
+          uint4 d[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (p + 8 * q < most)
+              d[q] = p + 8 * q + sub < pieces ? __ldg(row + p + 8 * q) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (p + 8 * q < most) {
+              const uint4 m = T4[p + 8 * q + sub];
+              cnt += __popc(d[q].x & m.x) + __popc(d[q].y & m.y) + __popc(d[q].z & m.z) + __popc(d[q].w & m.w);
+            }
+        }
+      }
+      __syncwarp();
+      if (__shfl_sync(0xffffffffu, v, 31) >= rows) break;  // ascending
+    }
+    total += cnt;
+    if (filled) {
+      __syncwarp();
+      for (int j = lane; j < du; j += 32) {
+        const int32_t x = __ldg(rcols + b + j);
+        if (x < (1 << 15)) T[x >> 5] = 0u;
+      }
+      __syncwarp();
+    }
   }
   warp_add_count(total, out);
 }
@@ -606,6 +735,9 @@ atc_status build_ranked(const atc_csr* csr, bool bitmaps, RankedCopy* rc, cudaSt
   // with bitmaps few targets are left for lists, and they have few entries
   const int warp_chunk = bitmaps ? kWarpChunk : chunk, block_chunk = bitmaps ? kBlockChunk : 4 * chunk;
   const int64_t lcap = !bitmaps || n > kRank16 ? max_items(n, m, std::min(warp_chunk, block_chunk)) : 0;
+  // Bitmaps of rows take no more room than the ids once more: rows^2 / 16 against 4 m bytes.
+  int rows = 0, sources = 0;
+  if (bitmaps) rows = (int)std::min<double>(8.0 * std::sqrt((double)m), (double)std::min<int64_t>(n, kDenseRows));
   Arena ar;
   const size_t a_ka = ar.add<uint64_t>(n), a_kb = ar.add<uint64_t>(n);
   const size_t a_tmp = ar.add<char>(std::max(sort_tmp, scan_tmp));
@@ -621,9 +753,14 @@ atc_status build_ranked(const atc_csr* csr, bool bitmaps, RankedCopy* rc, cudaSt
                a_19 = ar.add<int2>(cap19), a_list = ar.add<int2>(lcap);
   const size_t a_pieces = ar.add<int32_t>(bitmaps ? n + 1 : 0), a_roff8 = ar.add<int64_t>(bitmaps ? n + 1 : 0);
   const size_t a_r16 = ar.add<uint16_t>(bitmaps ? m + 8 * std::min(n, m) : 0);
-  if (rc->mem.alloc(ar.bytes, s) != ATC_OK) {  // no room for the copy: the caller counts in place
+  const size_t plain = ar.bytes, a_dense = ar.add<uint4>(rows ? dense_start(rows) : 0);
+  if (rc->mem.alloc(ar.bytes, s) != ATC_OK) {
     cudaGetLastError();
-    return ATC_OK;
+    rows = 0;
+    if (rc->mem.alloc(plain, s) != ATC_OK) {  // no room for the copy: the caller counts in place
+      cudaGetLastError();
+      return ATC_OK;
+    }
   }
   char* p = rc->mem.p;
   uint64_t* ka = reinterpret_cast<uint64_t*>(p + a_ka);
@@ -633,6 +770,7 @@ atc_status build_ranked(const atc_csr* csr, bool bitmaps, RankedCopy* rc, cudaSt
   int32_t* deg = reinterpret_cast<int32_t*>(p + a_deg);
   int32_t* cnt = reinterpret_cast<int32_t*>(p + a_cnt);
   int32_t* gcur = reinterpret_cast<int32_t*>(p + a_gcur);
+  uint4* dense = reinterpret_cast<uint4*>(p + a_dense);
   int64_t* roff = reinterpret_cast<int64_t*>(p + a_roff);
   int64_t* gstart = reinterpret_cast<int64_t*>(p + a_gstart);
   int32_t* rcols = reinterpret_cast<int32_t*>(p + a_rcols);
@@ -676,10 +814,16 @@ atc_status build_ranked(const atc_csr* csr, bool bitmaps, RankedCopy* rc, cudaSt
                                                                                                       ctr);
     *launches += 1;
   }
+  if (rows) {
+    sources = (int)std::min<int64_t>(n, (int64_t)kDenseSources * rows);
+    rank_dense_kernel<<<(rows + kDenseWarps - 1) / kDenseWarps, kDenseWarps * 32, 0, s>>>(roff, rcols, rows, dense);
+    *launches += 1;
+  }
   rank_piece_rows_kernel<<<grid_for(n, 256), 256, 0, s>>>(roff, n, piece_row);
   rank_entries_kernel<<<grid_for(m, kTile, 2), kEntryThreads, 0, s>>>(roff, n, m, rcols, piece_row, gstart, roff8,
-                                                                        bitmaps ? kRank16 : 0, gcur, r16, ent);
-  rank_items_kernel<<<grid_for(n, 256), 256, 0, s>>>(roff, gstart, n, li, bitmaps, ctr);
+                                                                        bitmaps ? kRank16 : 0, rows, sources, gcur,
+                                                                        r16, ent);
+  rank_items_kernel<<<grid_for(n, 256), 256, 0, s>>>(roff, gstart, gcur, n, li, bitmaps, ctr);
   ATC_CK(cudaGetLastError());
   *launches += 17;
   rc->n = n;
@@ -689,6 +833,10 @@ atc_status build_ranked(const atc_csr* csr, bool bitmaps, RankedCopy* rc, cudaSt
   rc->r16 = reinterpret_cast<const uint4*>(r16);
   rc->gstart = gstart;
   rc->ent = ent;
+  rc->nids = gcur;
+  rc->dense = rows ? dense : nullptr;
+  rc->dense_rows = rows;
+  rc->dense_sources = sources;
   rc->ctr = ctr;
   rc->li = li;
   rc->long_rows = long_rows != 0;
@@ -738,16 +886,23 @@ atc_status count_ranked(const atc_csr* csr, unsigned long long* out, bool* done,
     ATC_CK(cudaGetLastError());
     *launches += 2;
   }
+  if (rc.dense) {
+    rank_words_kernel<<<sm_count() * blocks_per_sm((const void*)rank_words_kernel, 256, 0), 256, 0, s>>>(
+        rc.roff, rc.rcols, rc.dense, rc.dense_rows, rc.dense_sources, ctr + kcNextDense, too, out);
+    ATC_CK(cudaGetLastError());
+    *launches += 1;
+  }
   const bool wide = csr->wedges_min >= kWideMean * m;
   if (n > kRank15) {
     const auto kern = wide ? rank_warp_kernel<1 << 16, 4, 16> : rank_warp_kernel<1 << 16, 4, 8>;
     kern<<<sm_count() * blocks_per_sm((const void*)kern, 128, 0), 128, 0, s>>>(
-        rc.roff, rc.rcols, rc.r16, ent, li.t16, gstart, li.chunk, ctr + kc16, ctr + kcNext16, too, out);
+        rc.roff, rc.rcols, rc.r16, ent, li.t16, gstart, rc.nids, li.chunk, ctr + kc16, ctr + kcNext16, too, out);
     *launches += 1;
   }
-  const auto kern = wide ? rank_warp_kernel<1 << 15, 8, 16> : rank_warp_kernel<1 << 15, 8, 8>;
+  const auto kern =
+      csr->wedges_min >= kWideMean15 * m ? rank_warp_kernel<1 << 15, 8, 8> : rank_warp_kernel<1 << 15, 8, 4>;
   kern<<<sm_count() * blocks_per_sm((const void*)kern, 256, 0), 256, 0, s>>>(
-      rc.roff, rc.rcols, rc.r16, ent, li.t15, gstart, li.chunk, ctr + kc15, ctr + kcNext15, too, out);
+      rc.roff, rc.rcols, rc.r16, ent, li.t15, gstart, rc.nids, li.chunk, ctr + kc15, ctr + kcNext15, too, out);
   ATC_CK(cudaGetLastError());
   *launches += 1;
   int too_long = 0;

@@ -8,7 +8,7 @@ namespace atc {
 
 // counters of one copy; the first six are the kinds of work items
 enum { kc15, kc16, kc17, kc19, kcWarp, kcBlock, kcNext15, kcNext16, kcNext17, kcNext19, kcNextWarp, kcNextBlock, kcMid,
-       kcBig, kcNextMid, kcNextBig, kcTooLong, kcMaxRow, kcError, kcCount };
+       kcBig, kcNextMid, kcNextBig, kcTooLong, kcMaxRow, kcError, kcNextDense, kcCount };
 
 // Work items (target, chunk): the bitmap kinds of ranked.cu, and the targets that take a warp or
 // a CTA with N+(v) as a list (`list`: warp items from the front, CTA items from the back).
@@ -29,6 +29,9 @@ struct RankedCopy {
   const uint4* r16 = nullptr;       // rows of 16-bit ids, starting at multiples of eight
   const int64_t* gstart = nullptr;  // n + 1: the entries of every target
   const uint2* ent = nullptr;       // (row start, prefix length)
+  const int32_t* nids = nullptr;    // n: how many of them a target has; the rest of its edges are tested as words
+  const uint4* dense = nullptr;     // rows of the ranks below dense_rows as bitmaps (null: none)
+  int dense_rows = 0, dense_sources = 0;
   int* ctr = nullptr;               // kcCount
   RankItemLists li{};
   bool long_rows = false;           // rows above the register sorts may exist (ctr[kcTooLong])
