@@ -19,20 +19,20 @@
 //   a long prefix before a target of low rank: the source's and the target's rows as bitmaps, ANDed
 //   word by word, 128 candidates per 16 bytes against eight ids; such edges need no entry.  Other
 //   targets of rank below 2^16: a warp per chunk of entries, its own bitmap of 4 or 8 KB, rows
-//   read as 16-bit ids; below 2^17 with enough entries: a CTA of four warps per chunk, a bitmap
-//   of 16 KB; the rest (a tenth of the tests at R-MAT scale 24): the hash kernels of bisson.cuh
-//   over the same entries, or a CTA's 64 KB bitmap for rows too long for a warp's table.
+//   read as 16-bit ids; the rest (a quarter of the tests at R-MAT scale 24): a warp's bitmap that is
+//   exact for low ids and a filter for the others, or, with many entries, a CTA's of 16 KB.
 //
 // Measured (R-MAT scale 24, A-direction + A-order; whole lists grouped at the longer endpoint ->
-// this path): 117.5 -> 40.0 ms, of which the passes take 12.8 ms (entries 4.9, group sizes 2.3,
-// row sorts 3.1, rows 1.4) and the count 27.1: words 4, other ranks below 2^15 6, 2^16 5.5, 2^17 3.2,
-// hash 9.2.  Without the words the ranks below 2^15 took 15.7 and the entries 5.7 (47.1 in all):
+// this path): 117.5 -> 37.5 ms, of which the passes take 12.8 ms (entries 4.9, group sizes 2.3,
+// row sorts 3.1, rows 1.4) and the count 24.6: words 4, other ranks below 2^15 5, 2^16 5.5, 2^17 3.2,
+// the filter 6.7.  Without the words the ranks below 2^15 took 15.7 and the entries 5.7 (47.1 in all):
 // bound by the shared and L1 pipe (two wavefronts per 32 tests, one of them bank conflicts) and by
-// issue (10 warp instructions per 32 tests).  Scale 22: 8.6 -> 7.0 ms by the words, scale 20: 1.86 ->
-// 1.47 (4.45 by whole lists); Chung-Lu n = 700 001, which has few dense rows: 1.30 -> 1.26.
+// issue (10 warp instructions per 32 tests).  Scale 22: 8.6 -> 6.5 ms, scale 20: 1.86 ->
+// 1.46 (4.45 by whole lists); Chung-Lu n = 700 001, which has few dense rows: 1.30 -> 1.25.
 // Tried: 32-bit rows and one entry a warp at a time 68 ms; 32-lane scans of short prefixes
 // instead of lane groups 88 ms; rows on 128-byte lines 1-4 % for twice the copy.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 
 #include "ranked.cuh"
@@ -46,14 +46,14 @@ constexpr int kHubEntry = 1024;         // ranks whose group cursors are reserve
 constexpr int kTile = 4096;             // edges per tile of the entry pass
 constexpr int kRank15 = (1 << 15) - 1;  // targets below: a warp's bitmap of 4 KB
 constexpr int kRank16 = (1 << 16) - 1;  // below: a warp's bitmap of 8 KB; ids in 16 bits
-constexpr int kRank17 = 1 << 17;        // below, with entries: a small CTA's bitmap of 16 KB
-constexpr int kRank19 = kTabWords * 32; // below, with a row too long for a warp's hash table: 64 KB
+constexpr int kRank17 = 1 << 17;        // below, with entries, on wide graphs: a small CTA's bitmap of 16 KB
 constexpr int kRankBlockChunk = 1024;   // entries per CTA item
-constexpr int kRankMidMin = 24;         // fewer entries than these do not pay for a CTA's bitmap
-constexpr int kRankBlockMin = 48;
+constexpr int kRankMidMin = 96;         // fewer entries than these do not pay for a CTA's bitmap
 // Lanes that read a prefix, by the mean of min(d+u, d+v).  Targets below 2^15, whose long prefixes are
 // words: four, from kWideMean15 eight (R-MAT scale 20, mean 132: 1.47 and 1.51 ms; scale 22, 187: 7.1 and
-// 7.0; scale 24, 270: 41.0 and 40.2; Chung-Lu 1.26 and 1.31).  Below 2^16: eight, from kWideMean 16.
+// 7.0; scale 24, 270: 41.0 and 40.2; Chung-Lu 1.26 and 1.31); the filter likewise.  Targets below 2^16:
+// eight, from kWideMean 16; from there too, targets below 2^17 take a CTA's bitmap (scale 24: 37.5 ms,
+// 38.5 with the filter; scale 22: 6.7 and 6.5).
 constexpr int64_t kWideMean15 = 160, kWideMean = 224;
 constexpr int kDenseRows = 1 << 15;     // rows that may be kept as bitmaps
 constexpr int kDenseSources = 4;        // times as many rows are looked at for targets among them
@@ -399,12 +399,9 @@ __global__ void rank_items_kernel(const int64_t* roff, const int64_t* gstart, co
                      : !bitmaps ? (dv <= li.warp_max ? kcWarp : kcBlock)
                      : v < kRank15 ? kc15
                      : v < kRank16 ? kc16
-                     : v < kRank17 && ne >= kRankMidMin ? kc17
-                     : dv <= li.warp_max ? kcWarp  // R-MAT scale 24, ranks 2^17..2^19: 9.2 ms by hash
-                                                   // tables, 21 ms by 64 KB bitmaps a CTA
-                     : v < kRank19 && ne >= kRankBlockMin ? kc19 : kcBlock;
-    const int64_t chunk = kind <= kc16 ? li.chunk : kind <= kc19 ? kRankBlockChunk
-                          : kind == kcWarp ? li.warp_chunk : li.block_chunk;
+                     : v < kRank17 && ne >= li.mid_min ? kc17 : kcFilter;
+    const int64_t chunk = kind == kc17 ? kRankBlockChunk : kind == kcWarp ? li.warp_chunk
+                          : kind == kcBlock ? li.block_chunk : li.chunk;
     const int k = any ? (int)((ne + chunk - 1) / chunk) : 0;
     if (any) longest = max(longest, (int)dv);
 #pragma unroll
@@ -412,7 +409,7 @@ __global__ void rank_items_kernel(const int64_t* roff, const int64_t* gstart, co
       if (!__any_sync(0xffffffffu, kind == q)) continue;
       const int at = warp_reserve(&ctr[q], kind == q ? k : 0);
       if (kind != q) continue;
-      int2* to = q == kc15 ? li.t15 : q == kc16 ? li.t16 : q == kc17 ? li.t17 : q == kc19 ? li.t19 : li.list;
+      int2* to = q == kc15 ? li.t15 : q == kc16 ? li.t16 : q == kc17 ? li.t17 : q == kcFilter ? li.filter : li.list;
       for (int c = 0; c < k; ++c)
         to[q == kcBlock ? li.lcap - 1 - (at + c) : (int64_t)(at + c)] = make_int2((int32_t)v, c);
     }
@@ -658,14 +655,161 @@ __global__ void __launch_bounds__(256) rank_words_kernel(const int64_t* __restri
   warp_add_count(total, out);
 }
 
-// Targets of larger rank: a CTA per chunk of entries, ids in 32 bits.
-template <int THREADS>
-__global__ void __launch_bounds__(THREADS) rank_block_kernel(CsrView g, const uint2* __restrict__ ent,
-                                                             const int2* __restrict__ items,
-                                                             const int64_t* __restrict__ gstart, uint32_t words,
-                                                             const int* nitems_dev, int* next, const int* too_long,
-                                                             unsigned long long* out) {
-  extern __shared__ __align__(16) uint32_t T[];  // words
+// Targets of larger rank: a warp per chunk of entries.  Ids below 2^14 have a bit each in the first
+// half of the warp's table, the others share the bits of the second half by their low 14 bits: a
+// hit there is kept on the lane's stack and looked up in the list N+(v) when a stack fills.
+// Groups of kLanes lanes read a prefix, four ids a lane from the 16-byte line they lie in; ids
+// outside the prefix are masked off by position.  Bound by latency (a few dozen lines per item,
+// then the next): what pays are warps in flight and the next item's header loaded early.  Halves of
+// 2^15 bits, six CTAs per SM instead of nine: 42.2 against 38.5 ms at R-MAT scale 24; of 2^13 39.7; eleven
+// CTAs with fewer registers, or stacks of 12 and 16: 1 ms more.  Hash tables of N+(v) instead of all
+// of this (31 instructions per 32 tests): 39.7 against 37.5 at scale 24, 7.0 and 6.5 at scale 22,
+// Chung-Lu n = 4 M 6.6 and 6.3.
+constexpr int kStack = 8;
+constexpr int kLowBits = 14;
+template <int WARPS, int kLanes>
+__global__ void __launch_bounds__(WARPS * 32, 9) rank_filter_kernel(const int64_t* __restrict__ roff,
+                                                                 const int32_t* __restrict__ rcols,
+                                                                 const uint2* __restrict__ ent,
+                                                                 const int2* __restrict__ items,
+                                                                 const int64_t* __restrict__ gstart, int chunk,
+                                                                 const int* nitems_dev, int* next, const int* too_long,
+                                                                 unsigned long long* out) {
+  constexpr uint32_t kHalf = (1u << kLowBits) / 8, kBytes = 2 * kHalf;
+  __shared__ __align__(16) unsigned char smem[WARPS * kBytes];
+  __shared__ int32_t stacks[WARPS][kStack][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const uint32_t base = w * kBytes;
+  const uint4* ids = reinterpret_cast<const uint4*>(rcols);
+  uint32_t* T = reinterpret_cast<uint32_t*>(smem + base);
+  for (int j = lane; j < (int)(kBytes / 4); j += 32) T[j] = 0u;
+  __syncwarp();
+  const int nitems = *too_long ? 0 : *nitems_dev;  // an unsorted row's prefix is no prefix
+  const int sub = lane % kLanes;
+  // byte of id x's word
+  auto place = [&](uint32_t x) {
+    return ((x >> 3) & (kHalf - 4)) + (x >> kLowBits ? base + kHalf : base);
+  };
+  auto word = [&](uint32_t x) { return *reinterpret_cast<uint32_t*>(smem + place(x)); };
+  struct Head {
+    int32_t v;
+    int ne, dh;
+    int64_t g0, hb;
+  };
+  auto head = [&]() {
+    int it = 0;
+    if (lane == 0) it = atomicAdd(next, 1);
+    it = __shfl_sync(0xffffffffu, it, 0);
+    Head h{-1, 0, 0, 0, 0};
+    if (it < nitems) {
+      const int2 c = __ldg(items + it);
+      h.v = c.x;
+      h.g0 = __ldg(gstart + c.x) + (int64_t)c.y * chunk;
+      h.ne = (int)min(__ldg(gstart + c.x + 1) - h.g0, (int64_t)chunk);
+      h.hb = __ldg(roff + c.x);
+      h.dh = (int)(__ldg(roff + c.x + 1) - h.hb);
+    }
+    return h;
+  };
+  unsigned long long total = 0;
+  Head nh = head();
+  while (nh.v >= 0) {
+    const int ne = nh.ne, dh = nh.dh;
+    const uint2* en = ent + nh.g0;
+    const int64_t hb = nh.hb;
+    nh = head();  // the next item's loads run under this one's
+    int i = lane / kLanes;
+    uint2 nq = i < ne ? __ldg(en + i) : make_uint2(0u, 0u);
+    for (int j = lane; j < dh; j += 32) {
+      const uint32_t x = (uint32_t)__ldg(rcols + hb + j);
+      atomicOr(reinterpret_cast<uint32_t*>(smem + place(x)), 0x80000000u >> (x & 31));
+    }
+    __syncwarp();
+    uint32_t at = 0;  // the lane's next line
+    int left = 0;     // ids from its start to the end of the group's prefix
+    int skip = 0;     // ids of it before the prefix
+    unsigned cnt = 0;
+    int sp = 0;
+    // loads the lane's next line; returns its ids that count, the first as bit 3
+    auto fetch = [&](uint4& d) -> unsigned {
+      if (left + 4 * sub <= 0 && i < ne) {  // the group's prefix is done
+        at = (nq.x >> 2) + sub;
+        skip = (int)(nq.x & 3u);
+        left = (int)nq.y + skip - 4 * sub;
+        if (sub) skip = 0;
+        i += 32 / kLanes;
+        if (i < ne) nq = __ldg(en + i);
+      }
+      unsigned valid = 0;
+      d = make_uint4(0u, 0u, 0u, 0u);
+      if (left > 0) {
+        d = __ldg(ids + at);
+        valid = (0xf0u >> min(left, 4)) & (0xfu >> skip);
+      }
+      at += kLanes;
+      left -= 4 * kLanes;
+      skip = 0;
+      return valid;
+    };
+    auto tests = [&](const uint4& d, unsigned valid) {
+      const uint32_t b0 = word(d.x), b1 = word(d.y), b2 = word(d.z), b3 = word(d.w);
+      auto fold = [](uint32_t acc, uint32_t b, uint32_t r) {
+        return __funnelshift_l(__funnelshift_l(b, b, r), acc, 1);
+      };
+      const unsigned hit = fold(fold(fold(fold(0u, b0, d.x), b1, d.y), b2, d.z), b3, d.w) & valid;
+      const unsigned high = hit & ((d.x >> kLowBits ? 8u : 0u) | (d.y >> kLowBits ? 4u : 0u) | (d.z >> kLowBits ? 2u : 0u) |
+                                  (d.w >> kLowBits ? 1u : 0u));
+      cnt += __popc(hit ^ high);
+      if (high) {
+        auto push = [&](unsigned bit, uint32_t x) {
+          if (high & bit) stacks[w][sp++][lane] = (int32_t)x;
+        };
+        push(8u, d.x);
+        push(4u, d.y);
+        push(2u, d.z);
+        push(1u, d.w);
+      }
+    };
+    auto settle = [&]() {
+      const int most = __reduce_max_sync(0xffffffffu, sp);
+      for (int k = 0; k < most; ++k)
+        if (k < sp) {
+          const int32_t x = stacks[w][k][lane];
+          int a = 0, b = dh;  // the first id not below x
+          while (a < b) {
+            const int mid = (a + b) >> 1;
+            if (__ldg(rcols + hb + mid) < x) a = mid + 1; else b = mid;
+          }
+          cnt += a < dh && __ldg(rcols + hb + a) == x;
+        }
+      sp = 0;
+    };
+    uint4 d0, d1;
+    unsigned v0 = fetch(d0), v1;
+    do {
+      v1 = fetch(d1);
+      tests(d0, v0);
+      if (__any_sync(0xffffffffu, sp > kStack - 4)) settle();
+      v0 = fetch(d0);
+      tests(d1, v1);
+      if (__any_sync(0xffffffffu, sp > kStack - 4)) settle();
+    } while (__any_sync(0xffffffffu, v0 != 0 || left > 0 || i < ne));
+    settle();
+    total += cnt;
+    __syncwarp();
+    for (int j = lane; j < dh; j += 32) *reinterpret_cast<uint32_t*>(smem + place((uint32_t)__ldg(rcols + hb + j))) = 0u;
+    __syncwarp();
+  }
+  warp_add_count(total, out);
+}
+
+// Targets below kRank17 with many entries on wide graphs: a CTA per chunk of them, ids in 32 bits.
+__global__ void __launch_bounds__(128) rank_block_kernel(CsrView g, const uint2* __restrict__ ent,
+                                                         const int2* __restrict__ items,
+                                                         const int64_t* __restrict__ gstart, const int* nitems_dev,
+                                                         int* next, const int* too_long, unsigned long long* out) {
+  constexpr uint32_t words = kRank17 / 32;
+  __shared__ __align__(16) uint32_t T[words];
   __shared__ int item;
   __shared__ unsigned long long bnext;
   const int lane = threadIdx.x & 31;
@@ -730,11 +874,10 @@ atc_status build_ranked(const atc_csr* csr, bool bitmaps, RankedCopy* rc, cudaSt
   auto item_cap = [&](int64_t below, int64_t per) { return std::min<int64_t>(n, below) + m / per + 1; };
   const int64_t cap15 = bitmaps ? item_cap(kRank15, chunk) : 0;
   const int64_t cap16 = bitmaps && n > kRank15 ? item_cap(kRank16, chunk) : 0;
-  const int64_t cap17 = bitmaps && n > kRank16 ? item_cap(kRank17, kRankBlockChunk) : 0;
-  const int64_t cap19 = bitmaps && n > kRank17 ? item_cap(kRank19, kRankBlockChunk) : 0;
-  // with bitmaps few targets are left for lists, and they have few entries
-  const int warp_chunk = bitmaps ? kWarpChunk : chunk, block_chunk = bitmaps ? kBlockChunk : 4 * chunk;
-  const int64_t lcap = !bitmaps || n > kRank16 ? max_items(n, m, std::min(warp_chunk, block_chunk)) : 0;
+  const bool wide = csr->wedges_min >= kWideMean * m;
+  const int64_t cap17 = bitmaps && wide && n > kRank16 ? item_cap(kRank17, kRankBlockChunk) : 0;
+  const int64_t cap_filter = bitmaps && n > kRank16 ? item_cap(n, chunk) : 0;
+  const int64_t lcap = !bitmaps ? max_items(n, m, chunk) : 0;
   // Bitmaps of rows take no more room than the ids once more: rows^2 / 16 against 4 m bytes.
   int rows = 0, sources = 0;
   if (bitmaps) rows = (int)std::min<double>(8.0 * std::sqrt((double)m), (double)std::min<int64_t>(n, kDenseRows));
@@ -750,7 +893,7 @@ atc_status build_ranked(const atc_csr* csr, bool bitmaps, RankedCopy* rc, cudaSt
   const size_t a_rcols = ar.add<int32_t>(m + 16), a_ent = ar.add<uint2>(m), a_piece = ar.add<int32_t>((m >> 5) + 1);
   const size_t a_mid = ar.add<int32_t>(m / 33 + 1), a_big = ar.add<int32_t>(m / (kRankWarpRow + 1) + 1);
   const size_t a_15 = ar.add<int2>(cap15), a_16 = ar.add<int2>(cap16), a_17 = ar.add<int2>(cap17),
-               a_19 = ar.add<int2>(cap19), a_list = ar.add<int2>(lcap);
+               a_filter = ar.add<int2>(cap_filter), a_list = ar.add<int2>(lcap);
   const size_t a_pieces = ar.add<int32_t>(bitmaps ? n + 1 : 0), a_roff8 = ar.add<int64_t>(bitmaps ? n + 1 : 0);
   const size_t a_r16 = ar.add<uint16_t>(bitmaps ? m + 8 * std::min(n, m) : 0);
   const size_t plain = ar.bytes, a_dense = ar.add<uint4>(rows ? dense_start(rows) : 0);
@@ -783,9 +926,9 @@ atc_status build_ranked(const atc_csr* csr, bool bitmaps, RankedCopy* rc, cudaSt
   int64_t* roff8 = reinterpret_cast<int64_t*>(p + a_roff8);
   uint16_t* r16 = reinterpret_cast<uint16_t*>(p + a_r16);
   const RankItemLists li{reinterpret_cast<int2*>(p + a_15), reinterpret_cast<int2*>(p + a_16),
-                         reinterpret_cast<int2*>(p + a_17), reinterpret_cast<int2*>(p + a_19),
-                         reinterpret_cast<int2*>(p + a_list), lcap, chunk, warp_chunk, block_chunk,
-                         bitmaps ? kWarpHashMax : kWarpMax};
+                         reinterpret_cast<int2*>(p + a_17), reinterpret_cast<int2*>(p + a_filter),
+                         reinterpret_cast<int2*>(p + a_list), lcap, chunk, chunk, 4 * chunk, kWarpMax,
+                         wide ? kRankMidMin : INT_MAX};
   ATC_CK(cudaMemsetAsync(p + a_zero, 0, zero_end - a_zero, s));
   rank_keys_kernel<<<grid_for(n, 256), 256, 0, s>>>(csr->offsets, pv->indeg, n, B, db, ka);
   ATC_CK(cudaGetLastError());
@@ -859,32 +1002,19 @@ atc_status count_ranked(const atc_csr* csr, unsigned long long* out, bool* done,
   const uint2* ent = rc.ent;
   int* ctr = rc.ctr;
   const int* too = ctr + kcTooLong;
-  auto block_launch = [&](auto kern, int threads, int64_t bits, const int2* items, int kind, int nxt) -> atc_status {
-    const size_t smem = (size_t)bits / 8;
-    ATC_CK(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<sm_count() * blocks_per_sm((const void*)kern, threads, smem), threads, smem, s>>>(
-        g, ent, items, gstart, (uint32_t)(bits / 32), ctr + kind, ctr + nxt, too, out);
+  const bool wide = csr->wedges_min >= kWideMean * m, wide15 = csr->wedges_min >= kWideMean15 * m;
+  if (n > kRank16) {
+    const auto kern = wide15 ? rank_filter_kernel<4, 8> : rank_filter_kernel<4, 4>;
+    kern<<<sm_count() * blocks_per_sm((const void*)kern, 128, 0), 128, 0, s>>>(
+        rc.roff, rc.rcols, ent, li.filter, gstart, li.chunk, ctr + kcFilter, ctr + kcNextFilter, too, out);
     ATC_CK(cudaGetLastError());
     *launches += 1;
-    return ATC_OK;
-  };
-  if (n > kRank17) ATC_TRY(block_launch(rank_block_kernel<256>, 256, kRank19, li.t19, kc19, kcNext19));
-  if (n > kRank16) {
-    ATC_TRY(block_launch(rank_block_kernel<128>, 128, kRank17, li.t17, kc17, kcNext17));
-    const auto hw = bisson_warp_kernel<RankedItems, kDefaultSlots, PrefixPartners>;
-    const auto hb = bisson_block_kernel<RankedItems, kDefaultSlots, PrefixPartners>;
-    const size_t hsmem = sizeof(int32_t) * kTabWords;
-    ATC_CK(cudaFuncSetAttribute((const void*)hb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsmem));
-    hb<<<sm_count() * blocks_per_sm((const void*)hb, kBgWarps * 32, hsmem), kBgWarps * 32, hsmem, s>>>(
-        g, PrefixPartners{ent}, RankedItems{li.list, gstart, li.lcap, li.block_chunk, true}, 0, ctr + kcBlock,
-        ctr + kcNextBlock,
-        (uint32_t)kTabWords, GraphTags{nullptr, 0, nullptr}, out);
-    hw<<<sm_count() * blocks_per_sm((const void*)hw, kBgWarps * 32, 0), kBgWarps * 32, 0, s>>>(
-        g, PrefixPartners{ent}, RankedItems{li.list, gstart, li.lcap, li.warp_chunk, false}, 0, ctr + kcWarp,
-        ctr + kcNextWarp,
-        GraphTags{nullptr, 0, nullptr}, out);
-    ATC_CK(cudaGetLastError());
-    *launches += 2;
+    if (wide) {
+      rank_block_kernel<<<sm_count() * blocks_per_sm((const void*)rank_block_kernel, 128, 0), 128, 0, s>>>(
+          g, ent, li.t17, gstart, ctr + kc17, ctr + kcNext17, too, out);
+      ATC_CK(cudaGetLastError());
+      *launches += 1;
+    }
   }
   if (rc.dense) {
     rank_words_kernel<<<sm_count() * blocks_per_sm((const void*)rank_words_kernel, 256, 0), 256, 0, s>>>(
@@ -892,15 +1022,13 @@ atc_status count_ranked(const atc_csr* csr, unsigned long long* out, bool* done,
     ATC_CK(cudaGetLastError());
     *launches += 1;
   }
-  const bool wide = csr->wedges_min >= kWideMean * m;
   if (n > kRank15) {
     const auto kern = wide ? rank_warp_kernel<1 << 16, 4, 16> : rank_warp_kernel<1 << 16, 4, 8>;
     kern<<<sm_count() * blocks_per_sm((const void*)kern, 128, 0), 128, 0, s>>>(
         rc.roff, rc.rcols, rc.r16, ent, li.t16, gstart, rc.nids, li.chunk, ctr + kc16, ctr + kcNext16, too, out);
     *launches += 1;
   }
-  const auto kern =
-      csr->wedges_min >= kWideMean15 * m ? rank_warp_kernel<1 << 15, 8, 8> : rank_warp_kernel<1 << 15, 8, 4>;
+  const auto kern = wide15 ? rank_warp_kernel<1 << 15, 8, 8> : rank_warp_kernel<1 << 15, 8, 4>;
   kern<<<sm_count() * blocks_per_sm((const void*)kern, 256, 0), 256, 0, s>>>(
       rc.roff, rc.rcols, rc.r16, ent, li.t15, gstart, rc.nids, li.chunk, ctr + kc15, ctr + kcNext15, too, out);
   ATC_CK(cudaGetLastError());

@@ -7,18 +7,20 @@
 namespace atc {
 
 // counters of one copy; the first six are the kinds of work items
-enum { kc15, kc16, kc17, kc19, kcWarp, kcBlock, kcNext15, kcNext16, kcNext17, kcNext19, kcNextWarp, kcNextBlock, kcMid,
+enum { kc15, kc16, kc17, kcFilter, kcWarp, kcBlock, kcNext15, kcNext16, kcNext17, kcNextFilter, kcNextWarp,
+       kcNextBlock, kcMid,
        kcBig, kcNextMid, kcNextBig, kcTooLong, kcMaxRow, kcError, kcNextDense, kcCount };
 
-// Work items (target, chunk): the bitmap kinds of ranked.cu, and the targets that take a warp or
-// a CTA with N+(v) as a list (`list`: warp items from the front, CTA items from the back).
+// Work items (target, chunk): the kinds of ranked.cu, or, for the searches, the targets that take a
+// warp or a CTA with N+(v) as a list (`list`: warp items from the front, CTA items from the back).
 struct RankItemLists {
-  int2 *t15, *t16, *t17, *t19, *list;
+  int2 *t15, *t16, *t17, *filter, *list;
   int64_t lcap;
-  int chunk;       // entries per warp item of the 15- and 16-bit kinds
+  int chunk;       // entries per warp item of the 15- and 16-bit kinds and the filter
   int warp_chunk;  // and of the list kinds
   int block_chunk;
   int warp_max;    // longest N+(v) of a warp's list item
+  int mid_min;     // fewest entries for which a target of rank below 2^17 takes a CTA's bitmap
 };
 
 struct RankedCopy {

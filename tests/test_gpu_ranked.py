@@ -146,3 +146,21 @@ def test_small_counts(n):
         assert atc.tc(csr, K.HU, tuning={"bisson_slots": 2})[0] == want
         assert atc.tc(csr, K.AUTO)[0] == want
         csr.free()
+
+
+@pytest.mark.parametrize("cliques,size", [(20000, 9), (4000, 50), (1400, 97), (300, 260), (110, 700)])
+def test_targets_of_large_rank(cliques, size):
+    """Disjoint cliques on scattered ids, joined in a path: rows of every alignment, members that share
+    a bit of the filter, more of them in one item than a stack holds, mean lists on both sides of
+    the lane and CTA rules."""
+    n = cliques * size
+    assert n > 1 << 16
+    i, j = torch.triu_indices(size, size, 1, device="cuda")
+    first = torch.arange(cliques, device="cuda") * size
+    e = torch.stack([(first[:, None] + i).flatten(), (first[:, None] + j).flatten()], 1)
+    link = torch.stack([first[:-1], first[1:] + size - 1], 1)  # closes no triangle
+    perm = torch.randperm(n, generator=torch.Generator().manual_seed(size)).cuda()
+    pairs = perm[torch.cat([e, link])].to(torch.int32).contiguous()
+    csr = _device(pairs, atc.Dir.ADIRECTION)
+    assert atc.tc(csr, K.BISSON)[0] == cliques * comb(size, 3)
+    csr.free()
