@@ -544,7 +544,7 @@ __global__ void __launch_bounds__(WARPS * 32) rank_warp_kernel(const int64_t* __
     }
     __syncwarp();
     uint32_t at = 0;  // the lane's next piece
-    int left = 0;     // ids from the lane's next piece to the end of the group's prefix
+    int left = -8 * sub;  // ids from the lane's next piece to the end of the group's prefix
     unsigned cnt = 0;
     // loads the lane's next piece; returns its valid ids (<= 0: none)
     auto fetch = [&](uint4& d) -> int {
@@ -726,7 +726,7 @@ __global__ void __launch_bounds__(WARPS * 32, 9) rank_filter_kernel(const int64_
     }
     __syncwarp();
     uint32_t at = 0;  // the lane's next line
-    int left = 0;     // ids from its start to the end of the group's prefix
+    int left = -4 * sub;  // ids from its start to the end of the group's prefix
     int skip = 0;     // ids of it before the prefix
     unsigned cnt = 0;
     int sp = 0;
