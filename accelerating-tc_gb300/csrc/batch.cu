@@ -202,6 +202,217 @@ extern "C" atc_status atc_batch_destroy(atc_batch* b) try {
 namespace atc {
 namespace {
 
+// Rows items: a warp per chunk of row u's members, whose lists are tested against N+(u), held in
+// 4 KB of shared memory per warp.  The ids of a graph are consecutive, which makes three forms of it:
+//   - up to 2^15 vertices: a bit per id;
+//   - more: 1024 words of four 8-bit tags, or three of 10 or two of 16 where the graph's ids need
+//     them.  The word is id + (id / 1024 + 1) * odd mod 1024 and the tag id / 1024 + 1 (ids from the
+//     graph's first), which together name the id;
+//   - rows of which more members share a word than it has tags (and graphs above 2^26 vertices): a bit
+//     by the low 15 bits of the id, and the members among the hits looked up in the list, from a stack
+//     per lane.
+// Groups of kLanes lanes read a list, four ids a lane from the 16-byte line they lie in; ids
+// outside the list are masked off by position.
+// The lists are short (20 ids in the mean), so what counts is that the groups stay busy: the warp
+// loads 32 members' list bounds at once and a group whose list is done takes the next.  48 Chung-Lu
+// graphs, 25 M edges, 9e8 tests: hash tables and 32 elements a round 2.95 ms; this with members dealt
+// out in advance and every hit looked up 2.33, dealt out in turn 2.17 (8 lanes 2.22, 2 lanes 2.45), with
+// tags 1.75 (1.34 if no hit had to be told from a shared bit).  Bound by issue.
+constexpr int kRowsChunk = 64;  // members an item: one row's members, so the longest rows set the tail
+constexpr int kRowsLanes = 4;
+constexpr int kRowStack = 12;
+template <int kLanes>
+__global__ void __launch_bounds__(128, 9) rows_kernel(CsrView g, CompactItems items, const int* nitems_dev, int* next,
+                                                      GraphTags tags) {
+  constexpr uint32_t kBytes = 1 << 12;
+  __shared__ __align__(16) unsigned char smem[4 * kBytes];
+  __shared__ int32_t stacks[4][kRowStack][32];
+  __shared__ GraphAccSlot acc[4];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const uint32_t base = w * kBytes;
+  const uint4* ids = reinterpret_cast<const uint4*>(g.cols);
+  uint32_t* T = reinterpret_cast<uint32_t*>(smem + base);
+  for (int j = lane; j < (int)(kBytes / 4); j += 32) T[j] = 0u;
+  graph_acc_init(&acc[w]);
+  const int nitems = *nitems_dev;
+  const int sub = lane % kLanes;
+  auto word = [&](uint32_t x) {
+    return reinterpret_cast<uint32_t*>(smem + (((x >> 3) & (kBytes - 4)) | base));
+  };
+  int it = 0, it_end = 0;
+  auto take = [&]() {
+    if (it == it_end) {
+      int first = 0;
+      if (lane == 0) first = atomicAdd(next, kWarpGrab);
+      it = __shfl_sync(0xffffffffu, first, 0);
+      it_end = it + kWarpGrab;
+    }
+    return it < nitems ? items.get(g, it++) : GroupItem{-1, 0, 0, 0};
+  };
+  GroupItem ni = take();
+  while (ni.h >= 0) {
+    const GroupItem gi = ni;
+    const int64_t hb = __ldg(g.off + gi.h);
+    const int dh = (int)(__ldg(g.off + gi.h + 1) - hb);
+    ni = take();  // the next item's loads run under this one's
+    if (dh < 2) continue;
+    graph_acc_enter(tags, &acc[w], gi.h);
+    const int size = acc[w].hi - acc[w].lo;
+    const bool exact = size <= (1 << 15);
+    // four times (id - the graph's first + 1024)
+    const uint32_t shift4 = 4u * (1024u - (uint32_t)acc[w].lo);
+    auto tag_word = [&](uint32_t x4, uint32_t tag) {
+      return reinterpret_cast<uint32_t*>(smem + (((x4 + tag * (4u * 661u)) & (kBytes - 4)) | base));
+    };
+    // tags of `bits` bits: one in each field, and each field's top bit
+    const int bits = size <= 255 << 10 ? 8 : size <= 1023 << 10 ? 10 : 16;
+    const uint32_t ones = bits == 8 ? 0x01010101u : bits == 10 ? 0x00100401u : 0x00010001u;
+    const uint32_t tops = ones << (bits - 1);
+    bool tagged = !exact && size <= 65535 << 10;
+    const int ne = (int)(gi.e - gi.b);
+    const int32_t* en = g.cols + gi.b;
+    if (tagged) {
+      bool full = false;
+      for (int j = lane; j < dh; j += 32) {
+        const uint32_t x4 = 4u * (uint32_t)__ldg(g.cols + hb + j) + shift4, tag = x4 >> 12;
+        uint32_t* at = tag_word(x4, tag);
+        uint32_t old = 0;
+        for (int k = 0;;) {  // into the first free field, counting from the low end
+          if (k + bits > 32) {
+            full = true;
+            break;
+          }
+          if (old >> k & ((1u << bits) - 1)) {
+            k += bits;
+            continue;
+          }
+          const uint32_t seen = atomicCAS(at, old, old | tag << k);
+          if (seen == old) break;
+          old = seen;
+        }
+      }
+      if (__any_sync(0xffffffffu, full)) {
+        for (int j = lane; j < dh; j += 32) {
+          const uint32_t x4 = 4u * (uint32_t)__ldg(g.cols + hb + j) + shift4;
+          *tag_word(x4, x4 >> 12) = 0u;
+        }
+        tagged = false;
+      }
+      __syncwarp();
+    }
+    if (!tagged)
+      for (int j = lane; j < dh; j += 32) {
+        const uint32_t x = (uint32_t)__ldg(g.cols + hb + j);
+        atomicOr(word(x), 0x80000000u >> (x & 31));
+      }
+    __syncwarp();
+    // 32 members' lists at a time, one per lane: first line, and ids from its start to the list's end
+    // (times four, plus those before the list)
+    uint32_t line = 0, span = 0;
+    int from = 0, lim = 0, given = 0;  // next members to load; lists loaded, and handed out
+    uint32_t at = 0;  // the lane's next line
+    int left = -4 * sub;  // ids from its start to the end of the group's list
+    int skip = 0;     // ids of it before the list
+    unsigned cnt = 0;
+    int sp = 0;
+    // Loads the lane's next line; returns its ids that count, the first as bit 3.  Groups whose list
+    // is done take the next ones in turn, so that lists of uneven lengths keep all of them busy.
+    auto fetch = [&](uint4& d) -> unsigned {
+      const bool need = left + 4 * sub <= 0;
+      const unsigned groups = __ballot_sync(0xffffffffu, need && sub == 0);
+      if (groups) {
+        if (given >= lim && from < ne) {
+          span = 0;
+          if (from + lane < ne) {
+            const int32_t v = __ldg(en + from + lane);
+            const int64_t b = __ldg(g.off + v), e = __ldg(g.off + v + 1);
+            line = (uint32_t)(b >> 2);
+            if (e > b) span = (uint32_t)(e - (b & ~3ll)) << 2 | (uint32_t)(b & 3);
+          }
+          lim = min(ne - from, 32);
+          from += 32;
+          given = 0;
+        }
+        const int k = given + __popc(groups & ((1u << (lane - sub)) - 1));
+        const uint32_t l = __shfl_sync(0xffffffffu, line, k), sk = __shfl_sync(0xffffffffu, span, k);
+        if (need) {
+          const bool some = k < lim;
+          at = l + sub;
+          skip = some && sub == 0 ? (int)(sk & 3u) : 0;
+          left = (some ? (int)(sk >> 2) : 0) - 4 * sub;
+        }
+        given = min(given + __popc(groups), lim);
+      }
+      unsigned valid = 0;
+      d = make_uint4(0u, 0u, 0u, 0u);
+      if (left > 0) {
+        d = __ldg(ids + at);
+        valid = (0xf0u >> min(left, 4)) & (0xfu >> skip);
+      }
+      at += kLanes;
+      left -= 4 * kLanes;
+      skip = 0;
+      return valid;
+    };
+    auto tests = [&](const uint4& d, unsigned valid) {
+      if (tagged) {
+        auto in = [&](uint32_t x) {
+          const uint32_t x4 = 4u * x + shift4, tag = x4 >> 12, y = *tag_word(x4, tag) ^ tag * ones;
+          return ((y - ones) & ~y & tops) != 0;  // a field of zeros
+        };
+        cnt += __popc(valid & ((in(d.x) ? 8u : 0u) | (in(d.y) ? 4u : 0u) | (in(d.z) ? 2u : 0u) | (in(d.w) ? 1u : 0u)));
+        return;
+      }
+      const uint32_t b0 = *word(d.x), b1 = *word(d.y), b2 = *word(d.z), b3 = *word(d.w);
+      auto fold = [](uint32_t a, uint32_t b, uint32_t r) { return __funnelshift_l(__funnelshift_l(b, b, r), a, 1); };
+      const unsigned hit = fold(fold(fold(fold(0u, b0, d.x), b1, d.y), b2, d.z), b3, d.w) & valid;
+      if (exact) {
+        cnt += __popc(hit);
+      } else if (hit) {
+        auto push = [&](unsigned bit, uint32_t x) {
+          if (hit & bit) stacks[w][sp++][lane] = (int32_t)x;
+        };
+        push(8u, d.x);
+        push(4u, d.y);
+        push(2u, d.z);
+        push(1u, d.w);
+      }
+    };
+    auto settle = [&]() {
+      const int most = __reduce_max_sync(0xffffffffu, sp);
+      for (int k = 0; k < most; ++k)
+        if (k < sp) {
+          const int32_t x = stacks[w][k][lane];
+          int a = 0, b = dh;  // the first member not below x
+          while (a < b) {
+            const int mid = (a + b) >> 1;
+            if (__ldg(g.cols + hb + mid) < x) a = mid + 1; else b = mid;
+          }
+          cnt += a < dh && __ldg(g.cols + hb + a) == x;
+        }
+      sp = 0;
+    };
+    uint4 d0, d1;
+    unsigned v0 = fetch(d0), v1;
+    do {
+      v1 = fetch(d1);
+      tests(d0, v0);
+      v0 = fetch(d0);
+      tests(d1, v1);
+      if (!exact && !tagged && __any_sync(0xffffffffu, sp > kRowStack - 8)) settle();
+    } while (__any_sync(0xffffffffu, v0 != 0 || left > 0) || given < lim || from < ne);
+    if (!exact && !tagged) settle();
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    if (lane == 0) acc[w].part += cnt;
+    for (int j = lane; j < dh; j += 32) {
+      const uint32_t x = (uint32_t)__ldg(g.cols + hb + j), x4 = 4u * x + shift4;
+      *(tagged ? tag_word(x4, x4 >> 12) : word(x)) = 0u;
+    }
+    __syncwarp();
+  }
+  graph_acc_flush(tags, &acc[w]);
+}
+
 bool same_shape(const ItemShape& a, const ItemShape& b) {
   return a.cutover == b.cutover && a.warp_max == b.warp_max && a.warp_chunk == b.warp_chunk &&
          a.block_chunk == b.block_chunk && a.by_source == b.by_source;
@@ -218,6 +429,7 @@ ItemShape shape_from(const atc_tuning* t, const ItemShape& base) {
   // every partner list is streamed through a row's set: the sorted copy only for the shortest rows,
   // as in the single-graph Hu count, unless the tuning says otherwise
   if (sh.by_source == 1 && t->bisson_cutover <= 0) sh.cutover = std::min(sh.cutover, 8);
+  if (sh.by_source == 1 && t->bisson_warp_chunk <= 0) sh.warp_chunk = std::min(sh.warp_chunk, kRowsChunk);
   if (sh.cutover > sh.warp_max) sh.cutover = sh.warp_max;
   return sh;
 }
@@ -231,13 +443,10 @@ atc_status build_pipeline(atc_batch* b, const ItemShape& sh, cudaStream_t s) {
   // block items of lists longer than kBlockSmallList: one per such list (at most
   // m / (kBlockSmallList + 1) of them) plus one per chunk boundary
   const int64_t big_cap = m / (kBlockSmallList + 1) + m / sh.block_chunk + 1;
-  // rows items of mode 2: a row's partners are its own members, so a chunk is a share of one row
-  // and the longest rows set the tail; 64 partners an item (Chung-Lu batch of 26M edges: rows items
-  // of 512 4.36 ms, of 64 4.22)
+  // rows items of mode 2
   ItemShape shr = sh;
   shr.by_source = 1;
-  shr.cutover = std::min(sh.cutover, 8);  // the rows items' sorted copy, as the single-graph Hu count
-  shr.warp_chunk = std::min(sh.warp_chunk, 64);
+  shr.warp_chunk = std::min(sh.warp_chunk, kRowsChunk);
   const int64_t cap_rows = max_items(n, m, std::min(shr.warp_chunk, shr.block_chunk));
   if (b->built_n != n || b->built_m != m || b->built_graphs != ng || b->items_cap < cap_items ||
       b->rows_cap < cap_rows || b->big_cap < big_cap) {
@@ -314,10 +523,10 @@ atc_status build_pipeline(atc_batch* b, const ItemShape& sh, cudaStream_t s) {
     for (int q = 0; q < ng; ++q) {
       const double m_q = (double)b->gm[q];
       // ps, fitted to R-MAT and Chung-Lu graphs alone and in batches.  Grouping's 250 ps an edge
-      // holds the contended cursors of the hubs: measured by rows / grouped, R-MAT scale 18 342 / 330 ps
-      // an edge in all, scale 20 395 / 305, scale 24 890 / 450, Chung-Lu 1M vertices 151 / 163, batches
-      // of 48 Chung-Lu graphs 120-130 / 165-196
-      const bool rows = 1.25 * (double)b->gw[q] + 60.0 * m_q < 1.2 * (double)b->gwmin[q] + 250.0 * m_q;
+      // holds the contended cursors of the hubs: measured by rows / grouped, R-MAT scale 14 113 / 521 ps
+      // an edge in all, 16 165 / 647, 18 534 / 958, 20 1101 / 569, 22 1470 / 452, Chung-Lu 1M vertices
+      // 124 / 268, 4M 165 / 183, a batch of 48 Chung-Lu graphs 73 / 166
+      const bool rows = 1.3 * (double)b->gw[q] + 30.0 * m_q < 1.2 * (double)b->gwmin[q] + 250.0 * m_q;
       if (rows && b->vbase[q + 1] > b->vbase[q]) {
         ATC_CK(cudaMemsetAsync(b->vrows + b->vbase[q], 1, (size_t)(b->vbase[q + 1] - b->vbase[q]), s));
         ++nrows;
@@ -373,8 +582,12 @@ atc_status build_pipeline(atc_batch* b, const ItemShape& sh, cudaStream_t s) {
     kernels += 1;
     stage("batch.block.long");
   }
-  bisson_warp_kernel<CompactItems, kDefaultSlots><<<grid_warp, kBgWarps * 32, 0, c>>>(g, ListPartners{plist}, witems, 0, b->counters,
-                                                                       b->counters + 4, tags, b->gcounts);
+  const int grid_rows = sm_count() * blocks_per_sm((const void*)rows_kernel<kRowsLanes>, 128, 0);
+  if (sh.by_source == 1)
+    rows_kernel<kRowsLanes><<<grid_rows, 128, 0, c>>>(g, witems, b->counters, b->counters + 4, tags);
+  else
+    bisson_warp_kernel<CompactItems, kDefaultSlots><<<grid_warp, kBgWarps * 32, 0, c>>>(
+        g, ListPartners{plist}, witems, 0, b->counters, b->counters + 4, tags, b->gcounts);
   stage("batch.warp");
   if (mixed && nrows > 0) {
     cudaMemsetAsync(b->counters_r, 0, sizeof(int) * 8, c);
@@ -391,8 +604,7 @@ atc_status build_pipeline(atc_batch* b, const ItemShape& sh, cudaStream_t s) {
       kernels += 1;
       stage("batch.rows.block.long");
     }
-    bisson_warp_kernel<CompactItems, kDefaultSlots><<<grid_warp, kBgWarps * 32, 0, c>>>(
-        g, ListPartners{b->cols}, witems_r, 0, b->counters_r, b->counters_r + 4, tags, b->gcounts);
+    rows_kernel<kRowsLanes><<<grid_rows, 128, 0, c>>>(g, witems_r, b->counters_r, b->counters_r + 4, tags);
     stage("batch.rows.warp");
   }
   cudaError_t launch_err = cudaGetLastError();

@@ -402,20 +402,22 @@ __device__ __forceinline__ void graph_acc_flush(const GraphTags& t, GraphAccSlot
   if ((threadIdx.x & 31) == 0 && a->part && a->g >= 0) atomicAdd(&t.counts[a->g], a->part);
   __syncwarp();
 }
-__device__ __forceinline__ void graph_acc_add(const GraphTags& t, GraphAccSlot* a, int64_t h, unsigned c) {
-  unsigned long long w = c;
-  for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-  if ((threadIdx.x & 31) == 0) {
-    if (h < a->lo || h >= a->hi) {
-      if (a->part && a->g >= 0) atomicAdd(&t.counts[a->g], a->part);
-      const int g = graph_of(t, h);
-      *a = GraphAccSlot{g, (int32_t)t.vbase[g], (int32_t)t.vbase[g + 1], 0ull};
-    }
-    a->part += w;
+// Makes h's graph the slot's, which receives the counts until the next call for another graph.
+__device__ __forceinline__ void graph_acc_enter(const GraphTags& t, GraphAccSlot* a, int64_t h) {
+  if ((threadIdx.x & 31) == 0 && (h < a->lo || h >= a->hi)) {
+    if (a->part && a->g >= 0) atomicAdd(&t.counts[a->g], a->part);
+    const int g = graph_of(t, h);
+    *a = GraphAccSlot{g, (int32_t)t.vbase[g], (int32_t)t.vbase[g + 1], 0ull};
   }
   __syncwarp();
 }
-
+__device__ __forceinline__ void graph_acc_add(const GraphTags& t, GraphAccSlot* a, int64_t h, unsigned c) {
+  unsigned long long w = c;
+  for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+  graph_acc_enter(t, a, h);
+  if ((threadIdx.x & 31) == 0) a->part += w;
+  __syncwarp();
+}
 
 // Hash tables of N+(h): linear probing over buckets of S slots (S = 1, 2 or 4; 4-, 8- or
 // 16-byte aligned), empty slots hold -1.  The home bucket of x is given by Fibonacci
