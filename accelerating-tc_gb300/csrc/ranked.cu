@@ -57,6 +57,11 @@ constexpr int kRankMidMin = 96;         // fewer entries than these do not pay f
 constexpr int64_t kWideMean15 = 160, kWideMean = 224;
 constexpr int kDenseRows = 1 << 15;     // rows that may be kept as bitmaps
 constexpr int kDenseSources = 4;        // times as many rows are looked at for targets among them
+// Small items (filter, middle rows to sort, rows with few words) per atomic on their counter: one
+// address takes about one atomic per ns, which was the whole time of the filter's 470 000 items on
+// Chung-Lu n = 700 001 (303 us; 189 by fours) and of the words' 105 000 rows there (104; 80).  The larger
+// items of the ranks below 2^16 lose by it (103 -> 125 us): their tail.
+constexpr int kGrab = 4;
 constexpr int kRankRowMax = kTabWords;  // longest row the CTA sort holds (64 KB)
 constexpr int kRankWarpRow = 1024;      // longest row a warp sorts in registers
 
@@ -217,10 +222,12 @@ __global__ void __launch_bounds__(256) rank_sort_mid_kernel(const int64_t* roff,
                                                             int* ctr) {
   const int lane = threadIdx.x & 31;
   const int total = ctr[kcMid];
-  for (;;) {
-    int it = 0;
-    if (lane == 0) it = atomicAdd(&ctr[kcNextMid], 1);
-    it = __shfl_sync(0xffffffffu, it, 0);
+  for (int it = 0, it_end = 0;; ++it) {
+    if (it == it_end) {
+      if (lane == 0) it = atomicAdd(&ctr[kcNextMid], kGrab);
+      it = __shfl_sync(0xffffffffu, it, 0);
+      it_end = it + kGrab;
+    }
     if (it >= total) break;
     const int32_t u = mid[it];
     const int64_t b = __ldg(roff + u);
@@ -597,10 +604,14 @@ __global__ void __launch_bounds__(256) rank_words_kernel(const int64_t* __restri
   __syncwarp();
   if (*too_long) return;  // an unsorted row's prefix is no prefix
   unsigned long long total = 0;
+  int u = -1, u_end = 0;
   for (;;) {
-    int u = 0;
-    if (lane == 0) u = atomicAdd(next, 1);
-    u = __shfl_sync(0xffffffffu, u, 0);
+    if (++u >= u_end) {
+      const int grab = u < rows ? 1 : kGrab;  // the longest rows one at a time
+      if (lane == 0) u = atomicAdd(next, grab);
+      u = __shfl_sync(0xffffffffu, u, 0);
+      u_end = u + grab;
+    }
     if (u >= sources) break;
     const int64_t b = __ldg(roff + u);
     const int du = (int)(__ldg(roff + u + 1) - b);
@@ -696,13 +707,16 @@ __global__ void __launch_bounds__(WARPS * 32, 9) rank_filter_kernel(const int64_
     int ne, dh;
     int64_t g0, hb;
   };
+  int it = 0, it_end = 0;
   auto head = [&]() {
-    int it = 0;
-    if (lane == 0) it = atomicAdd(next, 1);
-    it = __shfl_sync(0xffffffffu, it, 0);
+    if (it == it_end) {
+      if (lane == 0) it = atomicAdd(next, kGrab);
+      it = __shfl_sync(0xffffffffu, it, 0);
+      it_end = it + kGrab;
+    }
     Head h{-1, 0, 0, 0, 0};
     if (it < nitems) {
-      const int2 c = __ldg(items + it);
+      const int2 c = __ldg(items + it++);
       h.v = c.x;
       h.g0 = __ldg(gstart + c.x) + (int64_t)c.y * chunk;
       h.ne = (int)min(__ldg(gstart + c.x + 1) - h.g0, (int64_t)chunk);
