@@ -126,9 +126,13 @@ __global__ void rank_rows_kernel(const int32_t* esrc, const int32_t* cols, int64
 
 // Rows of up to 32 elements: a warp takes 32 consecutive rows, cuts them into windows of whole
 // rows of at most 32 elements together and sorts each window by (row, id) across its lanes.
-// Longer rows go on a list each for the warp and the CTA sort.
+// Longer rows go on a list each for the warp and the CTA sort.  Key: 32 bits, five for the row of
+// the window and 27 for the id, 64 for more than 2^27 vertices
+// (Chung-Lu n = 700 001, 11 M edges: 80 us with 64, 64 with 32).
+template <class Key>
 __global__ void rank_sort_small_kernel(const int64_t* roff, int64_t n, int32_t* rcols, int32_t* mid, int32_t* big,
                                        int* ctr) {
+  constexpr int kIdBits = sizeof(Key) == 4 ? 27 : 32;
   const int lane = threadIdx.x & 31;
   const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t rb = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; rb * 32 < n; rb += warps) {
@@ -163,16 +167,16 @@ __global__ void rank_sort_small_kernel(const int64_t* roff, int64_t n, int32_t* 
 #pragma unroll
       for (int step = 16; step > 0; step >>= 1)
         if (__shfl_sync(0xffffffffu, rel, k + step) <= lane) k += step;
-      uint64_t key = valid ? (uint64_t)k << 32 | (uint32_t)rcols[s0 + lane] : ~0ull;
+      Key key = valid ? (Key)k << kIdBits | (uint32_t)rcols[s0 + lane] : ~(Key)0;
 #pragma unroll
       for (int kk = 2; kk <= 32; kk <<= 1)
 #pragma unroll
         for (int j = kk >> 1; j > 0; j >>= 1) {
-          const uint64_t y = __shfl_xor_sync(0xffffffffu, key, j);
+          const Key y = __shfl_xor_sync(0xffffffffu, key, j);
           const bool keep_min = ((lane & j) == 0) == ((lane & kk) == 0);
           key = keep_min == (key < y) ? key : y;
         }
-      if (valid) rcols[s0 + lane] = (int32_t)(uint32_t)key;
+      if (valid) rcols[s0 + lane] = (int32_t)(uint32_t)(key & (((Key)1 << kIdBits) - 1));
       c = last + 1;
     }
   }
@@ -959,7 +963,8 @@ atc_status build_ranked(const atc_csr* csr, bool bitmaps, RankedCopy* rc, cudaSt
     *launches += 3;
   }
   rank_rows_kernel<<<grid_for(m, 256), 256, 0, s>>>(pv->esrc, csr->cols, m, rank, slot, roff, rcols);
-  rank_sort_small_kernel<<<grid_for(n, 256), 256, 0, s>>>(roff, n, rcols, mid, big, ctr);
+  if (n <= 1 << 27) rank_sort_small_kernel<uint32_t><<<grid_for(n, 256), 256, 0, s>>>(roff, n, rcols, mid, big, ctr);
+  else rank_sort_small_kernel<uint64_t><<<grid_for(n, 256), 256, 0, s>>>(roff, n, rcols, mid, big, ctr);
   rank_sort_mid_kernel<<<sm_count() * blocks_per_sm((const void*)rank_sort_mid_kernel, 256, 0), 256, 0, s>>>(
       roff, mid, rcols, ctr);
   const int64_t long_rows = m / (kRankWarpRow + 1);
