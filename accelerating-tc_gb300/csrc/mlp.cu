@@ -282,14 +282,24 @@ __global__ void __launch_bounds__(kFusedThreads) mlp_tile_kernel(FusedArgs a) {
   }
 }
 
-// grads[i] = sum over the CTAs / sum of M;  grads[nparams] = the loss.
+// grads[i] = sum over the CTAs / sum of M;  grads[nparams] = the loss.  Compensated sums (the
+// rounding of every addition is added up apart), in float: FP64 runs at a small fraction of its rate.
+__device__ __forceinline__ float column_sum(const float* partial, int ctas, int64_t stride) {
+  float acc = 0.0f, low = 0.0f;
+#pragma unroll 8
+  for (int c = 0; c < ctas; ++c) {
+    const float x = partial[c * stride], sum = __fadd_rn(acc, x), back = __fsub_rn(sum, acc);
+    low = __fadd_rn(low, __fadd_rn(__fsub_rn(acc, __fsub_rn(sum, back)), __fsub_rn(x, back)));
+    acc = sum;
+  }
+  return acc + low;
+}
+
 __global__ void mlp_reduce_kernel(const float* partial, int ctas, int nparams, float* grads) {
-  float cnt = 0.0f;
-  for (int c = 0; c < ctas; ++c) cnt += partial[(int64_t)c * (nparams + 2) + nparams + 1];
+  float cnt = column_sum(partial + nparams + 1, ctas, nparams + 2);
   if (!(cnt > 0.0f)) cnt = 1.0f;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= nparams; i += gridDim.x * blockDim.x) {
-    float acc = 0.0f;
-    for (int c = 0; c < ctas; ++c) acc += partial[(int64_t)c * (nparams + 2) + i];
+    const float acc = column_sum(partial + i, ctas, nparams + 2);
     grads[i] = i < nparams ? acc / cnt : 0.5f * acc / cnt;
   }
 }
