@@ -17,17 +17,20 @@ namespace atc {
 // faster (figures in radix.cuh; the two cross between 16000 and 32000 keys).
 constexpr size_t kOwnSort = 1 << 15;
 
+static atc_status library_sort(void* tmp, size_t* bytes, uint64_t* keys, uint64_t* alt, size_t n, int begin_bit,
+                               int end_bit, uint64_t** sorted, cudaStream_t s) {
+  cub::DoubleBuffer<uint64_t> db(keys, alt);
+  ATC_CK(cub::DeviceRadixSort::SortKeys(tmp, *bytes, db, (int64_t)n, begin_bit, end_bit, s));
+  if (sorted) *sorted = db.Current();
+  return ATC_OK;
+}
+
 // Sorts with caller-provided temporary storage; *sorted = the buffer that holds the result.
 // tmp == nullptr: *bytes receives the size needed.
 atc_status sort_keys_u64_tmp(void* tmp, size_t* bytes, uint64_t* keys, uint64_t* alt, size_t n, int begin_bit,
                              int end_bit, uint64_t** sorted, cudaStream_t s) {
-  if (n >= kOwnSort && end_bit > begin_bit) {
-    ATC_CK(radix_sort_keys(tmp, bytes, keys, alt, n, begin_bit, end_bit, sorted, s));
-    return ATC_OK;
-  }
-  cub::DoubleBuffer<uint64_t> db(keys, alt);
-  ATC_CK(cub::DeviceRadixSort::SortKeys(tmp, *bytes, db, (int64_t)n, begin_bit, end_bit, s));
-  if (sorted) *sorted = db.Current();
+  if (n < kOwnSort || end_bit <= begin_bit) return library_sort(tmp, bytes, keys, alt, n, begin_bit, end_bit, sorted, s);
+  ATC_CK(radix_sort_keys(tmp, bytes, keys, alt, n, begin_bit, end_bit, sorted, s));
   return ATC_OK;
 }
 
@@ -36,9 +39,16 @@ atc_status sort_keys_u64(uint64_t*& keys, uint64_t*& alt, size_t n, int begin_bi
   size_t tmp = 0;
   ATC_TRY(sort_keys_u64_tmp(nullptr, &tmp, keys, alt, n, begin_bit, end_bit, nullptr, s));
   DevBuf<char> t;
-  ATC_TRY(t.alloc(tmp, s));
   uint64_t* sorted = nullptr;
-  ATC_TRY(sort_keys_u64_tmp(t.p, &tmp, keys, alt, n, begin_bit, end_bit, &sorted, s));
+  if (t.alloc(tmp, s) == ATC_OK) {
+    ATC_TRY(sort_keys_u64_tmp(t.p, &tmp, keys, alt, n, begin_bit, end_bit, &sorted, s));
+  } else {
+    // up to 2^20 keys the library's scratch is the smaller one (0.18 bytes a key to 0.25)
+    cudaGetLastError();
+    ATC_TRY(library_sort(nullptr, &tmp, keys, alt, n, begin_bit, end_bit, nullptr, s));
+    ATC_TRY(t.alloc(tmp, s));
+    ATC_TRY(library_sort(t.p, &tmp, keys, alt, n, begin_bit, end_bit, &sorted, s));
+  }
   if (sorted != keys) {
     alt = keys;
     keys = sorted;
