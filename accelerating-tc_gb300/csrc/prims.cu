@@ -12,10 +12,9 @@
 
 namespace atc {
 
-// The framework's own sort (radix.cuh) from here on: it needs a histogram, an offsets and a clearing
-// launch besides its passes, so below this CUB's single-tile or smaller-tile kernels are as fast or
-// faster (figures in radix.cuh; the two cross between 16000 and 32000 keys).
-constexpr size_t kOwnSort = 1 << 15;
+// The framework's own sort (radix.cuh) from here on; fewer keys are a single launch in CUB, against a
+// clearing, a histogram, an offsets launch and the passes (figures in radix.cuh).
+constexpr size_t kOwnSort = 1 << 12;
 
 static atc_status library_sort(void* tmp, size_t* bytes, uint64_t* keys, uint64_t* alt, size_t n, int begin_bit,
                                int end_bit, uint64_t** sorted, cudaStream_t s) {
@@ -43,7 +42,8 @@ atc_status sort_keys_u64(uint64_t*& keys, uint64_t*& alt, size_t n, int begin_bi
   if (t.alloc(tmp, s) == ATC_OK) {
     ATC_TRY(sort_keys_u64_tmp(t.p, &tmp, keys, alt, n, begin_bit, end_bit, &sorted, s));
   } else {
-    // up to 2^20 keys the library's scratch is the smaller one (0.18 bytes a key to 0.25)
+    // up to 2^20 keys the library's scratch is the smaller one (0.18 bytes a key to 0.25 or, up to
+    // 2^18, one)
     cudaGetLastError();
     ATC_TRY(library_sort(nullptr, &tmp, keys, alt, n, begin_bit, end_bit, nullptr, s));
     ATC_TRY(t.alloc(tmp, s));

@@ -14,8 +14,8 @@
 // two.  A look at eight earlier tiles per step gave 3-7 % over one; 512 x 16 keys in two CTAs per SM
 // and 384 x 16 in three are equal, nine-bit digits gain at 44 bits and lose at 40 and 48.
 // Measured against CUB's sort (ms): 2^24 keys of 40 bits 0.58 to 0.89, 2^26 of 44 2.3 to 3.9, 2^28 of
-// 48 9.1 to 15.4; 1.5 M of 34 0.11 to 0.15; 32000 of 20 bits 0.046 to 0.049, and below that CUB's
-// fewer launches win (2000 keys: 0.044 to 0.010).
+// 48 9.1 to 15.4; 1.5 M of 34 0.11 to 0.15; 200 000 of 28 0.050 to 0.073, 8000 of 20 0.035 to 0.042, 4000 0.033
+// to 0.038; fewer are one launch in CUB (2000 keys: 0.031 to 0.010).
 //
 // A wait for an earlier tile's counts ends by itself: tiles start in order and publish before they
 // wait.  A thread that has still waited kWaitNs counts the tile's keys of its digit from the
@@ -32,9 +32,11 @@ namespace radix {
 constexpr int kDigitBits = 8;
 constexpr int kDigits = 1 << kDigitBits;
 constexpr int kThreads = 512;
-constexpr int kItems = 16;
+// Keys a thread: 16, or four up to kSmallSort keys, where tiles of 8192 would leave most SMs idle (200 000
+// keys of 28 bits 58 -> 50 us, 32 000 of 20 bits 46 -> 35; 400 000 of 34 bits 70 and 70, 800 000 78 -> 91).
+constexpr int kSmallItems = 4;
+constexpr size_t kSmallSort = 1 << 18;
 constexpr int kWarps = kThreads / 32;
-constexpr int kTileKeys = kThreads * kItems;
 constexpr int kMaxPasses = 8;
 constexpr int kLook = 8;
 constexpr uint64_t kWaitNs = 10000000ull;
@@ -95,7 +97,9 @@ __device__ __forceinline__ uint64_t clock_ns() {
   return t;
 }
 
+template <int kItems>
 struct PassSmem {
+  static constexpr int kTileKeys = kThreads * kItems;
   // a warp's match table (a word per digit, zero between uses) while ranking, then the tile's keys
   union {
     uint64_t keys[kTileKeys];
@@ -110,13 +114,14 @@ struct PassSmem {
 // state[tile * kDigits + digit]: the tile's keys of the digit with flag kCount, then those of all
 // tiles up to it with kSum; the flags are S's top bits, and n < 2^(bits of S - 2).  ticket: the
 // next tile.  next: the state of the next pass, cleared here when it is a buffer of its own.
-template <typename S>
+template <typename S, int kItems>
 __global__ void __launch_bounds__(kThreads, 2)
     pass_kernel(const uint64_t* __restrict__ in, uint64_t* __restrict__ out, uint64_t n, int shift, int bits,
                 const unsigned long long* __restrict__ offsets, S* state, S* next, unsigned* ticket) {
+  constexpr int kTileKeys = kThreads * kItems;
   constexpr S kSum = (S)1 << (8 * sizeof(S) - 1), kCount = kSum >> 1, kValue = kCount - 1;
   extern __shared__ __align__(16) unsigned char raw[];
-  PassSmem& sm = *reinterpret_cast<PassSmem*>(raw);
+  PassSmem<kItems>& sm = *reinterpret_cast<PassSmem<kItems>*>(raw);
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   const unsigned below = (1u << lane) - 1, mask = (1u << bits) - 1;
   if (t == 0) sm.tile = atomicAdd(ticket, 1u);
@@ -239,7 +244,8 @@ inline cudaError_t radix_sort_keys(void* tmp, size_t* bytes, uint64_t* keys, uin
                                    uint64_t** sorted, cudaStream_t s) {
   using namespace radix;
   const Passes ps = cut(begin, end);
-  const size_t tiles = (n + kTileKeys - 1) / kTileKeys;
+  const int items = n <= kSmallSort ? kSmallItems : 16;
+  const size_t tile = (size_t)kThreads * items, tiles = (n + tile - 1) / tile;
   const size_t head = 256;  // a ticket per pass
   const size_t hist = sizeof(unsigned long long) * kMaxPasses * kDigits;
   const bool wide = n >= (1ull << 30);
@@ -264,10 +270,10 @@ inline cudaError_t radix_sort_keys(void* tmp, size_t* bytes, uint64_t* keys, uin
   histogram_kernel<<<(unsigned)(hgrid < (size_t)sms * 4 ? hgrid : (size_t)sms * 4), 512, 0, s>>>(keys, n, ps, h);
   offsets_kernel<<<ps.n, kDigits, 0, s>>>(h);
   uint64_t *a = keys, *b = alt;
-  auto run = [&](auto kernel, auto zero) -> cudaError_t {
+  auto run = [&](auto kernel, auto zero, size_t smem) -> cudaError_t {
     using S = decltype(zero);
     const cudaError_t r =
-        cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PassSmem));
+        cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (r != cudaSuccess) return r;
     for (int i = 0; i < ps.n; ++i) {
       S* const mine = reinterpret_cast<S*>(st + (two && (i & 1) ? state : 0));
@@ -276,7 +282,7 @@ inline cudaError_t radix_sort_keys(void* tmp, size_t* bytes, uint64_t* keys, uin
         const cudaError_t c = cudaMemsetAsync(st, 0, state, s);
         if (c != cudaSuccess) return c;
       }
-      kernel<<<(unsigned)tiles, kThreads, sizeof(PassSmem), s>>>(a, b, n, ps.shift[i], ps.bits[i], h + i * kDigits, mine,
+      kernel<<<(unsigned)tiles, kThreads, smem, s>>>(a, b, n, ps.shift[i], ps.bits[i], h + i * kDigits, mine,
                                                                  next, ticket + i);
       uint64_t* x = a;
       a = b;
@@ -284,7 +290,9 @@ inline cudaError_t radix_sort_keys(void* tmp, size_t* bytes, uint64_t* keys, uin
     }
     return cudaSuccess;
   };
-  e = wide ? run(pass_kernel<unsigned long long>, 0ull) : run(pass_kernel<unsigned>, 0u);
+  e = items != 16 ? run(pass_kernel<unsigned, kSmallItems>, 0u, sizeof(PassSmem<kSmallItems>))
+      : wide      ? run(pass_kernel<unsigned long long, 16>, 0ull, sizeof(PassSmem<16>))
+                  : run(pass_kernel<unsigned, 16>, 0u, sizeof(PassSmem<16>));
   if (e != cudaSuccess) return e;
   if (sorted) *sorted = a;
   return cudaGetLastError();

@@ -1,5 +1,5 @@
-"""The key sort under preTC at its edges: around the size where it takes over, whole tiles of 8192
-keys, the size where the tile states share one buffer, id widths from one pass to eight-bit digits
+"""The key sort under preTC at its edges: around the size where it takes over, whole tiles of 2048
+and 8192 keys, the size where the tile states share one buffer, id widths from one pass to eight-bit digits
 of every width, and keys that agree in most digits."""
 import numpy as np
 import pytest
@@ -9,7 +9,7 @@ import atc
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("m", [32767, 32768, 32769, 40960, 40961, 73728, (1 << 20), (1 << 20) + 1, (1 << 20) + 8192])
+@pytest.mark.parametrize("m", [4095, 4096, 4097, 6144, 6145, 32769, 73728, (1 << 18), (1 << 18) + 1, (1 << 20), (1 << 20) + 1, (1 << 20) + 8192])
 @pytest.mark.parametrize("bits", [3, 8, 9, 17, 22])
 @pytest.mark.parametrize("skew", [0, 1])
 def test_rows_of_the_sorted_edges(m, bits, skew):
