@@ -479,6 +479,14 @@ constexpr int kRowBlock = 512;     // k = 5: C0 up to this size by the CTA that 
 constexpr int kRowThreads = 512;
 constexpr int kRowParts = 2048;    // part table of N+(u): two parts a member
 constexpr int kRowBuckets = 4;     // lists by length, longest first (row_bucket)
+constexpr int kRowCounts = 4;      // the first of their counts among the queues
+// Sources of the longer half that a warp each would take, up to which they are split over CTAs
+// instead, from k = 5 on: one such row's search held a whole count up where the GPU had little else to
+// do.  Chung-Lu n = 128 000, 0.9 M edges: k = 5 517 -> 202 us, k = 6 850 -> 345; R-MAT scale 11 of 31 000
+// edges 307 -> 182 and 752 -> 456.  k >= 6: with 2048 instead Chung-Lu n = 7000 k = 6 takes 511 us (188);
+// with 65536 RGG n = 128 000 5.6 ms (2.6); Chung-Lu n = 32 000 of 0.5 M edges 970 with 8192, 650 with 16384.
+constexpr int kFewRows = 2048;
+constexpr int kFewRowsDeep = 16384;  // k >= 6, or n / 16
 constexpr int kRowSearch = 128;    // lists longer than this are searched for the members of
                                    // N+(u), not streamed, where N+(u) fits one warp's masks
 
@@ -562,12 +570,13 @@ __device__ __forceinline__ void for_members(const int32_t* cols, int64_t xb, int
 }
 
 // A warp per source u with lo < |N+(u)| <= R (R = bits of M), k - 1 <= |N+(u)|, over the edges
-// of [e0, e1).  KD = k - 3: the members to choose below an induced edge (0: k = 3; above
+// of [e0, e1).  Sources above few_lo are left to kcl_rows_block_kernel where they are few (*few).  KD = k - 3: the members to choose below an induced edge (0: k = 3; above
 // kRowUnroll: any k).  Sources are taken `grab` (<= 32) at a time from `queue`.
 template <class M, int KD>
 __global__ void __launch_bounds__(kKcWarps * 32) kcl_rows_warp_kernel(const int64_t* off, const int32_t* cols, int64_t n,
-                                                                    int64_t e0, int64_t e1, int k, int lo, int grab,
-                                                                    int* queue, unsigned long long* out) {
+                                                                    int64_t e0, int64_t e1, int k, int lo, int few_lo,
+                                                                    const int* few, int few_max, int grab, int* queue,
+                                                                    unsigned long long* out) {
   constexpr int R = 8 * (int)sizeof(M);
   constexpr int kPairs = R * (R - 1) / 2;  // induced edges of a DAG; other digraphs may hold more
   __shared__ int32_t Ssm[kKcWarps][R];
@@ -580,6 +589,8 @@ __global__ void __launch_bounds__(kKcWarps * 32) kcl_rows_warp_kernel(const int6
   uint16_t* pairs = psm[w];
   const unsigned below = (1u << lane) - 1;
   unsigned long long cnt = 0, bytes = 0;
+  const int hi = *few <= few_max ? min(few_lo, R) : R;
+  if (hi <= lo) return;
   for (;;) {
     int chunk = 0;
     if (lane == 0) chunk = atomicAdd(queue, 1);
@@ -587,7 +598,7 @@ __global__ void __launch_bounds__(kKcWarps * 32) kcl_rows_warp_kernel(const int6
     if ((int64_t)chunk * grab >= n) break;
     const int64_t row = min((int64_t)chunk * grab + lane, n);
     const int64_t rb = __ldg(off + row), re = __ldg(off + min(row + 1, n));
-    unsigned todo = __ballot_sync(0xffffffffu, lane < grab && re - rb > lo && re - rb <= R && re - rb >= k - 1 &&
+    unsigned todo = __ballot_sync(0xffffffffu, lane < grab && re - rb > lo && re - rb <= hi && re - rb >= k - 1 &&
                                                    min(re, e1) > max(rb, e0));
     while (todo) {
       const int q = __ffs(todo) - 1;
@@ -663,25 +674,27 @@ __global__ void __launch_bounds__(kKcWarps * 32) kcl_rows_warp_kernel(const int6
   }
 }
 
-// Sources with lo < |N+(u)| <= hi and an edge in [e0, e1), longest bucket first:
-// lists[b * cap ...], counts[b].
+// Sources with mid < |N+(u)| <= hi and an edge in [e0, e1), longest bucket first: lists[b * cap ...],
+// counts[b].  Those with lo < |N+(u)| <= mid, which a warp each takes where they are many, are
+// counted in counts[kRowBuckets] and listed (lists[kRowBuckets * cap ...]) up to few_max.
 __device__ __forceinline__ int row_bucket(int64_t d) { return d > 384 ? 0 : d > 192 ? 1 : d > 96 ? 2 : 3; }
-__global__ void kcl_rows_list_kernel(const int64_t* off, int64_t n, int64_t e0, int64_t e1, int lo, int hi, int64_t cap,
-                                     int32_t* lists, int* counts) {
+__global__ void kcl_rows_list_kernel(const int64_t* off, int64_t n, int64_t e0, int64_t e1, int lo, int mid, int hi,
+                                     int64_t cap, int few_max, int32_t* lists, int* counts) {
   const int lane = threadIdx.x & 31;
   const int64_t n_pad = (n + 31) & ~31ll;
   for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < n_pad; u += (int64_t)gridDim.x * blockDim.x) {
     int mine = -1;
     if (u < n) {
       const int64_t b = off[u], e = off[u + 1];
-      if (e - b > lo && e - b <= hi && min(e, e1) > max(b, e0)) mine = row_bucket(e - b);
+      if (e - b > lo && e - b <= hi && min(e, e1) > max(b, e0)) mine = e - b > mid ? row_bucket(e - b) : kRowBuckets;
     }
-    for (int q = 0; q < kRowBuckets; ++q) {  // one atomic per warp and bucket
+    for (int q = 0; q <= kRowBuckets; ++q) {  // one atomic per warp and bucket
       const unsigned m = __ballot_sync(0xffffffffu, mine == q);
       int at = 0;
       if (m && lane == 0) at = atomicAdd(&counts[q], __popc(m));
       at = __shfl_sync(0xffffffffu, at, 0);
-      if (mine == q) lists[q * cap + at + __popc(m & ((1u << lane) - 1))] = (int32_t)u;
+      at += __popc(m & ((1u << lane) - 1));
+      if (mine == q && (q < kRowBuckets || at < few_max)) lists[q * cap + at] = (int32_t)u;
     }
   }
 }
@@ -724,7 +737,7 @@ __device__ __forceinline__ void row_members(const uint32_t* r32, int halves, uin
 template <int MODE>
 __global__ void __launch_bounds__(kRowThreads) kcl_rows_block_kernel(const int64_t* off, const int32_t* cols, int64_t e0,
                                                                     int64_t e1, int k, const int32_t* lists, int64_t cap,
-                                                                    const int* counts, int dmax, int* queue,
+                                                                    const int* counts, int few_max, int dmax, int* queue,
                                                                     unsigned long long* dense,
                                                                     unsigned long long* out) {
   extern __shared__ __align__(16) unsigned char rsm[];
@@ -735,12 +748,17 @@ __global__ void __launch_bounds__(kRowThreads) kcl_rows_block_kernel(const int64
   __shared__ uint32_t ptab[kRowParts];
   __shared__ uint16_t part_start[kRowParts + 1];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = kRowThreads / 32;
-  int first[kRowBuckets + 1];
+  int first[kRowBuckets + 2];
   first[0] = 0;
 #pragma unroll
   for (int b = 0; b < kRowBuckets; ++b) first[b + 1] = first[b] + counts[b];
-  const int sources = first[kRowBuckets];
-  const int nsplit = MODE < 2 ? 1 : min(max(8 * (int)gridDim.x / max(sources, 1), 1), 32);
+  first[kRowBuckets + 1] = first[kRowBuckets] + (counts[kRowBuckets] <= few_max ? counts[kRowBuckets] : 0);
+  // the long sources (the lists but the last) and the others are split by their own numbers
+  const int sources = first[kRowBuckets + 1], longs = first[kRowBuckets];
+  // Parts of fewer than four edges only build the rows once more: four of a CTA's sixteen warps
+  // already have a scheduler each.
+  const int split_long = MODE < 2 ? 1 : min(max(6 * (int)gridDim.x / max(longs, 1), 1), min(max(dmax / 4, 1), 32));
+  const int split_few = MODE < 2 ? 1 : min(max(3 * (int)gridDim.x / max(sources - longs, 1), 1), 8);
   unsigned long long cnt = 0, bytes = 0;
   for (;;) {
     if (threadIdx.x == 0) {
@@ -749,11 +767,13 @@ __global__ void __launch_bounds__(kRowThreads) kcl_rows_block_kernel(const int64
       next_row = 0;
     }
     __syncthreads();
-    const int it = item / nsplit, part = item - it * nsplit;
+    const bool is_long = item < longs * split_long;
+    const int nsplit = is_long ? split_long : split_few, at_item = is_long ? item : item - longs * split_long;
+    const int it = at_item / nsplit + (is_long ? 0 : longs), part = at_item % nsplit;
     if (it >= sources) break;
     int b = 0, fb = 0;
 #pragma unroll
-    for (int q = 1; q < kRowBuckets; ++q)
+    for (int q = 1; q <= kRowBuckets; ++q)
       if (it >= first[q]) {
         b = q;
         fb = first[q];
@@ -957,10 +977,11 @@ using namespace atc;
 
 // Rows of up to R = 32 or 64 members (M's bits): one warp launch for the given k.
 template <class M>
-static atc_status launch_rows_warp(const atc_csr* csr, int64_t e0, int64_t e1, int k, int lo, int* queue,
+static atc_status launch_rows_warp(const atc_csr* csr, int64_t e0, int64_t e1, int k, int lo, int few_lo, const int* few,
+                                   int few_max, int* queue,
                                    unsigned long long* out, cudaStream_t s) {
-  using Kernel = void (*)(const int64_t*, const int32_t*, int64_t, int64_t, int64_t, int, int, int, int*,
-                          unsigned long long*);
+  using Kernel = void (*)(const int64_t*, const int32_t*, int64_t, int64_t, int64_t, int, int, int, const int*, int,
+                          int, int*, unsigned long long*);
   static const Kernel kernels[kRowUnroll + 2] = {
       kcl_rows_warp_kernel<M, 0>, kcl_rows_warp_kernel<M, 1>, kcl_rows_warp_kernel<M, 2>, kcl_rows_warp_kernel<M, 3>,
       kcl_rows_warp_kernel<M, 4>, kcl_rows_warp_kernel<M, 5>, kcl_rows_warp_kernel<M, kRowUnroll + 1>};
@@ -972,14 +993,15 @@ static atc_status launch_rows_warp(const atc_csr* csr, int64_t e0, int64_t e1, i
   const int64_t warps = (int64_t)sm_count() * std::max(bps, 1) * kKcWarps;
   const int grab = (int)std::min<int64_t>(std::max<int64_t>(csr->n / (4 * warps), 1), 32);
   const int64_t grid = std::min<int64_t>(warps, (csr->n + grab - 1) / grab) / kKcWarps + 1;
-  kern<<<(unsigned)grid, kKcWarps * 32, 0, s>>>(csr->offsets, csr->cols, csr->n, e0, e1, k, lo, grab, queue, out);
+  kern<<<(unsigned)grid, kKcWarps * 32, 0, s>>>(csr->offsets, csr->cols, csr->n, e0, e1, k, lo, few_lo, few,
+                                                    few_max, grab, queue, out);
   ATC_CK(cudaGetLastError());
   return ATC_OK;
 }
 
 template <int MODE>
 static atc_status launch_rows_block(const atc_csr* csr, int64_t e0, int64_t e1, int k, int dmax, const int32_t* lists,
-                                    int64_t cap, int* counts, int* queue, unsigned long long* dense,
+                                    int64_t cap, int* counts, int few_max, int* queue, unsigned long long* dense,
                                     unsigned long long* out, cudaStream_t s) {
   const size_t smem = RowsSmem(dmax, MODE).bytes;
   ATC_CK(cudaFuncSetAttribute((const void*)kcl_rows_block_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -987,13 +1009,36 @@ static atc_status launch_rows_block(const atc_csr* csr, int64_t e0, int64_t e1, 
   int bps = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kcl_rows_block_kernel<MODE>, kRowThreads, smem);
   kcl_rows_block_kernel<MODE><<<(unsigned)(sm_count() * std::max(bps, 1)), kRowThreads, smem, s>>>(
-      csr->offsets, csr->cols, e0, e1, k, lists, cap, counts, dmax, queue, dense, out);
+      csr->offsets, csr->cols, e0, e1, k, lists, cap, counts, few_max, dmax, queue, dense, out);
   ATC_CK(cudaGetLastError());
   return ATC_OK;
 }
 
+// Whether every edge is better walked (with the dense kernel from k = 5 on): one or two launches
+// against up to six, which is what small graphs take.  Measured rows / walk in us: k = 3 R-MAT of
+// 14 000 edges 74 / 41, 114 000 124 / 73, RGG of 245 000 117 / 122; k = 4 R-MAT of 2900 51 / 47, Chung-Lu of 14 000
+// 67 / 52, R-MAT of 31 000 119 / 159; k = 5 R-MAT of 6000 67 / 48, 27 000 140 / 85, Chung-Lu of 114 000 140 / 110, R-MAT of 68 000 (W = 45 m)
+// 244 / 461; k = 6 R-MAT of 6000 115 / 61, Chung-Lu of 48 000 116 / 72, R-MAT of 14 000 (W = 25 m) 226 / 360.
+// The walk's warp per edge also balances a few very long rows better (K-core orientations: W = 2.5 W_min and
+// more): R-MAT scale 14 of 177 000 edges k = 6 4.8 / 3.8 ms, of 259 000 k = 5 4.4 / 2.9; by degree (1.7 W_min) 1.8 /
+// 2.6 and 0.62 / 2.0.  From k = 7 on any skewed graph: Chung-Lu of 2.3 M edges 43 / 31 ms, RGG of 2.5 M 10.8 /
+// 21.2.
+static bool walk_pays(const atc_csr* csr, int k) {
+  const int64_t m = csr->m, w = csr->wedges;
+  if (csr->max_outdeg <= (k >= 6 ? 16 : 32)) return false;  // rows by one launch
+  if (k == 3) return m <= 240000;
+  if (k == 4) return m <= 16000;
+  if (csr->max_outdeg > 192 && w >= csr->wedges_min * 12 / 5 && (k >= 6 || m > 200000)) return true;
+  if (k == 5) return m <= 32000 || (m <= 120000 && w <= 36 * m);
+  if (m <= 50000 && w <= 21 * m) return true;
+  // short rows with few cliques below them: Chung-Lu of 290 000 edges (exponent 2.85) 250 / 133 us; RGG
+  // (W = W_min) of 150 000 447 / 700
+  if (m > 120000 && m <= 320000 && w <= 28 * m && w >= csr->wedges_min + 3 * (csr->wedges_min / 20)) return true;
+  return k >= 7 && m > 200000 && w >= csr->wedges_min + 3 * (csr->wedges_min / 10);
+}
+
 // k-cliques whose first two vertices (in orientation order) form an edge of [e0, e1).  by_rows:
-// sources of up to kRowMax members by rows, longer ones by the walk;
+// where walk_pays says no, sources of up to kRowMax members by rows and longer ones by the walk;
 // otherwise every edge by the walk alone.
 static atc_status kcl_window(const atc_csr* csr, uint32_t k, int64_t e0, int64_t e1, uint64_t* count, atc_stats* stats,
                              cudaStream_t s, bool by_rows = true) {
@@ -1005,12 +1050,14 @@ static atc_status kcl_window(const atc_csr* csr, uint32_t k, int64_t e0, int64_t
     CsrPriv* pv = static_cast<CsrPriv*>(csr->priv);
     const int cap = std::max(csr->max_outdeg, 1);
     const int levels = (int)k - 2;
+    const bool walk_dense = by_rows && walk_pays(csr, (int)k);
+    if (walk_dense) by_rows = false;
     const int row_max = by_rows ? kRowMax : 0;
     const bool walk = cap > row_max;  // some source is too long for rows
     int64_t grid = 0;
     DevBuf<int32_t> scratch, lists;
     DevBuf<unsigned long long> dense;
-    DevBuf<int> q;  // queues: 32-bit rows, 64-bit rows, block rows; [4..7] the block lists' counts
+    DevBuf<int> q;  // queues: 32-bit rows, 64-bit rows, block rows; from kRowCounts on the block lists' counts
     if (walk) {
       int bps = 0;
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kcl_kernel, kKcWarps * 32, 0);
@@ -1023,18 +1070,21 @@ static atc_status kcl_window(const atc_csr* csr, uint32_t k, int64_t e0, int64_t
     }
     // edges with 65..1024 members in C0 go to the dense kernel from k = 5 on (at k = 4 the walk
     // does one intersection per member of C0 as fast)
-    const bool use_dense = by_rows && k >= 5 && cap > kMaskMax;
+    const bool use_dense = (by_rows || walk_dense) && k >= 5 && cap > kMaskMax;
     if (use_dense) ATC_TRY(dense.alloc((size_t)csr->m + 2, s));
     // k >= 6: the search below one source of 33..64 members is long enough for a CTA (one warp
     // of it held R-MAT scale 14's k = 6 count at 12.8 ms, 3.8 by the walk)
     const int warp_max = k >= 6 ? 32 : kMaskMax;  // longest rows a warp takes
+    // from k = 5 on the upper half of them goes to CTAs too where they are few
+    const int few_lo = k >= 5 ? warp_max / 2 : warp_max;
+    const int few_max = k >= 6 ? (int)std::max<int64_t>(kFewRowsDeep, csr->n / 16) : kFewRows;
     const int64_t lcap = csr->m / (warp_max + 1) + 1;
-    const bool blocks = by_rows && cap > warp_max;
-    ATC_TRY(q.alloc(8, s));
-    if (blocks) ATC_TRY(lists.alloc((size_t)lcap * kRowBuckets, s));
+    const bool blocks = by_rows && cap > few_lo;
+    if (by_rows) ATC_TRY(q.alloc(kRowCounts + kRowBuckets + 1, s));
+    if (blocks) ATC_TRY(lists.alloc((size_t)lcap * kRowBuckets + few_max, s));
     tm.start(s);
     ATC_CK(cudaMemsetAsync(pv->counter, 0, 2 * sizeof(unsigned long long), s));
-    ATC_CK(cudaMemsetAsync(q.p, 0, 8 * sizeof(int), s));
+    if (by_rows) ATC_CK(cudaMemsetAsync(q.p, 0, (kRowCounts + kRowBuckets + 1) * sizeof(int), s));
     if (use_dense) ATC_CK(cudaMemsetAsync(dense.p, 0, 2 * sizeof(unsigned long long), s));
     if (walk) {
       kcl_kernel<<<(unsigned)grid, kKcWarps * 32, 0, s>>>(csr->offsets, csr->cols, pv->esrc, e0, e1, (int)k, cap,
@@ -1045,12 +1095,12 @@ static atc_status kcl_window(const atc_csr* csr, uint32_t k, int64_t e0, int64_t
     }
     if (blocks) {
       const int dmax = std::min(cap, row_max);
-      kcl_rows_list_kernel<<<grid_for(csr->n, 256), 256, 0, s>>>(csr->offsets, csr->n, e0, e1, warp_max, row_max, lcap,
-                                                                lists.p, q.p + 4);
+      kcl_rows_list_kernel<<<grid_for(csr->n, 256), 256, 0, s>>>(csr->offsets, csr->n, e0, e1, few_lo, warp_max, row_max,
+                                                                lcap, few_max, lists.p, q.p + kRowCounts);
       ATC_CK(cudaGetLastError());
       const auto launch = k == 3 ? launch_rows_block<0> : k == 4 ? launch_rows_block<1>
                           : k == 5 ? launch_rows_block<2> : launch_rows_block<3>;
-      ATC_TRY(launch(csr, e0, e1, (int)k, dmax, lists.p, lcap, q.p + 4, q.p + 2, use_dense ? dense.p + 1 : nullptr,
+      ATC_TRY(launch(csr, e0, e1, (int)k, dmax, lists.p, lcap, q.p + kRowCounts, few_max, q.p + 2, use_dense ? dense.p + 1 : nullptr,
                      pv->counter, s));
       launches += 2;
     }
@@ -1069,11 +1119,13 @@ static atc_status kcl_window(const atc_csr* csr, uint32_t k, int64_t e0, int64_t
       ++launches;
     }
     if (by_rows && cap > 32 && warp_max > 32) {
-      ATC_TRY(launch_rows_warp<unsigned long long>(csr, e0, e1, (int)k, 32, q.p + 1, pv->counter, s));
+      ATC_TRY(launch_rows_warp<unsigned long long>(csr, e0, e1, (int)k, 32, few_lo, q.p + kRowCounts + kRowBuckets, few_max, q.p + 1,
+                                                   pv->counter, s));
       ++launches;
     }
     if (by_rows) {
-      ATC_TRY(launch_rows_warp<uint32_t>(csr, e0, e1, (int)k, 0, q.p, pv->counter, s));
+      ATC_TRY(launch_rows_warp<uint32_t>(csr, e0, e1, (int)k, 0, few_lo, q.p + kRowCounts + kRowBuckets, few_max, q.p,
+                                         pv->counter, s));
       ++launches;
     }
     tm.stop(s);
