@@ -18,10 +18,11 @@
 //   longer rows up to kRowMax members (kcl_rows_block_kernel): a CTA per u, rows of 64-bit
 //     words; at k = 4 each induced edge is one AND / popc over the words, from k = 5 on a row's
 //     C0 is renumbered into shorter rows of its own by a warp (up to kRowWarp members) or, at
-//     k = 5, by the CTA; what is left goes to kcl_dense_kernel, a CTA per edge;
+//     k = 5, by the CTA; what is left goes to kcl_dense_kernel, a CTA per edge; few such rows, and
+//     from k = 5 on a few of the longer half a warp takes, are split over CTAs;
 //   longer rows still: a warp walks the search tree of one oriented edge depth first with
 //     binary searches in global memory (kcl_kernel), its C0 of 65..1024 members counted by
-//     kcl_dense_kernel from k = 5 on.  atc_tuning.kcl_dense = -1 puts every edge on that warp
+//     kcl_dense_kernel from k = 5 on; every edge so where walk_pays says.  atc_tuning.kcl_dense = -1 puts every edge on that warp
 //     search, without the dense kernel.
 //
 // Orientation is acyclic, so every k-clique is found once, from its first two vertices
@@ -30,7 +31,7 @@
 // Measured (ms, one call; the per-edge walk with its dense kernel -> rows): RGG 2^20 of mean
 // degree 32, k = 4 / 5 / 6 / 7: 22.0 / 25.2 / 39.7 / 72.8 -> 0.87 / 1.25 / 4.3 / 16.8; R-MAT
 // scale 18, k = 4 / 5 / 6: 53.7 / 69.4 / 360 -> 2.7 / 15.0 / 171; scale 20, k = 4 / 5 / 6: 424 /
-// 547 / 3697 -> 16.2 / 169 / 2464; scale 14, k = 6 / 7: 3.8 / 37.5 -> 2.3 / 30.5.  Of that, the CTA
+// 547 / 3697 -> 16.2 / 169 / 2464; scale 14, k = 6: 3.8 -> 2.3.  Of that, the CTA
 // kernel's binary searches in all of N+(u) and its grabs of 32 lists (few of its warps had any)
 // took scale 18, k = 4 from 3.8 to 2.7 when a part table and smaller grabs replaced them.
 #include <algorithm>

@@ -12,7 +12,8 @@
 //                                        table, bitmap or sorted copy in shared memory,
 //                                        the partner's shorter list streamed through it
 //                                        (sum of min(d+u, d+v) tests).  Kernels in
-//                                        bisson.cuh.
+//                                        bisson.cuh.  Whole counts of CSRs that preTC built:
+//                                        a degree-ranked copy (ranked.cu) where it pays.
 //   Fox-style     Fox/tc.cu:18-125,     per-edge work min*log2(max+2); edges binned on
 //                 316-384                the device into 1,2,4,...,32 threads per edge;
 //                                        each thread searches a slice of the shorter list
@@ -21,6 +22,7 @@
 //                                        in shared memory bracket each element of the
 //                                        shorter list, then a binary search inside the
 //                                        bracket.
+// The Fox- and TriCore-style searches run on the ranked copy too, under the same conditions.
 #include <cmath>
 #include <mutex>
 #include <vector>
@@ -261,7 +263,8 @@ __global__ void fox_deal_kernel(const uint64_t* keys, const int64_t* list, int64
 // to end stores the total and leaves the accumulator and the ticket at zero.
 // Measured, the whole call, items -> this kernel (us): R-MAT of 4.9K, 23K, 102K, 441K edges 55 -> 30,
 // 78 -> 31, 118 -> 50, 232 -> 175; Chung-Lu of 35K, 380K 93 -> 31, 115 -> 69; RGG of 45K, 473K
-// 80 -> 30, 106 -> 70, 1.6M 160 -> 180.  Bound by launches below 50K edges, then by the searches'
+// 80 -> 30, 106 -> 70, 1.6M 160 -> 180; the total stored to the caller's memory instead of copied
+// takes another 5 to 10 us off (R-MAT scale 10 27).  Bound by launches below 50K edges, then by the searches'
 // dependent loads.
 constexpr int64_t kSmallEdges = 1 << 19;
 template <int G>
@@ -847,7 +850,7 @@ static atc_status group_edges(const CsrView& g, const ItemShape& sh, Grouping* g
 // than grouping whole lists, which in turn is slow where hubs are (contended group cursors, long
 // lists).  Measured whole lists / ranked in ms: Bisson on R-MAT of 5K, 23K, 910K, 16M edges 0.12 /
 // 0.16, 0.19 / 0.16, 0.64 / 0.28, 4.8 / 1.9, Chung-Lu of 35K, 1.3M, 14M 0.21 / 0.18, 0.73 / 0.34,
-// 2.25 / 1.66, RGG (mean degree 32, W = 1.04 W_min) of 45K, 1.6M, 16M 0.11 / 0.18, 0.21 / 0.39,
+// 2.25 / 1.2, RGG (mean degree 32, W = 1.04 W_min) of 45K, 1.6M, 16M 0.11 / 0.18, 0.21 / 0.39,
 // 1.19 / 1.96.  Even degrees with long lists pay too: a test costs a third.
 static bool ranked_pays(const atc_csr* csr) {
   return csr->m >= 16384 && (csr->wedges >= csr->wedges_min + csr->wedges_min / 2 || csr->wedges_min >= 48 * csr->m);
@@ -1157,11 +1160,12 @@ atc_status atc::part_edge_range(const atc_csr* csr, uint32_t part, uint32_t npar
 // GB300 times predicts is faster.  Hu-style: 2 ps per wedge (W; 1.2 at scale 20 and above, where
 // it loses anyway) + 45 ps per edge + 0.06 ms.
 // Bisson-style, ranked: 0.37 ps per element of the shorter lists (W_min) + 85 ps per edge (the
-// ranked copy) + 0.17 ms of launches.  By whole lists (parts, loaded CSRs): 1.232 ps per
+// ranked copy) + 0.17 ms of launches (since then faster at large scales, where it wins anyway).  By whole lists (parts, loaded CSRs): 1.232 ps per
 // element of W_min + 117.5 ps per edge + 0.3 ms, against Hu's 1.097 ps and 103.5 ps, the fit of
-// the two that it was made with.  Measured Hu / ranked in ms: R-MAT scale 14 0.15 / 0.21, 16 0.37 /
-// 0.26, 18 1.30 / 0.55, 20 6.2 / 1.8, 24 231 / 47; Chung-Lu 1.3M edges 0.21 / 0.33, 9.6M 1.39 /
-// 1.18; RGG 1.6M 0.14 / 0.36, 16M 0.93 / 1.9.
+// the two that it was made with.  Measured Hu / ranked in ms: R-MAT scale 14 0.09 / 0.23, 15 0.18 /
+// 0.24, 16 0.39 / 0.27, 18 1.32 / 0.47, 20 6.4 / 1.35, 22 36 / 6.2; Chung-Lu 1.3M edges 0.27 / 0.34, 4.0M 0.68 /
+// 0.53, 9.6M 1.52 / 0.98; of exponent 3 8.0M 0.74 / 0.89; RGG 1.6M 0.17 / 0.21, 16M 0.92 / 1.18.  The model
+// picks the faster one in all of them, A-direction + A-order and by degree.
 static atc_kernel auto_kernel(const atc_csr* csr, bool ranked) {
   const double m = (double)csr->m, w = (double)csr->wedges, wmin = (double)csr->wedges_min;
   const double bisson_ps = ranked ? 0.37 * wmin + 85.0 * m + 1.7e8 : 1.232 * wmin + 117.5 * m + 3.0e8;

@@ -125,7 +125,8 @@ typedef enum atc_kernel {
   ATC_KERNEL_AUTO = 0,    /* Bisson- or Hu-style, whichever a cost model of their GB300 times
                              (W, W_min and m of the CSR) predicts is faster */
   ATC_KERNEL_HU = 1,      /* wedge walk, N+(u) staged in shared memory (Hu/tc.cu:69-201) */
-  ATC_KERNEL_BISSON = 2,  /* bitmap for large N+(u), search otherwise (Bisson/tc.cu:18-104) */
+  ATC_KERNEL_BISSON = 2,  /* lists streamed through a set of N+(v): bitmaps over a degree-ranked copy
+                             of the edges where that pays (Bisson/tc.cu:18-104) */
   ATC_KERNEL_FOX = 3,     /* edge bins with 1..32 threads per edge (Fox/tc.cu:64-125,316-384) */
   ATC_KERNEL_TRICORE = 4  /* warp per edge, 32 pivots + binary search (tricount_gpu.cu:215-290) */
 } atc_kernel;
@@ -136,7 +137,8 @@ typedef struct atc_tuning {
   int32_t prune_deg1;        /* drop degree<=1 vertices, compact ids (Hu/preTC.cu:135-169) */
   int32_t hu_blocks;         /* unused: the Hu-style kernel drains a work queue (layout kept) */
   int32_t hu_stage_ints;     /* unused: N+(u) is staged per work item (layout kept) */
-  int32_t bisson_cutover;    /* warp items: sorted copy up to this out-degree, hash above (32) */
+  int32_t bisson_cutover;    /* warp items: sorted copy up to this out-degree, hash above (32); any
+                                bisson_* value asks for grouped lists, not the ranked copy */
   int32_t fox_rearrange;     /* interleave each bin's edges (Fox/tc.cu:127-183) */
   int32_t fox_work_per_thread; /* bin base of the threads-per-edge bins (8) */
   int32_t tricore_blocks;    /* CTAs of the TriCore-style kernel (0: auto) */
@@ -148,10 +150,10 @@ typedef struct atc_tuning {
   int32_t group_by_source;   /* batches: 1 = every edge at its source, the items index the
                                 CSR rows (Hu-style wedge tests, no grouping passes); 0 = at
                                 the endpoint with the longer list (Bisson-style); 2 = each
-                                graph the way the Hu/Bisson cost model predicts faster */
-  int32_t kcl_dense;         /* k-cliques (atc_kcl_part_tuned): 0 = candidate sets of 65..1024
-                                members on the dense kernel from k = 5 on; -1 = every edge on
-                                the warp search */
+                                graph the way a cost model of the two predicts faster */
+  int32_t kcl_dense;         /* k-cliques (atc_kcl_part_tuned): 0 = sources by rows, candidate sets of
+                                65..1024 members on the dense kernel from k = 5 on; -1 = every
+                                edge on the warp search */
   int32_t edge_kernels;      /* TriCore- and Fox-style: 1 = per-edge kernels searching the longer
                                 list in global memory, as the reference kernels do (a warp per
                                 edge with 32 pivots; 1..32 threads per edge in work bins);
