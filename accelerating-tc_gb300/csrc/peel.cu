@@ -341,18 +341,18 @@ __global__ void __launch_bounds__(kPeelThreads, 2) peel_kernel(PeelArgs a) {
 struct PeelGraph {
   DevBuf<int64_t> off;
   DevBuf<int32_t> adj;
+  DevBuf<unsigned long long> cur;  // n: the scatter's cursors, then the peel's lists of the unpeeled
 };
 
 atc_status sym_graph(const SimpleEdges& e, const int32_t* deg, PeelGraph* g, cudaStream_t s) {
   const int64_t n = e.n_in, m = e.m, total = 2 * m;
-  DevBuf<unsigned long long> cur;
   ATC_TRY(g->off.alloc(n + 1, s));
   ATC_TRY(exclusive_scan_i32_to_i64(deg, g->off.p, n, s));
   ATC_CK(cudaMemcpyAsync(g->off.p + n, &total, sizeof(total), cudaMemcpyHostToDevice, s));
-  ATC_TRY(cur.alloc(n, s));
-  ATC_CK(cudaMemcpyAsync(cur.p, g->off.p, sizeof(int64_t) * n, cudaMemcpyDeviceToDevice, s));
+  ATC_TRY(g->cur.alloc(n, s));
+  ATC_CK(cudaMemcpyAsync(g->cur.p, g->off.p, sizeof(int64_t) * n, cudaMemcpyDeviceToDevice, s));
   ATC_TRY(g->adj.alloc(total, s));
-  if (m) sym_scatter_kernel<<<grid_for(m, 256), 256, 0, s>>>(e.keys.p, m, e.bits, cur.p, g->adj.p);
+  if (m) sym_scatter_kernel<<<grid_for(m, 256), 256, 0, s>>>(e.keys.p, m, e.bits, g->cur.p, g->adj.p);
   ATC_CK(cudaGetLastError());
   return ATC_OK;
 }
@@ -362,16 +362,15 @@ atc_status run_peel(const SimpleEdges& e, const PeelGraph& g, int32_t* rt, int32
                     PeelState* out, cudaStream_t s) {
   const int64_t n = e.n_in, m = e.m;
   DevBuf<int2> queue;
-  DevBuf<int32_t> alive;
   DevBuf<PeelState> st;
   // every vertex is queued once, in at most one piece more than its list has full ones
   ATC_TRY(queue.alloc((size_t)(n + 2 * m / kPeelPiece + 1), s));
-  ATC_TRY(alive.alloc(2 * (size_t)n, s));
   ATC_TRY(st.alloc(1, s));
   *out = PeelState{};
   out->step[0].smallest = INT_MAX;
   ATC_CK(cudaMemcpyAsync(st.p, out, sizeof(PeelState), cudaMemcpyHostToDevice, s));
-  PeelArgs a{g.off.p, g.adj.p, n, rt, label, queue.p, {alive.p, alive.p + n}, threshold, grow, st.p};
+  int32_t* const alive = reinterpret_cast<int32_t*>(g.cur.p);
+  PeelArgs a{g.off.p, g.adj.p, n, rt, label, queue.p, {alive, alive + n}, threshold, grow, st.p};
   int bps = 0;
   ATC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, peel_kernel<CORE>, kPeelThreads, 0));
   // about four vertices or sixteen neighbours a thread: more blocks only make the barrier dearer
