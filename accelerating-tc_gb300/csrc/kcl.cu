@@ -340,6 +340,8 @@ __device__ __forceinline__ unsigned long long pair_word_cliques(const unsigned l
 // heavy rows are spread over every thread.
 constexpr int kDenseRows = kDenseMax / kDenseThreads;  // rows a thread sums in the row scan
 static_assert(kDenseRows * kDenseThreads == kDenseMax, "the row scan covers kDenseMax rows");
+// DEEP: k >= 6, short rows with the candidate sets in registers (their code in the kernel of k = 5 cost it 20 %).
+template <bool DEEP>
 __global__ void __launch_bounds__(kDenseThreads) kcl_dense_kernel(const int64_t* off, const int32_t* cols,
                                                                   const int32_t* esrc, const unsigned long long* dense,
                                                                   int k, int cmax, unsigned long long* next,
@@ -453,8 +455,8 @@ __global__ void __launch_bounds__(kDenseThreads) kcl_dense_kernel(const int64_t*
         r -= pc;
       }
       const int j = x * 64 + select_bit(Ri[x], r);
-      if (words <= 2 && k <= 7) cnt += pair_word_cliques<2>(dsm, words, i, j, k - 4);
-      else if (words <= 4 && k <= 7) cnt += pair_word_cliques<4>(dsm, words, i, j, k - 4);
+      if (DEEP && words <= 2 && k <= 7) cnt += pair_word_cliques<2>(dsm, words, i, j, k - 4);
+      else if (DEEP && words <= 4 && k <= 7) cnt += pair_word_cliques<4>(dsm, words, i, j, k - 4);
       else cnt += pair_cliques(dsm, words, i, j, k - 4);
     }
     __syncthreads();
@@ -486,7 +488,7 @@ constexpr int kRowCounts = 4;      // the first of their counts among the queues
 // do.  Chung-Lu n = 128 000, 0.9 M edges: k = 5 517 -> 202 us, k = 6 850 -> 345; R-MAT scale 11 of 31 000
 // edges 307 -> 182 and 752 -> 456.  k >= 6: with 2048 instead Chung-Lu n = 7000 k = 6 takes 511 us (188);
 // with 65536 RGG n = 128 000 5.6 ms (2.6); Chung-Lu n = 32 000 of 0.5 M edges 970 with 8192, 650 with 16384.
-constexpr int kFewRows = 2048;
+constexpr int kFewRows = 2048;       // k = 5, or n / 32 (Chung-Lu n = 300 000 of mean degree 14 1.46 -> 1.2 ms or less)
 constexpr int kFewRowsDeep = 16384;  // k >= 6, or n / 16
 constexpr int kRowSearch = 128;    // lists longer than this are searched for the members of
                                    // N+(u), not streamed, where N+(u) fits one warp's masks
@@ -1028,8 +1030,10 @@ static bool walk_pays(const atc_csr* csr, int k) {
   const int64_t m = csr->m, w = csr->wedges;
   if (csr->max_outdeg <= (k >= 6 ? 16 : 32)) return false;  // rows by one launch
   if (k == 3) return m <= 240000;
-  if (k == 4) return m <= 16000;
-  if (csr->max_outdeg > 192 && w >= csr->wedges_min * 12 / 5 && (k >= 6 || m > 200000)) return true;
+  // up to 45 000 where few wedges close (Chung-Lu of 38 000, exponent 2.87, 81 / 67; RGG, W = W_min, 64 / 110)
+  if (k == 4) return m <= 16000 || (m <= 45000 && w <= 32 * m && w >= csr->wedges_min + 3 * (csr->wedges_min / 20));
+  if (csr->max_outdeg > 192 && w >= csr->wedges_min * 12 / 5 && (k >= 6 || m > 200000 || w >= 110 * m))
+    return true;
   if (k == 5) return m <= 32000 || (m <= 120000 && w <= 36 * m);
   if (m <= 50000 && w <= 21 * m) return true;
   // short rows with few cliques below them: Chung-Lu of 290 000 edges (exponent 2.85) 250 / 133 us; RGG
@@ -1051,14 +1055,28 @@ static atc_status kcl_window(const atc_csr* csr, uint32_t k, int64_t e0, int64_t
     CsrPriv* pv = static_cast<CsrPriv*>(csr->priv);
     const int cap = std::max(csr->max_outdeg, 1);
     const int levels = (int)k - 2;
-    const bool walk_dense = by_rows && walk_pays(csr, (int)k);
+    DevBuf<int> q;  // queues: 32-bit rows, 64-bit rows, block rows; from kRowCounts on the block lists' counts
+    DevBuf<int32_t> scratch, lists;
+    // k >= 6: the search below one source of 33..64 members is long enough for a CTA (one warp
+    // of it held R-MAT scale 14's k = 6 count at 12.8 ms, 3.8 by the walk)
+    const int warp_max = k >= 6 ? 32 : kMaskMax;  // longest rows a warp takes
+    // from k = 5 on the upper half of them goes to CTAs too where they are few
+    const int few_lo = k >= 5 ? warp_max / 2 : warp_max;
+    const int few_max =
+        (int)(k >= 6 ? std::max<int64_t>(kFewRowsDeep, csr->n / 16) : std::max<int64_t>(kFewRows, csr->n / 32));
+    const int64_t lcap = csr->m / (warp_max + 1) + 1;
+    bool walk_dense = by_rows && walk_pays(csr, (int)k);
+    if (by_rows && !walk_dense &&
+        (q.alloc(kRowCounts + kRowBuckets + 1, s) != ATC_OK ||
+         (cap > few_lo && lists.alloc((size_t)lcap * kRowBuckets + few_max, s) != ATC_OK))) {
+      cudaGetLastError();  // no room for the lists of rows: the walk needs none
+      walk_dense = true;
+    }
     if (walk_dense) by_rows = false;
     const int row_max = by_rows ? kRowMax : 0;
     const bool walk = cap > row_max;  // some source is too long for rows
     int64_t grid = 0;
-    DevBuf<int32_t> scratch, lists;
     DevBuf<unsigned long long> dense;
-    DevBuf<int> q;  // queues: 32-bit rows, 64-bit rows, block rows; from kRowCounts on the block lists' counts
     if (walk) {
       int bps = 0;
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kcl_kernel, kKcWarps * 32, 0);
@@ -1073,16 +1091,7 @@ static atc_status kcl_window(const atc_csr* csr, uint32_t k, int64_t e0, int64_t
     // does one intersection per member of C0 as fast)
     const bool use_dense = (by_rows || walk_dense) && k >= 5 && cap > kMaskMax;
     if (use_dense) ATC_TRY(dense.alloc((size_t)csr->m + 2, s));
-    // k >= 6: the search below one source of 33..64 members is long enough for a CTA (one warp
-    // of it held R-MAT scale 14's k = 6 count at 12.8 ms, 3.8 by the walk)
-    const int warp_max = k >= 6 ? 32 : kMaskMax;  // longest rows a warp takes
-    // from k = 5 on the upper half of them goes to CTAs too where they are few
-    const int few_lo = k >= 5 ? warp_max / 2 : warp_max;
-    const int few_max = k >= 6 ? (int)std::max<int64_t>(kFewRowsDeep, csr->n / 16) : kFewRows;
-    const int64_t lcap = csr->m / (warp_max + 1) + 1;
     const bool blocks = by_rows && cap > few_lo;
-    if (by_rows) ATC_TRY(q.alloc(kRowCounts + kRowBuckets + 1, s));
-    if (blocks) ATC_TRY(lists.alloc((size_t)lcap * kRowBuckets + few_max, s));
     tm.start(s);
     ATC_CK(cudaMemsetAsync(pv->counter, 0, 2 * sizeof(unsigned long long), s));
     if (by_rows) ATC_CK(cudaMemsetAsync(q.p, 0, (kRowCounts + kRowBuckets + 1) * sizeof(int), s));
@@ -1109,12 +1118,13 @@ static atc_status kcl_window(const atc_csr* csr, uint32_t k, int64_t e0, int64_t
       // rows for the largest C0 this graph can have
       const int cmax = std::min(cap, kDenseMax);
       const size_t smem = sizeof(unsigned long long) * ((size_t)cmax * ((cmax + 63) / 64) + kDensePad);
-      ATC_CK(cudaFuncSetAttribute((const void*)kcl_dense_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      const auto kern = k >= 6 ? kcl_dense_kernel<true> : kcl_dense_kernel<false>;
+      ATC_CK(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)smem));
       int dbps = 0;
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&dbps, kcl_dense_kernel, kDenseThreads, smem);
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&dbps, kern, kDenseThreads, smem);
       if (dbps < 1) dbps = 1;
-      kcl_dense_kernel<<<(unsigned)(sm_count() * dbps), kDenseThreads, smem, s>>>(
+      kern<<<(unsigned)(sm_count() * dbps), kDenseThreads, smem, s>>>(
           csr->offsets, csr->cols, pv->esrc, dense.p + 1, (int)k, cmax, dense.p, pv->counter);
       ATC_CK(cudaGetLastError());
       ++launches;

@@ -39,3 +39,25 @@ def test_complete(n, k):
     csr = atc.pretc(np.stack([i, j], 1).astype(np.int32), atc.Dir.ID)
     assert atc.kcl(csr, k)[0] == comb(n, k)
     csr.free()
+
+
+@pytest.mark.parametrize("k", [4, 5, 6])
+def test_no_room_for_the_lists(k):
+    """Whatever the budget holds, the count is right or refused, by rows or, where only their lists do not
+    fit, by the walk."""
+    csr = atc.pretc(_planted(40000, 2200, 35, 60000, 3), atc.Dir.ADIRECTION)
+    want = atc.kcl(csr, k)[0]
+    counted = False
+    try:
+        for b in range(12, 27):
+            for f in (4, 5, 6, 7):
+                atc.set_alloc_budget(f << (b - 2))
+                try:
+                    assert atc.kcl(csr, k)[0] == want
+                    counted = True
+                except atc.ATCError as e:
+                    assert "allocation budget" in str(e)
+    finally:
+        atc.set_alloc_budget(None)
+    assert counted
+    csr.free()
