@@ -488,7 +488,7 @@ constexpr int kRowCounts = 4;      // the first of their counts among the queues
 // do.  Chung-Lu n = 128 000, 0.9 M edges: k = 5 517 -> 202 us, k = 6 850 -> 345; R-MAT scale 11 of 31 000
 // edges 307 -> 182 and 752 -> 456.  k >= 6: with 2048 instead Chung-Lu n = 7000 k = 6 takes 511 us (188);
 // with 65536 RGG n = 128 000 5.6 ms (2.6); Chung-Lu n = 32 000 of 0.5 M edges 970 with 8192, 650 with 16384.
-constexpr int kFewRows = 2048;       // k = 5, or n / 32 (Chung-Lu n = 300 000 of mean degree 14 1.46 -> 1.2 ms or less)
+constexpr int kFewRows = 2048;       // k = 5, or n / 32 (Chung-Lu n = 300 000 of mean degree 14 1.46 -> 0.60 ms)
 constexpr int kFewRowsDeep = 16384;  // k >= 6, or n / 16
 constexpr int kRowSearch = 128;    // lists longer than this are searched for the members of
                                    // N+(u), not streamed, where N+(u) fits one warp's masks
