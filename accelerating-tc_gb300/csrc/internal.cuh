@@ -108,11 +108,10 @@ atc_status gro_lookup(const int2* pairs, uint64_t ne, int64_t n_v, int32_t* look
 atc_status count_ranked(const atc_csr* csr, unsigned long long* out, bool* done, cudaStream_t s, int* launches);
 
 // Private part of an atc_csr.
-constexpr int kCsrCounters = 6;
+constexpr int kCsrCounters = 4;
 struct CsrPriv {
   int32_t* esrc = nullptr;       // m: source vertex of every edge, in edge order
-  // kCsrCounters u64: [0], [1] scratch for counting kernels; [4], [5] the small count's
-  // accumulator and ticket, zero between calls
+  // kCsrCounters u64, scratch of the call that runs on the CSR: nothing is kept in them between calls
   unsigned long long* counter = nullptr;
   int bits = 1;
   // n: in-degrees of a CSR built by preTC, which orients every edge of a simple graph once;

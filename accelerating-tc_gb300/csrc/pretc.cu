@@ -912,7 +912,6 @@ static atc_status csr_load_impl(const char* path, bool host_resident, atc_csr* o
   HostMapped hcols, hesrc;
   ATC_TRY(doff.alloc(n + 1, s));
   ATC_TRY(counter.alloc(kCsrCounters, s));
-  ATC_CK(cudaMemsetAsync(counter.p, 0, sizeof(unsigned long long) * kCsrCounters, s));
   ATC_CK(cudaMemcpyAsync(doff.p, off.data(), sizeof(int64_t) * (n + 1), cudaMemcpyHostToDevice, s));
   int32_t* cols_dev;
   int32_t* esrc_dev;

@@ -259,17 +259,17 @@ __global__ void fox_deal_kernel(const uint64_t* keys, const int64_t* list, int64
 // Graphs of a few thousand edges are counted before a launch's items could be made: G lanes take
 // an edge, each every G-th element of the shorter list, and binary-search it in the longer
 // one, where both lists sit in L1 or L2 (Hu/tc.cu:69-201 searches a staged run the same way).  One
-// launch, no scratch, no item lists, no wait before the result, and no memset: the last block
-// to end stores the total and leaves the accumulator and the ticket at zero.
+// launch, no item lists, no wait before the result and no memset: every block stores its sum to a
+// place of its own in memory of the call, and the host adds them up, so that nothing outlives the call
+// and calls that overlap share nothing.
 // Measured, the whole call, items -> this kernel (us): R-MAT of 4.9K, 23K, 102K, 441K edges 55 -> 30,
 // 78 -> 31, 118 -> 50, 232 -> 175; Chung-Lu of 35K, 380K 93 -> 31, 115 -> 69; RGG of 45K, 473K
-// 80 -> 30, 106 -> 70, 1.6M 160 -> 180; the total stored to the caller's memory instead of copied
-// takes another 5 to 10 us off (R-MAT scale 10 27).  Bound by launches below 50K edges, then by the searches'
+// 80 -> 30, 106 -> 70, 1.6M 160 -> 180; the sums stored to the caller's memory instead of copied
+// take another 5 to 10 us off (R-MAT scale 10 27).  Bound by launches below 50K edges, then by the searches'
 // dependent loads.
 constexpr int64_t kSmallEdges = 1 << 19;
 template <int G>
-__global__ void __launch_bounds__(256) small_edges_kernel(CsrView g, unsigned long long* out, unsigned long long* acc,
-                                                         volatile unsigned long long* host) {
+__global__ void __launch_bounds__(256) small_edges_kernel(CsrView g, volatile unsigned long long* sums) {
   const int sub = threadIdx.x % G;
   const int64_t groups = (int64_t)gridDim.x * 256 / G;
   unsigned cnt = 0;
@@ -298,15 +298,7 @@ __global__ void __launch_bounds__(256) small_edges_kernel(CsrView g, unsigned lo
   if (threadIdx.x == 0) {
     unsigned long long t = 0;
     for (int i = 0; i < 8; ++i) t += part[i];
-    if (t) atomicAdd(&acc[0], t);
-    __threadfence();
-    if (atomicAdd(&acc[1], 1ull) == gridDim.x - 1) {  // the last block
-      __threadfence();
-      const unsigned long long total = atomicExch(&acc[0], 0ull);
-      *out = total;
-      if (host) *host = total;
-      acc[1] = 0ull;
-    }
+    sums[blockIdx.x] = t;
   }
 }
 
@@ -785,20 +777,33 @@ static bool small_pays(const atc_csr* csr, int64_t edges) {
   return part * (5.5 * (double)csr->wedges_min + 15.0 * (double)csr->m) < part * 2.0 * (double)csr->wedges + 4.7e7;
 }
 
-// host (nullable): the caller's variable, stored by the kernel (host_stores()).
-static atc_status run_small(const CsrView& g, int64_t mean_min, unsigned long long* ctr, unsigned long long* acc,
-                            unsigned long long* host, cudaStream_t s, int* launches) {
-  Phase ph("tc.count", s);
-  const int64_t edges = g.e1 - g.e0;
-  auto launch = [&](auto kern, int lanes) {
-    const int64_t want = (edges * lanes + 255) / 256;
-    kern<<<(unsigned)std::min<int64_t>(want, (int64_t)sm_count() * 8), 256, 0, s>>>(g, ctr, acc, host);
-  };
-  if (mean_min <= 8) launch(small_edges_kernel<8>, 8);
-  else if (mean_min <= 32) launch(small_edges_kernel<16>, 16);
-  else launch(small_edges_kernel<32>, 32);
+// Counts the window into *count and waits for it; tm is stopped behind the kernel.  The blocks' sums
+// go to host memory where the kernel can store there, else to device memory of the call.
+static atc_status run_small(const CsrView& g, int64_t mean_min, uint64_t* count, EventTimer* tm, cudaStream_t s,
+                            int* launches) {
+  const int lanes = mean_min <= 8 ? 8 : mean_min <= 32 ? 16 : 32;
+  const int64_t want = ((g.e1 - g.e0) * lanes + 255) / 256;
+  const unsigned grid = (unsigned)std::min<int64_t>(want, (int64_t)sm_count() * 8);
+  const bool stored = host_stores();
+  std::vector<unsigned long long> sums(grid);
+  DevBuf<unsigned long long> dev;
+  if (!stored) ATC_TRY(dev.alloc(grid, s));
+  unsigned long long* to = stored ? sums.data() : dev.p;
+  {
+    Phase ph("tc.count", s);
+    if (lanes == 8) small_edges_kernel<8><<<grid, 256, 0, s>>>(g, to);
+    else if (lanes == 16) small_edges_kernel<16><<<grid, 256, 0, s>>>(g, to);
+    else small_edges_kernel<32><<<grid, 256, 0, s>>>(g, to);
+  }
   *launches += 1;
-  return ATC_OK;  // the caller's read_bytes checks the launch
+  tm->stop(s);
+  Phase ph("tc.readback", s);
+  ATC_TRY(read_bytes(sums.data(), dev.p, sizeof(unsigned long long) * grid, stored, s));
+  const volatile unsigned long long* v = sums.data();
+  uint64_t t = 0;
+  for (unsigned i = 0; i < grid; ++i) t += v[i];
+  *count = t;
+  return ATC_OK;
 }
 
 // The Bisson-style grouping of the edges of [e0, e1): every edge {u, v} at its endpoint h
@@ -1188,48 +1193,45 @@ static atc_status tc_window(const atc_csr* csr, atc_kernel kernel, const atc_tun
     unsigned long long* ctr = pv->counter;
     Phase ph("tc", s);
     tm.start(s);
-    const bool small = kernel == ATC_KERNEL_HU && !shaped(tuning) && small_pays(csr, e1 - e0);
-    const bool stored = small && host_stores();  // the kernel itself stores the count to h
-    unsigned long long h = 0;
-    if (!small) ATC_CK(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), s));
-    switch (kernel) {
-      case ATC_KERNEL_HU:
-        if (small) ATC_TRY(run_small(g, csr->wedges_min / csr->m, ctr, pv->counter + 4, stored ? &h : nullptr, s, &launches));
-        else ATC_TRY(run_hu(g, tuning, ctr, s, &launches));
-        break;
-      case ATC_KERNEL_BISSON: {
-        bool done = false;
-        if (ranked) ATC_TRY(count_ranked(csr, ctr, &done, s, &launches));
-        if (!done) {
-          ATC_CK(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), s));
-          ATC_TRY(run_bisson(g, tuning, ctr, s, &launches));
-        }
-        break;
-      }
-      default: {
-        const bool fox = kernel == ATC_KERNEL_FOX;
-        if (tuning && tuning->edge_kernels) {
-          ATC_TRY(fox ? run_fox(g, tuning, ctr, s, &launches) : run_tricore(g, tuning, ctr, s, &launches));
+    if (kernel == ATC_KERNEL_HU && !shaped(tuning) && small_pays(csr, e1 - e0)) {
+      ATC_TRY(run_small(g, csr->wedges_min / csr->m, count, &tm, s, &launches));
+    } else {
+      ATC_CK(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), s));
+      switch (kernel) {
+        case ATC_KERNEL_HU: ATC_TRY(run_hu(g, tuning, ctr, s, &launches)); break;
+        case ATC_KERNEL_BISSON: {
+          bool done = false;
+          if (ranked) ATC_TRY(count_ranked(csr, ctr, &done, s, &launches));
+          if (!done) {
+            ATC_CK(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), s));
+            ATC_TRY(run_bisson(g, tuning, ctr, s, &launches));
+          }
           break;
         }
-        bool done = false;
-        if (ranked)
-          ATC_TRY(fox ? run_sorted_ranked<1>(csr, ctr, &done, s, &launches)
-                      : run_sorted_ranked<0>(csr, ctr, &done, s, &launches));
-        if (!done) {
-          const bool bulk = pv->host_cols == nullptr;
-          ATC_TRY(fox ? run_sorted<1>(g, csr->max_outdeg, bulk, ctr, s, &launches)
-                      : run_sorted<0>(g, csr->max_outdeg, bulk, ctr, s, &launches));
+        default: {
+          const bool fox = kernel == ATC_KERNEL_FOX;
+          if (tuning && tuning->edge_kernels) {
+            ATC_TRY(fox ? run_fox(g, tuning, ctr, s, &launches) : run_tricore(g, tuning, ctr, s, &launches));
+            break;
+          }
+          bool done = false;
+          if (ranked)
+            ATC_TRY(fox ? run_sorted_ranked<1>(csr, ctr, &done, s, &launches)
+                        : run_sorted_ranked<0>(csr, ctr, &done, s, &launches));
+          if (!done) {
+            const bool bulk = pv->host_cols == nullptr;
+            ATC_TRY(fox ? run_sorted<1>(g, csr->max_outdeg, bulk, ctr, s, &launches)
+                        : run_sorted<0>(g, csr->max_outdeg, bulk, ctr, s, &launches));
+          }
+          break;
         }
-        break;
       }
-    }
-    tm.stop(s);
-    {
+      tm.stop(s);
       Phase ph_rb("tc.readback", s);
-      ATC_TRY(read_bytes(&h, ctr, sizeof(h), stored, s));
+      unsigned long long h = 0;
+      ATC_TRY(read_bytes(&h, ctr, sizeof(h), false, s));
+      *count = h;
     }
-    *count = *static_cast<volatile unsigned long long*>(&h);
   }
   if (stats) {
     stats->kernel_ms = e1 > e0 ? tm.ms() : 0.0f;
