@@ -97,22 +97,25 @@ void phase_add(const char* name, float ms) {
   L.recs.push_back(r);
 }
 
-Phase::Phase(const char* name, cudaStream_t s) : s_(s) {
+Phase::Phase(const char* name, cudaStream_t s) noexcept : s_(s) {
   nvtxRangePushA(name);
   PhaseLog& L = g_phases;
   if (!L.on) return;
   PhaseRec r{};
   snprintf(r.name, sizeof(r.name), "%s", name);
-  r.depth = L.depth++;
-  if (cudaEventCreate(&r.a) != cudaSuccess || cudaEventCreate(&r.b) != cudaSuccess ||
-      cudaEventRecord(r.a, s) != cudaSuccess) {
-    if (r.a) cudaEventDestroy(r.a);
-    if (r.b) cudaEventDestroy(r.b);
-    --L.depth;
-    return;
+  r.depth = L.depth;
+  if (cudaEventCreate(&r.a) == cudaSuccess && cudaEventCreate(&r.b) == cudaSuccess &&
+      cudaEventRecord(r.a, s) == cudaSuccess) {
+    try {
+      L.recs.push_back(r);
+      ++L.depth;
+      slot_ = (int)L.recs.size() - 1;
+      return;
+    } catch (const std::exception&) {  // no host memory for the record
+    }
   }
-  slot_ = (int)L.recs.size();
-  L.recs.push_back(r);
+  if (r.a) cudaEventDestroy(r.a);
+  if (r.b) cudaEventDestroy(r.b);
 }
 
 Phase::~Phase() {

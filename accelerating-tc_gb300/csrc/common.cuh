@@ -82,10 +82,12 @@ void phase_add(const char* name, float ms);
 // A named phase of a call: an NVTX range (visible to Nsight tools and ncu's NVTX filters)
 // and, when phase timing is on for the calling thread (atc_phase_timing), a pair of CUDA
 // events on the phase's stream, read back by atc_phase_times.  Phases nest; a phase is
-// recorded with its nesting depth.
+// recorded with its nesting depth.  A phase that cannot be recorded (no event, no host memory) is left
+// out: it never throws, for it may open between a kernel that stores to the call's host memory and the
+// wait for it.
 class Phase {
  public:
-  Phase(const char* name, cudaStream_t s);
+  Phase(const char* name, cudaStream_t s) noexcept;
   ~Phase();
   Phase(const Phase&) = delete;
   Phase& operator=(const Phase&) = delete;
