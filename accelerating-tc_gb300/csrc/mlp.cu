@@ -141,9 +141,11 @@ __global__ void standardise_kernel(float* X, const float* mean, const float* inv
 // parameters in shared memory and takes tiles of kTileRows rows through the forward pass, the
 // masked error, the backward pass and the weight gradients; each CTA adds up its tiles'
 // gradients in shared memory and writes them once, and a second kernel adds the CTAs' sums in
-// order and divides by the mask's sum.  The order of every sum is fixed by the sizes alone, so
-// results are deterministic.  Networks whose parameters and gradients do not fit shared memory
-// use the layer kernels above.
+// order and divides by the mask's sum.  The order of every sum is fixed by the sizes and the GPU's
+// number of SMs, so results are deterministic.  The mask's sum is known only at the end, so the errors
+// are scaled by a power of two near 1 / (B O) (exact) on the way, which keeps the sums in the range that
+// dividing first would.  Networks whose parameters and gradients do not fit shared memory use the layer
+// kernels above.
 // Measured, gradients of 480 rows of the 6-64-64-24 network, the whole call from host arrays: 349 us
 // with a kernel per layer and gradient (183 us in the weight gradients' serial sums) and
 // thirteen buffers, 75 us so, 59 with the rows read and the results stored in host memory in place; error
@@ -164,6 +166,7 @@ struct FusedArgs {
   const float *x, *t, *mask;  // mask: null = all ones
   const int32_t* pick;        // rows of x, t and mask to use (null: rows 0..B-1)
   int B, I, H, O;
+  float scale;                // grad: of the errors
   float* y;                   // forward only: B x O
   float* partial;             // grad: per CTA nparams gradients, sum of M (Y - T)^2, sum of M
 };
@@ -220,7 +223,7 @@ __global__ void __launch_bounds__(kFusedThreads) mlp_tile_kernel(FusedArgs a) {
       const int r = i / O;
       const int64_t at = row(r) * O + (i - r * O);
       const float m = a.mask ? a.mask[at] : 1.0f, d = Y[i] - a.t[at];
-      DY[i] = m * d;
+      DY[i] = m * d * a.scale;
       err += m * d * d;
       cnt += m;
     }
@@ -283,8 +286,9 @@ __global__ void __launch_bounds__(kFusedThreads) mlp_tile_kernel(FusedArgs a) {
   }
 }
 
-// grads[i] = sum over the CTAs / sum of M;  grads[nparams] = the loss.  Compensated sums (the
+// grads[i] = sum over the CTAs / (sum of M * scale);  grads[nparams] = the loss.  Compensated sums (the
 // rounding of every addition is added up apart), in float: FP64 runs at a small fraction of its rate.
+// Of a sum that has left the range nothing is left to add up: it stays an infinity.
 __device__ __forceinline__ float column_sum(const float* partial, int ctas, int64_t stride) {
   float acc = 0.0f, low = 0.0f;
 #pragma unroll 8
@@ -293,15 +297,15 @@ __device__ __forceinline__ float column_sum(const float* partial, int ctas, int6
     low = __fadd_rn(low, __fadd_rn(__fsub_rn(acc, __fsub_rn(sum, back)), __fsub_rn(x, back)));
     acc = sum;
   }
-  return acc + low;
+  return isfinite(acc) ? acc + low : acc;
 }
 
-__global__ void mlp_reduce_kernel(const float* partial, int ctas, int nparams, float* grads) {
+__global__ void mlp_reduce_kernel(const float* partial, int ctas, int nparams, float unscale, float* grads) {
   float cnt = column_sum(partial + nparams + 1, ctas, nparams + 2);
   if (!(cnt > 0.0f)) cnt = 1.0f;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= nparams; i += gridDim.x * blockDim.x) {
     const float acc = column_sum(partial + i, ctas, nparams + 2);
-    grads[i] = i < nparams ? acc / cnt : 0.5f * acc / cnt;
+    grads[i] = i < nparams ? acc / cnt * unscale : 0.5f * acc / cnt;
   }
 }
 
@@ -324,10 +328,12 @@ atc_status launch_tiles(const atc_mlp* net, FusedArgs a, cudaStream_t st) {
 }
 
 // grads: nparams + 1 floats (the loss last); partial: fused_ctas(B) * (nparams + 2).
-atc_status fused_gradients(const atc_mlp* net, const FusedArgs& a, float* grads, cudaStream_t st) {
+atc_status fused_gradients(const atc_mlp* net, FusedArgs a, float* grads, cudaStream_t st) {
+  const int bits = std::ilogb((double)a.B * net->O);
+  a.scale = std::ldexp(1.0f, -bits);
   ATC_TRY(launch_tiles<true>(net, a, st));
   const int n = (int)net->nparams;
-  mlp_reduce_kernel<<<(n + 128) / 128, 128, 0, st>>>(a.partial, fused_ctas(a.B), n, grads);
+  mlp_reduce_kernel<<<(n + 128) / 128, 128, 0, st>>>(a.partial, fused_ctas(a.B), n, std::ldexp(1.0f, bits), grads);
   ATC_CK(cudaGetLastError());
   return ATC_OK;
 }
