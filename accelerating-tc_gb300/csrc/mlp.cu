@@ -193,9 +193,9 @@ __global__ void __launch_bounds__(kFusedThreads) mlp_tile_kernel(FusedArgs a) {
   float *gW1 = G, *gb1 = gW1 + I * H, *gW2 = gb1 + H, *gb2 = gW2 + H * H, *gW3 = gb2 + H, *gb3 = gW3 + H * O;
   float err = 0.0f, cnt = 0.0f;
   __syncthreads();
-  for (int r0 = blockIdx.x * kTileRows; r0 < a.B; r0 += gridDim.x * kTileRows) {
-    const int R = min(kTileRows, a.B - r0);
-    auto row = [&](int r) { return (int64_t)(a.pick ? a.pick[r0 + r] : r0 + r); };
+  for (int64_t r0 = blockIdx.x * kTileRows; r0 < a.B; r0 += gridDim.x * kTileRows) {
+    const int R = (int)min((int64_t)kTileRows, a.B - r0);
+    auto row = [&](int r) { return a.pick ? (int64_t)a.pick[r0 + r] : r0 + r; };
     for (int i = t; i < R * I; i += kFusedThreads) {
       const int r = i / I, k = i - r * I;
       const float v = a.x[row(r) * I + k];
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(kFusedThreads) mlp_tile_kernel(FusedArgs a) {
     layer(A1, H, W2, b2, A2, H, true);
     layer(A2, H, W3, b3, Y, O, false);
     if (!GRAD) {
-      for (int i = t; i < R * O; i += kFusedThreads) a.y[(int64_t)r0 * O + i] = Y[i];
+      for (int i = t; i < R * O; i += kFusedThreads) a.y[r0 * O + i] = Y[i];
       continue;
     }
     for (int i = t; i < R * O; i += kFusedThreads) {
@@ -311,7 +311,7 @@ __global__ void mlp_reduce_kernel(const float* partial, int ctas, int nparams, f
 
 bool fused_fits(const atc_mlp* net, bool grad) { return fused_smem(net->I, net->H, net->O, grad) <= kFusedSmemMax; }
 
-int fused_ctas(int B) { return std::min((B + kTileRows - 1) / kTileRows, sm_count()); }
+int fused_ctas(int B) { return std::min((B - 1) / kTileRows + 1, sm_count()); }
 
 template <bool GRAD>
 atc_status launch_tiles(const atc_mlp* net, FusedArgs a, cudaStream_t st) {
