@@ -144,8 +144,8 @@ __global__ void standardise_kernel(float* X, const float* mean, const float* inv
 // order and divides by the mask's sum.  The order of every sum is fixed by the sizes and the GPU's
 // number of SMs, so results are deterministic.  The mask's sum is known only at the end, so the errors
 // are scaled by a power of two near 1 / (B O) (exact) on the way, which keeps the sums in the range that
-// dividing first would.  Networks whose parameters and gradients do not fit shared memory use the layer
-// kernels above.
+// dividing first would.  Networks whose parameters and gradients do not fit shared memory, and calls
+// whose scratch is refused, use the layer kernels above.
 // Measured, gradients of 480 rows of the 6-64-64-24 network, the whole call from host arrays: 349 us
 // with a kernel per layer and gradient (183 us in the weight gradients' serial sums) and
 // thirteen buffers, 75 us so, 59 with the rows read and the results stored in host memory in place; error
@@ -345,18 +345,30 @@ bool direct_io(int rows, const atc_mlp* net) {
   return host_stores() && (size_t)rows * (net->I + 2 * net->O) <= (1u << 18);
 }
 
+// mean, then 1 / std: 2 I floats.
+void pack_scaling(const atc_mlp* net, float* to) {
+  for (int i = 0; i < net->I; ++i) {
+    to[i] = net->mean[i];
+    to[net->I + i] = net->stdv[i] > 0 ? 1.0f / net->stdv[i] : 1.0f;
+  }
+}
+
 // One host array of the call's inputs, so that they take one copy: mean, 1 / std, x, t, mask.
 std::vector<float> pack_inputs(const atc_mlp* net, const float* x, const float* t, const float* mask, int B) {
   const size_t I = net->I, O = net->O, nx = (size_t)B * I, nt = t ? (size_t)B * O : 0;
   std::vector<float> h(2 * I + nx + nt + (mask ? nt : 0));
-  for (size_t i = 0; i < I; ++i) {
-    h[i] = net->mean[i];
-    h[I + i] = net->stdv[i] > 0 ? 1.0f / net->stdv[i] : 1.0f;
-  }
+  pack_scaling(net, h.data());
   memcpy(h.data() + 2 * I, x, sizeof(float) * nx);
   if (t) memcpy(h.data() + 2 * I + nx, t, sizeof(float) * nt);
   if (mask) memcpy(h.data() + 2 * I + nx + nt, mask, sizeof(float) * nt);
   return h;
+}
+
+// Room for the tile kernels' sums; false where it is refused: the layer kernels need less.
+bool tiles_alloc(DevBuf<float>* mem, size_t count, cudaStream_t s) {
+  if (mem->alloc(count, s) == ATC_OK) return true;
+  cudaGetLastError();
+  return false;
 }
 
 unsigned grid_small(int64_t work) { return (unsigned)std::min<int64_t>((work + 255) / 256, 4096); }
@@ -603,7 +615,7 @@ extern "C" atc_status atc_mlp_scaling(atc_mlp* net, float* get_mean, float* get_
 extern "C" atc_status atc_mlp_forward(atc_mlp* net, const float* x, int32_t rows, float* y, atc_stream st) try {
   ATC_CHECK_ARG(net != nullptr && x != nullptr && y != nullptr && rows > 0, "bad argument");
   cudaStream_t s = as_stream(st);
-  if (fused_fits(net, false)) {
+  if (fused_fits(net, false)) {  // needs less device memory than the layers
     const std::vector<float> in = pack_inputs(net, x, nullptr, nullptr, rows);
     const size_t ny = (size_t)rows * net->O;
     const bool direct = direct_io(rows, net);
@@ -639,13 +651,14 @@ extern "C" atc_status atc_mlp_gradients(atc_mlp* net, const float* x, const floa
                                         float* grads, float* loss, atc_stream st) try {
   ATC_CHECK_ARG(net != nullptr && x != nullptr && t != nullptr && rows > 0, "bad argument");
   cudaStream_t s = as_stream(st);
-  if (fused_fits(net, true)) {
+  const size_t np = (size_t)net->nparams, nx = (size_t)rows * net->I, nt = (size_t)rows * net->O;
+  const bool direct = direct_io(rows, net);
+  const size_t n_in = direct ? 0 : 2 * (size_t)net->I + nx + (mask ? 2 : 1) * nt;
+  DevBuf<float> mem;
+  if (fused_fits(net, true) &&
+      tiles_alloc(&mem, (direct ? 0 : n_in + np + 1) + (size_t)fused_ctas(rows) * (np + 2), s)) {
     const std::vector<float> in = pack_inputs(net, x, t, mask, rows);
-    const size_t np = (size_t)net->nparams, nx = (size_t)rows * net->I, nt = (size_t)rows * net->O;
-    const bool direct = direct_io(rows, net);
     std::vector<float> out(np + 1);
-    DevBuf<float> mem;
-    ATC_TRY(mem.alloc((direct ? 0 : in.size() + np + 1) + (size_t)fused_ctas(rows) * (np + 2), s));
     float* g = direct ? out.data() : mem.p + in.size();
     if (!direct) ATC_CK(cudaMemcpyAsync(mem.p, in.data(), sizeof(float) * in.size(), cudaMemcpyHostToDevice, s));
     const float* src = direct ? in.data() : mem.p;
@@ -694,19 +707,28 @@ extern "C" atc_status atc_mlp_train(atc_mlp* net, const float* x, const float* t
     net->mean[i] = (float)mu;
     net->stdv[i] = (float)std::sqrt(var / rows) > 1e-6f ? (float)std::sqrt(var / rows) : 1.0f;
   }
-  const bool fused = fused_fits(net, true);
   Scratch sc;
-  ATC_TRY(alloc_scratch(sc, net, batch, s));
   DevBuf<float> X, T, M, G;
   DevBuf<int32_t> idx;
-  if (fused) ATC_TRY(G.alloc((size_t)net->nparams + 1 + (size_t)fused_ctas(batch) * (net->nparams + 2), s));
-  float* const grads = fused ? G.p : sc.grads.p;
   ATC_TRY(X.alloc((size_t)rows * I, s));
   ATC_TRY(T.alloc((size_t)rows * O, s));
   ATC_TRY(M.alloc((size_t)rows * O, s));
   ATC_TRY(idx.alloc(batch, s));
+  // the gradients and the loss, the CTAs' sums, mean and 1 / std
+  const size_t sums = (size_t)net->nparams + 1 + (size_t)fused_ctas(batch) * (net->nparams + 2);
+  const bool fused = fused_fits(net, true) && tiles_alloc(&G, sums + 2 * (size_t)I, s);
+  if (fused) {
+    std::vector<float> in(2 * (size_t)I);
+    pack_scaling(net, in.data());
+    ATC_CK(cudaMemcpyAsync(G.p + sums, in.data(), sizeof(float) * in.size(), cudaMemcpyHostToDevice, s));
+    ATC_CK(cudaStreamSynchronize(s));  // `in` ends here
+  } else {
+    ATC_TRY(alloc_scratch(sc, net, batch, s));
+  }
+  float* const grads = fused ? G.p : sc.grads.p;
+  const float* const mean = fused ? G.p + sums : sc.mean.p;
   ATC_CK(cudaMemcpyAsync(X.p, x, sizeof(float) * rows * I, cudaMemcpyHostToDevice, s));
-  standardise_kernel<<<grid_small((int64_t)rows * I), 256, 0, s>>>(X.p, sc.mean.p, sc.inv.p, rows, I);
+  standardise_kernel<<<grid_small((int64_t)rows * I), 256, 0, s>>>(X.p, mean, fused ? mean + I : sc.inv.p, rows, I);
   ATC_CK(cudaMemcpyAsync(T.p, t, sizeof(float) * rows * O, cudaMemcpyHostToDevice, s));
   if (mask) {
     ATC_CK(cudaMemcpyAsync(M.p, mask, sizeof(float) * rows * O, cudaMemcpyHostToDevice, s));

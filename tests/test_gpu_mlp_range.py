@@ -1,5 +1,5 @@
-"""The selector's network where sums leave the range, and its forward pass over several tiles a CTA and odd
-layers."""
+"""The selector's network where sums leave the range, where the tile kernels' scratch is refused, and its
+forward pass over several tiles a CTA and odd layers."""
 import numpy as np
 import pytest
 
@@ -59,6 +59,26 @@ def test_one_infinite_target():
     assert loss == np.inf
     b3 = g[-24:]
     assert b3[5] == -np.inf and np.isfinite(np.delete(b3, 5)).all()
+
+
+@pytest.mark.parametrize("B,H", [(30, 64), (480, 64), (480, 100)])
+def test_no_room_for_the_tiles(B, H):
+    """The layer kernels take over where the tile kernels' sums are refused; the values agree within the
+    tolerance of both against the oracle."""
+    net, x, t, _, _ = _case(B, 6, H, 24, 3)
+    loss, g = net.gradients(x, t)
+    p = net.params()
+    # what the layers hold: rows of 6, 24 and H values several times over, and the gradients
+    layers = 4 * (B * (6 + 4 * 24 + 4 * H) + p.size + 64)
+    try:
+        atc.set_alloc_budget(layers)
+        loss2, g2 = net.gradients(x, t)
+        atc.set_alloc_budget(2 * layers)
+        net.train(x, t, epochs=1, batch=B, seed=1)
+    finally:
+        atc.set_alloc_budget(None)
+    assert abs(loss - loss2) <= 1e-4 * max(1.0, abs(loss))
+    assert np.abs(g - g2).max() <= 2e-4 * max(np.abs(g).max(), 1e-3)
 
 
 @pytest.mark.parametrize("B", [1, 7, 8, 9, 480, 1217, 1300, 5000])
