@@ -24,6 +24,7 @@ struct atc_batch {
   int32_t* cols = nullptr;     // ecap + 16
   std::vector<int64_t> vbase{0};
   std::vector<int64_t> gm, gw, gwmin;  // per graph: edges, W, sum of min(d+u, d+v)
+  std::vector<int32_t> gmax;           // per graph: longest list
   int32_t max_outdeg = 0;
   bool dirty = true;
   int rows_graphs = 0;  // graphs of the last built pipeline counted by rows
@@ -175,6 +176,7 @@ extern "C" atc_status atc_batch_add(atc_batch* b, const atc_csr* csr, int32_t* i
   b->gm.push_back(csr->m);
   b->gw.push_back(csr->wedges);
   b->gwmin.push_back(csr->wedges_min);
+  b->gmax.push_back(csr->max_outdeg);
   b->max_outdeg = std::max(b->max_outdeg, csr->max_outdeg);
   b->dirty = true;
   return ATC_OK;
@@ -440,6 +442,32 @@ ItemShape rows_shape(ItemShape sh) {
   return sh;
 }
 
+// Mode 2: the graphs counted by rows.  ps, fitted to 105 batches of 1 to 48 R-MAT, Chung-Lu and random geometric
+// graphs, each in both modes: rows cost per wedge (more in graphs of many ids, whose tags are wider), edge
+// and vertex; grouping per element of the shorter lists, edge and vertex, and once for the whole batch
+// what its hubs' cursors take, 8 us per member of the longest list (R-MAT scale 18, grouped, 1, 2 and 6 graphs 3.7,
+// 4.3 and 7.5 ms).  In no batch slower than the choice by 1.097 W + 103.5 m against 1.232 W_min + 117.5 m that the
+// earlier kernels were given; R-MAT scale 20 by rows / grouped: of 15.7M edges 17.1 / 8.6 ms, of 4.1M 1.65 / 2.3, six of those
+// 7.1 / 5.4; 48 Chung-Lu graphs 2.3 / 5.2.
+std::vector<bool> rows_graphs(const atc_batch* b) {
+  constexpr double kHubPs = 8.0e6;
+  const size_t ng = b->gm.size();
+  std::vector<bool> rows(ng, true);
+  double gain = 0.0;
+  int32_t longest = 0;
+  for (size_t q = 0; q < ng; ++q) {
+    const double n = (double)(b->vbase[q + 1] - b->vbase[q]), m = (double)b->gm[q];
+    const double by_rows = (n > 300000.0 ? 2.1 : 1.3) * (double)b->gw[q] + 10.0 * m + 350.0 * n;
+    const double grouped = 1.2 * (double)b->gwmin[q] + 100.0 * m + 60.0 * n;
+    if (by_rows <= grouped) continue;
+    rows[q] = false;
+    gain += by_rows - grouped;
+    longest = std::max(longest, b->gmax[q]);
+  }
+  if (gain <= kHubPs * longest) rows.assign(ng, true);
+  return rows;
+}
+
 // Sizes the scratch for the union and records the counting pipeline into a CUDA graph
 // on the batch's own stream (capture is not allowed on the legacy default stream).
 atc_status build_pipeline(atc_batch* b, const ItemShape& sh, cudaStream_t s) {  // by_source == 1: of rows_shape
@@ -513,9 +541,7 @@ atc_status build_pipeline(atc_batch* b, const ItemShape& sh, cudaStream_t s) {  
   CompactItems bitems{b->items, gstart, cap_items, true, true, sh};
   CompactItems litems{b->big, gstart, big_cap, false, true, sh};
   // mode 2: each graph counts by rows (every wedge tested at its source, W tests, no grouping)
-  // or grouped at the longer endpoint (sum of min(d+u, d+v) tests plus the grouping passes),
-  // whichever the per-graph cost model of the two kernels predicts faster (the per-call terms
-  // of the single-graph model do not apply inside one replay)
+  // or grouped at the longer endpoint (sum of min(d+u, d+v) tests plus the grouping passes): rows_graphs
   const bool mixed = sh.by_source == 2;
   CompactItems witems_r{b->items_r, b->off, cap_rows, false, false, shr};
   CompactItems bitems_r{b->items_r, b->off, cap_rows, true, true, shr};
@@ -523,18 +549,12 @@ atc_status build_pipeline(atc_batch* b, const ItemShape& sh, cudaStream_t s) {  
   int nrows = 0;
   if (mixed) {
     ATC_CK(cudaMemsetAsync(b->vrows, 0, (size_t)n + 1, s));
-    for (int q = 0; q < ng; ++q) {
-      const double m_q = (double)b->gm[q];
-      // ps, fitted to R-MAT and Chung-Lu graphs alone and in batches.  Grouping's 250 ps an edge
-      // holds the contended cursors of the hubs: measured by rows / grouped, R-MAT scale 14 113 / 521 ps
-      // an edge in all, 16 165 / 647, 18 534 / 958, 20 1101 / 569, 22 1470 / 452, Chung-Lu 1M vertices
-      // 124 / 268, 4M 165 / 183, a batch of 48 Chung-Lu graphs 73 / 166
-      const bool rows = 1.3 * (double)b->gw[q] + 30.0 * m_q < 1.2 * (double)b->gwmin[q] + 250.0 * m_q;
-      if (rows && b->vbase[q + 1] > b->vbase[q]) {
+    const std::vector<bool> rows = rows_graphs(b);
+    for (int q = 0; q < ng; ++q)
+      if (rows[q] && b->vbase[q + 1] > b->vbase[q]) {
         ATC_CK(cudaMemsetAsync(b->vrows + b->vbase[q], 1, (size_t)(b->vbase[q + 1] - b->vbase[q]), s));
         ++nrows;
       }
-    }
     ATC_CK(cudaStreamSynchronize(s));
   }
   b->rows_graphs = mixed ? nrows : (sh.by_source == 1 ? ng : 0);

@@ -596,6 +596,17 @@ BATCH_CANDIDATES = [{}, {"bisson_warp_max": 128}, {"bisson_warp_max": 64, "bisso
                     {"group_by_source": 2}, {"group_by_source": 2, "bisson_cutover": 64}]
 
 
+def rows_graphs(gstats):
+    """The graphs of (m, W, sum of min, n, longest list) that group_by_source = 2 counts by rows
+    (rows_graphs in csrc/batch.cu)."""
+    by_rows = [(2.1 if n > 300000 else 1.3) * w + 10.0 * m + 350.0 * n for m, w, _, n, _ in gstats]
+    grouped = [1.2 * wm + 100.0 * m + 60.0 * n for m, _, wm, n, _ in gstats]
+    rows = [r <= g for r, g in zip(by_rows, grouped)]
+    gain = sum(r - g for r, g, by in zip(by_rows, grouped, rows) if not by)
+    longest = max((x[4] for x, by in zip(gstats, rows) if not by), default=0)
+    return rows if gain > 8.0e6 * longest else [True] * len(gstats)
+
+
 def batch_leg(a, indices, plain_kernels, sp, stream=None, candidates=None):
     """Graphs `indices` of the seeded Chung-Lu batch (batch_params(4096, seed)) counted in one
     CUDA-graph replay (autotuned items) and, for comparison, one atc_tc call per graph with each
@@ -619,7 +630,7 @@ def batch_leg(a, indices, plain_kernels, sp, stream=None, candidates=None):
     plain_dev = [[] for _ in kfixed]  # device time of the counting kernels of each call
     plain_counts = []
     dirs = []
-    gstats = []  # (m, W, sum of min) of every graph as added
+    gstats = []  # (m, W, sum of min, n, longest list) of every graph as added
     wmin_adir = wmin_sel = 0
     # the per-graph calls are timed with L2 flushed before each (a graph counted right after
     # it was built or warmed would otherwise be read from L2, which a pass over many graphs,
@@ -649,7 +660,7 @@ def batch_leg(a, indices, plain_kernels, sp, stream=None, candidates=None):
             if alt.wedges_min < csr.wedges_min:
                 chosen, dsel = alt, "degree"
         wmin_sel += chosen.wedges_min
-        gstats.append((chosen.m, chosen.wedges, chosen.wedges_min))
+        gstats.append((chosen.m, chosen.wedges, chosen.wedges_min, chosen.n, chosen.max_outdeg))
         dirs.append(dsel)
         batch.add(chosen, stream=sp)
         csr.free()
@@ -684,7 +695,7 @@ def batch_leg(a, indices, plain_kernels, sp, stream=None, candidates=None):
     names = [kf.name.lower() for kf in kfixed]
     if "hu" in names and "bisson" in names:
         hu_dev, bi_dev = plain_dev[names.index("hu")], plain_dev[names.index("bisson")]
-        rows = [1.097 * w + 103.5 * m < 1.232 * wm + 117.5 * m for m, w, wm in gstats]
+        rows = rows_graphs(gstats)
         split = {"rows_graphs": int(sum(rows)), "rows_edges": int(sum(g[0] for g, r in zip(gstats, rows) if r)),
                  "hu_device_ms_rows_graphs": float(sum(t for t, r in zip(hu_dev, rows) if r)),
                  "bisson_device_ms_grouped_graphs": float(sum(t for t, r in zip(bi_dev, rows) if not r)),

@@ -1,8 +1,9 @@
-// Rules of the library that show in times only: a batch's item shapes.  One section per argument; prints
-// "ok" or what differs.
+// Rules of the library that show in times only: a batch's item shapes, and which of its graphs are counted
+// by rows.  One section per argument; prints "ok" or what differs.
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <vector>
 
 #include "batch.cu"
 
@@ -35,10 +36,42 @@ static int shapes() {
   return 0;
 }
 
+// Which graphs of a batch are counted by rows, for batches of `graphs` equal graphs whose two modes were
+// measured (ms by rows / grouped beside each).
+static bool by_rows(int graphs, int64_t n, int64_t m, double w, double wmin, int32_t longest) {
+  atc_batch b;
+  for (int q = 0; q < graphs; ++q) {
+    b.vbase.push_back(b.vbase.back() + n);
+    b.gm.push_back(m);
+    b.gw.push_back((int64_t)(w * (double)m));
+    b.gwmin.push_back((int64_t)(wmin * (double)m));
+    b.gmax.push_back(longest);
+  }
+  const std::vector<bool> rows = rows_graphs(&b);
+  return rows.size() == (size_t)graphs && rows[0] && rows[graphs - 1];
+}
+
+static int choice() {
+  REQUIRE(!by_rows(1, 1048576, 15701789, 286.8, 127.6, 615));  // R-MAT scale 20: 17.1 / 8.6
+  REQUIRE(!by_rows(2, 1048576, 15700815, 292.3, 129.6, 615));  // 33.1 / 12.9
+  REQUIRE(by_rows(1, 1048576, 4087819, 94.7, 39.3, 200));      // 1.65 / 2.34
+  REQUIRE(!by_rows(6, 1048576, 4087656, 96.1, 39.7, 204));     // 7.1 / 5.4
+  REQUIRE(by_rows(1, 262144, 3805211, 178.7, 86.9, 375));      // scale 18: 2.1 / 3.7
+  REQUIRE(by_rows(6, 262144, 3805306, 181.6, 87.8, 375));      // 6.6 / 7.5
+  REQUIRE(!by_rows(6, 262144, 7253730, 300.3, 150.4, 588));    // 18.9 / 16.5
+  REQUIRE(by_rows(1, 2000000, 38453316, 51.3, 23.2, 136));     // Chung-Lu: 3.1 / 6.0
+  REQUIRE(by_rows(48, 20000, 357849, 29.1, 18.9, 54));         // 1.0 / 2.6
+  REQUIRE(by_rows(12, 500000, 5979693, 8.8, 8.4, 24));         // RGG: 4.0 / 5.5
+  atc_batch none;
+  REQUIRE(rows_graphs(&none).empty());
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const char* const what = argc > 1 ? argv[1] : "";
   int r = 2;
   if (!strcmp(what, "shapes")) r = shapes();
+  if (!strcmp(what, "choice")) r = choice();
   if (r == 0) std::printf("ok\n");
   return r;
 }

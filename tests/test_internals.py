@@ -34,3 +34,15 @@ def _run(program, section):
 
 def test_batch_shapes(program):
     _run(program, "shapes")
+
+
+def test_batch_choice(program):
+    """Also the benchmark's copy of the rule, on the same batches."""
+    _run(program, "choice")
+    import bench
+    for graphs, n, m, w, wmin, longest, rows in ((1, 1048576, 15701789, 286.8, 127.6, 615, False),
+                                                 (1, 1048576, 4087819, 94.7, 39.3, 200, True),
+                                                 (6, 1048576, 4087656, 96.1, 39.7, 204, False),
+                                                 (48, 20000, 357849, 29.1, 18.9, 54, True)):
+        assert bench.rows_graphs([(m, w * m, wmin * m, n, longest)] * graphs) == [rows] * graphs
+    assert bench.rows_graphs([]) == []
