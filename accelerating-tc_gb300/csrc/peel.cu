@@ -375,9 +375,19 @@ atc_status run_peel(const SimpleEdges& e, const PeelGraph& g, int32_t* rt, int32
   ATC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, peel_kernel<CORE>, kPeelThreads, 0));
   // about four vertices or sixteen neighbours a thread: more blocks only make the barrier dearer
   const int64_t want = (n / 4 + m / 8) / kPeelThreads + 1;
-  const unsigned grid = (unsigned)std::min<int64_t>(want, (int64_t)sm_count() * std::min(std::max(bps, 1), 2));
+  unsigned grid = (unsigned)std::min<int64_t>(want, (int64_t)sm_count() * std::min(std::max(bps, 1), 2));
   void* args[] = {&a};
-  ATC_CK(cudaLaunchCooperativeKernel((const void*)peel_kernel<CORE>, dim3(grid), dim3(kPeelThreads), args, 0, s));
+  for (;;) {
+    const cudaError_t launched =
+        cudaLaunchCooperativeKernel((const void*)peel_kernel<CORE>, dim3(grid), dim3(kPeelThreads), args, 0, s);
+    // the stream may have fewer SMs than the device (a green context's): fewer blocks do as well
+    if (launched != cudaErrorCooperativeLaunchTooLarge || grid == 1) {
+      ATC_CK(launched);
+      break;
+    }
+    cudaGetLastError();
+    grid = (grid + 1) / 2;
+  }
   ATC_CK(cudaMemcpyAsync(out, st.p, sizeof(PeelState), cudaMemcpyDeviceToHost, s));
   ATC_CK(cudaStreamSynchronize(s));
   if (out->timed_out) {
