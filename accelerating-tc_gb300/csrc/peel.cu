@@ -67,7 +67,7 @@ __global__ void peel_init_kernel(const int32_t* deg, int64_t n, int32_t* rt, int
 //     end over its lanes, four rounds of loads and atomics in flight;
 //   - a scan goes over the vertices that the last scan left unpeeled, and finds their smallest
 //     remaining degree: the outer steps that would admit nobody are passed over;
-//   - every wait at the barrier is bounded by the global timer: a block that gives up records it
+//   - every wait at the barrier is bounded by the time it has polled: a block that gives up records it
 //     and returns, and so do the others, one after another.
 // Data that other blocks write is read past L1 (ld.global.cg).
 // Measured, the whole peel (adjacency and loop): R-MAT scale 22 12.3 -> 4.0 ms (89 waves and 57
@@ -75,6 +75,10 @@ __global__ void peel_init_kernel(const int32_t* deg, int64_t n, int32_t* rt, int
 constexpr int kPeelThreads = 512;
 constexpr int kPeelPiece = 256;
 constexpr uint64_t kPeelWaitNs = 2000000000ull;  // two seconds for one step of the other blocks
+// The time between two looks at the clock counts as at most this: they are microseconds apart, unless the
+// whole kernel was off the GPU in between (time slices of other processes, a debugger), which is no block's delay.
+constexpr uint64_t kPeelPollNs = 1000000ull;
+constexpr unsigned kPeelPolls = 16;  // polls per look at the clock
 
 struct PeelStep {  // what one step's blocks count
   int admitted, alive, smallest;
@@ -100,7 +104,19 @@ struct PeelArgs {
   int32_t* alive[2];
   float threshold;   // A-direction
   int grow;          // A-direction: what the threshold grows by
+  uint64_t wait_ns;  // limit of a wait at the barrier
   PeelState* st;
+};
+
+// A wait's time, poll by poll.
+struct PeelWait {
+  uint64_t last, waited;
+  __host__ __device__ bool over(uint64_t now, uint64_t limit) {
+    const uint64_t gap = now - last;
+    waited += gap < kPeelPollNs ? gap : kPeelPollNs;
+    last = now;
+    return waited > limit;
+  }
 };
 
 __device__ __forceinline__ uint64_t peel_clock_ns() {
@@ -110,20 +126,21 @@ __device__ __forceinline__ uint64_t peel_clock_ns() {
 }
 
 // All blocks of the (cooperative) launch; false when the wait ran out.
-__device__ __forceinline__ bool peel_barrier(PeelState* st, unsigned* epoch) {
+__device__ __forceinline__ bool peel_barrier(PeelState* st, uint64_t limit, unsigned* epoch) {
   __shared__ int ok;
   __syncthreads();
   if (threadIdx.x == 0) {
     *epoch += gridDim.x;
     __threadfence();
     atomicAdd(&st->arrived, 1u);
-    const uint64_t t0 = peel_clock_ns();
+    PeelWait wait{peel_clock_ns(), 0};
     ok = 1;
-    for (;;) {
+    for (unsigned polls = 1;; ++polls) {
       unsigned a;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(a) : "l"(&st->arrived) : "memory");
       if ((int)(a - *epoch) >= 0) break;
-      if (peel_clock_ns() - t0 > kPeelWaitNs) {
+      // the clock only now and then: on each poll it made a step of 3.6 us 3.9
+      if (polls % kPeelPolls == 0 && wait.over(peel_clock_ns(), limit)) {
         st->timed_out = 1;
         ok = 0;
         break;
@@ -181,7 +198,7 @@ __global__ void __launch_bounds__(kPeelThreads, 2) peel_kernel(PeelArgs a) {
     PeelStep* c = &st->step[t % 3];
     admitted = __reduce_add_sync(0xffffffffu, admitted);
     if (lane == 0 && admitted) atomicAdd(&c->admitted, admitted);
-    if (!peel_barrier(st, &epoch)) return false;
+    if (!peel_barrier(st, a.wait_ns, &epoch)) return false;
     got->admitted = __ldcg(&c->admitted);
     got->alive = __ldcg(&c->alive);
     got->smallest = __ldcg(&c->smallest);
@@ -359,7 +376,7 @@ atc_status sym_graph(const SimpleEdges& e, const int32_t* deg, PeelGraph* g, cud
 
 template <bool CORE>
 atc_status run_peel(const SimpleEdges& e, const PeelGraph& g, int32_t* rt, int32_t* label, float threshold, int grow,
-                    PeelState* out, cudaStream_t s) {
+                    PeelState* out, cudaStream_t s, uint64_t wait_ns = kPeelWaitNs) {
   const int64_t n = e.n_in, m = e.m;
   DevBuf<int2> queue;
   DevBuf<PeelState> st;
@@ -370,7 +387,7 @@ atc_status run_peel(const SimpleEdges& e, const PeelGraph& g, int32_t* rt, int32
   out->step[0].smallest = INT_MAX;
   ATC_CK(cudaMemcpyAsync(st.p, out, sizeof(PeelState), cudaMemcpyHostToDevice, s));
   int32_t* const alive = reinterpret_cast<int32_t*>(g.cur.p);
-  PeelArgs a{g.off.p, g.adj.p, n, rt, label, queue.p, {alive, alive + n}, threshold, grow, st.p};
+  PeelArgs a{g.off.p, g.adj.p, n, rt, label, queue.p, {alive, alive + n}, threshold, grow, wait_ns, st.p};
   int bps = 0;
   ATC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, peel_kernel<CORE>, kPeelThreads, 0));
   // about four vertices or sixteen neighbours a thread: more blocks only make the barrier dearer

@@ -1,11 +1,13 @@
-// Rules of the library that show in times only: a batch's item shapes, and which of its graphs are counted
-// by rows.  One section per argument; prints "ok" or what differs.
+// Parts of the library that no call reaches at a test's size: rules that show in times only (a batch's item
+// shapes, and which of its graphs are counted by rows), and a peel whose barrier wait runs out.  One
+// section per argument; prints "ok" or what differs.
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <vector>
 
 #include "batch.cu"
+#include "peel.cu"
 
 using namespace atc;
 
@@ -67,11 +69,70 @@ static int choice() {
   return 0;
 }
 
+static int wait() {
+  const uint64_t limit = 2000000000ull;
+  PeelWait w{1000, 0};
+  uint64_t now = 1000;
+  // polls a microsecond apart reach the limit after that time
+  int64_t polls = 0;
+  while (!w.over(now += 1000, limit)) REQUIRE(++polls < 3000000);
+  REQUIRE(now - 1000 > limit && now - 1000 <= limit + 2000);
+  // a gap of any length between two polls is no delay of the other blocks
+  w = PeelWait{1000, 0};
+  REQUIRE(!w.over(60000000000ull, limit));
+  REQUIRE(!w.over(60000001000ull, limit));
+  return 0;
+}
+
+// ---- on the device -------------------------------------------------------------------
+// A ring of n vertices with chords; its cores by the peel, with a wait that runs out and without.
+static int peel() {
+  const int64_t n = 1 << 18;
+  SimpleEdges e;
+  e.n_in = n;
+  e.bits = id_bits(n);
+  std::vector<uint64_t> keys;
+  std::vector<int32_t> deg(n, 0);
+  for (int64_t a = 0; a < n; ++a)
+    for (int64_t s : {1, 2, 5}) {
+      const int64_t b = a + s;
+      if (b >= n) continue;
+      keys.push_back((uint64_t)a << e.bits | (uint64_t)b);
+      ++deg[a];
+      ++deg[b];
+    }
+  e.m = (int64_t)keys.size();
+  DevBuf<int32_t> d, rt, core;
+  REQUIRE(e.keys.alloc(e.m, nullptr) == ATC_OK && d.alloc(n, nullptr) == ATC_OK && rt.alloc(n, nullptr) == ATC_OK &&
+          core.alloc(n, nullptr) == ATC_OK);
+  cudaMemcpy(e.keys.p, keys.data(), 8 * e.m, cudaMemcpyHostToDevice);
+  cudaMemcpy(d.p, deg.data(), 4 * n, cudaMemcpyHostToDevice);
+  std::vector<int32_t> want, got(n);
+  for (int round = 0; round < 3; ++round) {
+    PeelGraph g;
+    REQUIRE(sym_graph(e, d.p, &g, nullptr) == ATC_OK);
+    cudaMemcpy(rt.p, deg.data(), 4 * n, cudaMemcpyHostToDevice);
+    cudaMemset(core.p, 0xff, 4 * n);
+    PeelState st;
+    const atc_status s = run_peel<true>(e, g, rt.p, core.p, 0.0f, 0, &st, nullptr, round == 1 ? 0 : kPeelWaitNs);
+    REQUIRE(s == (round == 1 ? ATC_ERR_TIMEOUT : ATC_OK));
+    if (round == 1) continue;
+    cudaMemcpy(got.data(), core.p, 4 * n, cudaMemcpyDeviceToHost);
+    if (round == 0) want = got;
+    REQUIRE(got == want);
+  }
+  for (int64_t v = 1; v < n - 1; ++v) REQUIRE(want[v] == want[n / 2]);
+  REQUIRE(want[n / 2] == 3);
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const char* const what = argc > 1 ? argv[1] : "";
   int r = 2;
   if (!strcmp(what, "shapes")) r = shapes();
   if (!strcmp(what, "choice")) r = choice();
+  if (!strcmp(what, "wait")) r = wait();
+  if (!strcmp(what, "peel")) r = peel();
   if (r == 0) std::printf("ok\n");
   return r;
 }

@@ -46,3 +46,13 @@ def test_batch_choice(program):
                                                  (48, 20000, 357849, 29.1, 18.9, 54, True)):
         assert bench.rows_graphs([(m, w * m, wmin * m, n, longest)] * graphs) == [rows] * graphs
     assert bench.rows_graphs([]) == []
+
+
+def test_barrier_wait_counts_polls(program):
+    _run(program, "wait")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("section", ["peel"])
+def test_on_the_device(program, section):
+    _run(program, section)
