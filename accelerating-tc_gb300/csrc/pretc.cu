@@ -894,11 +894,14 @@ static atc_status csr_load_impl(const char* path, bool host_resident, atc_csr* o
   }
   fclose(f);
   // the arrays must form a CSR: offsets from 0 to m, non-decreasing, rows strictly
-  // increasing ids in [0, n)
+  // increasing ids in [0, n).  The longest row, which sizes the kernels' buffers, is theirs, whatever the
+  // header says.
   const int64_t n = ok ? h64[0] : 0, m = ok ? h64[1] : 0;
+  int64_t longest = 0;
   if (ok) ok = off[0] == 0 && off[n] == m;
   for (int64_t u = 0; ok && u < n; ++u) {
     if (off[u + 1] < off[u]) ok = false;
+    longest = std::max(longest, off[u + 1] - off[u]);
     for (int64_t j = off[u]; ok && j < off[u + 1]; ++j)
       if (cols[j] < 0 || cols[j] >= n || (j > off[u] && cols[j] <= cols[j - 1])) ok = false;
   }
@@ -954,7 +957,7 @@ static atc_status csr_load_impl(const char* path, bool host_resident, atc_csr* o
   out->dir = h32[0];
   out->order = h32[1];
   out->pruned = h32[2];
-  out->max_outdeg = h32[3];
+  out->max_outdeg = (int32_t)longest;
   out->priv = pv;
   return ATC_OK;
 }
