@@ -267,28 +267,75 @@ __global__ void fox_deal_kernel(const uint64_t* keys, const int64_t* list, int64
 // 80 -> 30, 106 -> 70, 1.6M 160 -> 180; the sums stored to the caller's memory instead of copied
 // take another 5 to 10 us off (R-MAT scale 10 27).  Bound by launches below 50K edges, then by the searches'
 // dependent loads.
+// An edge whose shorter list has more than kSmallEach elements a lane is left to the whole block, four
+// searches a thread under way at once: one group's chain of dependent searches would hold the call up
+// (two hubs with the same 100 000 neighbours: 11.2 ms by one group).  Edges of one row lie in several
+// blocks, so that a hub's long ones do not meet in one.
 constexpr int64_t kSmallEdges = 1 << 19;
+constexpr int kSmallEach = 16;
+constexpr int kSmallLong = 128;  // edges a block can keep for all of it
 template <int G>
 __global__ void __launch_bounds__(256) small_edges_kernel(CsrView g, volatile unsigned long long* sums) {
+  __shared__ int32_t held[kSmallLong];
+  __shared__ int nheld;
+  if (threadIdx.x == 0) nheld = 0;
+  __syncthreads();
   const int sub = threadIdx.x % G;
   const int64_t groups = (int64_t)gridDim.x * 256 / G;
+  const int64_t warp = (threadIdx.x >> 5) * (int64_t)gridDim.x + blockIdx.x;
+  const unsigned group = 0xffffffffu >> (32 - G) << ((threadIdx.x & 31) - sub);
   unsigned cnt = 0;
-  for (int64_t e = g.e0 + (blockIdx.x * 256ll + threadIdx.x) / G; e < g.e1; e += groups) {
+  struct Lists {
+    const int32_t *L, *S;
+    int dl, ds;
+  };
+  auto lists = [&](int64_t e) {
     const int32_t u = __ldg(g.esrc + e), v = __ldg(g.cols + e);
     const int64_t au = __ldg(g.off + u), av = __ldg(g.off + v);
     const int du = (int)(__ldg(g.off + u + 1) - au), dv = (int)(__ldg(g.off + v + 1) - av);
-    const int32_t* L = g.cols + (du >= dv ? au : av);
-    const int32_t* S = g.cols + (du >= dv ? av : au);
-    const int dl = max(du, dv), ds = min(du, dv);
-    for (int j = sub; j < ds; j += G) {
-      const int32_t x = __ldg(S + j);
-      int lo = 0, n = dl;
+    return Lists{g.cols + (du >= dv ? au : av), g.cols + (du >= dv ? av : au), max(du, dv), min(du, dv)};
+  };
+  for (int64_t e = g.e0 + warp * (32 / G) + (threadIdx.x & 31) / G; e < g.e1; e += groups) {
+    const Lists x = lists(e);
+    if (x.ds > kSmallEach * G) {
+      int at = kSmallLong;
+      if (sub == 0) at = atomicAdd(&nheld, 1);
+      at = __shfl_sync(group, at, (threadIdx.x & 31) - sub);
+      if (at < kSmallLong) {
+        if (sub == 0) held[at] = (int32_t)(e - g.e0);
+        continue;
+      }
+    }
+    for (int j = sub; j < x.ds; j += G) {
+      const int32_t y = __ldg(x.S + j);
+      int lo = 0, n = x.dl;
       while (n > 1) {  // branch-free lower bound
         const int half = n >> 1;
-        lo = __ldg(L + lo + half - 1) < x ? lo + half : lo;
+        lo = __ldg(x.L + lo + half - 1) < y ? lo + half : lo;
         n -= half;
       }
-      cnt += __ldg(L + lo) == x;
+      cnt += __ldg(x.L + lo) == y;
+    }
+  }
+  __syncthreads();
+  for (int h = 0; h < min(nheld, kSmallLong); ++h) {
+    const Lists x = lists(g.e0 + held[h]);
+    for (int j = threadIdx.x; j < x.ds; j += 4 * 256) {
+      int32_t y[4];
+      int lo[4], n = x.dl;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        y[q] = j + 256 * q < x.ds ? __ldg(x.S + j + 256 * q) : -1;  // no id
+        lo[q] = 0;
+      }
+      while (n > 1) {
+        const int half = n >> 1;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) lo[q] = __ldg(x.L + lo[q] + half - 1) < y[q] ? lo[q] + half : lo[q];
+        n -= half;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) cnt += __ldg(x.L + lo[q]) == y[q];
     }
   }
   __shared__ unsigned long long part[8];
