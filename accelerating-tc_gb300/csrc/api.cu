@@ -61,6 +61,8 @@ bool alloc_budget_take(size_t bytes) {
   }
 }
 
+int64_t alloc_budget_left() { return g_budget.load(std::memory_order_relaxed); }
+
 // ---- phases --------------------------------------------------------------------------
 namespace {
 struct PhaseRec {

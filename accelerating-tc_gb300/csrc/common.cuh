@@ -72,6 +72,9 @@ bool host_stores();
 // returns true, or returns false (and takes nothing) when the budget would go below zero.
 // Unlimited unless a budget was set.
 bool alloc_budget_take(size_t bytes);
+// What is left of the budget, -1 without one: what a call takes for speed alone is not there for its later
+// allocations.
+int64_t alloc_budget_left();
 
 // Phase timing on for the calling thread (atc_phase_timing).
 bool phase_timing_on();

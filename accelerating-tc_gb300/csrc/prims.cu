@@ -35,19 +35,21 @@ atc_status sort_keys_u64_tmp(void* tmp, size_t* bytes, uint64_t* keys, uint64_t*
 
 atc_status sort_keys_u64(uint64_t*& keys, uint64_t*& alt, size_t n, int begin_bit, int end_bit, cudaStream_t s) {
   if (n <= 1) return ATC_OK;
-  size_t tmp = 0;
+  size_t tmp = 0, lib = 0;
   ATC_TRY(sort_keys_u64_tmp(nullptr, &tmp, keys, alt, n, begin_bit, end_bit, nullptr, s));
   DevBuf<char> t;
   uint64_t* sorted = nullptr;
-  if (t.alloc(tmp, s) == ATC_OK) {
+  // up to 2^20 keys the library's scratch is the smaller one (0.18 bytes a key to 0.25 or, up to 2^18, one):
+  // taken where the own one is refused, and under a budget, whose bytes do not come back
+  const bool capped = alloc_budget_left() >= 0;
+  if (capped) ATC_TRY(library_sort(nullptr, &lib, keys, alt, n, begin_bit, end_bit, nullptr, s));
+  if ((!capped || tmp <= lib) && t.alloc(tmp, s) == ATC_OK) {
     ATC_TRY(sort_keys_u64_tmp(t.p, &tmp, keys, alt, n, begin_bit, end_bit, &sorted, s));
   } else {
-    // up to 2^20 keys the library's scratch is the smaller one (0.18 bytes a key to 0.25 or, up to
-    // 2^18, one)
     cudaGetLastError();
-    ATC_TRY(library_sort(nullptr, &tmp, keys, alt, n, begin_bit, end_bit, nullptr, s));
-    ATC_TRY(t.alloc(tmp, s));
-    ATC_TRY(library_sort(t.p, &tmp, keys, alt, n, begin_bit, end_bit, &sorted, s));
+    ATC_TRY(library_sort(nullptr, &lib, keys, alt, n, begin_bit, end_bit, nullptr, s));
+    ATC_TRY(t.alloc(lib, s));
+    ATC_TRY(library_sort(t.p, &lib, keys, alt, n, begin_bit, end_bit, &sorted, s));
   }
   if (sorted != keys) {
     alt = keys;
