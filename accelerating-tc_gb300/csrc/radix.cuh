@@ -117,7 +117,8 @@ struct PassSmem {
 template <typename S, int kItems>
 __global__ void __launch_bounds__(kThreads, 2)
     pass_kernel(const uint64_t* __restrict__ in, uint64_t* __restrict__ out, uint64_t n, int shift, int bits,
-                const unsigned long long* __restrict__ offsets, S* state, S* next, unsigned* ticket) {
+                const unsigned long long* __restrict__ offsets, S* state, S* next, unsigned* ticket,
+                uint64_t wait_ns) {
   constexpr int kTileKeys = kThreads * kItems;
   constexpr S kSum = (S)1 << (8 * sizeof(S) - 1), kCount = kSum >> 1, kValue = kCount - 1;
   extern __shared__ __align__(16) unsigned char raw[];
@@ -204,7 +205,7 @@ __global__ void __launch_bounds__(kThreads, 2)
         p -= used;
         if (used) {
           t0 = clock_ns();
-        } else if (clock_ns() - t0 > kWaitNs) {
+        } else if (clock_ns() - t0 > wait_ns) {
           const uint64_t* const q = in + p * kTileKeys;  // a tile before this one is full
           for (int j = 0; j < kTileKeys; ++j) before += ((unsigned)(q[j] >> shift) & mask) == (unsigned)t;
           found = --p < 0;
@@ -239,16 +240,17 @@ __global__ void __launch_bounds__(kThreads, 2)
 }  // namespace radix
 
 // Sorts n keys by bits [begin, end), end > begin; *sorted = the buffer holding the result.  tmp ==
-// nullptr: *bytes receives the scratch needed.
+// nullptr: *bytes receives the scratch needed.  wide: 64-bit tile states whatever n, for tests, as wait_ns is.
 inline cudaError_t radix_sort_keys(void* tmp, size_t* bytes, uint64_t* keys, uint64_t* alt, size_t n, int begin, int end,
-                                   uint64_t** sorted, cudaStream_t s) {
+                                   uint64_t** sorted, cudaStream_t s, bool wide = false,
+                                   uint64_t wait_ns = radix::kWaitNs) {
   using namespace radix;
   const Passes ps = cut(begin, end);
-  const int items = n <= kSmallSort ? kSmallItems : 16;
+  wide = wide || n >= (1ull << 30);
+  const int items = n <= kSmallSort && !wide ? kSmallItems : 16;
   const size_t tile = (size_t)kThreads * items, tiles = (n + tile - 1) / tile;
   const size_t head = 256;  // a ticket per pass
   const size_t hist = sizeof(unsigned long long) * kMaxPasses * kDigits;
-  const bool wide = n >= (1ull << 30);
   const size_t state = (wide ? 8 : 4) * kDigits * tiles;
   // Up to 2^20 keys a launch to clear the state costs more than a second buffer; beyond, one
   // buffer (an eighth of a byte per key) is cleared between passes.
@@ -283,7 +285,7 @@ inline cudaError_t radix_sort_keys(void* tmp, size_t* bytes, uint64_t* keys, uin
         if (c != cudaSuccess) return c;
       }
       kernel<<<(unsigned)tiles, kThreads, smem, s>>>(a, b, n, ps.shift[i], ps.bits[i], h + i * kDigits, mine,
-                                                                 next, ticket + i);
+                                         next, ticket + i, wait_ns);
       uint64_t* x = a;
       a = b;
       b = x;

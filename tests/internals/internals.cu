@@ -1,13 +1,17 @@
 // Parts of the library that no call reaches at a test's size: rules that show in times only (a batch's item
-// shapes, and which of its graphs are counted by rows), and a peel whose barrier wait runs out.  One
+// shapes, and which of its graphs are counted by rows), the sort's wide tile states and its recount of an
+// earlier tile, the 64-bit row sort of the ranked copy, and a peel whose barrier wait runs out.  One
 // section per argument; prints "ok" or what differs.
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <random>
 #include <vector>
 
 #include "batch.cu"
 #include "peel.cu"
+#include "radix.cuh"
+#include "ranked.cu"
 
 using namespace atc;
 
@@ -85,6 +89,76 @@ static int wait() {
 }
 
 // ---- on the device -------------------------------------------------------------------
+static int sort_case(size_t n, int bits, bool wide, uint64_t wait_ns, unsigned seed) {
+  std::mt19937_64 rng(seed);
+  std::vector<uint64_t> h(n);
+  for (auto& x : h) x = rng() & ((1ull << bits) - 1);
+  DevBuf<uint64_t> a, b;
+  REQUIRE(a.alloc(n, nullptr) == ATC_OK && b.alloc(n, nullptr) == ATC_OK);
+  REQUIRE(cudaMemcpy(a.p, h.data(), 8 * n, cudaMemcpyHostToDevice) == cudaSuccess);
+  size_t bytes = 0;
+  uint64_t* sorted = nullptr;
+  REQUIRE(radix_sort_keys(nullptr, &bytes, a.p, b.p, n, 0, bits, nullptr, nullptr, wide, wait_ns) == cudaSuccess);
+  DevBuf<char> tmp;
+  REQUIRE(tmp.alloc(bytes, nullptr) == ATC_OK);
+  REQUIRE(radix_sort_keys(tmp.p, &bytes, a.p, b.p, n, 0, bits, &sorted, nullptr, wide, wait_ns) == cudaSuccess);
+  std::vector<uint64_t> got(n);
+  REQUIRE(cudaMemcpy(got.data(), sorted, 8 * n, cudaMemcpyDeviceToHost) == cudaSuccess);
+  std::sort(h.begin(), h.end());
+  REQUIRE(got == h);
+  return 0;
+}
+
+static int sorts() {
+  for (size_t n : {size_t(1), size_t(2047), size_t(2049), size_t(1) << 18, (size_t(1) << 18) + 1, size_t(700001),
+                   (size_t(1) << 20) + 8193, size_t(3) << 20})
+    for (int wide = 0; wide < 2; ++wide)
+      for (uint64_t wait_ns : {radix::kWaitNs, uint64_t(0)})
+        if (sort_case(n, 21, wide != 0, wait_ns, (unsigned)n)) return 1;
+  return 0;
+}
+
+// Rows of 0..40 ids (those above 32 are left to other kernels, as lists) by both key widths.
+template <class Key>
+static int row_sort(const std::vector<int64_t>& off, std::vector<int32_t> cols) {
+  const int64_t n = (int64_t)off.size() - 1;
+  DevBuf<int64_t> roff;
+  DevBuf<int32_t> rcols, mid, big;
+  DevBuf<int> ctr;
+  REQUIRE(roff.alloc(n + 1, nullptr) == ATC_OK && rcols.alloc(cols.size(), nullptr) == ATC_OK &&
+          mid.alloc(n, nullptr) == ATC_OK && big.alloc(n, nullptr) == ATC_OK && ctr.alloc(kcCount, nullptr) == ATC_OK);
+  cudaMemcpy(roff.p, off.data(), 8 * off.size(), cudaMemcpyHostToDevice);
+  cudaMemcpy(rcols.p, cols.data(), 4 * cols.size(), cudaMemcpyHostToDevice);
+  cudaMemset(ctr.p, 0, sizeof(int) * kcCount);
+  rank_sort_small_kernel<Key><<<grid_for(n, 256), 256>>>(roff.p, n, rcols.p, mid.p, big.p, ctr.p);
+  REQUIRE(cudaDeviceSynchronize() == cudaSuccess);
+  std::vector<int32_t> got(cols.size());
+  cudaMemcpy(got.data(), rcols.p, 4 * cols.size(), cudaMemcpyDeviceToHost);
+  for (int64_t u = 0; u < n; ++u)
+    if (off[u + 1] - off[u] <= 32) std::sort(cols.begin() + off[u], cols.begin() + off[u + 1]);
+  REQUIRE(got == cols);
+  return 0;
+}
+
+static int rows() {
+  std::mt19937 rng(5);
+  for (int64_t n : {1, 31, 33, 5000}) {
+    std::vector<int64_t> off(1, 0);
+    std::vector<int32_t> cols;
+    for (int64_t u = 0; u < n; ++u) {
+      const int len = rng() % 4 ? rng() % 9 : rng() % 41;
+      for (int j = 0; j < len; ++j) cols.push_back((int32_t)(rng() & 0x7ffffff));
+      off.push_back((int64_t)cols.size());
+    }
+    cols.push_back(0);  // no row is empty-handed
+    off.push_back((int64_t)cols.size());
+    if (row_sort<uint32_t>(off, cols) || row_sort<uint64_t>(off, cols)) return 1;
+    for (auto& x : cols) x |= 0x40000000;  // beyond the 27 bits of the narrow keys
+    if (row_sort<uint64_t>(off, cols)) return 1;
+  }
+  return 0;
+}
+
 // A ring of n vertices with chords; its cores by the peel, with a wait that runs out and without.
 static int peel() {
   const int64_t n = 1 << 18;
@@ -132,6 +206,8 @@ int main(int argc, char** argv) {
   if (!strcmp(what, "shapes")) r = shapes();
   if (!strcmp(what, "choice")) r = choice();
   if (!strcmp(what, "wait")) r = wait();
+  if (!strcmp(what, "sorts")) r = sorts();
+  if (!strcmp(what, "rows")) r = rows();
   if (!strcmp(what, "peel")) r = peel();
   if (r == 0) std::printf("ok\n");
   return r;

@@ -53,6 +53,6 @@ def test_barrier_wait_counts_polls(program):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("section", ["peel"])
+@pytest.mark.parametrize("section", ["sorts", "rows", "peel"])
 def test_on_the_device(program, section):
     _run(program, section)
