@@ -265,23 +265,24 @@ __global__ void fox_deal_kernel(const uint64_t* keys, const int64_t* list, int64
 // Measured, the whole call, items -> this kernel (us): R-MAT of 4.9K, 23K, 102K, 441K edges 55 -> 30,
 // 78 -> 31, 118 -> 50, 232 -> 175; Chung-Lu of 35K, 380K 93 -> 31, 115 -> 69; RGG of 45K, 473K
 // 80 -> 30, 106 -> 70, 1.6M 160 -> 180; the sums stored to the caller's memory instead of copied
-// take another 5 to 10 us off (R-MAT scale 10 27).  Bound by launches below 50K edges, then by the searches'
+// take another 5 to 10 us off (R-MAT scale 10 26; 441K edges 125).  Bound by launches below 50K edges, then by the searches'
 // dependent loads.
 // An edge whose shorter list has more than kSmallEach elements a lane is left to the whole block, four
 // searches a thread under way at once: one group's chain of dependent searches would hold the call up
-// (two hubs with the same 100 000 neighbours: 11.2 ms by one group).  Edges of one row lie in several
-// blocks, so that a hub's long ones do not meet in one.
+// (two hubs with the same 2000, 10 000, 100 000 neighbours: 0.20, 1.02, 11.3 ms by one group, 0.030, 0.035, 0.115 so; work
+// items 0.08, 0.09, 0.37).  Edges of one row lie in several blocks, so that a hub's long ones do not meet in one.
 constexpr int64_t kSmallEdges = 1 << 19;
 constexpr int kSmallEach = 16;
 constexpr int kSmallLong = 128;  // edges a block can keep for all of it
 template <int G>
-__global__ void __launch_bounds__(256) small_edges_kernel(CsrView g, volatile unsigned long long* sums) {
+__global__ void __launch_bounds__(1024, 2) small_edges_kernel(CsrView g, volatile unsigned long long* sums) {
   __shared__ int32_t held[kSmallLong];
   __shared__ int nheld;
   if (threadIdx.x == 0) nheld = 0;
   __syncthreads();
   const int sub = threadIdx.x % G;
-  const int64_t groups = (int64_t)gridDim.x * 256 / G;
+  const int threads = blockDim.x;
+  const int64_t groups = (int64_t)gridDim.x * threads / G;
   const int64_t warp = (threadIdx.x >> 5) * (int64_t)gridDim.x + blockIdx.x;
   const unsigned group = 0xffffffffu >> (32 - G) << ((threadIdx.x & 31) - sub);
   unsigned cnt = 0;
@@ -320,12 +321,12 @@ __global__ void __launch_bounds__(256) small_edges_kernel(CsrView g, volatile un
   __syncthreads();
   for (int h = 0; h < min(nheld, kSmallLong); ++h) {
     const Lists x = lists(g.e0 + held[h]);
-    for (int j = threadIdx.x; j < x.ds; j += 4 * 256) {
+    for (int j = threadIdx.x; j < x.ds; j += 4 * threads) {
       int32_t y[4];
       int lo[4], n = x.dl;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        y[q] = j + 256 * q < x.ds ? __ldg(x.S + j + 256 * q) : -1;  // no id
+        y[q] = j + threads * q < x.ds ? __ldg(x.S + j + threads * q) : -1;  // no id
         lo[q] = 0;
       }
       while (n > 1) {
@@ -338,14 +339,14 @@ __global__ void __launch_bounds__(256) small_edges_kernel(CsrView g, volatile un
       for (int q = 0; q < 4; ++q) cnt += __ldg(x.L + lo[q]) == y[q];
     }
   }
-  __shared__ unsigned long long part[8];
+  __shared__ unsigned part[32];
   const unsigned w = __reduce_add_sync(0xffffffffu, cnt);
   if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = w;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned long long t = 0;
-    for (int i = 0; i < 8; ++i) t += part[i];
-    sums[blockIdx.x] = t;
+  if (threadIdx.x < 32) {
+    unsigned long long t = (int)threadIdx.x < threads / 32 ? part[threadIdx.x] : 0u;
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (threadIdx.x == 0) sums[blockIdx.x] = t;
   }
 }
 
@@ -829,8 +830,11 @@ static bool small_pays(const atc_csr* csr, int64_t edges) {
 static atc_status run_small(const CsrView& g, int64_t mean_min, uint64_t* count, EventTimer* tm, cudaStream_t s,
                             int* launches) {
   const int lanes = mean_min <= 8 ? 8 : mean_min <= 32 ? 16 : 32;
-  const int64_t want = ((g.e1 - g.e0) * lanes + 255) / 256;
-  const unsigned grid = (unsigned)std::min<int64_t>(want, (int64_t)sm_count() * 8);
+  // blocks of 256 up to two an SM, then of 1024: the fewer sums, the less the host has to add up (1216 of them
+  // took 3 us)
+  const int64_t all = (g.e1 - g.e0) * lanes, two = (int64_t)sm_count() * 2;
+  const int threads = all <= 256 * two ? 256 : 1024;
+  const unsigned grid = (unsigned)std::min<int64_t>((all + threads - 1) / threads, two);
   const bool stored = host_stores();
   std::vector<unsigned long long> sums(grid);
   DevBuf<unsigned long long> dev;
@@ -838,9 +842,9 @@ static atc_status run_small(const CsrView& g, int64_t mean_min, uint64_t* count,
   unsigned long long* to = stored ? sums.data() : dev.p;
   {
     Phase ph("tc.count", s);
-    if (lanes == 8) small_edges_kernel<8><<<grid, 256, 0, s>>>(g, to);
-    else if (lanes == 16) small_edges_kernel<16><<<grid, 256, 0, s>>>(g, to);
-    else small_edges_kernel<32><<<grid, 256, 0, s>>>(g, to);
+    if (lanes == 8) small_edges_kernel<8><<<grid, threads, 0, s>>>(g, to);
+    else if (lanes == 16) small_edges_kernel<16><<<grid, threads, 0, s>>>(g, to);
+    else small_edges_kernel<32><<<grid, threads, 0, s>>>(g, to);
   }
   *launches += 1;
   tm->stop(s);
