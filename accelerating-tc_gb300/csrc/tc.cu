@@ -902,15 +902,28 @@ static atc_status group_edges(const CsrView& g, const ItemShape& sh, Grouping* g
   return ATC_OK;
 }
 
-// Whether the ranked copy pays for its passes: the passes cost about 60 ps an edge and 0.1 ms more
-// than grouping whole lists, which in turn is slow where hubs are (contended group cursors, long
-// lists).  Measured whole lists / ranked in ms: Bisson on R-MAT of 5K, 23K, 910K, 16M edges 0.12 /
-// 0.16, 0.19 / 0.16, 0.64 / 0.28, 4.8 / 1.9, Chung-Lu of 35K, 1.3M, 14M 0.21 / 0.18, 0.73 / 0.34,
-// 2.25 / 1.2, RGG (mean degree 32, W = 1.04 W_min) of 45K, 1.6M, 16M 0.11 / 0.18, 0.21 / 0.39,
-// 1.19 / 1.96.  Even degrees with long lists pay too: a test costs a third.
-static bool ranked_pays(const atc_csr* csr) {
-  return csr->m >= 16384 && (csr->wedges >= csr->wedges_min + csr->wedges_min / 2 || csr->wedges_min >= 48 * csr->m);
+// Predicted times (ps) of a whole count by grouped lists and on the ranked copy, per family: launches and
+// waits, per vertex, per edge, per element of the shorter lists; and for lists, where W well above W_min
+// tells of hubs, their contended group cursors and the longest item, whose 512 partners one warp streams.
+// Fitted to 150 graphs of 16K to 16M edges (R-MAT, Chung-Lu, RGG, stars; ids spread by 1 to 256; every orientation), each
+// counted both ways: following the faster prediction costs 1 % of the sum of the faster times, no graph more
+// than half its own, and is 17 (Bisson), 29 (TriCore) and 27 % (Fox) faster in the mean than lists.  Lists / ranked
+// in us, Bisson, stars (no wedge) of 3 M leaves 125 / 406, 4 M edges 173 / 554; R-MAT of 0.5 M edges on ids up to 7e7 1350 / 3800; RGG
+// (W = 1.06 W_min) of 0.5 M 151 / 291; R-MAT of 0.7 M, 3.1 M, 11 M 528 / 300, 1058 / 474, 2652 / 1026, scale 24
+// 117500 / 35700; Chung-Lu of 0.6 M, 14 M 387 / 295, 2232 / 1332; Fox, R-MAT scale 12 of 80 000 733 / 287.
+static double lists_ps(const atc_csr* csr, atc_kernel kernel) {
+  const double n = (double)csr->n, m = (double)csr->m, w = (double)csr->wedges, wmin = (double)csr->wedges_min;
+  const double test = kernel == ATC_KERNEL_TRICORE ? 3.9 : kernel == ATC_KERNEL_FOX ? 4.2 : 1.0;
+  const double tail = kernel == ATC_KERNEL_TRICORE ? 9.7e6 : kernel == ATC_KERNEL_FOX ? 1.44e7 : 4.6e6;
+  const double hubs = wmin > 0.0 ? std::min(std::max(2.0 * (w / wmin - 1.0), 0.0), 1.0) : 0.0;
+  return 9.2e7 + 15.0 * n + 32.0 * m + test * wmin +
+         hubs * (2.9e5 * std::sqrt(m) + tail * wmin / m * std::min(m / 20000.0, 1.0));
 }
+static double ranked_ps(const atc_csr* csr, atc_kernel kernel) {
+  const double test = kernel == ATC_KERNEL_TRICORE ? 1.1 : kernel == ATC_KERNEL_FOX ? 3.4 : 0.3;
+  return 1.95e8 + 52.0 * (double)csr->n + 87.0 * (double)csr->m + test * (double)csr->wedges_min;
+}
+static bool ranked_pays(const atc_csr* csr, atc_kernel kernel) { return ranked_ps(csr, kernel) < lists_ps(csr, kernel); }
 
 // The ranked count (csrc/ranked.cu) takes whole counts of CSRs that preTC built and that live on
 // the device.  Parts keep the CSR's own orientation (their counts are defined by it), as do CSRs
@@ -1211,30 +1224,27 @@ atc_status atc::part_edge_range(const atc_csr* csr, uint32_t part, uint32_t npar
   return ATC_OK;
 }
 
-// Counts the edges [e0, e1) of the CSR (every edge for the whole count).
-// ATC_KERNEL_AUTO: the Bisson-style or the Hu-style count, whichever this cost model of their
-// GB300 times predicts is faster.  Hu-style: 2 ps per wedge (W; 1.2 at scale 20 and above, where
-// it loses anyway) + 45 ps per edge + 0.06 ms.
-// Bisson-style, ranked: 0.37 ps per element of the shorter lists (W_min) + 85 ps per edge (the
-// ranked copy) + 0.17 ms of launches (since then faster at large scales, where it wins anyway).  By whole lists (parts, loaded CSRs): 1.232 ps per
-// element of W_min + 117.5 ps per edge + 0.3 ms, against Hu's 1.097 ps and 103.5 ps, the fit of
-// the two that it was made with.  Measured Hu / ranked in ms: R-MAT scale 14 0.09 / 0.23, 15 0.18 /
-// 0.24, 16 0.39 / 0.27, 18 1.32 / 0.47, 20 6.4 / 1.35, 22 36 / 6.2; Chung-Lu 1.3M edges 0.27 / 0.34, 4.0M 0.68 /
-// 0.53, 9.6M 1.52 / 0.98; of exponent 3 8.0M 0.74 / 0.89; RGG 1.6M 0.17 / 0.21, 16M 0.92 / 1.18.  The model
-// picks the faster one in all of them, A-direction + A-order and by degree.
+// ATC_KERNEL_AUTO: the Bisson-style or the Hu-style count, whichever is predicted faster.  Against the ranked
+// copy: Hu-style 2.3 ps per wedge (W; 1.2 at scale 20 and above, where it loses anyway) + 45 ps per edge + 9 ps
+// per vertex + 0.06 ms, or the small count.  Against grouped lists (parts, loaded CSRs, graphs that the copy does not pay
+// for): 1.097 ps per wedge + 103.5 ps per edge against 1.232 ps per element of W_min + 117.5 ps per edge + 0.3 ms, the fit
+// of the two that it was made with.  Measured Hu / ranked in ms: R-MAT scale 14 0.09 / 0.23, 15 0.18 / 0.24, 16 0.39 / 0.27, 18 1.32 /
+// 0.47, 20 6.4 / 1.35; Chung-Lu 1.3M edges 0.27 / 0.34, 4.0M 0.68 / 0.53, 9.6M 1.52 / 0.98.
 static atc_kernel auto_kernel(const atc_csr* csr, bool ranked) {
-  const double m = (double)csr->m, w = (double)csr->wedges, wmin = (double)csr->wedges_min;
-  const double bisson_ps = ranked ? 0.37 * wmin + 85.0 * m + 1.7e8 : 1.232 * wmin + 117.5 * m + 3.0e8;
-  double hu_ps = ranked ? 2.0 * w + 45.0 * m + 6.0e7 : 1.097 * w + 103.5 * m;
+  const double n = (double)csr->n, m = (double)csr->m, w = (double)csr->wedges, wmin = (double)csr->wedges_min;
+  const double bisson_ps = ranked ? ranked_ps(csr, ATC_KERNEL_BISSON) : 1.232 * wmin + 117.5 * m + 3.0e8;
+  double hu_ps = ranked ? 2.3 * w + 45.0 * m + 9.0 * n + 6.0e7 : 1.097 * w + 103.5 * m;
   if (small_pays(csr, csr->m)) hu_ps = std::min(hu_ps, 5.5 * wmin + 60.0 * m + 1.3e7);
   return hu_ps < bisson_ps ? ATC_KERNEL_HU : ATC_KERNEL_BISSON;
 }
 
+// Counts the edges [e0, e1) of the CSR (every edge for the whole count).
 static atc_status tc_window(const atc_csr* csr, atc_kernel kernel, const atc_tuning* tuning, int64_t e0, int64_t e1,
                             uint64_t* count, atc_stats* stats, cudaStream_t s) {
   CsrPriv* pv = static_cast<CsrPriv*>(csr->priv);
-  const bool ranked = pv && ranked_applies(csr, e0, e1, tuning) && ranked_pays(csr);
-  if (kernel == ATC_KERNEL_AUTO) kernel = auto_kernel(csr, ranked);
+  const bool applies = pv && ranked_applies(csr, e0, e1, tuning);
+  if (kernel == ATC_KERNEL_AUTO) kernel = auto_kernel(csr, applies && ranked_pays(csr, ATC_KERNEL_BISSON));
+  const bool ranked = applies && ranked_pays(csr, kernel);
   int launches = 0;
   EventTimer tm;
   if (e1 > e0) {
@@ -1253,10 +1263,9 @@ static atc_status tc_window(const atc_csr* csr, atc_kernel kernel, const atc_tun
         case ATC_KERNEL_BISSON: {
           bool done = false;
           if (ranked) ATC_TRY(count_ranked(csr, ctr, &done, s, &launches));
-          if (!done) {
-            ATC_CK(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), s));
-            ATC_TRY(run_bisson(g, tuning, ctr, s, &launches));
-          }
+          if (done) break;
+          if (ranked) ATC_CK(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), s));
+          ATC_TRY(run_bisson(g, tuning, ctr, s, &launches));
           break;
         }
         default: {
