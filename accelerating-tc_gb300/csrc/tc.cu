@@ -868,6 +868,15 @@ struct Grouping {
   int hc[4] = {0, 0, 0, 0};
 };
 
+// The device memory that group_edges allocates for `edges` edges.
+static atc_status grouping_bytes(const CsrView& g, int64_t edges, const ItemShape& sh, size_t* bytes, cudaStream_t s) {
+  ATC_TRY(exclusive_scan_i32_to_i64_tmp(nullptr, bytes, nullptr, nullptr, (size_t)g.n + 1, s));
+  const int64_t items = max_items(g.n, edges, std::min(sh.warp_chunk, sh.block_chunk));
+  *bytes += sizeof(int32_t) * (3 * (size_t)g.n + 2 + (size_t)edges + 32) + sizeof(int64_t) * ((size_t)g.n + 1) +
+            sizeof(int) * 8 + 2 * sizeof(GroupItem) * (size_t)items;
+  return ATC_OK;
+}
+
 static atc_status group_edges(const CsrView& g, const ItemShape& sh, Grouping* gr, cudaStream_t s, int* launches) {
   ATC_TRY(gr->cnt.alloc(g.n + 1, s));
   ATC_TRY(gr->cur.alloc(g.n, s));
@@ -1242,8 +1251,8 @@ static atc_kernel auto_kernel(const atc_csr* csr, bool ranked) {
 static atc_status tc_window(const atc_csr* csr, atc_kernel kernel, const atc_tuning* tuning, int64_t e0, int64_t e1,
                             uint64_t* count, atc_stats* stats, cudaStream_t s) {
   CsrPriv* pv = static_cast<CsrPriv*>(csr->priv);
-  const bool applies = pv && ranked_applies(csr, e0, e1, tuning);
-  if (kernel == ATC_KERNEL_AUTO) kernel = auto_kernel(csr, applies && ranked_pays(csr, ATC_KERNEL_BISSON));
+  const bool applies = pv && ranked_applies(csr, e0, e1, tuning), chosen = kernel == ATC_KERNEL_AUTO;
+  if (chosen) kernel = auto_kernel(csr, applies && ranked_pays(csr, ATC_KERNEL_BISSON));
   const bool ranked = applies && ranked_pays(csr, kernel);
   int launches = 0;
   EventTimer tm;
@@ -1265,7 +1274,23 @@ static atc_status tc_window(const atc_csr* csr, atc_kernel kernel, const atc_tun
           if (ranked) ATC_TRY(count_ranked(csr, ctr, &done, s, &launches));
           if (done) break;
           if (ranked) ATC_CK(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), s));
-          ATC_TRY(run_bisson(g, tuning, ctr, s, &launches));
+          // the choice was the library's: where the lists find no room, the Hu-style count, which groups none
+          atc_status st = ATC_OK;
+          if (chosen && alloc_budget_left() >= 0) {
+            ItemShape sh;
+            int slots;
+            size_t need = 0;
+            ATC_TRY(item_shape(tuning, &sh, &slots));
+            ATC_TRY(grouping_bytes(g, e1 - e0, sh, &need, s));
+            if ((size_t)alloc_budget_left() < need) st = ATC_ERR_OOM;
+          }
+          if (st == ATC_OK) st = run_bisson(g, tuning, ctr, s, &launches);
+          if (st == ATC_ERR_OOM && chosen) {
+            cudaGetLastError();
+            kernel = ATC_KERNEL_HU;
+            st = run_hu(g, tuning, ctr, s, &launches);
+          }
+          ATC_TRY(st);
           break;
         }
         default: {
