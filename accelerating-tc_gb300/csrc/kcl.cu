@@ -1024,29 +1024,34 @@ static atc_status launch_rows_block(const atc_csr* csr, int64_t e0, int64_t e1, 
   return ATC_OK;
 }
 
-// Whether every edge is better walked (with the dense kernel from k = 5 on): one or two launches
-// against up to six, which is what small graphs take.  Measured rows / walk in us: k = 3 R-MAT of
-// 14 000 edges 74 / 41, 114 000 124 / 73, RGG of 245 000 117 / 122; k = 4 R-MAT of 2900 51 / 47, Chung-Lu of 14 000
-// 67 / 52, R-MAT of 31 000 119 / 159; k = 5 R-MAT of 6000 67 / 48, 27 000 140 / 85, Chung-Lu of 114 000 140 / 110, R-MAT of 68 000 (W = 45 m)
-// 244 / 461; k = 6 R-MAT of 6000 115 / 61, Chung-Lu of 48 000 116 / 72, R-MAT of 14 000 (W = 25 m) 226 / 360.
-// The walk's warp per edge also balances a few very long rows better (K-core orientations: W = 2.5 W_min and
-// more): R-MAT scale 14 of 177 000 edges k = 6 4.8 / 3.8 ms, of 259 000 k = 5 4.4 / 2.9; by degree (1.7 W_min) 1.8 /
-// 2.6 and 0.62 / 2.0.  From k = 7 on any skewed graph: Chung-Lu of 2.3 M edges 43 / 31 ms, RGG of 2.5 M 10.8 /
-// 21.2.
-static bool walk_pays(const atc_csr* csr, int k) {
-  const int64_t m = csr->m, w = csr->wedges;
-  if (csr->max_outdeg <= (k >= 6 ? 16 : 32)) return false;  // rows by one launch
-  if (k == 3) return m <= 240000;
-  // up to 45 000 where few wedges close (Chung-Lu of 38 000, exponent 2.87, 81 / 67; RGG, W = W_min, 64 / 110)
-  if (k == 4) return m <= 16000 || (m <= 45000 && w <= 32 * m && w >= csr->wedges_min + 3 * (csr->wedges_min / 20));
-  if (csr->max_outdeg > 192 && w >= csr->wedges_min * 12 / 5 && (k >= 6 || m > 200000 || w >= 110 * m))
-    return true;
-  if (k == 5) return m <= 32000 || (m <= 120000 && w <= 36 * m);
-  if (m <= 50000 && w <= 21 * m) return true;
-  // short rows with few cliques below them: Chung-Lu of 290 000 edges (exponent 2.85) 250 / 133 us; RGG
-  // (W = W_min) of 150 000 447 / 700
-  if (m > 120000 && m <= 320000 && w <= 28 * m && w >= csr->wedges_min + 3 * (csr->wedges_min / 20)) return true;
-  return k >= 7 && m > 200000 && w >= csr->wedges_min + 3 * (csr->wedges_min / 10);
+// Whether the edges of a window are better walked (with the dense kernel from k = 5 on) than counted by rows:
+// by predicted times (ps) of the two.  The walk takes one launch or two, a little per edge (more where most
+// wedges close, as W near W_min tells) and dependent searches per wedge, more the longer the lists; rows take up
+// to six launches, a pass over all vertices, and less per wedge.  From k = 7 on the enumeration below the edges
+// is nearly all of either, which a warp per edge spreads better than a warp or CTA per source: rows are left to
+// graphs with hardly a wedge, at k = 7 also to those of few hubs (W below 2 W_min).
+// Fitted to 118 graphs of 8K to 2M edges (R-MAT, Chung-Lu, RGG, stars; ids spread by 1 to 256; every orientation), each
+// counted both ways, and tried on 94 others: k = 4..9 one call in ten or fewer is more than 5 % slower than by
+// the walk; by the windows of m and W that the choice was made with before, one in three.  Walk / rows in us, k = 4:
+// Chung-Lu of 1.4M edges (W = 3.2 m) 257 / 61, RGG of 1.5M (2.2 m) 344 / 75, of 96 000 (11 m) 175 / 69, R-MAT of 60 000 (42 m) 296 /
+// 135, of 32 000 (19 m) 85 / 131, a star of 39 000 36 / 62.
+static bool walk_pays(const atc_csr* csr, int k, int64_t edges) {
+  struct Cost {
+    double closed;           // walk: per edge where wedges close
+    double walk, walk_long;  // per wedge, and per wedge and 100 ids of the longest list
+    double rows, rows_long;
+  };
+  static const Cost costs[] = {{0.0, 5.4, 0.09, 4.5, 0.05}, {220.0, 16.0, 6.6, 7.5, 0.64}, {170.0, 18.6, 4.2, 11.7, 3.4},
+                               {130.0, 20.0, 14.0, 16.0, 12.2}, {130.0, 20.0, 126.0, 16.0, 112.0}};
+  const Cost& c = costs[std::min(k, 7) - 3];
+  const double n = (double)csr->n, m = (double)edges, longest = csr->max_outdeg, wmin = (double)csr->wedges_min;
+  const double w = (double)csr->wedges * m / (double)csr->m, lw = w * longest / 100.0;
+  const double close = wmin > 0.0 ? std::min(std::max((1.3 - (double)csr->wedges / wmin) / 0.2, 0.0), 1.0) : 0.0;
+  const double walk = 4.0e7 + (95.0 + c.closed * close) * m + c.walk * w + c.walk_long * lw;
+  double rows = 5.5e7 + 2.5 * n + 8.0 * m + c.rows * w + c.rows_long * lw;
+  if (k == 3) rows += (longest > 32 ? 1.5e7 : 0.0) + (longest > 64 ? 3.0e7 : 0.0);  // its launches
+  if (rows >= walk) return true;
+  return k >= 7 && w > 5.0 * m && (k > 7 || csr->wedges >= 2 * csr->wedges_min);
 }
 
 // k-cliques whose first two vertices (in orientation order) form an edge of [e0, e1).  by_rows:
@@ -1072,7 +1077,7 @@ static atc_status kcl_window(const atc_csr* csr, uint32_t k, int64_t e0, int64_t
     const int few_max =
         (int)(k >= 6 ? std::max<int64_t>(kFewRowsDeep, csr->n / 16) : std::max<int64_t>(kFewRows, csr->n / 32));
     const int64_t lcap = csr->m / (warp_max + 1) + 1;
-    bool walk_dense = by_rows && walk_pays(csr, (int)k);
+    bool walk_dense = by_rows && walk_pays(csr, (int)k, e1 - e0);
     if (by_rows && !walk_dense &&
         (q.alloc(kRowCounts + kRowBuckets + 1, s) != ATC_OK ||
          (cap > few_lo && lists.alloc((size_t)lcap * kRowBuckets + few_max, s) != ATC_OK))) {
