@@ -478,17 +478,20 @@ atc_status build_pipeline(atc_batch* b, const ItemShape& sh, cudaStream_t s) {  
   // m / (kBlockSmallList + 1) of them) plus one per chunk boundary
   const int64_t big_cap = m / (kBlockSmallList + 1) + m / sh.block_chunk + 1;
   const ItemShape shr = rows_shape(sh);  // rows items of mode 2
-  const int64_t cap_rows = max_items(n, m, std::min(shr.warp_chunk, shr.block_chunk));
-  if (b->built_n != n || b->built_m != m || b->built_graphs != ng || b->items_cap < cap_items ||
-      b->rows_cap < cap_rows || b->big_cap < big_cap) {
+  const int64_t cap_rows = sh.by_source == 2 ? max_items(n, m, std::min(shr.warp_chunk, shr.block_chunk)) : 0;
+  const bool same = b->built_n == n && b->built_m == m && b->built_graphs == ng;
+  if (!same || b->items_cap < cap_items || b->rows_cap < cap_rows || b->big_cap < big_cap) {
+    // room for the shapes of before too, so that a change back and forth allocates once
+    const int64_t items_cap = std::max(cap_items, same ? b->items_cap : 0);
+    const int64_t rows_cap = std::max(cap_rows, same ? b->rows_cap : 0);
     free_pipeline(b);
     ATC_TRY(dev_alloc(&b->cnt, (size_t)n + 1));
     ATC_TRY(dev_alloc(&b->cur, (size_t)n + 1));
     ATC_TRY(dev_alloc(&b->gstart, (size_t)n + 1));
     ATC_TRY(dev_alloc(&b->plist, (size_t)m + 32));
-    ATC_TRY(dev_alloc(&b->items, (size_t)cap_items));
+    ATC_TRY(dev_alloc(&b->items, (size_t)items_cap));
     ATC_TRY(dev_alloc(&b->counters, kBatchCounters));
-    ATC_TRY(dev_alloc(&b->items_r, (size_t)cap_rows));
+    ATC_TRY(dev_alloc(&b->items_r, (size_t)rows_cap));
     ATC_TRY(dev_alloc(&b->counters_r, 8));
     ATC_TRY(dev_alloc(&b->vrows, (size_t)n + 1));
     ATC_TRY(dev_alloc(&b->big, (size_t)big_cap));
@@ -502,8 +505,8 @@ atc_status build_pipeline(atc_batch* b, const ItemShape& sh, cudaStream_t s) {  
     b->built_n = n;
     b->built_m = m;
     b->built_graphs = ng;
-    b->items_cap = cap_items;
-    b->rows_cap = cap_rows;
+    b->items_cap = items_cap;
+    b->rows_cap = rows_cap;
     b->big_cap = big_cap;
   } else if (b->exec) {
     cudaGraphExecDestroy(b->exec);

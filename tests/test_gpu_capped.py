@@ -49,6 +49,40 @@ def test_auto_counts_where_the_hu_style_count_fits(scale, edge_factor):
     csr.free()
 
 
+@pytest.mark.parametrize("mode,before", [(0, 5361664), (1, 5361664)])
+def test_batches_take_no_more_than_before(mode, before):
+    """Three R-MAT graphs of scale 13: bytes that adding and counting them took before rows items had chunks of
+    their own (both modes), to 1 / 1024."""
+    csr = atc.pretc(atc.rmat_graph(13, 16, 1), atc.Dir.ADIRECTION)
+
+    def call():
+        b = atc.Batch()
+        try:
+            for _ in range(3):
+                b.add(csr)
+            return b.run({"group_by_source": mode} if mode else None)
+        finally:
+            b.free()
+
+    assert _least(call, 1 << 24) <= before * 1025 // 1024
+    csr.free()
+
+
+def test_batch_modes_in_turn():
+    """A change of the mode back and forth keeps its buffers; the counts stay."""
+    graphs = [atc.rmat_graph(9 + i % 3, 8, 40 + i) for i in range(6)]
+    want = [oracle.tc_count(g) for g in graphs]
+    b = atc.Batch()
+    for g in graphs:
+        c = atc.pretc(g, atc.Dir.ADIRECTION)
+        b.add(c)
+        c.free()
+    for mode in (2, 1, 2, None, 1, 2, None):
+        got, _ = b.run({"group_by_source": mode} if mode else None)
+        assert [int(x) for x in got] == want, mode
+    b.free()
+
+
 def test_small_sorts_take_the_smaller_scratch():
     """preTC of 32 768 pairs took 797 568 bytes with the library's sorts, 846 208 with the own ones."""
     g = atc.rmat_graph(10, 16, 1)
