@@ -771,14 +771,14 @@ def kcl_leg(sp):
 def select_leg():
     """The learned selector trained on the committed timings fixture (640 seeded graphs, every
     (direction, ordering, kernel) triple timed on a GB300): policies on its held-out quarter."""
-    path = os.path.join(ROOT, "tests", "golden", "select_timings.npz")
-    d = np.load(path)
+    name = "tests/golden/select_timings_ranked.npz"
+    d = np.load(os.path.join(ROOT, name))
     feats, times, costs = d["features"], d["times_ms"], d["costs"]
     ntr = int(0.75 * feats.shape[0])
     t0 = time.perf_counter()
     res = train_and_evaluate(feats, times, costs, ntr, seed=1)
     res["train_s"] = time.perf_counter() - t0
-    res["data"] = "tests/golden/select_timings.npz: %d training, %d held-out graphs" % (ntr, feats.shape[0] - ntr)
+    res["data"] = "%s: %d training, %d held-out graphs" % (name, ntr, feats.shape[0] - ntr)
     return res
 
 
