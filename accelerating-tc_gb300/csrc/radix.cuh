@@ -1,4 +1,6 @@
-// Least-significant-digit radix sort of 64-bit keys, one pass over memory per eight bits.
+// Least-significant-digit radix sort of 64-bit keys, one pass over memory per eight bits: the published
+// one-sweep method (Adinets and Merrill, "Onesweep: A Faster Least Significant Digit Radix Sort for GPUs",
+// 2022; the decoupled look-back is Merrill and Garland's, 2016), in code of its own.
 //
 // preTC sorts its edges as 64-bit keys, which was half of its time.  Each pass reads and writes the
 // keys once: a CTA takes a tile (tiles are handed out in order), ranks its keys by digit, learns

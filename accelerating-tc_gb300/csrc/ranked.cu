@@ -23,12 +23,12 @@
 //   exact for low ids and a filter for the others, or, with many entries, a CTA's of 16 KB.
 //
 // Measured (R-MAT scale 24, A-direction + A-order; whole lists grouped at the longer endpoint ->
-// this path): 117.5 -> 37.5 ms, of which the passes take 12.8 ms (entries 4.9, group sizes 2.3,
-// row sorts 3.1, rows 1.4) and the count 24.6: words 4, other ranks below 2^15 5, 2^16 5.5, 2^17 3.2,
-// the filter 6.7.  Without the words the ranks below 2^15 took 15.7 and the entries 5.7 (47.1 in all):
+// this path): 117.5 -> 35.6 ms, of which the passes take 12.3 ms (entries 4.8, group sizes 2.3,
+// row sorts 2.9, rows 1.4) and the count 23.3: words 4, other ranks below 2^15 5, 2^16 5.5, 2^17 3,
+// the filter 6.  Without the words the ranks below 2^15 took 15.7 and the entries 5.7 (47.1 in all):
 // bound by the shared and L1 pipe (two wavefronts per 32 tests, one of them bank conflicts) and by
-// issue (10 warp instructions per 32 tests).  Scale 22: 8.6 -> 6.5 ms, scale 20: 1.86 ->
-// 1.46 (4.45 by whole lists); Chung-Lu n = 700 001, which has few dense rows: 1.30 -> 1.25.
+// issue (10 warp instructions per 32 tests).  Scale 22: 8.6 -> 6.2 ms, scale 20: 1.86 ->
+// 1.4 (4.45 by whole lists); Chung-Lu n = 700 001, which has few dense rows: 1.30 -> 1.09.
 // Tried: 32-bit rows and one entry a warp at a time 68 ms; 32-lane scans of short prefixes
 // instead of lane groups 88 ms; rows on 128-byte lines 1-4 % for twice the copy.
 #include <algorithm>

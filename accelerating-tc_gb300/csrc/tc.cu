@@ -18,11 +18,13 @@
 //                 316-384                the device into 1,2,4,...,32 threads per edge;
 //                                        each thread searches a slice of the shorter list
 //                                        in the longer one.
-//   TriCore-style tricount_gpu.cu:215-290  warp per edge; 32 pivots of the longer list
-//                                        in shared memory bracket each element of the
+//   TriCore-style tricount_gpu.cu:215-290  the longer list staged in shared memory, a table
+//                                        over its id range brackets each element of the
 //                                        shorter list, then a binary search inside the
 //                                        bracket.
-// The Fox- and TriCore-style searches run on the ranked copy too, under the same conditions.
+// The Fox- and TriCore-style searches are staged per group item too, and run on the ranked copy under the same
+// conditions; the reference's forms of both, a warp or 1..32 threads per edge searching global memory, stay
+// behind atc_tuning.edge_kernels.
 #include <cmath>
 #include <mutex>
 #include <vector>

@@ -163,15 +163,16 @@ def measured_peak():
     return 6800.0, "fallback"
 
 
-def traffic_for(cfg, kernel_name):
-    """DRAM bytes per launch of the dominant kernel from the committed ncu summary."""
+def traffic_for(cfg, kernel_name, key="dram_bytes_per_launch"):
+    """DRAM bytes per launch of the dominant kernel, or of the whole step (dram_bytes_per_step), from the
+    committed ncu summary."""
     p = os.path.join(ROOT, "profiles", "traffic.json")
     if not os.path.exists(p):
         return None
     with open(p) as f:
         d = json.load(f)
     rec = d.get("%s|scale%d" % (kernel_name, cfg["scale"]))
-    return rec.get("dram_bytes_per_launch") if rec else None
+    return rec.get(key) if rec else None
 
 
 def sharded_throughput(units, ms, part_count, dist=None, device="cpu"):
@@ -457,6 +458,7 @@ def run_ours(a):
 
     cfg = workload_config(a)
     kname = {1: "hu", 2: "bisson", 3: "fox", 4: "tricore"}.get(st.kernel_used, "auto")
+    step_dram = traffic_for(cfg, kname, "dram_bytes_per_step")
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": a.steps, "warmup": a.warmup,
         "ms_per_step": ms_step, "higher_is_better": True, "scaling": "strong", "vs_baseline": None, "dtype": "int32",
@@ -465,7 +467,12 @@ def run_ours(a):
                   "max_outdeg": csr.max_outdeg, "triangles": head_count},
         "headline_kernel": kname, "fastest_kernel": best, "kernels": kernels,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "traffic": traffic_for(cfg, kname), "peak_source": peak_kind,
+                     "traffic": traffic_for(cfg, kname), "traffic_step": step_dram,
+                     "frac_dram": step_dram / (kern_ms * 1e-3) / 1e9 / peak if step_dram else None,
+                     "note": "frac: every candidate list read once per wedge, which the degree-ranked count does not "
+                             "do (fewer ids, dense rows as bitmaps), so it passes 1; frac_dram: the DRAM bytes ncu "
+                             "counted over the step's launches; traffic: the dominant one of them",
+                     "peak_source": peak_kind,
                      "alg_bytes_per_launch": alg, "kernel_ms": kern_ms,
                      "alg_bytes_min_per_launch": alg_min,
                      "achieved_min": alg_min / (kern_ms * 1e-3) / 1e9,

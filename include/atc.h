@@ -11,7 +11,9 @@
  * it in atc_csr_free.  Callers own their input arrays.  Host pointers are plain
  * pageable or pinned memory; "_device" variants take device pointers.  Streams are
  * cudaStream_t values passed as void* (NULL = the legacy default stream); every call
- * that returns a host result synchronises its stream before returning.
+ * that returns a host result synchronises its stream before returning.  An atc_csr carries scratch
+ * of the calls on it: calls on one CSR must not overlap (several threads or streams), except that small
+ * Hu-style counts share nothing.  The same holds for an atc_batch, and for training an atc_mlp.
  *
  * Vertex ids are int32 >= 0; an input pair is two consecutive int32 {src, dst}, the
  * little-endian layout of the reference's binary edge files (Hu/preTC.cu:29-32,84).
@@ -128,7 +130,8 @@ typedef enum atc_kernel {
   ATC_KERNEL_BISSON = 2,  /* lists streamed through a set of N+(v): bitmaps over a degree-ranked copy
                              of the edges where that pays (Bisson/tc.cu:18-104) */
   ATC_KERNEL_FOX = 3,     /* edge bins with 1..32 threads per edge (Fox/tc.cu:64-125,316-384) */
-  ATC_KERNEL_TRICORE = 4  /* warp per edge, 32 pivots + binary search (tricount_gpu.cu:215-290) */
+  ATC_KERNEL_TRICORE = 4  /* the longer list in shared memory, a bracket per element of the shorter one, then
+                             a binary search in it (tricount_gpu.cu:215-290) */
 } atc_kernel;
 
 /* Tuning knobs; zero means "library default".  The reference hard-codes these as
@@ -138,12 +141,13 @@ typedef struct atc_tuning {
   int32_t hu_blocks;         /* unused: the Hu-style kernel drains a work queue (layout kept) */
   int32_t hu_stage_ints;     /* unused: N+(u) is staged per work item (layout kept) */
   int32_t bisson_cutover;    /* warp items: sorted copy up to this out-degree, hash above (32); any
-                                bisson_* value asks for grouped lists, not the ranked copy */
+                                bisson_* value asks for grouped lists, not the ranked copy.  Batches:
+                                not used by items that index the rows (group_by_source) */
   int32_t fox_rearrange;     /* interleave each bin's edges (Fox/tc.cu:127-183) */
   int32_t fox_work_per_thread; /* bin base of the threads-per-edge bins (8) */
   int32_t tricore_blocks;    /* CTAs of the TriCore-style kernel (0: auto) */
   int32_t bisson_warp_max;   /* longest list a warp item handles, <= 512 (256) */
-  int32_t bisson_warp_chunk; /* partners per warp item (512) */
+  int32_t bisson_warp_chunk; /* partners per warp item (512; batches, items that index the rows: 64 at most) */
   int32_t bisson_block_chunk; /* partners per block item (2048) */
   int32_t bisson_slots;      /* hash slots per bucket of the tables: 1, 2 or 4 (0: default) */
   /* the bisson_* item shape applies to the Hu-style kernel too */
@@ -151,9 +155,10 @@ typedef struct atc_tuning {
                                 CSR rows (Hu-style wedge tests, no grouping passes); 0 = at
                                 the endpoint with the longer list (Bisson-style); 2 = each
                                 graph the way a cost model of the two predicts faster */
-  int32_t kcl_dense;         /* k-cliques (atc_kcl_part_tuned): 0 = sources by rows, candidate sets of
-                                65..1024 members on the dense kernel from k = 5 on; -1 = every
-                                edge on the warp search */
+  int32_t kcl_dense;         /* k-cliques (atc_kcl_part_tuned): 0 = sources by rows, or every edge by the
+                                warp search, as predicted times of the two say, and candidate sets of
+                                65..1024 members on the dense kernel from k = 5 on; -1 = every edge on
+                                the warp search alone */
   int32_t edge_kernels;      /* TriCore- and Fox-style: 1 = per-edge kernels searching the longer
                                 list in global memory, as the reference kernels do (a warp per
                                 edge with 32 pivots; 1..32 threads per edge in work bins);
@@ -339,7 +344,9 @@ atc_status atc_aorder(const int32_t* pairs, uint64_t n_pairs, int32_t* lookup, i
 /* ---- counting --------------------------------------------------------------------
    Triangle count of the oriented CSR: sum_u sum_{v in N+(u)} |N+(u) ∩ N+(v)|, exact in
    uint64.  Replaces the kernels' launch + host reduction in Hu/tc.cu:317-323,
-   Bisson/tc.cu:198-204, Fox/tc.cu:334-384, tricount_gpu.cu:337-408. */
+   Bisson/tc.cu:198-204, Fox/tc.cu:334-384, tricount_gpu.cu:337-408.  Scratch, freed with the call: the ranked
+   copy 14 to 18 bytes an edge and about 80 a vertex; grouped lists, taken where that is refused, 4 and 70;
+   the Hu-style count, which ATC_KERNEL_AUTO falls back on, about 50 a vertex, nothing for small counts. */
 atc_status atc_tc(const atc_csr* csr, atc_kernel kernel, const atc_tuning* tuning,
                   uint64_t* count, atc_stats* stats, atc_stream s);
 /* One part of the triangle count: the edges of the CSR are cut into `nparts` contiguous
