@@ -46,7 +46,7 @@ struct atc_batch {
   int64_t* vbase_d = nullptr;
   unsigned long long* gcounts = nullptr;
   void* scan_tmp = nullptr;
-  int64_t built_n = -1, built_m = -1, items_cap = 0, rows_cap = 0;
+  int64_t built_n = -1, built_m = -1, items_cap = 0, rows_cap = 0, plist_cap = 0;
   int built_graphs = -1;
   atc::ItemShape built_shape{};
   cudaStream_t cap_stream = nullptr;
@@ -473,22 +473,33 @@ std::vector<bool> rows_graphs(const atc_batch* b) {
 atc_status build_pipeline(atc_batch* b, const ItemShape& sh, cudaStream_t s) {  // by_source == 1: of rows_shape
   const int64_t n = b->n, m = b->m;
   const int ng = (int)(b->vbase.size() - 1);
-  const int64_t cap_items = max_items(n, m, std::min(sh.warp_chunk, sh.block_chunk));
+  const bool mixed = sh.by_source == 2;
+  const std::vector<bool> rows = mixed ? rows_graphs(b) : std::vector<bool>();
+  int64_t nr = 0, mr = 0;  // vertices and edges of mode 2's rows graphs, which have no groups and items of their own
+  for (int q = 0; mixed && q < ng; ++q)
+    if (rows[q]) {
+      nr += b->vbase[q + 1] - b->vbase[q];
+      mr += b->gm[q];
+    }
+  const int64_t cap_items = max_items(n - nr, m - mr, std::min(sh.warp_chunk, sh.block_chunk));
+  const int64_t cap_plist = sh.by_source == 1 ? 0 : m - mr;
   // block items of lists longer than kBlockSmallList: one per such list (at most
   // m / (kBlockSmallList + 1) of them) plus one per chunk boundary
   const int64_t big_cap = m / (kBlockSmallList + 1) + m / sh.block_chunk + 1;
   const ItemShape shr = rows_shape(sh);  // rows items of mode 2
-  const int64_t cap_rows = sh.by_source == 2 ? max_items(n, m, std::min(shr.warp_chunk, shr.block_chunk)) : 0;
+  const int64_t cap_rows = mixed ? max_items(nr, mr, std::min(shr.warp_chunk, shr.block_chunk)) : 0;
   const bool same = b->built_n == n && b->built_m == m && b->built_graphs == ng;
-  if (!same || b->items_cap < cap_items || b->rows_cap < cap_rows || b->big_cap < big_cap) {
+  if (!same || b->items_cap < cap_items || b->rows_cap < cap_rows || b->plist_cap < cap_plist ||
+      b->big_cap < big_cap) {
     // room for the shapes of before too, so that a change back and forth allocates once
     const int64_t items_cap = std::max(cap_items, same ? b->items_cap : 0);
     const int64_t rows_cap = std::max(cap_rows, same ? b->rows_cap : 0);
+    const int64_t plist_cap = std::max(cap_plist, same ? b->plist_cap : 0);
     free_pipeline(b);
     ATC_TRY(dev_alloc(&b->cnt, (size_t)n + 1));
     ATC_TRY(dev_alloc(&b->cur, (size_t)n + 1));
     ATC_TRY(dev_alloc(&b->gstart, (size_t)n + 1));
-    ATC_TRY(dev_alloc(&b->plist, (size_t)m + 32));
+    ATC_TRY(dev_alloc(&b->plist, (size_t)plist_cap + 32));
     ATC_TRY(dev_alloc(&b->items, (size_t)items_cap));
     ATC_TRY(dev_alloc(&b->counters, kBatchCounters));
     ATC_TRY(dev_alloc(&b->items_r, (size_t)rows_cap));
@@ -507,6 +518,7 @@ atc_status build_pipeline(atc_batch* b, const ItemShape& sh, cudaStream_t s) {  
     b->built_graphs = ng;
     b->items_cap = items_cap;
     b->rows_cap = rows_cap;
+    b->plist_cap = plist_cap;
     b->big_cap = big_cap;
   } else if (b->exec) {
     cudaGraphExecDestroy(b->exec);
@@ -545,14 +557,12 @@ atc_status build_pipeline(atc_batch* b, const ItemShape& sh, cudaStream_t s) {  
   CompactItems litems{b->big, gstart, big_cap, false, true, sh};
   // mode 2: each graph counts by rows (every wedge tested at its source, W tests, no grouping)
   // or grouped at the longer endpoint (sum of min(d+u, d+v) tests plus the grouping passes): rows_graphs
-  const bool mixed = sh.by_source == 2;
   CompactItems witems_r{b->items_r, b->off, cap_rows, false, false, shr};
   CompactItems bitems_r{b->items_r, b->off, cap_rows, true, true, shr};
   CompactItems litems_r{b->big_r, b->off, big_cap, false, true, shr};
   int nrows = 0;
   if (mixed) {
     ATC_CK(cudaMemsetAsync(b->vrows, 0, (size_t)n + 1, s));
-    const std::vector<bool> rows = rows_graphs(b);
     for (int q = 0; q < ng; ++q)
       if (rows[q] && b->vbase[q + 1] > b->vbase[q]) {
         ATC_CK(cudaMemsetAsync(b->vrows + b->vbase[q], 1, (size_t)(b->vbase[q + 1] - b->vbase[q]), s));

@@ -1,5 +1,6 @@
 """Calls under a device allocation budget: what the choice of the kernel or of the sort costs in memory
 does not refuse a call that a plainer choice would have room for."""
+import numpy as np
 import pytest
 
 import atc
@@ -66,6 +67,33 @@ def test_batches_take_no_more_than_before(mode, before):
 
     assert _least(call, 1 << 24) <= before * 1025 // 1024
     csr.free()
+
+
+@pytest.mark.parametrize("mode", [1, 2])
+@pytest.mark.parametrize("name", ["rmat13", "clique1200", "both"])
+def test_rows_items_fit_where_the_groups_did(name, mode):
+    """Items of 64 partners at most need no more room than the partner list that graphs counted by rows do not have:
+    modes 1 and 2 fit where mode 0 does, on long rows too."""
+    u, v = np.triu_indices(1200, 1)
+    clique = np.stack([u, v], 1).astype(np.int32)
+    graphs = {"rmat13": [atc.rmat_graph(13, 16, 1)], "clique1200": [clique], "both": [atc.rmat_graph(13, 16, 1), clique]}
+    csrs = [atc.pretc(g, atc.Dir.ADIRECTION) for g in graphs[name]]
+    want = [oracle.tc_count(g) for g in graphs[name]]
+
+    def call(m):
+        b = atc.Batch()
+        try:
+            for c in csrs:
+                b.add(c)
+            got = b.run({"group_by_source": m} if m else None)
+        finally:
+            b.free()
+        assert [int(x) for x in got[0]] == want
+        return got
+
+    assert _least(lambda: call(mode), 1 << 25) <= _least(lambda: call(0), 1 << 25)
+    for c in csrs:
+        c.free()
 
 
 def test_batch_modes_in_turn():
